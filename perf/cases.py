@@ -435,3 +435,80 @@ def tolerance(case):
         # 32-bit sums in varying order; a weight close to the soft threshold moves by more than the rest
         return {"rel": 1e-5, "max": 1e-3}
     return {"rel": 1e-5}                         # 32-bit sums in varying order
+
+
+# ------------------------------------------------------------------ the same results in 64 bits
+def _uindex(keys_list):
+    """Sorted (as unsigned numbers) different keys of the lists, and every list as indices into them."""
+    sign = -(1 << 63)
+    u, inv = torch.unique(torch.cat(keys_list) ^ sign, return_inverse=True)
+    return u ^ sign, torch.split(inv, [k.numel() for k in keys_list])
+
+
+def _row_sums(x, rp, z, rows):
+    if rp is None:
+        return x.view(rows, z).sum(1)
+    row = torch.repeat_interleave(torch.arange(rows, device=x.device), (rp[1:] - rp[:-1]).long())
+    return torch.zeros(rows, dtype=torch.float64, device=x.device).index_add_(0, row, x)
+
+
+def _exact_train(case, seed):
+    rows, z, app, algo = case["rows"], case["nnz"], case["source"] == "host_keys", case["algo"]
+    batches = []
+    for k in range(3):
+        ids, y, vals, rp = _rows(case, seed, k, ids64=app)
+        ids = _fix_unique(ids, case)
+        batches.append((_hash(ids) if app else _hash(ids.long(), 40), y.double(), None if vals is None else vals.double(), rp))
+    u, index = _uindex([b[0] for b in batches])
+    w, s0, s1 = (torch.zeros(u.numel(), dtype=torch.float64, device="cuda") for _ in range(3))
+    alpha, beta, l1, l2 = (0.1, 1.0, 1.0, 0.1) if algo == "ftrl" else (0.1, 1.0, 0.0, 0.01)
+    for at, (_, y, vals, rp) in zip(index, batches):
+        margin = _row_sums(w[at] if vals is None else w[at] * vals, rp, z, rows)
+        coef = -y * torch.sigmoid(-y * margin)
+        coef = coef.repeat_interleave(z) if rp is None else torch.repeat_interleave(coef, (rp[1:] - rp[:-1]).long())
+        g = torch.zeros_like(w).index_add_(0, at, coef if vals is None else coef * vals)
+        mine = torch.unique(at)
+        gm, wm, am, bm = g[mine], w[mine], s0[mine], s1[mine]
+        if algo == "ftrl":
+            n = torch.sqrt(bm * bm + gm * gm)
+            am, bm = am + gm - (n - bm) / alpha * wm, n
+            eta = alpha / (n + beta)
+            step = -am * eta
+        else:
+            am = am + (gm * gm if algo == "adagrad" else 1.0)
+            eta = alpha / (torch.sqrt(am) + beta)
+            step = wm - eta * gm
+        w[mine] = torch.sign(step) * (step.abs() - l1 * eta).clamp(min=0) / (1 + l2 * eta)
+        s0[mine], s1[mine] = am, bm
+    return {"keys": u[mine], "gradient": gm, "margin": margin}
+
+
+def _exact_evaluate(case, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    model = _hash(torch.arange(case["model"], dtype=torch.int64, device="cuda"))
+    weights = (torch.randn(case["model"], device="cuda", generator=g) * 0.1).double()
+    ids, _, vals, rp = _rows(case, seed, 0, ids64=True)
+    u, (mine, at) = _uindex([model, _hash(ids)])
+    w = torch.zeros(u.numel(), dtype=torch.float64, device="cuda")
+    w[mine] = weights
+    return _row_sums(w[at] if vals is None else w[at] * vals.double(), rp, case["nnz"], case["rows"])
+
+
+def exact(case, seed):
+    """What the first pass on ``prepare(case, seed)`` returns, in 64 bits."""
+    kind = case["kind"]
+    if kind == "train":
+        return _exact_train(case, seed)
+    if kind == "evaluate":
+        return _exact_evaluate(case, seed)
+    if kind == "kv":                             # one push into an empty table, pulled back
+        n, g = case["keys"], torch.Generator(device="cuda").manual_seed(seed)
+        keys = torch.unique(torch.randint(0, 1 << 40, (n + n // 20 + 64,), device="cuda", generator=g))
+        torch.randperm(keys.numel(), device="cuda", generator=g)
+        values = torch.randn(n, case["width"], device="cuda", generator=g).double()
+        return values if case["width"] > 1 else values.flatten()
+    if kind == "layers":                         # one push into zeros
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        return [torch.randn(n, device="cuda", generator=g).double() * (-0.1 if case["updater"] == "sgd" else 1.0)
+                for n in _sizes(case)]
+    return None                                  # wide: bf16 state rounded on the way; darlin: 512 dependent blocks
