@@ -233,6 +233,59 @@ __device__ __forceinline__ long long table_lookup_w(const Entry* tab, const Slot
   return -1;
 }
 
+// A whole entry moved by one 256-bit access (sm_100): one request and one sector instead of a load of the
+// key, one of (w, s0) and one of s1. Past L1: entries are shared with the peers' look-ups.
+struct __align__(32) EntryWords {
+  u64 key;     // Entry::key
+  u64 ws0;     // w (low half), s0
+  u64 s1pad;   // s1 (low half), pad
+  u64 acc;     // gacc, gcnt
+};
+static_assert(sizeof(EntryWords) == sizeof(Entry), "EntryWords mirrors Entry");
+__device__ __forceinline__ EntryWords ld_entry(const Entry* e) {
+  EntryWords v;
+  asm volatile("ld.relaxed.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(v.key), "=l"(v.ws0), "=l"(v.s1pad), "=l"(v.acc) : "l"(e) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_entry(Entry* e, const EntryWords& v) {
+  asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};"
+               :: "l"(e), "l"(v.key), "l"(v.ws0), "l"(v.s1pad), "l"(v.acc) : "memory");
+}
+
+// Q keys located (and inserted where absent) side by side: every trip probes one slot of each key that is
+// still open, the loads of a trip all issued before the first is looked at. A thread then waits for as many
+// trips as its longest probe sequence has, not for the sum of the four; in a table at half load a third of
+// the keys sit behind their first slot, so nearly every thread has such a key. `want` has bit q set for the
+// keys that are asked for; returns the bits of those found (a full table leaves some open). Only for the
+// owner's own table: an entry that was inserted just now is returned with the zeros it starts from.
+template <int Q>
+__device__ __forceinline__ u32 find_entries(Entry* tab, const SlotMap& sm, const u64 (&key)[Q], u32 want, u32 max_probe,
+                                            u32 (&slot)[Q], EntryWords (&e)[Q]) {
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if ((want >> q) & 1u) slot[q] = (u32)first_slot(sm, key[q]);
+  u32 open = want;
+  for (u32 p = 0; open && p < max_probe; ++p) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if ((open >> q) & 1u) e[q] = ld_entry(&tab[slot[q]]);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      if (!((open >> q) & 1u)) continue;
+      bool mine = e[q].key == key[q];
+      if (!mine && e[q].key == kEmptyKey) {
+        const u64 old = atomicCAS_system(&tab[slot[q]].key, kEmptyKey, key[q]);
+        mine = old == kEmptyKey || old == key[q];
+        e[q].key = key[q];
+      }
+      if (mine) open &= ~(1u << q);
+      else slot[q] = (slot[q] + 1) & (u32)sm.mask;
+    }
+  }
+  return want & ~open;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

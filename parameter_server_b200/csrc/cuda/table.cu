@@ -422,40 +422,26 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
       }
       continue;
     }
-    // Four keys per thread and trip. The first probe of each is one 16-byte load
-    // that returns key and weight, issued for all four before any is examined;
-    // only a miss on that slot (collision or new key) takes the probing path.
+    // Four keys per thread and trip, probed side by side: one load of an entry returns key and weight.
     for (u32 j0 = gtid; j0 < n; j0 += 4 * gsize) {
-      u64 key[4], slot[4], k0[4], hi[4];
+      u64 key[4];
+      u32 slot[4], want = 0;
+      EntryWords e[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        u32 j = j0 + q * gsize;
+        const u32 j = j0 + q * gsize;
         key[q] = j < n ? p.my_req_keys[r][j] : 0;
+        want |= j < n ? 1u << q : 0u;
       }
+      const u32 found = find_entries<4>(tab, sm, key, want, kMaxProbe, slot, e);
+      if (found != want) set_status(p.status, kTableFull);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        u32 j = j0 + q * gsize;
-        slot[q] = first_slot(sm, key[q]);
-        k0[q] = kEmptyKey; hi[q] = 0;
-        if (j < n)
-          asm volatile("ld.relaxed.sys.global.v2.u64 {%0, %1}, [%2];"
-                       : "=l"(k0[q]), "=l"(hi[q]) : "l"(&tab[slot[q]]) : "memory");
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        u32 j = j0 + q * gsize;
-        if (j >= n) break;
-        float w = __uint_as_float((u32)hi[q]);
-        u32 sc = (u32)slot[q];
-        if (k0[q] != key[q]) {
-          long long sl = table_find<true>(tab, sm, key[q], kMaxProbe);
-          w = 0.f;
-          sc = 0x7fffffffu;
-          if (sl >= 0) { w = __ldcg(&tab[sl].w); sc = (u32)sl; }
-          else set_status(p.status, kTableFull);
-        }
-        p.slot_cache[r][j] = sc;
-        p.resp_w[r][base + j] = w;
+        if (!((want >> q) & 1u)) continue;
+        const u32 j = j0 + q * gsize;
+        const bool ok = (found >> q) & 1u;
+        p.slot_cache[r][j] = ok ? slot[q] : 0x7fffffffu;
+        p.resp_w[r][base + j] = ok ? __uint_as_float((u32)e[q].ws0) : 0.f;
       }
     }
   }
@@ -738,7 +724,9 @@ __device__ __forceinline__ float inbox_value(const void* vals, int quant, u32 ca
   return scale * __half2float(((const __half*)(scales + scale_words(cap)))[j]);
 }
 
-__global__ void __launch_bounds__(kThreads) k_apply(const PsbApplyParams p) {
+// kWide: values of width k > 1. An instantiation of its own, so that neither path pays for the other's registers.
+template <bool kWide>
+__global__ void __launch_bounds__(kThreads, kWide ? 4 : 3) k_apply(const PsbApplyParams p) {
   __shared__ u32 s_wslot[kThreads], s_wsrc[kThreads], s_wrec[kThreads];   // a tile of the k-wide path
   __shared__ u32 s_pre[PSB_MAX_SHARDS + 1];
   __shared__ u32 s_cached[PSB_MAX_SHARDS];
@@ -785,11 +773,11 @@ __global__ void __launch_bounds__(kThreads) k_apply(const PsbApplyParams p) {
     if (p.alive[r] && !s_cached[r]) all_cached = false;
   }
   const bool single = n_src <= 1;
-  const bool merge = !single && p.tile_off != nullptr && all_cached && p.width <= 1;
+  const bool merge = !kWide && !single && p.tile_off != nullptr && all_cached;
   const SlotMap sm{p.mask, p.key_begin, p.slot_mult};
   StatAcc st;
 
-  if (p.width > 1) {
+  if constexpr (kWide) {
     // k values per key, sum entries: every record adds its k values to wide_vals[slot * k ..]. A CTA
     // takes tiles of blockDim.x records: one thread per record finds the slot, then the CTA adds the
     // tile's values with consecutive threads on consecutive values (coalesced inbox reads; 16 bytes
@@ -921,52 +909,63 @@ __global__ void __launch_bounds__(kThreads) k_apply(const PsbApplyParams p) {
   } else {
   // phase A: locate the slot of every record; single source -> update in place,
   // several sources -> accumulate into gacc and elect one leader per key
-  // four records per thread and trip: values and slots first, then the entries
+  // four records per thread and trip: values and slots (or keys) first, then the entries
   for (u32 i0 = gtid; i0 < total; i0 += 4 * gsize) {
-    long long slot[4];
+    u32 slot[4];
+    u64 key[4];
     float g[4];
     int rr[4];
-    u32 jj[4];
+    u32 known = 0, look = 0;                       // bit q: slot remembered / to be looked up by key
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      u32 i = i0 + q * gsize;
-      slot[q] = -1;
-      g[q] = 0.f; rr[q] = 0; jj[q] = 0;
+      const u32 i = i0 + q * gsize;
+      slot[q] = 0; key[q] = 0;
+      g[q] = 0.f; rr[q] = 0;
       if (i >= total) continue;
       int r = 0;
       while (r + 1 < S && i >= s_pre[r + 1]) ++r;
-      u32 j = i - s_pre[r];
-      rr[q] = r; jj[q] = j;
+      const u32 j = i - s_pre[r];
+      rr[q] = r;
       g[q] = inbox_value(p.inbox_vals[r], p.quant, p.inbox_cap, j);
       if (s_cached[r]) {
-        u32 sc = p.slot_cache[r][j] & 0x7fffffffu;
-        if (sc != 0x7fffffffu) slot[q] = sc;
+        slot[q] = p.slot_cache[r][j] & 0x7fffffffu;
+        if (slot[q] != 0x7fffffffu) known |= 1u << q;
       } else {
-        slot[q] = table_find<true>(tab, sm, p.inbox_keys[r][j], kMaxProbe);
-        if (slot[q] < 0) { set_status(p.status, kTableFull); if (p.slot_cache[r]) p.slot_cache[r][j] = 0x7fffffffu; }
+        key[q] = p.inbox_keys[r][j];
+        look |= 1u << q;
+      }
+    }
+    EntryWords e[4];
+    u32 got = known;
+    if (look) {
+      const u32 found = find_entries<4>(tab, sm, key, look, kMaxProbe, slot, e);
+      got |= found;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (!((look >> q) & 1u)) continue;
+        const bool ok = (found >> q) & 1u;
+        if (!ok) slot[q] = 0x7fffffffu;
+        if (!ok) set_status(p.status, kTableFull);
+        // remembered for a later round of the same keys (several sources: written below with the leader bit)
+        if ((single || !ok) && p.slot_cache[rr[q]]) p.slot_cache[rr[q]][i0 + q * gsize - s_pre[rr[q]]] = slot[q];
       }
     }
     if (single) {
-      float2 ws[4];
-      float s1[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if ((known >> q) & 1u) e[q] = ld_entry(&tab[slot[q]]);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        ws[q] = make_float2(0.f, 0.f); s1[q] = 0.f;
-        if (slot[q] >= 0) {
-          ws[q] = *reinterpret_cast<const float2*>(&tab[slot[q]].w);   // (w, s0): one 8-byte load
-          s1[q] = tab[slot[q]].s1;
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (slot[q] < 0) continue;
-        float w = ws[q].x, s0 = ws[q].y, t1 = s1[q], w_old = w;
+        if (!((got >> q) & 1u)) continue;
+        float w = __uint_as_float((u32)e[q].ws0), s0 = __uint_as_float((u32)(e[q].ws0 >> 32));
+        float t1 = __uint_as_float((u32)e[q].s1pad);
+        const float w_old = w;
         opt_step(p.opt, g[q], w, s0, t1);
-        Entry* e = &tab[slot[q]];
-        *reinterpret_cast<float2*>(&e->w) = make_float2(w, s0);
-        e->s1 = t1;
+        e[q].ws0 = (u64)__float_as_uint(w) | ((u64)__float_as_uint(s0) << 32);
+        e[q].s1pad = __float_as_uint(t1);
+        e[q].acc = 0;                               // the accumulators are zero between applies
+        st_entry(&tab[slot[q]], e[q]);
         st.add(w, w_old);
-        if (p.slot_cache[rr[q]]) p.slot_cache[rr[q]][jj[q]] = (u32)slot[q];
       }
     } else {
       // one vector atomic per record: gradient into gacc, one into gcnt; the record that finds
@@ -975,16 +974,17 @@ __global__ void __launch_bounds__(kThreads) k_apply(const PsbApplyParams p) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         seen[q] = 1.f;
-        if (slot[q] >= 0) seen[q] = atomic_add_f32x2(&tab[slot[q]].gacc, g[q], 1.f).y;
+        if ((got >> q) & 1u) seen[q] = atomic_add_f32x2(&tab[slot[q]].gacc, g[q], 1.f).y;
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (slot[q] >= 0) p.slot_cache[rr[q]][jj[q]] = (u32)slot[q] | (seen[q] == 0.f ? 0x80000000u : 0u);
+        if ((got >> q) & 1u)
+          p.slot_cache[rr[q]][i0 + q * gsize - s_pre[rr[q]]] = slot[q] | (seen[q] == 0.f ? 0x80000000u : 0u);
     }
   }
   }
   PSB_TSTAMP(2);
-  bool phase_b = !single && p.width <= 1;
+  bool phase_b = !kWide && !single;
   if (merge) {
     if (!grid_barrier(p.bar, p.status)) return;
     phase_b = __ldcg(p.slow) != 0;                 // only if a part went through the accumulators
@@ -1072,12 +1072,13 @@ extern "C" int psb_device_sm_count(void) {
 }
 
 extern "C" int psb_coop_grid(int which) {
-  static int g[4] = {0, 0, 0, 0};
-  if (which < 0 || which > 3) return 0;
+  static int g[5] = {0, 0, 0, 0, 0};
+  if (which < 0 || which > 4) return 0;
   if (!g[which]) {
     const void* fn = which == 0 ? (const void*)k_pull_margin
                    : which == 1 ? (const void*)k_push
-                   : which == 2 ? (const void*)k_apply : (const void*)k_pull_exchange;
+                   : which == 2 ? (const void*)k_apply<false>
+                   : which == 3 ? (const void*)k_pull_exchange : (const void*)k_apply<true>;
     g[which] = coop_grid_for(fn);
   }
   return g[which];
@@ -1138,7 +1139,8 @@ extern "C" int psb_push(const PsbPushParams* p, cudaStream_t stream) {
 }
 extern "C" int psb_apply(const PsbApplyParams* p, cudaStream_t stream) {
   if (p->S < 1 || p->S > PSB_MAX_SHARDS) return -(int)cudaErrorInvalidValue;
-  return launch_coop((const void*)k_apply, 2, p, stream);
+  if (p->width > 1) return launch_coop((const void*)k_apply<true>, 4, p, stream);
+  return launch_coop((const void*)k_apply<false>, 2, p, stream);
 }
 
 // sizeof of the parameter blocks, so that a binding can verify its mirror structs

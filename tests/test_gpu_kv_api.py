@@ -145,3 +145,26 @@ def test_buffered_kv_vector_aggregation_idiom(cuda_lib):
     t2 = kv.pull(keys)
     kv.wait(t2)
     assert np.array_equal(kv.result(t2).cpu().numpy(), 2 * vals)
+
+
+@pytest.mark.parametrize("n", [1, 3, 1025, 4095, 4096])
+def test_crowded_table_probes_past_collisions(cuda_lib, n):
+    """Keys far from their first slot (up to a completely full table, with wrap-around): look-ups and updates
+    of four keys side by side find and insert every one of them, whatever the keys of a thread collide with."""
+    from parameter_server_b200.parameter.kv import DeviceKVVector
+    rng = np.random.default_rng(n)
+    kv = DeviceKVVector.create(None, table_capacity=4096, max_keys=4096)
+    keys = np.sort(rng.choice(1 << 40, size=n, replace=False).astype(np.uint64))
+    vals = rng.integers(-8, 9, size=n).astype(np.float32)
+    ts = kv.push(keys, vals)                               # inserted by the push
+    ts = kv.push(keys, 2 * vals, wait=[ts])                # found by the push
+    got = kv.pull(keys, wait=[ts])                         # found by the pull
+    kv.wait(got)
+    np.testing.assert_array_equal(kv.result(got).cpu().numpy(), 3 * vals)
+    kv = DeviceKVVector.create(None, table_capacity=4096, max_keys=4096)
+    got = kv.pull(keys)                                    # inserted by the pull
+    kv.wait(got)
+    assert not kv.result(got).any()
+    kv.wait(kv.push(keys, vals))
+    have = dict(zip(*(t.tolist() for t in kv.plane.dump_nonzero())))
+    assert have == {int(k): float(v) for k, v in zip(keys, vals) if v}
