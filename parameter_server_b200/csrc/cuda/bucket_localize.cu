@@ -59,6 +59,7 @@ static constexpr int kWalkThreads = 1024;         // count / scatter CTAs
 static constexpr int kBucketThreads = 256;
 static constexpr u32 kRunMax = 64;                // longest probe sequence / run of adjacent occupied slots
 static constexpr u32 kMaxBuckets = 8192;
+static constexpr int kHintShift = 5;              // one row hint per 32 positions
 // A bucket's table comes in two sizes. 2^11 home slots (35 KB of shared memory, six CTAs per SM) serve
 // minibatches in which keys repeat, the usual case; 2^12 (55 KB, four per SM) those in which nearly
 // every nonzero has its own key. The sample decides (k_bl_plan), both kernels are launched and the
@@ -109,6 +110,7 @@ struct BLP {
   u32* bucket_hot_off;    // [NB + 1]
   u32* hot_u; u32* hot_seg;         // [kHotMax]
   u32* bstate;            // [NB]
+  u32* row_hint;          // [n / 32 + 2], with row_ptr only: the row of every 32nd position
   u64* cold_words; u32* cold_pos; u32* hot_pos;
   // outputs
   u64* ukeys; u32* seg_off; u32* csr_col; u32* csc_row; float* csc_val;
@@ -124,23 +126,35 @@ __device__ __forceinline__ u64 bl_key_of(const BLP& p, u32 i) {
 __device__ __forceinline__ u32 hot_home(u64 key) {
   return (((u32)(key >> 32) ^ (u32)key) * 0x9E3779B1u) >> 20;   // 12 bits = kHotSlots
 }
+// Largest r in [lo, hi) with row_ptr[r] <= pos; row_ptr[lo] <= pos.
+__device__ __forceinline__ u32 row_search(const u32* __restrict__ row_ptr, u32 lo, u32 hi, u32 pos) {
+  while (hi - lo > 1) {
+    const u32 mid = (lo + hi) >> 1;
+    if (row_ptr[mid] <= pos) lo = mid; else hi = mid;
+  }
+  return lo;
+}
 __device__ __forceinline__ u32 row_of_pos(const BLP& p, u32 pos, u32 zinv) {
   if (p.row_ptr == nullptr) {
     u32 r = __umulhi(pos, zinv);
     while (pos - r * p.fixed_z >= p.fixed_z) ++r;              // the estimate is at most two short
     return r;
   }
-  u32 lo = 0, hi = p.n_rows;                                   // largest r with row_ptr[r] <= pos
-  while (hi - lo > 1) {
-    u32 mid = (lo + hi) >> 1;
-    if (p.row_ptr[mid] <= pos) lo = mid; else hi = mid;
-  }
-  return lo;
+  // Ragged rows: the hints of the position's block of 32 and of the next one bracket the row, so that the
+  // search takes a step or two instead of log2(n_rows) dependent loads per nonzero (3.9 M nonzeros in 100,000
+  // rows: localisation and margins 579 -> 466 us).
+  const u32 b = pos >> kHintShift;
+  return row_search(p.row_ptr, p.row_hint[b], min(p.row_hint[b + 1] + 1, p.n_rows), pos);
 }
 
 // ---------------------------------------------------------------- 1. sample
 __global__ void __launch_bounds__(256) k_bl_sample(const BLP p) {
   const u32 j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p.row_ptr != nullptr) {
+    // row hints for steps 5 and 6, up to the block behind the last position
+    const u32 nh = ((p.n - 1) >> kHintShift) + 2;
+    for (u32 h = j; h < nh; h += gridDim.x * blockDim.x) p.row_hint[h] = row_search(p.row_ptr, 0, p.n_rows, h << kHintShift);
+  }
   const bool valid = j < p.samp_m;
   const u64 key = valid ? bl_key_of(p, j * p.samp_stride) : kEmptyKey;
   // equal keys of a warp count once (the most frequent key would otherwise take thousands of
@@ -755,10 +769,10 @@ struct BlLayout {
   size_t zero_begin, samp_cnt, ctl, bstate, zero_end;
   size_t ff_begin, samp_key, hot_tab, ff_end;
   size_t hot_idx, hot_key, part, bin_total, cold_base, pos_base, hot_base, shot_key, shot_h, bucket_hot_off,
-      hot_u, hot_seg, total;
+      hot_u, hot_seg, row_hint, total;
 };
 static size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
-static BlLayout bl_layout(u32 NB, u32 G) {
+static BlLayout bl_layout(u32 NB, u32 G, u32 n) {
   BlLayout L;
   size_t o = 0;
   const u32 NBINS = NB + kHotMax;
@@ -783,6 +797,7 @@ static BlLayout bl_layout(u32 NB, u32 G) {
   L.bucket_hot_off = o; o = al(o + (size_t)(NB + 1) * 4);
   L.hot_u = o; o = al(o + kHotMax * 4);
   L.hot_seg = o; o = al(o + kHotMax * 4);
+  L.row_hint = o; o = al(o + ((size_t)(n >> kHintShift) + 2) * 4);
   L.total = o;
   return L;
 }
@@ -806,8 +821,8 @@ static int bl_walk_ctas() {
 using namespace psb;
 
 extern "C" size_t psb_bucket_localize_scratch_bytes(uint32_t max_n) {
-  (void)max_n;   // the layout is sized for the largest bucket count; the per-nonzero buffers are the caller's
-  return bl_layout(kMaxBuckets, (u32)bl_walk_ctas()).total;
+  // sized for the largest bucket count; the per-nonzero buffers are the caller's
+  return bl_layout(kMaxBuckets, (u32)bl_walk_ctas(), max_n).total;
 }
 
 // Groups the n nonzeros of a minibatch by key. Inputs as for psb_sort_pairs (in, in_kind, seed);
@@ -851,7 +866,7 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   p.hot_thresh = max(4u, p.samp_m / p.NB / 2);
   p.cold_limit = max(32768u, 16u * (n / p.NB));
   p.row_ptr = row_ptr; p.n_rows = n_rows; p.fixed_z = fixed_z; p.vals = vals;
-  const BlLayout L = bl_layout(p.NB, p.G);
+  const BlLayout L = bl_layout(p.NB, p.G, n);
   unsigned char* sc = (unsigned char*)scratch;
   p.samp_key = (u64*)(sc + L.samp_key); p.samp_cnt = (u32*)(sc + L.samp_cnt);
   p.hot_tab = (u64*)(sc + L.hot_tab); p.hot_idx = (unsigned short*)(sc + L.hot_idx);
@@ -860,7 +875,7 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   p.cold_base = (u32*)(sc + L.cold_base); p.pos_base = (u32*)(sc + L.pos_base);
   p.hot_base = (u32*)(sc + L.hot_base); p.shot_key = (u64*)(sc + L.shot_key); p.shot_h = (u32*)(sc + L.shot_h);
   p.bucket_hot_off = (u32*)(sc + L.bucket_hot_off); p.hot_u = (u32*)(sc + L.hot_u);
-  p.hot_seg = (u32*)(sc + L.hot_seg); p.bstate = (u32*)(sc + L.bstate);
+  p.hot_seg = (u32*)(sc + L.hot_seg); p.row_hint = (u32*)(sc + L.row_hint); p.bstate = (u32*)(sc + L.bstate);
   p.cold_words = (u64*)cold_words; p.cold_pos = cold_pos; p.hot_pos = hot_pos;
   p.ukeys = (u64*)ukeys; p.seg_off = seg_off; p.csr_col = csr_col; p.csc_row = csc_row; p.csc_val = csc_val;
   p.flagbits = flagbits; p.wordbase = wordbase; p.n_unique = n_unique; p.status = status;

@@ -269,3 +269,23 @@ def test_auto_falls_back_to_sort_on_clustered_keys(cuda_lib):
     torch.cuda.synchronize()
     assert int(b.gate.item()) == 0 and int(b.status.item()) == 0
     _check_grouped(b, keys2, np.arange(rows + 1) * z, None, bounds_h, rows)
+
+
+@pytest.mark.parametrize("lens", ["one_row", "empty_rows", "one_each", "last_rows_empty", "long_then_short"])
+def test_bucket_localize_rows_of_all_lengths(cuda_lib, lens):
+    """The row of a nonzero, found between the hints of its block of 32 positions and of the next one."""
+    from parameter_server_b200.ops.localize import LocalBatch
+    rng = np.random.default_rng(5)
+    n = {"one_row": [5003], "empty_rows": (rng.random(40000) < 0.13) * rng.integers(1, 3, 40000), "one_each": np.ones(4097, int),
+         "last_rows_empty": np.concatenate([rng.integers(0, 9, 1500), np.zeros(700, int)]),
+         "long_then_short": np.concatenate([[6000], rng.integers(0, 4, 900)])}[lens]
+    row_ptr = np.concatenate([[0], np.cumsum(n)])
+    rows, nnz = len(n), int(row_ptr[-1])
+    keys = _rand_keys(nnz, rng, skew=True)
+    bounds_h, bounds = _bounds(2)
+    b = LocalBatch(rows, nnz, 2, "cuda")
+    b.localize(torch.from_numpy(keys.view(np.int64)).cuda(), None, bounds,
+               row_ptr=torch.from_numpy(row_ptr.astype(np.int32)).cuda(), hash_seed=None, method="bucket")
+    torch.cuda.synchronize()
+    assert nnz >= b.BUCKET_MIN_NNZ and int(b.gate.item()) == 0 and int(b.status.item()) == 0
+    _check_grouped(b, keys, row_ptr, None, bounds_h, rows)
