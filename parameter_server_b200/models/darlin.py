@@ -90,6 +90,7 @@ class DarlinRank:
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         self.violation = torch.zeros(1, dtype=torch.float32, device=dev)
         self.stage = torch.zeros(self.R * 2 * cfg.block_cols, dtype=torch.float32, device=dev)   # one area per ring slot
+        self._row_state: Optional[torch.Tensor] = None   # work space of the passes of a rank that is alone
         self.kkt_threshold = 1e20
         self.step = 0
         self.phase_ns: Optional[torch.Tensor] = None   # int64[4]: set to have run_pass add up its phase times
@@ -302,6 +303,10 @@ class DarlinRank:
         p.kkt_threshold, p.wait_iters = self.kkt_threshold, wait_iters
         p.bar, p.status = ptr(self._pass_bar), ptr(self.status)
         p.phase_ns = ptr(self.phase_ns) if self.phase_ns is not None else None
+        if self.S == 1 and tau == 0:
+            if self._row_state is None:
+                self._row_state = torch.empty(2 * max(1, self.n_rows), dtype=torch.float32, device=self.dev)
+            p.row_state, p.n_rows, p.steps = ptr(self._row_state), self.n_rows, self._pass_bar.data_ptr() + 8
         check(_lib.lib().psb_darlin_pass(C.byref(p), stream_ptr(stream)), "darlin_pass")
         self._pass_order = od          # keep the schedule alive until the launch has run
 

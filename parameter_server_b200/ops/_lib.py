@@ -139,6 +139,7 @@ class DarlinPass(C.Structure):
         ("n_steps", _u32), ("ts_base", _u32), ("tau", _i32), ("ring", _i32),
         ("kkt_threshold", _f32), ("wait_iters", _u32), ("bar", _vp), ("status", _vp),
         ("phase_ns", _vp),
+        ("row_state", _vp), ("n_rows", _u32), ("steps", _vp),
     ]
 
 

@@ -159,3 +159,45 @@ def test_device_preprocessing_tail_filter_groups_and_blocks(cuda_lib):
         gid, c0, c1 = space.groups[g]
         assert c0 <= b0 and b1 <= c1
     assert (covered == 1).all()
+
+
+@pytest.mark.parametrize("rows,z,n_feat,cols,real", [(1, 1, 40, 64, False), (257, 3, 90, 7, True), (4000, 40, 3000, 512, True),
+                                                    (20000, 50, 400, 300, False)])
+def test_pass_of_a_lone_rank_equals_its_blocks_one_by_one(cuda_lib, rows, z, n_feat, cols, real):
+    """One rank without delay takes a pass kernel of its own (no slices, no flags, label and margin as pairs);
+    the single-block kernels of the general path give the same state, over columns without data, deactivated
+    columns and columns of one to a few hundred thousand nonzeros."""
+    from parameter_server_b200.models.darlin import DarlinConfig, DarlinRank, darlin_heap_bytes
+    from parameter_server_b200.parallel.fabric import Fabric
+    rng = np.random.default_rng(rows)
+    keys, y, vals = _data(rng, rows, z, n_feat, real)
+    gk = np.unique(np.concatenate([keys, rng.integers(1, 1 << 62, 50).astype(np.uint64)]))
+    cfg = DarlinConfig(lambda_l1=0.5, eta=0.9, block_cols=cols)
+    a, b = (DarlinRank(Fabric.single(darlin_heap_bytes(cfg, 1)), cfg, torch.from_numpy(keys.view(np.int64)).cuda(),
+                       torch.from_numpy(y).cuda(), fixed_z=z, vals=None if vals is None else torch.from_numpy(vals).cuda(),
+                       global_keys=torch.from_numpy(gk.view(np.int64)).cuda()) for _ in range(2))
+    ts, n = 0, len(a.blocks)
+    for it in range(3):
+        order = np.random.default_rng(it).permutation(n).tolist()
+        a.run_pass(order, ts, 0)
+        for i, blk in enumerate(order):
+            b.grad(blk, ts + i)
+            b.update(blk, ts + i)
+            b.dual(blk, ts + i)
+        ts += n
+        torch.cuda.synchronize()
+        a.check_status(), b.check_status()
+        # 32-bit sums in another order: a column's sum of n terms is good to about n^0.5 * 2^-24 of their size
+        for name in ("margin", "w_cur", "w_own", "delta_w", "delta_own", "violation"):
+            x, w = getattr(a, name).double(), getattr(b, name).double()
+            assert (x - w).norm() <= 1e-4 * w.norm() + 1e-6, (it, name)
+        for name in ("active_w", "active_own"):
+            assert (getattr(a, name) != getattr(b, name)).sum() <= 1, (it, name)
+        assert not a.stage.any()
+        e = a.evaluate()
+        m, w, yy = a.margin.double(), a.w_own[:a.n_cols].double(), a.y.double()
+        want = [torch.nn.functional.softplus(-yy * m).sum().item(), cfg.lambda_l1 * w.abs().sum().item(),
+                int((w != 0).sum()), int(a.active_own[:a.n_cols].sum())]
+        assert np.allclose(e[:4], want, rtol=1e-5, atol=1e-5)
+        b.violation.zero_()
+        a.kkt_threshold = b.kkt_threshold = e[4] / rows * 10
