@@ -39,6 +39,13 @@ __device__ __forceinline__ float ld_sys_f1(const float* p) {
   return v;
 }
 
+// A slice of more elements than this (64 MB, half of L2) is written past L2's working set: it would be evicted
+// before the next kernel reads it in any case. (Seven layers of 4 KB to 709 MB pushed, applied and pulled: 1058 us
+// with two loads per thread in flight, one fence per thread and no streaming stores, 1009 us like this; the
+// 5.5 GB that the three calls move take 834 us at copy speed.)
+static constexpr u64 kStreamElems = 16u << 20;
+static constexpr int kLayerCtas = 5;               // resident CTAs per SM of the three kernels: the grid is one wave of them
+
 struct LayerPushArgs {
   int S;
   uint32_t ts1;
@@ -53,7 +60,7 @@ struct LayerPushArgs {
   uint32_t* status;
 };
 
-__global__ void __launch_bounds__(256) k_layer_push(const LayerPushArgs p) {
+__global__ void __launch_bounds__(256, kLayerCtas) k_layer_push(const LayerPushArgs p) {
   __shared__ u32 s_last;
   __shared__ u32 s_ok[PSB_MAX_SHARDS];
   if (threadIdx.x == 0) {
@@ -80,20 +87,29 @@ __global__ void __launch_bounds__(256) k_layer_push(const LayerPushArgs p) {
     const float* src = p.data + b;
     float* dst = p.inbox[s];
     const u64 n4 = ((((size_t)src | (size_t)dst) & 15) == 0) ? n / 4 : 0;
-    // two 16-byte loads in flight per thread
-    for (u64 i = gtid; i < n4; i += 2 * gsize) {
-      const u64 j = i + gsize;
-      const float4 a = __ldcs(reinterpret_cast<const float4*>(src) + i);
-      float4 c = a;
-      if (j < n4) c = __ldcs(reinterpret_cast<const float4*>(src) + j);
-      reinterpret_cast<float4*>(dst)[i] = a;
-      if (j < n4) reinterpret_cast<float4*>(dst)[j] = c;
+    // four 16-byte loads in flight per thread
+    const bool stream = n > kStreamElems;
+    for (u64 i = gtid; i < n4; i += 4 * gsize) {
+      float4 v[4];
+#pragma unroll
+      for (int k4 = 0; k4 < 4; ++k4)
+        if (i + k4 * gsize < n4) v[k4] = __ldcs(reinterpret_cast<const float4*>(src) + i + k4 * gsize);
+#pragma unroll
+      for (int k4 = 0; k4 < 4; ++k4) {
+        if (i + k4 * gsize >= n4) break;
+        float4* d = reinterpret_cast<float4*>(dst) + i + k4 * gsize;
+        if (stream) __stcs(d, v[k4]); else *d = v[k4];
+      }
     }
     for (u64 i = 4 * n4 + gtid; i < n; i += gsize) dst[i] = src[i];
   }
-  __threadfence_system();
+  // One system fence per CTA: the block barrier orders every thread's stores before thread 0's fence (fences
+  // are cumulative), and that fence precedes the arrival count.
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(p.done, 1u) + 1 == gridDim.x;
+  if (threadIdx.x == 0) {
+    __threadfence_system();
+    s_last = atomicAdd(p.done, 1u) + 1 == gridDim.x;
+  }
   __syncthreads();
   if (s_last && threadIdx.x < p.S) {
     __threadfence_system();
@@ -122,7 +138,7 @@ __device__ __forceinline__ float layer_update(int updater, float lr, float d, fl
   return updater == 0 ? s : (updater == 1 ? d + s : d - lr * s);
 }
 
-__global__ void __launch_bounds__(256) k_layer_apply(const LayerApplyArgs p) {
+__global__ void __launch_bounds__(256, kLayerCtas) k_layer_apply(const LayerApplyArgs p) {
   __shared__ u32 s_last;
   if (threadIdx.x == 0) {
     const u32 iters = p.wait_iters ? p.wait_iters : kPeerWaitIters;
@@ -134,27 +150,49 @@ __global__ void __launch_bounds__(256) k_layer_apply(const LayerApplyArgs p) {
   bool aligned = (((size_t)p.data) & 15) == 0;
   for (int r = 0; r < p.S; ++r) aligned = aligned && ((((size_t)p.inbox[r]) & 15) == 0);
   const u64 n4 = aligned ? p.n / 4 : 0;
-  for (u64 i = gtid; i < n4; i += gsize) {
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  const bool stream = p.n > kStreamElems;
+  // two groups of four per thread and trip, all their loads first; what the inbox held is not read again
+  for (u64 i = gtid; i < n4; i += 2 * gsize) {
+    const bool two = i + gsize < n4;
+    float4 s[2], d[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      s[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (k && !two) continue;
+      if (p.updater != 0) d[k] = reinterpret_cast<const float4*>(p.data)[i + k * gsize];
+    }
     for (int r = 0; r < p.S; ++r)
       if (p.alive[r]) {
-        // the inbox was filled by peer stores that the ready flag ordered: read past L1
-        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.inbox[r]) + i);
-        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        // filled by peer stores that the ready flag ordered, and read once: no line of it is in L1 before
+        float4 v[2];
+        v[0] = __ldcs(reinterpret_cast<const float4*>(p.inbox[r]) + i);
+        v[1] = two ? __ldcs(reinterpret_cast<const float4*>(p.inbox[r]) + i + gsize) : v[0];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) { s[k].x += v[k].x; s[k].y += v[k].y; s[k].z += v[k].z; s[k].w += v[k].w; }
       }
-    float4 d = reinterpret_cast<float4*>(p.data)[i];
-    d.x = layer_update(p.updater, p.lr, d.x, s.x); d.y = layer_update(p.updater, p.lr, d.y, s.y);
-    d.z = layer_update(p.updater, p.lr, d.z, s.z); d.w = layer_update(p.updater, p.lr, d.w, s.w);
-    reinterpret_cast<float4*>(p.data)[i] = d;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (k && !two) break;
+      if (p.updater == 0) {
+        d[k] = s[k];
+      } else {
+        d[k].x = layer_update(p.updater, p.lr, d[k].x, s[k].x); d[k].y = layer_update(p.updater, p.lr, d[k].y, s[k].y);
+        d[k].z = layer_update(p.updater, p.lr, d[k].z, s[k].z); d[k].w = layer_update(p.updater, p.lr, d[k].w, s[k].w);
+      }
+      float4* out = reinterpret_cast<float4*>(p.data) + i + k * gsize;
+      if (stream) __stcs(out, d[k]); else *out = d[k];
+    }
   }
   for (u64 i = 4 * n4 + gtid; i < p.n; i += gsize) {
     float s = 0.f;
     for (int r = 0; r < p.S; ++r) if (p.alive[r]) s += __ldcg(&p.inbox[r][i]);
     p.data[i] = layer_update(p.updater, p.lr, p.data[i], s);
   }
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(p.done, 1u) + 1 == gridDim.x;
+  if (threadIdx.x == 0) {
+    __threadfence();                               // one per CTA (see k_layer_push)
+    s_last = atomicAdd(p.done, 1u) + 1 == gridDim.x;
+  }
   __syncthreads();
   if (s_last && threadIdx.x == 0) {
     __threadfence_system();
@@ -174,7 +212,7 @@ struct LayerPullArgs {
   uint32_t* status;
 };
 
-__global__ void __launch_bounds__(256) k_layer_pull(const LayerPullArgs p) {
+__global__ void __launch_bounds__(256, kLayerCtas) k_layer_pull(const LayerPullArgs p) {
   if (threadIdx.x == 0 && p.need_applied) {
     const u32 iters = p.wait_iters ? p.wait_iters : kPeerWaitIters;
     for (int s = 0; s < p.S; ++s)
@@ -189,13 +227,14 @@ __global__ void __launch_bounds__(256) k_layer_pull(const LayerPullArgs p) {
     const float* src = p.data[s];
     float* dst = p.out + b;
     const u64 n4 = ((((size_t)src | (size_t)dst) & 15) == 0) ? n / 4 : 0;
-    for (u64 i = gtid; i < n4; i += 2 * gsize) {
-      const u64 j = i + gsize;
-      const float4 a = ld_sys_f4(src + 4 * i);
-      float4 c = a;
-      if (j < n4) c = ld_sys_f4(src + 4 * j);
-      __stcs(reinterpret_cast<float4*>(dst) + i, a);
-      if (j < n4) __stcs(reinterpret_cast<float4*>(dst) + j, c);
+    for (u64 i = gtid; i < n4; i += 4 * gsize) {
+      float4 v[4];
+#pragma unroll
+      for (int k4 = 0; k4 < 4; ++k4)
+        if (i + k4 * gsize < n4) v[k4] = ld_sys_f4(src + 4 * (i + k4 * gsize));
+#pragma unroll
+      for (int k4 = 0; k4 < 4; ++k4)
+        if (i + k4 * gsize < n4) __stcs(reinterpret_cast<float4*>(dst) + i + k4 * gsize, v[k4]);
     }
     for (u64 i = 4 * n4 + gtid; i < n; i += gsize) dst[i] = ld_sys_f1(src + i);
   }
@@ -232,7 +271,7 @@ using namespace psb;
 
 static int layer_grid(psb_u64 n) {
   const psb_u64 b = (n / 4 + 255) / 256;
-  const psb_u64 mx = (psb_u64)psb_device_sm_count() * 8;
+  const psb_u64 mx = (psb_u64)psb_device_sm_count() * kLayerCtas;
   return (int)(b < 1 ? 1 : (b > mx ? mx : b));
 }
 extern "C" int psb_layer_push(const void* args, cudaStream_t stream) {

@@ -68,3 +68,23 @@ def test_kvlayer_ring_bounds_a_fast_worker(cuda_lib):
     kv[1].check_status()
     # the push that timed out touched nothing: rounds 0 and 1 of both workers sum to (1 + 2) * (1 + 2)
     assert torch.equal(out, torch.full_like(out, 9.0))
+
+
+@pytest.mark.parametrize("updater", ["assign", "add", "sgd"])
+@pytest.mark.parametrize("n", [3, 5 * 256 * 148 * 4 + 1, (16 << 20) - 4, (16 << 20) + 7])
+def test_kvlayer_slice_sizes(cuda_lib, n, updater):
+    """One owner: a few elements, a little more than one trip of the grid, and slices at both sides of the
+    size from which they are streamed past L2. One addition (and one product) per element and round."""
+    from parameter_server_b200.parallel.fabric import Fabric
+    from parameter_server_b200.parameter.kv_layer import DeviceKVLayer
+    kv = DeviceKVLayer(Fabric.single(DeviceKVLayer.heap_bytes({0: n}, 1)), {0: n}, updater=updater, lr=0.5)
+    kv.segment(0).zero_()
+    want, out = torch.zeros(n, device="cuda"), torch.empty(n, device="cuda")
+    for rnd in range(3):
+        g = torch.randn(n, device="cuda")
+        kv.push(0, g)
+        kv.apply(0)
+        kv.pull(0, out, wait_for_round=rnd + 1)
+        want = g if updater == "assign" else want + (g if updater == "add" else -0.5 * g)
+        kv.check_status()
+        assert torch.equal(out, want)
