@@ -420,9 +420,12 @@ __global__ void __launch_bounds__(128) k_wide_pull_xgemm(const __grid_constant__
       u32 j = u - s_off[s];
       if (j < p.req_cap) p.req_keys[s][j] = p.ukeys[u];
     }
-    __threadfence_system();
+    // one system fence per CTA, behind the block barrier (fences are cumulative)
     __syncthreads();
-    if (tid == 0) s_last = atomicAdd(&p.done[0], 1u) + 1 == gridDim.x;
+    if (tid == 0) {
+      __threadfence_system();
+      s_last = atomicAdd(&p.done[0], 1u) + 1 == gridDim.x;
+    }
     __syncthreads();
     if (s_last && tid < S) {
       int s = tid;
@@ -495,9 +498,11 @@ __global__ void __launch_bounds__(128) k_wide_pull_xgemm(const __grid_constant__
         }
       }
     }
-    __threadfence_system();
     __syncthreads();
-    if (tid == 0) s_last = atomicAdd(&p.done[1], 1u) + 1 == gridDim.x;
+    if (tid == 0) {
+      __threadfence_system();
+      s_last = atomicAdd(&p.done[1], 1u) + 1 == gridDim.x;
+    }
     __syncthreads();
     if (s_last && tid < S && p.alive[tid]) {
       __threadfence_system();
@@ -536,22 +541,51 @@ __global__ void __launch_bounds__(128) k_wide_pull_xgemm(const __grid_constant__
   if (warp == 0) tmem_dealloc(c.tmem_base, (u32)N);
 }
 
+// Block sums of three doubles, one atomic per CTA and value: with one per warp the tens of thousands of atomics
+// on the same three addresses take longer than the rows.
+__device__ __forceinline__ void block_add3(double a, double b, double c, double* out) {
+  __shared__ double s_acc[3];
+  if (threadIdx.x < 3) s_acc[threadIdx.x] = 0;
+  __syncthreads();
+  a = warp_sum_d(a); b = warp_sum_d(b); c = warp_sum_d(c);
+  if ((threadIdx.x & 31) == 0) { atomicAdd(&s_acc[0], a); atomicAdd(&s_acc[1], b); atomicAdd(&s_acc[2], c); }
+  __syncthreads();
+  if (threadIdx.x < 3 && out && s_acc[threadIdx.x] != 0) atomicAdd(&out[threadIdx.x], s_acc[threadIdx.x]);
+}
+
 // ---------------------------------------------------------------- rows: prediction, loss, gcoef
+// Eight lanes per row, four nonzeros of each lane in flight: bound by the two dependent gathers (column, product).
 __global__ void __launch_bounds__(256) k_wide_rowsum(const float* __restrict__ P, int N, const u32* __restrict__ row_ptr,
                                                      u32 n_rows, u32 fixed_z, const u32* __restrict__ csr_col,
                                                      const u32* __restrict__ row_ctx, const float* __restrict__ y,
                                                      float* __restrict__ gcoef, float* __restrict__ margin,
                                                      double* __restrict__ stats) {
-  const int lane = threadIdx.x & 31;
-  const u32 gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+  const u32 sub = threadIdx.x & 7;
+  const u32 ggroup = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, ngroups = (gridDim.x * blockDim.x) >> 3;
   double loss = 0, correct = 0, seen = 0;
-  for (u32 r = gwarp; r < n_rows; r += nwarps) {
-    u32 b = row_ptr ? row_ptr[r] : r * fixed_z, e = row_ptr ? row_ptr[r + 1] : b + fixed_z;
-    u32 ctx = row_ctx ? row_ctx[r] : r % (u32)N;
+  // (the bound is the same for all lanes of a warp: the shuffles need all of them)
+  for (u32 r0 = ggroup & ~3u; r0 < n_rows; r0 += ngroups) {
+    const u32 r = r0 + (ggroup & 3u);
+    const bool have = r < n_rows;
+    u32 b = 0, e = 0, ctx = 0;
+    if (have) {
+      b = row_ptr ? row_ptr[r] : r * fixed_z;
+      e = row_ptr ? row_ptr[r + 1] : b + fixed_z;
+      ctx = row_ctx ? row_ctx[r] : r % (u32)N;
+    }
     float acc = 0.f;
-    for (u32 j = b + lane; j < e; j += 32) acc += P[(size_t)csr_col[j] * N + ctx];
-    acc = warp_sum(acc);
-    if (lane == 0) {
+    for (u32 j0 = b + sub; j0 < e; j0 += 32) {
+      u32 col[4];
+      float v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) col[q] = j0 + 8 * q < e ? csr_col[j0 + 8 * q] : 0xffffffffu;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = col[q] != 0xffffffffu ? P[(size_t)col[q] * N + ctx] : 0.f;
+      acc += (v[0] + v[1]) + (v[2] + v[3]);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (have && sub == 0) {
       float yy = y[r], ym = yy * acc;
       float en = expf(-fabsf(ym));
       float tau = ym > 0 ? en / (1.f + en) : 1.f / (1.f + en);
@@ -562,8 +596,7 @@ __global__ void __launch_bounds__(256) k_wide_rowsum(const float* __restrict__ P
       seen += 1;
     }
   }
-  loss = warp_sum_d(loss); correct = warp_sum_d(correct); seen = warp_sum_d(seen);
-  if (lane == 0 && stats && seen > 0) { atomicAdd(&stats[0], loss); atomicAdd(&stats[1], correct); atomicAdd(&stats[2], seen); }
+  block_add3(loss, correct, seen, stats);
 }
 
 // The long segments that the fused pull listed: chunks of kPullLongSeg nonzeros, one per warp and trip
@@ -599,7 +632,6 @@ __global__ void __launch_bounds__(256) k_wide_long_margins(const unsigned long l
 __global__ void __launch_bounds__(256) k_wide_rowloss(const float* __restrict__ margin, const float* __restrict__ y,
                                                       u32 n_rows, float* __restrict__ gcoef, double* __restrict__ stats,
                                                       unsigned long long* plong_n) {
-  const int lane = threadIdx.x & 31;
   if (plong_n != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *plong_n = 0ull;   // the list is used up
   double loss = 0, correct = 0, seen = 0;
   for (u32 r = blockIdx.x * blockDim.x + threadIdx.x; r < n_rows; r += gridDim.x * blockDim.x) {
@@ -611,8 +643,7 @@ __global__ void __launch_bounds__(256) k_wide_rowloss(const float* __restrict__ 
     correct += ym > 0 ? 1 : 0;
     seen += 1;
   }
-  loss = warp_sum_d(loss); correct = warp_sum_d(correct); seen = warp_sum_d(seen);
-  if (lane == 0 && stats && seen > 0) { atomicAdd(&stats[0], loss); atomicAdd(&stats[1], correct); atomicAdd(&stats[2], seen); }
+  block_add3(loss, correct, seen, stats);
 }
 
 // ---------------------------------------------------------------- push: per-key gradient rows to the owners
@@ -640,6 +671,13 @@ struct WidePushArgs {
   float* long_acc;                             // long_cap x 64 floats, zero on entry, left zero
   uint32_t long_cap;
 };
+
+// Keys (or records) that a warp takes at a time: a power of two, no more than keeps every warp busy.
+__device__ __forceinline__ u32 tile_size(u32 n, u32 nwarps, u32 most) {
+  u32 t = 4;
+  while (t < most && t * nwarps < n) t <<= 1;
+  return t;
+}
 
 // Segments longer than this are reduced by many warps (under a Zipf law one key can
 // own a fifth of all nonzeros; a single warp walking it would take milliseconds).
@@ -687,24 +725,79 @@ __global__ void __launch_bounds__(256) k_wide_push(const WidePushArgs p) {
     reinterpret_cast<__nv_bfloat162*>(p.inbox_vals[s] + (size_t)j * kWide)[lane] = __floats2bfloat162_rn(g0, g1);
     if (lane == 0) p.inbox_keys[s][j] = p.ukeys[u];
   };
-  // ---- phase 1: one warp per key; long segments are only listed, with the number of their
-  // first chunk (one 64-bit atomic hands out list position and chunk numbers together, so the
-  // list is sorted by first chunk)
-  for (u32 u = gwarp; u < U; u += nwarps) {
-    const u32 i0 = p.seg_off[u], i1 = p.seg_off[u + 1];
-    if (i1 - i0 > kWideLongSeg && p.long_cap) {
-      if (lane == 0) {
-        const u32 nch = (i1 - i0 + kWideLongSeg - 1) / kWideLongSeg;
+  auto emit_zero = [&](u32 u) {                     // by one lane: a key without nonzeros
+    const int s = owner_of(s_off, p.S, u);
+    const u32 j = u - s_off[s];
+    if (j >= p.inbox_cap) { set_status(p.status, kInboxOverflow); return; }
+    for (int q = 0; q < kWide / 8; ++q) reinterpret_cast<uint4*>(p.inbox_vals[s] + (size_t)j * kWide)[q] = make_uint4(0, 0, 0, 0);
+    p.inbox_keys[s][j] = p.ukeys[u];
+  };
+  // ---- phase 1: a warp takes tiles of 4 to 16 keys. Their nonzeros, laid end to end, are fetched 32 at a time
+  // (row, coefficient and context are a chain of dependent loads; most keys own one or two nonzeros, and a
+  // warp per key spent its time on one such chain per key) and then added one by one, in order. Long segments
+  // are only listed, with the number of their first chunk (one 64-bit atomic hands out list position and
+  // chunk numbers together, so the list is sorted by first chunk).
+  const u32 tile = tile_size(U, nwarps, 16);
+  for (u32 t0 = gwarp * tile; t0 < U; t0 += nwarps * tile) {
+    const u32 u = t0 + lane;
+    const bool have = (u32)lane < tile && u < U;
+    u32 i0 = 0, len = 0;
+    if (have) {
+      i0 = p.seg_off[u];
+      len = p.seg_off[u + 1] - i0;
+      if (len > kWideLongSeg && p.long_cap) {
+        const u32 nch = (len + kWideLongSeg - 1) / kWideLongSeg;
         const unsigned long long old = atomicAdd(p.n_long, 1ull | ((unsigned long long)nch << 32));
         const u32 k = (u32)old;
-        if (k < p.long_cap) p.long_list[k] = make_uint4(u, (u32)(old >> 32), i0, i1);
+        if (k < p.long_cap) p.long_list[k] = make_uint4(u, (u32)(old >> 32), i0, i0 + len);
         else set_status(p.status, kInboxOverflow);
+        len = 0;
+      } else if (len == 0) {
+        emit_zero(u);
       }
-      continue;
     }
+    u32 inc = len;                                  // inclusive prefix of the lengths
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    const u32 total = __shfl_sync(0xffffffffu, inc, 31);
     float g0 = 0.f, g1 = 0.f;   // lane handles dimensions 2*lane, 2*lane+1
-    wide_seg_accumulate(p, s_ctx, i0, i1, lane, g0, g1);
-    emit(u, g0, g1);
+    u32 cur = 32;               // the key of the tile whose sum is open
+    for (u32 base = 0; base < total; base += 32) {
+      const u32 x = base + lane;
+      u32 k = 0;                                    // the key of element x: the number of keys that end at or before it
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const u32 v = __shfl_sync(0xffffffffu, inc, k + o - 1);
+        if (v <= x) k += o;
+      }
+      const u32 start = __shfl_sync(0xffffffffu, inc - len, k), first = __shfl_sync(0xffffffffu, i0, k);
+      float gc = 0.f;
+      u32 n = 0;
+      if (x < total) {
+        const u32 r = __ldcs(&p.csc_row[first + (x - start)]);
+        gc = __ldg(&p.gcoef[r]);
+        n = p.row_ctx ? p.row_ctx[r] : r % (u32)p.N;
+      }
+      const u32 before = __shfl_up_sync(0xffffffffu, k, 1);
+      const u32 heads = __ballot_sync(0xffffffffu, k != (lane ? before : cur));
+      const int cnt = (int)min(32u, total - base);
+      for (int e = 0; e < cnt; ++e) {
+        if ((heads >> e) & 1u) {
+          if (cur != 32) emit(t0 + cur, g0, g1);
+          cur = __shfl_sync(0xffffffffu, k, e);
+          g0 = g1 = 0.f;
+        }
+        const float gce = __shfl_sync(0xffffffffu, gc, e);
+        const u32 ne = __shfl_sync(0xffffffffu, n, e);
+        const __nv_bfloat162 c2 = s_ctx[ne * (kWide / 2) + lane];
+        g0 += gce * __bfloat162float(c2.x);
+        g1 += gce * __bfloat162float(c2.y);
+      }
+    }
+    if (cur != 32) emit(t0 + cur, g0, g1);
   }
   if (p.long_cap) {
     if (!grid_barrier(p.bar, p.status)) return;
@@ -737,9 +830,12 @@ __global__ void __launch_bounds__(256) k_wide_push(const WidePushArgs p) {
       emit(__ldcg(&p.long_list[k].x), g.x, g.y);
     }
   }
-  __threadfence_system();
+  // one system fence per CTA, behind the block barrier (fences are cumulative)
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(p.done, 1u) + 1 == gridDim.x;
+  if (threadIdx.x == 0) {
+    __threadfence_system();
+    s_last = atomicAdd(p.done, 1u) + 1 == gridDim.x;
+  }
   __syncthreads();
   if (s_last && threadIdx.x == 0 && p.n_long) *p.n_long = 0ull;
   if (s_last && threadIdx.x < p.S) {
@@ -794,27 +890,47 @@ __global__ void __launch_bounds__(256) k_wide_apply(const WideApplyArgs p) {
     if (!p.alive[r]) continue;
     // a key pushed by two sources is updated twice, once per source: keep the passes apart
     if (applied_sources++ > 0) { if (!grid_barrier(p.bar, p.status)) return; }
-    for (u32 j = gwarp; j < s_cnt[r]; j += nwarps) {
-      long long slot = 0;
-      if (lane == 0) slot = wide_find<true>((u64*)p.keys, sm, p.inbox_keys[r][j]);
-      slot = __shfl_sync(0xffffffffu, slot, 0);
-      if (slot < 0) { if (lane == 0) set_status(p.status, kTableFull); continue; }
-      __nv_bfloat162 g2 = reinterpret_cast<const __nv_bfloat162*>(p.inbox_vals[r] + (size_t)j * kWide)[lane];
-      float g0 = __bfloat162float(g2.x), g1 = __bfloat162float(g2.y);
-      float2* ap = reinterpret_cast<float2*>(p.acc + (size_t)slot * kWide) + lane;
-      __nv_bfloat162* wp = reinterpret_cast<__nv_bfloat162*>(p.vals + (size_t)slot * kWide) + lane;
-      float2 a = *ap;
-      __nv_bfloat162 w2 = *wp;
-      a.x += g0 * g0; a.y += g1 * g1;
-      float w0 = __bfloat162float(w2.x) - p.alpha / (sqrtf(a.x) + p.beta) * g0;
-      float w1 = __bfloat162float(w2.y) - p.alpha / (sqrtf(a.y) + p.beta) * g1;
-      *ap = a;
-      *wp = __floats2bfloat162_rn(w0, w1);
+    // A warp takes tiles of 4 to 32 records: their slots are looked up side by side, one per lane, then the rows
+    // of four records are in flight at a time (a source's keys are unique, so no two records share a row).
+    const u32 total = s_cnt[r], tile = tile_size(total, nwarps, 32);
+    for (u32 t0 = gwarp * tile; t0 < total; t0 += nwarps * tile) {
+      const u32 cnt = min(tile, total - t0);
+      long long mine = -1;
+      if ((u32)lane < cnt) {
+        mine = wide_find<true>((u64*)p.keys, sm, p.inbox_keys[r][t0 + lane]);
+        if (mine < 0) set_status(p.status, kTableFull);
+      }
+      for (u32 k0 = 0; k0 < cnt; k0 += 4) {
+        long long slot[4];
+        __nv_bfloat162 g2[4], w2[4];
+        float2 a[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          slot[q] = __shfl_sync(0xffffffffu, mine, min(k0 + q, 31u));
+          if (k0 + q >= cnt) slot[q] = -1;
+          if (slot[q] < 0) continue;
+          g2[q] = reinterpret_cast<const __nv_bfloat162*>(p.inbox_vals[r] + (size_t)(t0 + k0 + q) * kWide)[lane];
+          a[q] = reinterpret_cast<const float2*>(p.acc + (size_t)slot[q] * kWide)[lane];
+          w2[q] = reinterpret_cast<const __nv_bfloat162*>(p.vals + (size_t)slot[q] * kWide)[lane];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (slot[q] < 0) continue;
+          const float g0 = __bfloat162float(g2[q].x), g1 = __bfloat162float(g2[q].y);
+          a[q].x += g0 * g0; a[q].y += g1 * g1;
+          const float w0 = __bfloat162float(w2[q].x) - p.alpha / (sqrtf(a[q].x) + p.beta) * g0;
+          const float w1 = __bfloat162float(w2[q].y) - p.alpha / (sqrtf(a[q].y) + p.beta) * g1;
+          reinterpret_cast<float2*>(p.acc + (size_t)slot[q] * kWide)[lane] = a[q];
+          reinterpret_cast<__nv_bfloat162*>(p.vals + (size_t)slot[q] * kWide)[lane] = __floats2bfloat162_rn(w0, w1);
+        }
+      }
     }
   }
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(p.done, 1u) + 1 == gridDim.x;
+  if (threadIdx.x == 0) {
+    __threadfence();                                // one per CTA, as in k_wide_push
+    s_last = atomicAdd(p.done, 1u) + 1 == gridDim.x;
+  }
   __syncthreads();
   if (s_last && threadIdx.x == 0) {
     __threadfence_system();
@@ -950,7 +1066,7 @@ extern "C" int psb_wide_rowsum(const float* P, int N, const uint32_t* row_ptr, u
                                const uint32_t* csr_col, const uint32_t* row_ctx, const float* y, float* gcoef,
                                float* margin, double* stats, cudaStream_t stream) {
   if (n_rows == 0) return 0;
-  k_wide_rowsum<<<psb_device_sm_count() * 4, 256, 0, stream>>>(P, N, row_ptr, n_rows, fixed_z, csr_col, row_ctx, y, gcoef, margin, stats);
+  k_wide_rowsum<<<psb_device_sm_count() * 8, 256, 0, stream>>>(P, N, row_ptr, n_rows, fixed_z, csr_col, row_ctx, y, gcoef, margin, stats);
   return -(int)cudaGetLastError();
 }
 // After a fused pull: add the listed long segments into the margins, then loss and d loss / d margin per row.

@@ -143,3 +143,36 @@ def test_wide_exchange_pull_matches_fp32_matmul(cuda_lib, S, N):
             margin = Pref[torch.from_numpy(col), torch.from_numpy(n_of_row)[:, None]].sum(1)
             assert torch.allclose(b.margin[:rows].cpu(), margin, rtol=2e-3, atol=2e-3)
         Ps[0].zero_()
+
+
+@pytest.mark.parametrize("rows,z,N", [(1, 1, 64), (3, 70, 128), (37, 5, 64), (2050, 9, 128)])
+def test_wide_rows_push_and_apply_sizes(cuda_lib, rows, z, N):
+    """Row sums, gradient rows and AdaGrad steps at sizes around the tiles that a warp takes (4 to 32 keys or
+    records, eight lanes per row), with keys of one to thousands of nonzeros, against fp64."""
+    planes, b, ctx, table, known, all_keys, ids, y, rows, z = _setup(1, N, rows=rows, z=z, seed=rows)
+    w = planes[0]
+    U = int(b.n_unique.item())
+    P = torch.zeros(b.max_nnz, N, device="cuda")
+    w.pull_gemm(b, ctx, P)
+    w.rowsum(b, P, N)
+    w.push(b, ctx, 0)
+    w.apply(0)
+    torch.cuda.synchronize()
+    w.check_status()
+    col = b.csr_col[:rows * z].long()
+    cx = torch.arange(rows, device="cuda") % N
+    margin = P.double()[col, cx.repeat_interleave(z)].view(rows, z).sum(1)
+    assert (b.margin[:rows] - margin).norm() <= 1e-6 * margin.norm() + 1e-6      # 32-bit sums of z terms
+    yy = torch.from_numpy(y).cuda().double()
+    gcoef = -yy * torch.sigmoid(-yy * margin)
+    assert torch.allclose(b.gcoef[:rows].double(), gcoef, rtol=1e-5, atol=1e-6)
+    C = ctx.double()
+    G = torch.zeros(U, 64, dtype=torch.float64, device="cuda").index_add_(0, col, (gcoef[:, None] * C[cx]).repeat_interleave(z, 0))
+    uk = b.ukeys[:U].cpu().numpy().view(np.uint64)
+    at = np.searchsorted(all_keys, uk, sorter=np.argsort(all_keys))
+    at = np.argsort(all_keys)[at]
+    V = torch.where(torch.from_numpy(known[at])[:, None], table[torch.from_numpy(at)].double(), 0.0).cuda()
+    want = V - 0.1 / (G.abs() + 1.0) * G
+    # the gradient travels as bf16 (2^-9 of |G|, whose step is at most 0.1 |G|) and the weight is stored as bf16
+    err = (w.lookup(uk).cuda().double() - want).abs()
+    assert (err <= 0.1 * G.abs() * 2.0 ** -8 + want.abs() * 2.0 ** -8 + 1e-5).all()
