@@ -102,6 +102,8 @@ typedef struct {
   uint32_t* auc_hist;         // nullable: [2][4096] histogram of sigmoid(margin) by label
   uint32_t* bar;              // 2 words, grid barrier
   uint32_t* status;
+  // upper bound of the number of values this call handles on this GPU (0: not known); sizes the grid
+  uint32_t work;
 } PsbPullParams;
 
 // Worker half of a push (kernel F1a): X^T g over CSC segments, range partition,
@@ -138,6 +140,8 @@ typedef struct {
   // k > 1: `grad` holds k values per unique key (key-major) and nnz must be 0. The inbox then holds
   // count * k values per source, quantised in groups of 32 consecutive values.
   int width;
+  // upper bound of the number of values this call handles on this GPU (0: not known); sizes the grid
+  uint32_t work;
 } PsbPushParams;
 
 // Server half of a push (kernel F1b): wait for the sources' flags, reduce
@@ -177,6 +181,8 @@ typedef struct {
   const uint32_t* tile_off;
   int tiles;
   uint32_t* slow;
+  // upper bound of the number of values this call handles on this GPU (0: not known); sizes the grid
+  uint32_t work;
 } PsbApplyParams;
 
 // Two-sided pull fused with the margins (kernel F2, exchange form). One launch on
@@ -249,6 +255,8 @@ typedef struct {
   const uint32_t* tile_off_prev;
   int tiles;
   psb_u64 key_end;
+  // upper bound of the number of values this call handles on this GPU (0: not known); sizes the grid
+  uint32_t work;
 } PsbPullExchangeParams;
 
 int psb_pull_exchange(const PsbPullExchangeParams* p, cudaStream_t stream);

@@ -47,6 +47,7 @@ class PullParams(C.Structure):
         ("csr_col", _vp), ("csr_val", _vp), ("y", _vp), ("loss", _i32),
         ("gcoef", _vp), ("margin", _vp), ("stats", _vp), ("auc_hist", _vp),
         ("bar", _vp), ("status", _vp),
+        ("work", _u32),
     ]
 
 
@@ -67,6 +68,7 @@ class PullExchangeParams(C.Structure):
         ("key_cache", _i32), ("kc_state", _vp), ("bar", _vp), ("slot_cache_prev", _vp * MAX_SHARDS),
         ("width", _i32), ("wide_vals", _vp),
         ("tile_off", _vp), ("tile_off_prev", _vp), ("tiles", _i32), ("key_end", _u64),
+        ("work", _u32),
     ]
 
 
@@ -81,6 +83,7 @@ class PushParams(C.Structure):
         ("nnz", _u32), ("csc_row", _vp), ("csc_val", _vp), ("flagbits", _vp), ("wordbase", _vp),
         ("gcoef", _vp), ("grad", _vp), ("bar", _vp), ("done", _vp), ("status", _vp),
         ("width", _i32),
+        ("work", _u32),
     ]
 
 
@@ -97,6 +100,7 @@ class ApplyParams(C.Structure):
         ("bar", _vp), ("done", _vp), ("status", _vp),
         ("width", _i32), ("wide_vals", _vp),
         ("tile_off", _vp), ("tiles", _i32), ("slow", _vp),
+        ("work", _u32),
     ]
 
 

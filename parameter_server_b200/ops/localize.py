@@ -81,6 +81,7 @@ class LocalBatch:
         self.margin = torch.empty(max_rows, dtype=f32, device=dev)
         self.csc_val_buf = torch.empty(max_nnz, dtype=f32, device=dev) if real_values else None
         # set per batch
+        self.n_keys_max = 0                                      # bound of the number of unique keys (0: not known)
         self.n_rows = 0
         self.nnz = 0
         self.fixed_z = 0
@@ -123,7 +124,7 @@ class LocalBatch:
             ids = self._ids32[:n]
         n = ids.numel()
         assert n <= self.max_nnz
-        self.nnz = n
+        self.nnz = self.n_keys_max = n
         if row_ptr is not None:
             self.n_rows = row_ptr.numel() - 1
             self.fixed_z = 0
@@ -214,7 +215,7 @@ class LocalBatch:
             # thread_local: other threads of the process (loaders, node threads) may call the runtime meanwhile
             with torch.cuda.graph(g, stream=stream, capture_error_mode="thread_local"):
                 self.localize(ids, y, bounds, row_ptr=row_ptr, vals=vals, stream=torch.cuda.current_stream(), **kw)
-            state = {a: getattr(self, a) for a in ("nnz", "n_rows", "fixed_z", "row_ptr", "csr_val", "y", "pack_bits",
+            state = {a: getattr(self, a) for a in ("nnz", "n_keys_max", "n_rows", "fixed_z", "row_ptr", "csr_val", "y", "pack_bits",
                                                    "csc_val", "csc_row")}
             ent = graphs[key] = (g, state, _lib.LAUNCHES - before, (ids, y, bounds, row_ptr, vals))
             _lib.LAUNCHES = before                             # the capture launched nothing
@@ -238,4 +239,5 @@ class LocalBatch:
                                            ptr(self.own_off), stream_ptr(stream)), "owner offsets")
         self.n_rows = 0
         self.nnz = 0
+        self.n_keys_max = n
         return self

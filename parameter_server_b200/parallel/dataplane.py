@@ -135,6 +135,7 @@ class DataPlane:
             m = (cfg.table_capacity << 64) // size if (cfg.ordered_slots and size > cfg.table_capacity) else 0
             self.slot_mult.append(m if m < (1 << 64) else 0)
         self.applied_ts1 = 0
+        self._round_work = {}                             # ring slot -> (round, bound of the values pushed in it)
         self.ctrl = fabric.view(self.layout["ctrl"], (CTRL_WORDS,), torch.int32)
         self.width = max(1, cfg.width)
         assert self.width == 1 or (cfg.pull_cap and opt.algo in ("sum", "keep")), \
@@ -220,6 +221,7 @@ class DataPlane:
         p.loss = loss
         p.stats, p.auc_hist = ptr(self.pull_stats), ptr(auc_hist)
         p.bar, p.status = self._bar(0), ptr(self.status)
+        p.work = min(b.n_keys_max, 0xffffffff)
         check(_lib.lib().psb_pull_margin(C.byref(p), stream_ptr(stream)), "pull_margin")
 
     # ---------------------------------------------------------------- two-sided pull (+ margins)
@@ -276,6 +278,8 @@ class DataPlane:
         p.ts1, p.need_applied, p.wait_iters, p.phases = ts + 1, need_applied, wait_iters, phases
         assert self.width == 1 or not with_margins, "margins need scalar values"
         p.ukeys, p.n_unique, p.own_off, p.grad_zero = ptr(b.ukeys), ptr(b.n_unique), ptr(b.own_off), ptr(b.grad)
+        # with several ranks this GPU also serves the others' requests, whose lengths the host does not know
+        p.work = min(b.n_keys_max * self.width, 0xffffffff) if self.S == 1 else 0
         if with_margins:
             p.row_ptr, p.n_rows, p.fixed_z = ptr(b.row_ptr), b.n_rows, b.fixed_z
             p.csr_col, p.csr_val, p.y = ptr(b.csr_col), ptr(b.csr_val), ptr(b.y)
@@ -325,6 +329,8 @@ class DataPlane:
         else:
             p.nnz = 0
         p.grad = ptr(b.grad)
+        p.work = min(b.n_keys_max * self.width, 0xffffffff)
+        self._round_work[q] = (ts, p.work)
         assert self.width == 1 or not with_gradient
         check(_lib.lib().psb_push(C.byref(p), stream_ptr(stream)), "push")
 
@@ -360,6 +366,8 @@ class DataPlane:
         for r in range(self.S):
             p.cached[r] = 1 if (cached is not None and cached[r]) else 0
         p.opt = (opt or self.opt).to_c()
+        if self.S == 1 and self._round_work.get(q, (None, 0))[0] == ts:
+            p.work = self._round_work[q][1]               # what this rank, the only source, pushed in the round
         check(_lib.lib().psb_apply(C.byref(p), stream_ptr(stream)), "apply")
         self.applied_ts1 = ts + 1
 
