@@ -244,12 +244,21 @@ __global__ void __launch_bounds__(kThreads) k_pull_margin(const PsbPullParams p)
   block_add4(loss_sum, n_correct, n_seen, 0.0, p.stats);
 }
 
+// Where a lane stands in a tile of 32 items x `width` columns that a warp walks in steps of 32 columns.
+struct WarpTile {
+  u32 item, col, width, di, dc;
+  __device__ __forceinline__ WarpTile(u32 lane, u32 w) : item(lane / w), col(lane % w), width(w), di(32u / w), dc(32u % w) {}
+  __device__ __forceinline__ void step() {
+    item += di; col += dc;
+    if (col >= width) { col -= width; ++item; }
+  }
+};
+
 // ------------------------------------------------------------------ F2 (exchange form)
 __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchangeParams p) {
   __shared__ u32 s_off[PSB_MAX_SHARDS + 1];
   __shared__ u32 s_last;
   __shared__ u32 s_n, s_base;
-  __shared__ u32 s_wslot[kThreads];                // slots of a tile of the k-wide owner path
   const int S = p.S;
   const u32 U = *p.n_unique;
   const u32 iters = p.wait_iters ? p.wait_iters : kPeerWaitIters;
@@ -375,43 +384,60 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
       }
     }
     if (kw > 1) {
-      // k values per key. A CTA takes tiles of blockDim.x keys: one thread per key finds the slot
-      // (remembered slots on a key-cache hit at the source), then the whole CTA copies the tile's
-      // k-wide rows with consecutive threads on consecutive values (16 bytes each when k % 4 == 0),
-      // so that the peer stores of a warp form whole lines.
+      // k values per key. A warp takes tiles of 32 keys: one lane per key finds the slot (remembered slots on
+      // a key-cache hit at the source), then the warp copies the tile's k-wide rows with consecutive lanes on
+      // consecutive values (16 bytes each when k % 4 == 0), so that its peer stores form whole lines, the
+      // loads of four steps issued together.
       const bool hit = (s_n & 0x80000000u) != 0;
-      for (u32 t0 = blockIdx.x * blockDim.x; t0 < n; t0 += gridDim.x * blockDim.x) {
-        const u32 j = t0 + threadIdx.x;
+      const u32 lane = threadIdx.x & 31;
+      for (u32 t0 = (gtid >> 5) * 32; t0 < n; t0 += gsize) {
+        const u32 j = t0 + lane;
+        u32 sc = 0x7fffffffu;
         if (j < n) {
-          u32 sc;
           if (hit) {
             sc = p.slot_cache_prev[r][j] & 0x7fffffffu;
           } else {
             const long long sl = table_find<true>(tab, sm, p.my_req_keys[r][j], kMaxProbe);
-            sc = sl >= 0 ? (u32)sl : 0x7fffffffu;
-            if (sl < 0) set_status(p.status, kTableFull);
+            if (sl >= 0) sc = (u32)sl;
+            else set_status(p.status, kTableFull);
           }
           p.slot_cache[r][j] = sc;
-          s_wslot[threadIdx.x] = sc;
         }
-        __syncthreads();
-        const u32 cnt = min((u32)blockDim.x, n - t0);
+        const u32 cnt = min(32u, n - t0);
         float* dst = p.resp_w[r] + (size_t)(base + t0) * kw;
         if ((kw & 3) == 0) {
           const u32 q4 = (u32)kw >> 2;
-          for (u32 idx = threadIdx.x; idx < cnt * q4; idx += blockDim.x) {
-            const u32 jj = idx / q4, c4 = idx - jj * q4, sc = s_wslot[jj];
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (sc != 0x7fffffffu) v = __ldcg(reinterpret_cast<const float4*>(p.wide_vals + (size_t)sc * kw) + c4);
-            reinterpret_cast<float4*>(dst)[idx] = v;
+          WarpTile at(lane, q4);
+          for (u32 x0 = lane; x0 - lane < cnt * q4; x0 += 128) {
+            float4 v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const u32 slot = __shfl_sync(0xffffffffu, sc, min(at.item, 31u));
+              v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (at.item < cnt && slot != 0x7fffffffu)
+                v[q] = __ldcg(reinterpret_cast<const float4*>(p.wide_vals + (size_t)slot * kw) + at.col);
+              at.step();
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (x0 + 32 * q < cnt * q4) reinterpret_cast<float4*>(dst)[x0 + 32 * q] = v[q];
           }
         } else {
-          for (u32 idx = threadIdx.x; idx < cnt * (u32)kw; idx += blockDim.x) {
-            const u32 jj = idx / (u32)kw, c = idx - jj * (u32)kw, sc = s_wslot[jj];
-            dst[idx] = sc != 0x7fffffffu ? __ldcg(&p.wide_vals[(size_t)sc * kw + c]) : 0.f;
+          WarpTile at(lane, (u32)kw);
+          for (u32 x0 = lane; x0 - lane < cnt * (u32)kw; x0 += 128) {
+            float v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const u32 slot = __shfl_sync(0xffffffffu, sc, min(at.item, 31u));
+              v[q] = 0.f;
+              if (at.item < cnt && slot != 0x7fffffffu) v[q] = __ldcg(&p.wide_vals[(size_t)slot * kw + at.col]);
+              at.step();
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (x0 + 32 * q < cnt * (u32)kw) dst[x0 + 32 * q] = v[q];
           }
         }
-        __syncthreads();
       }
       continue;
     }
@@ -531,12 +557,6 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
 }
 
 // ------------------------------------------------------------------ F1a: worker push
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
 // Value region of one inbox, by quantisation mode (cap = records per inbox):
 //   NONE : float v[cap]
 //   INT8 : float scale[ceil(cap/32)] followed by int8 code[cap]
@@ -545,7 +565,6 @@ __device__ __forceinline__ u32 scale_words(u32 cap) { return (cap + 31) / 32; }
 
 __global__ void __launch_bounds__(kThreads) k_push(const PsbPushParams p) {
   __shared__ u32 s_off[PSB_MAX_SHARDS + 1];
-  __shared__ u32 s_gp[PSB_MAX_SHARDS + 1];  // group prefix per owner
   __shared__ u32 s_last;
   const int S = p.S;
   if (threadIdx.x <= S) s_off[threadIdx.x] = p.own_off[threadIdx.x];
@@ -555,17 +574,7 @@ __global__ void __launch_bounds__(kThreads) k_push(const PsbPushParams p) {
         set_status(p.status, kWaitTimeout);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    u32 acc = 0;
-    for (int s = 0; s < S; ++s) {
-      s_gp[s] = acc;
-      u32 c = s_off[s + 1] - s_off[s];
-      if (c > p.inbox_cap) { set_status(p.status, kInboxOverflow); c = p.inbox_cap; }
-      acc += (c + 31) / 32;
-    }
-    s_gp[S] = acc;
-  }
-  __syncthreads();
+  if (threadIdx.x < S && s_off[threadIdx.x + 1] - s_off[threadIdx.x] > p.inbox_cap) set_status(p.status, kInboxOverflow);
   const int lane = threadIdx.x & 31;
   const u32 gsize = gridDim.x * blockDim.x;
   const u32 gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -642,61 +651,96 @@ __global__ void __launch_bounds__(kThreads) k_push(const PsbPushParams p) {
   }
   PSB_TSTAMP(2);
 
-  // phase 2: range partition + (quantise) + peer stores, 32 values per warp step. With value width k
-  // an owner's slice is cnt keys and cnt * k values (key-major); the group prefix counts value groups.
+  // phase 2: range partition + (quantise) + peer stores. With value width k an owner's slice is cnt keys and
+  // cnt * k values (key-major), quantised in groups of 32 consecutive values. A warp step takes 128 values,
+  // four consecutive ones per lane (a group is eight lanes), two steps' loads issued together: one value per
+  // lane and step left the kernel waiting for memory (262,145 keys of width 64 as int8, pushed, applied and
+  // pulled with the warp tiles of k_apply and k_pull_exchange: 460 -> 285 us; 1 M of width 8, plain: 250 -> 227).
   const bool omit_keys = !p.send_keys || (p.key_hit && *p.key_hit);
   const u32 kw = p.width > 1 ? (u32)p.width : 1u;
-  if (kw > 1) {
-    // group prefix over values instead of keys (recomputed by every CTA's thread 0)
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      u32 acc = 0;
-      for (int s = 0; s < S; ++s) {
-        s_gp[s] = acc;
-        acc += (min(s_off[s + 1] - s_off[s], p.inbox_cap) * kw + 31) / 32;
-      }
-      s_gp[S] = acc;
-    }
-    __syncthreads();
-    if (!omit_keys)
-      for (u32 u = gtid; u < s_off[S]; u += gsize) {
-        const int s = owner_of(s_off, S, u);
-        const u32 j = u - s_off[s];
-        if (j < p.inbox_cap) p.inbox_keys[s][j] = p.ukeys[u];
-      }
-  }
-  // owners in a per-CTA order, each owner's groups divided over the whole grid (see k_pull_exchange)
+  // owners in a per-CTA order, each owner's values divided over the whole grid (see k_pull_exchange)
   for (int kk = 0; kk < S; ++kk) {
-  const int s = (int)((blockIdx.x + (u32)kk) % (u32)S);
-  const u32 ng = s_gp[s + 1] - s_gp[s];
-  for (u32 gi = gwarp; gi < ng; gi += nwarps) {
-    const u32 g = s_gp[s] + gi;
-    u32 cnt = min(s_off[s + 1] - s_off[s], p.inbox_cap) * kw;       // values of this owner's slice
-    u32 j0 = (g - s_gp[s]) * 32, j = j0 + lane;
-    bool valid = j < cnt;
-    size_t u = (size_t)s_off[s] * kw + j;
-    float v = valid ? __ldcg(&p.grad[u]) : 0.f;
-    if (kw == 1 && !omit_keys && valid) p.inbox_keys[s][j] = p.ukeys[u];
-    const u32 vcap = p.inbox_cap * kw;
-    if (p.quant == PSB_QUANT_NONE) {
-      if (valid) ((float*)p.inbox_vals[s])[j] = v;
-    } else {
-      float amax = warp_max(fabsf(v));
-      float* scales = (float*)p.inbox_vals[s];
-      if (p.quant == PSB_QUANT_INT8) {
-        float scale = amax / 127.f;
-        int code = amax > 0.f ? __float2int_rn(v / scale) : 0;
-        signed char* codes = (signed char*)(scales + scale_words(vcap));
-        if (valid) codes[j] = (signed char)max(-127, min(127, code));
-        if (lane == 0) scales[j0 >> 5] = scale;
-      } else {
-        float scale = amax > 0.f ? amax : 1.f;
-        __half* codes = (__half*)(scales + scale_words(vcap));
-        if (valid) codes[j] = __float2half_rn(v / scale);
-        if (lane == 0) scales[j0 >> 5] = scale;
+    const int s = (int)((blockIdx.x + (u32)kk) % (u32)S);
+    const u32 nkeys = min(s_off[s + 1] - s_off[s], p.inbox_cap);
+    const u32 cnt = nkeys * kw, vcap = p.inbox_cap * kw;            // values of this owner's slice
+    const float* src = p.grad + (size_t)s_off[s] * kw;
+    if (!omit_keys)
+      for (u32 j0 = gtid; j0 < nkeys; j0 += 4 * gsize) {
+        u64 k[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) k[q] = j0 + q * gsize < nkeys ? p.ukeys[s_off[s] + j0 + q * gsize] : 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (j0 + q * gsize < nkeys) p.inbox_keys[s][j0 + q * gsize] = k[q];
+      }
+    // (a slice that starts off a 16-byte boundary, possible with several owners, is loaded value by value)
+    const bool src16 = (((size_t)src) & 15) == 0, dst16 = (((size_t)p.inbox_vals[s]) & 15) == 0;
+    const u32 steps = (cnt + 127) / 128;
+    for (u32 g0 = gwarp; g0 < steps; g0 += 2 * nwarps) {
+      float4 v[2];
+      u32 m[2];                                                    // values of this lane
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const u32 j = (g0 + q * nwarps) * 128 + 4 * lane;
+        m[q] = g0 + q * nwarps < steps && j < cnt ? min(4u, cnt - j) : 0u;
+        v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (m[q] == 4 && src16) {
+          v[q] = __ldcg(reinterpret_cast<const float4*>(src + j));
+        } else {
+          if (m[q] > 0) v[q].x = __ldcg(src + j);
+          if (m[q] > 1) v[q].y = __ldcg(src + j + 1);
+          if (m[q] > 2) v[q].z = __ldcg(src + j + 2);
+          if (m[q] > 3) v[q].w = __ldcg(src + j + 3);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const u32 j = (g0 + q * nwarps) * 128 + 4 * lane;
+        if (p.quant == PSB_QUANT_NONE) {
+          float* out = (float*)p.inbox_vals[s] + j;
+          if (m[q] == 4 && dst16) {
+            *reinterpret_cast<float4*>(out) = v[q];
+          } else {
+            if (m[q] > 0) out[0] = v[q].x;
+            if (m[q] > 1) out[1] = v[q].y;
+            if (m[q] > 2) out[2] = v[q].z;
+            if (m[q] > 3) out[3] = v[q].w;
+          }
+          continue;
+        }
+        float amax = fmaxf(fmaxf(fabsf(v[q].x), fabsf(v[q].y)), fmaxf(fabsf(v[q].z), fabsf(v[q].w)));
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        float* scales = (float*)p.inbox_vals[s];
+        const float x[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+        float scale;
+        if (p.quant == PSB_QUANT_INT8) {
+          scale = amax / 127.f;
+          signed char c[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            c[i] = (signed char)max(-127, min(127, amax > 0.f ? __float2int_rn(x[i] / scale) : 0));
+          signed char* out = (signed char*)(scales + scale_words(vcap)) + j;
+          if (m[q] == 4) {
+            *reinterpret_cast<char4*>(out) = make_char4(c[0], c[1], c[2], c[3]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) if ((u32)i < m[q]) out[i] = c[i];
+          }
+        } else {
+          scale = amax > 0.f ? amax : 1.f;
+          __half* out = (__half*)(scales + scale_words(vcap)) + j;
+          if (m[q] == 4) {
+            reinterpret_cast<__half2*>(out)[0] = __floats2half2_rn(x[0] / scale, x[1] / scale);
+            reinterpret_cast<__half2*>(out)[1] = __floats2half2_rn(x[2] / scale, x[3] / scale);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) if ((u32)i < m[q]) out[i] = __float2half_rn(x[i] / scale);
+          }
+        }
+        if ((lane & 7) == 0 && m[q]) scales[j >> 5] = scale;
       }
     }
-  }
   }
   // signal: all of this CTA's peer stores are ordered before its arrival, the
   // last CTA to arrive publishes counts and the release flags
@@ -729,10 +773,24 @@ __device__ __forceinline__ float inbox_value(const void* vals, int quant, u32 ca
   return scale * __half2float(((const __half*)(scales + scale_words(cap)))[j]);
 }
 
+// Four consecutive values from index j on, j a multiple of four (the region is 16-byte aligned when it holds
+// plain floats of a width that is a multiple of four; codes start on a 4-byte boundary).
+__device__ __forceinline__ float4 inbox_value4(const void* vals, int quant, u32 cap, u32 j) {
+  if (quant == PSB_QUANT_NONE) return *reinterpret_cast<const float4*>((const float*)vals + j);
+  const float* scales = (const float*)vals;
+  const float scale = scales[j >> 5];
+  if (quant == PSB_QUANT_INT8) {
+    const char4 c = *reinterpret_cast<const char4*>((const signed char*)(scales + scale_words(cap)) + j);
+    return make_float4(scale * (float)c.x, scale * (float)c.y, scale * (float)c.z, scale * (float)c.w);
+  }
+  const __half2* h = reinterpret_cast<const __half2*>((const __half*)(scales + scale_words(cap)) + j);
+  const float2 a = __half22float2(h[0]), b = __half22float2(h[1]);
+  return make_float4(scale * a.x, scale * a.y, scale * b.x, scale * b.y);
+}
+
 // kWide: values of width k > 1. An instantiation of its own, so that neither path pays for the other's registers.
 template <bool kWide>
-__global__ void __launch_bounds__(kThreads, kWide ? 4 : 3) k_apply(const PsbApplyParams p) {
-  __shared__ u32 s_wslot[kThreads], s_wsrc[kThreads], s_wrec[kThreads];   // a tile of the k-wide path
+__global__ void __launch_bounds__(kThreads, 3) k_apply(const PsbApplyParams p) {
   __shared__ u32 s_pre[PSB_MAX_SHARDS + 1];
   __shared__ u32 s_cached[PSB_MAX_SHARDS];
   __shared__ u32 s_last;
@@ -783,19 +841,19 @@ __global__ void __launch_bounds__(kThreads, kWide ? 4 : 3) k_apply(const PsbAppl
   StatAcc st;
 
   if constexpr (kWide) {
-    // k values per key, sum entries: every record adds its k values to wide_vals[slot * k ..]. A CTA
-    // takes tiles of blockDim.x records: one thread per record finds the slot, then the CTA adds the
-    // tile's values with consecutive threads on consecutive values (coalesced inbox reads; 16 bytes
-    // per thread where the inbox holds plain floats and k % 4 == 0). One source: plain
-    // read-modify-write (a slot belongs to one record); several: atomic adds.
+    // k values per key, sum entries: every record adds its k values to wide_vals[slot * k ..]. A warp takes
+    // tiles of 32 records: one lane per record finds the slot, then the warp adds the tile's values with
+    // consecutive lanes on consecutive values, four per lane where k % 4 == 0, the loads of four steps issued
+    // together. No warp waits for another. One source: plain read-modify-write (a slot belongs to one
+    // record); several: atomic adds.
     const u32 kw = (u32)p.width, vcap = p.inbox_cap * kw;
-    for (u32 t0 = blockIdx.x * blockDim.x; t0 < total; t0 += gridDim.x * blockDim.x) {
-      const u32 i = t0 + threadIdx.x;
+    const u32 lane = threadIdx.x & 31;
+    for (u32 t0 = (gtid >> 5) * 32; t0 < total; t0 += gsize) {
+      const u32 i = t0 + lane;
+      u32 sc = 0x7fffffffu, r = 0, j = 0;
       if (i < total) {
-        int r = 0;
-        while (r + 1 < S && i >= s_pre[r + 1]) ++r;
-        const u32 j = i - s_pre[r];
-        u32 sc;
+        while (r + 1 < (u32)S && i >= s_pre[r + 1]) ++r;
+        j = i - s_pre[r];
         if (s_cached[r]) {
           sc = p.slot_cache[r][j] & 0x7fffffffu;
         } else {
@@ -803,40 +861,64 @@ __global__ void __launch_bounds__(kThreads, kWide ? 4 : 3) k_apply(const PsbAppl
           sc = sl >= 0 ? (u32)sl : 0x7fffffffu;
           if (sl < 0) set_status(p.status, kTableFull);
         }
-        s_wslot[threadIdx.x] = sc;
-        s_wsrc[threadIdx.x] = (u32)r;
-        s_wrec[threadIdx.x] = j;
         if (sc != 0x7fffffffu) st.n += 1;
       }
-      __syncthreads();
-      const u32 cnt = min((u32)blockDim.x, total - t0);
-      if (p.opt.algo != PSB_ALGO_KEEP) {
-        if ((kw & 3) == 0 && p.quant == PSB_QUANT_NONE) {
-          const u32 q4 = kw >> 2;
-          for (u32 idx = threadIdx.x; idx < cnt * q4; idx += blockDim.x) {
-            const u32 jj = idx / q4, c4 = idx - jj * q4, sc = s_wslot[jj];
-            if (sc == 0x7fffffffu) continue;
-            const float4 g = reinterpret_cast<const float4*>((const float*)p.inbox_vals[s_wsrc[jj]] + (size_t)s_wrec[jj] * kw)[c4];
-            float4* dst = reinterpret_cast<float4*>(p.wide_vals + (size_t)sc * kw) + c4;
+      if (p.opt.algo == PSB_ALGO_KEEP) continue;
+      const u32 cnt = min(32u, total - t0);
+      if ((kw & 3) == 0) {
+        WarpTile at(lane, kw >> 2);
+        for (u32 x0 = lane; x0 - lane < cnt * (kw >> 2); x0 += 128) {
+          float4 g[4], o[4];
+          float* dst[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const u32 jj = min(at.item, 31u), c = at.col * 4;
+            const u32 slot = __shfl_sync(0xffffffffu, sc, jj), src = __shfl_sync(0xffffffffu, r, jj),
+                      rec = __shfl_sync(0xffffffffu, j, jj);
+            dst[q] = nullptr;
+            if (at.item < cnt && slot != 0x7fffffffu) {
+              dst[q] = p.wide_vals + (size_t)slot * kw + c;
+              g[q] = inbox_value4(p.inbox_vals[src], p.quant, vcap, rec * kw + c);
+              if (single) o[q] = *reinterpret_cast<const float4*>(dst[q]);
+            }
+            at.step();
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            if (dst[q] == nullptr) continue;
             if (single) {
-              float4 o = *dst;
-              o.x += g.x; o.y += g.y; o.z += g.z; o.w += g.w;
-              *dst = o;
+              o[q].x += g[q].x; o[q].y += g[q].y; o[q].z += g[q].z; o[q].w += g[q].w;
+              *reinterpret_cast<float4*>(dst[q]) = o[q];
             } else {
-              atomicAdd(dst, g);
+              atomicAdd(reinterpret_cast<float4*>(dst[q]), g[q]);
             }
           }
-        } else {
-          for (u32 idx = threadIdx.x; idx < cnt * kw; idx += blockDim.x) {
-            const u32 jj = idx / kw, c = idx - jj * kw, sc = s_wslot[jj];
-            if (sc == 0x7fffffffu) continue;
-            const float g = inbox_value(p.inbox_vals[s_wsrc[jj]], p.quant, vcap, s_wrec[jj] * kw + c);
-            float* dst = p.wide_vals + (size_t)sc * kw + c;
-            if (single) *dst += g; else atomicAdd(dst, g);
+        }
+      } else {
+        WarpTile at(lane, kw);
+        for (u32 x0 = lane; x0 - lane < cnt * kw; x0 += 128) {
+          float g[4], o[4];
+          float* dst[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const u32 jj = min(at.item, 31u);
+            const u32 slot = __shfl_sync(0xffffffffu, sc, jj), src = __shfl_sync(0xffffffffu, r, jj),
+                      rec = __shfl_sync(0xffffffffu, j, jj);
+            dst[q] = nullptr;
+            if (at.item < cnt && slot != 0x7fffffffu) {
+              dst[q] = p.wide_vals + (size_t)slot * kw + at.col;
+              g[q] = inbox_value(p.inbox_vals[src], p.quant, vcap, rec * kw + at.col);
+              if (single) o[q] = *dst[q];
+            }
+            at.step();
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            if (dst[q] == nullptr) continue;
+            if (single) *dst[q] = o[q] + g[q]; else atomicAdd(dst[q], g[q]);
           }
         }
       }
-      __syncthreads();
     }
   } else if (merge) {
     // Several sources whose slots are all remembered: one key-range part at a time, the records of all

@@ -168,3 +168,25 @@ def test_crowded_table_probes_past_collisions(cuda_lib, n):
     kv.wait(kv.push(keys, vals))
     have = dict(zip(*(t.tolist() for t in kv.plane.dump_nonzero())))
     assert have == {int(k): float(v) for k, v in zip(keys, vals) if v}
+
+
+@pytest.mark.parametrize("n", [1, 31, 129, 5000])
+@pytest.mark.parametrize("k,quant", [(1, "none"), (1, "int8"), (3, "none"), (3, "fp16"), (8, "none"), (8, "int8"), (64, "int8"),
+                                     (64, "fp16")])
+def test_request_sizes_widths_and_filters(cuda_lib, n, k, quant):
+    """Requests of a few to thousands of keys on one plane, values that start off a 16-byte boundary, groups of
+    32 values that end inside a row. Each of the two pushes is off by at most half a code step of its group."""
+    from parameter_server_b200.parameter.kv import DeviceKVVector
+    rng = np.random.default_rng(n * k)
+    kv = DeviceKVVector.create(table_capacity=1 << 14, max_keys=5001, k=k, quant=quant)
+    keys = np.unique(rng.integers(1, 1 << 60, 2 * n + 8).astype(np.uint64))[:n]
+    vals = torch.randn(n * k + 1, device="cuda")[1:].view(n, k)
+    t0 = kv.push(keys, vals)
+    t1 = kv.push(keys, vals, wait=[t0])
+    got = kv.pull(keys, wait=[t1])
+    kv.wait(got)
+    got = kv.result(got).view(n, k)
+    flat = torch.nn.functional.pad(vals.flatten(), (0, -n * k % 32)).view(-1, 32)
+    step = {"none": 0.0, "int8": 1 / 254, "fp16": 2.0 ** -11}[quant]
+    bound = (flat.abs().amax(1, keepdim=True) * 2 * step * 1.001 + flat.abs() * 2.0 ** -22).expand_as(flat).flatten()[:n * k].view(n, k)
+    assert ((got - 2 * vals).abs() <= bound).all()
