@@ -51,8 +51,9 @@
 
 namespace psb {
 
-static constexpr u32 kSampSlots = 1u << 17;       // sample hash table (global memory)
-static constexpr u32 kSampMax = 1u << 16;         // elements sampled
+static constexpr u32 kSampMin = 1u << 14;         // elements sampled: a quarter of them, between these two
+static constexpr u32 kSampMax = 1u << 16;
+static constexpr u32 kSampSlots = 2 * kSampMax;   // sample hash table (global memory), largest
 static constexpr u32 kHotSlots = 4096;            // hot-key lookup table (open addressing)
 static constexpr u32 kHotMax = 2048;              // hot keys at most
 static constexpr int kWalkThreads = 1024;         // count / scatter CTAs
@@ -93,7 +94,7 @@ struct BLP {
   int nb_bits;            // log2(number of buckets)
   u32 NB, NBINS;          // buckets; NB + kHotMax
   u32 G, chunk;           // walk CTAs and elements per CTA
-  u32 samp_m, samp_stride, hot_thresh, cold_limit;
+  u32 samp_m, samp_stride, samp_slots, hot_thresh, cold_limit;
   // rows
   const u32* row_ptr; u32 n_rows, fixed_z;
   const float* vals;
@@ -147,31 +148,40 @@ __device__ __forceinline__ u32 row_of_pos(const BLP& p, u32 pos, u32 zinv) {
   return row_search(p.row_ptr, p.row_hint[b], min(p.row_hint[b + 1] + 1, p.n_rows), pos);
 }
 
-// ---------------------------------------------------------------- 1. sample
-__global__ void __launch_bounds__(256) k_bl_sample(const BLP p) {
-  const u32 j = blockIdx.x * blockDim.x + threadIdx.x;
+// ---------------------------------------------------------------- 0. clean scratch
+// Everything that starts as zeros or ones, and the row hints, in one launch instead of one per region.
+__global__ void __launch_bounds__(256) k_bl_clear(const BLP p, uint4* zero, u32 zero4, uint4* ones, u32 ones4, u32 flag_words) {
+  const u32 gsize = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x;
+  for (u32 i = gtid; i < zero4; i += gsize) zero[i] = make_uint4(0, 0, 0, 0);
+  for (u32 i = gtid; i < ones4; i += gsize) ones[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+  for (u32 i = gtid; i < flag_words; i += gsize) p.flagbits[i] = 0;
   if (p.row_ptr != nullptr) {
     // row hints for steps 5 and 6, up to the block behind the last position
     const u32 nh = ((p.n - 1) >> kHintShift) + 2;
-    for (u32 h = j; h < nh; h += gridDim.x * blockDim.x) p.row_hint[h] = row_search(p.row_ptr, 0, p.n_rows, h << kHintShift);
+    for (u32 h = gtid; h < nh; h += gsize) p.row_hint[h] = row_search(p.row_ptr, 0, p.n_rows, h << kHintShift);
   }
+}
+
+// ---------------------------------------------------------------- 1. sample
+__global__ void __launch_bounds__(256) k_bl_sample(const BLP p) {
+  const u32 j = blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = j < p.samp_m;
   const u64 key = valid ? bl_key_of(p, j * p.samp_stride) : kEmptyKey;
   // equal keys of a warp count once (the most frequent key would otherwise take thousands of
   // atomics on one address)
   const u32 m = __match_any_sync(0xffffffffu, key);
   if (!valid || (int)(threadIdx.x & 31) != __ffs(m) - 1) return;
-  u32 slot = (u32)(fmix64(key) & (kSampSlots - 1));
-  for (u32 probe = 0; probe < kSampSlots; ++probe) {
+  u32 slot = (u32)(fmix64(key) & (p.samp_slots - 1));
+  for (u32 probe = 0; probe < p.samp_slots; ++probe) {
     u64 old = atomicCAS(&p.samp_key[slot], kEmptyKey, key);
     if (old == kEmptyKey || old == key) { atomicAdd(&p.samp_cnt[slot], (u32)__popc(m)); return; }
-    slot = (slot + 1) & (kSampSlots - 1);
+    slot = (slot + 1) & (p.samp_slots - 1);
   }
 }
 
 __global__ void __launch_bounds__(256) k_bl_hot(const BLP p) {
   const u32 s = blockIdx.x * blockDim.x + threadIdx.x;
-  const u32 c = s < kSampSlots ? p.samp_cnt[s] : 0u;
+  const u32 c = s < p.samp_slots ? p.samp_cnt[s] : 0u;
   // distinct keys of the sample (how much keys repeat decides the size of the buckets' tables)
   const u32 occ = __ballot_sync(0xffffffffu, c > 0);
   if ((threadIdx.x & 31) == 0 && occ) atomicAdd(&p.ctl[kCtlSampleDistinct], (u32)__popc(occ));
@@ -611,7 +621,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
     my_rank[k] = r; my_start[k] = st;
   }
   if (bad) s_ovf = 1;
-  // unique keys in all buckets before this one: look back over the published counts, 32 buckets per trip
+  // unique keys in all buckets before this one: look back over the published counts
   if (w == 0) {
     u32 ex = 0;
     if (b > 0) {
@@ -619,23 +629,35 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
       u32 spins = 0;
       bool done = false;
       while (!done && q >= 0) {
-        const long long idx = q - lane;
-        u32 v = kFlagIncl;
-        if (idx >= 0) asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.bstate + idx));
-        const u32 f = v & ~kValMask;
-        const u32 empty = __ballot_sync(0xffffffffu, f == 0);
-        const u32 incl = __ballot_sync(0xffffffffu, f == kFlagIncl);
-        const int first_empty = empty ? __ffs(empty) - 1 : 32;
-        const int first_incl = incl ? __ffs(incl) - 1 : 32;
-        const int upto = first_incl < first_empty ? first_incl + 1 : first_empty;   // lanes [0, upto) are usable
-        u32 add = lane < upto ? (v & kValMask) : 0u;
+        // 4 x 32 buckets are fetched per round trip to L2 and consumed from the nearest on
+        u32 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const long long idx = q - 32 * k - lane;
+          v[k] = kFlagIncl;
+          if (idx >= 0) v[k] = ld_relaxed_gpu(p.bstate + idx);
+        }
+        u32 add = 0;
+        int taken = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (done || taken < 32 * k) continue;    // warp-uniform
+          const u32 f = v[k] & ~kValMask;
+          const u32 empty = __ballot_sync(0xffffffffu, f == 0);
+          const u32 incl = __ballot_sync(0xffffffffu, f == kFlagIncl);
+          const int first_empty = empty ? __ffs(empty) - 1 : 32;
+          const int first_incl = incl ? __ffs(incl) - 1 : 32;
+          const int upto = first_incl < first_empty ? first_incl + 1 : first_empty;   // lanes [0, upto) are usable
+          if (lane < upto) add += v[k] & kValMask;
+          taken += upto;
+          if (first_incl < first_empty) done = true;
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
         ex += add;
-        if (first_incl < first_empty) done = true;
-        else {
-          q -= upto;
-          if (upto == 0) {
+        if (!done) {
+          q -= taken;
+          if (taken == 0) {
             // a bucket that gave up (or never started because of that) publishes nothing: stop waiting
             if (ld_relaxed_gpu(&p.ctl[kCtlFallback])) break;
             if (++spins > kGridWaitIters) { if (lane == 0) set_status(p.status, kLookbackTimeout); break; }
@@ -762,8 +784,6 @@ __global__ void __launch_bounds__(256) k_bl_hot_emit(const BLP p) {
   }
 }
 
-__global__ void k_bl_gate(const u32* ctl, u32* gate) { *gate = ctl[kCtlFallback]; }
-
 // scratch layout (bytes), shared by the size query and the launcher
 struct BlLayout {
   size_t zero_begin, samp_cnt, ctl, bstate, zero_end;
@@ -772,17 +792,17 @@ struct BlLayout {
       hot_u, hot_seg, row_hint, total;
 };
 static size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
-static BlLayout bl_layout(u32 NB, u32 G, u32 n) {
+static BlLayout bl_layout(u32 NB, u32 G, u32 n, u32 samp_slots) {
   BlLayout L;
   size_t o = 0;
   const u32 NBINS = NB + kHotMax;
   L.zero_begin = o;
-  L.samp_cnt = o; o = al(o + kSampSlots * 4);
+  L.samp_cnt = o; o = al(o + (size_t)samp_slots * 4);
   L.ctl = o; o = al(o + kCtlWords * 4);
   L.bstate = o; o = al(o + (size_t)NB * 4);
   L.zero_end = o;
   L.ff_begin = o;
-  L.samp_key = o; o = al(o + (size_t)kSampSlots * 8);
+  L.samp_key = o; o = al(o + (size_t)samp_slots * 8);
   L.hot_tab = o; o = al(o + (size_t)kHotSlots * 8);
   L.ff_end = o;
   L.hot_idx = o; o = al(o + kHotSlots * 2);
@@ -807,6 +827,10 @@ static u32 bl_num_buckets(u32 n) {
   // fills a bucket's table to 40 % only, so runs of adjacent occupied slots stay short
   u32 nb = 64;
   while (nb < kMaxBuckets && (size_t)nb * 1600 < n) nb <<= 1;
+  // a small minibatch gets more and smaller buckets, so that its few CTAs' worth of work is spread over the
+  // SMs (390,000 nonzeros in 256 buckets kept 256 CTAs busy for 49 us; with the smaller sample and walk grid the
+  // training step on them went from 231 to 180 us)
+  while (nb < 512 && (size_t)nb * 512 <= n) nb <<= 1;
   return nb;
 }
 static int bl_walk_ctas() {
@@ -822,7 +846,7 @@ using namespace psb;
 
 extern "C" size_t psb_bucket_localize_scratch_bytes(uint32_t max_n) {
   // sized for the largest bucket count; the per-nonzero buffers are the caller's
-  return bl_layout(kMaxBuckets, (u32)bl_walk_ctas(), max_n).total;
+  return bl_layout(kMaxBuckets, (u32)bl_walk_ctas(), max_n, kSampSlots).total;
 }
 
 // Groups the n nonzeros of a minibatch by key. Inputs as for psb_sort_pairs (in, in_kind, seed);
@@ -858,15 +882,19 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   p.nb_bits = 0;
   while ((1u << p.nb_bits) < p.NB) ++p.nb_bits;
   p.NBINS = p.NB + kHotMax;
-  p.G = (u32)bl_walk_ctas();
+  // walk CTAs: one per SM, and no more than get a full trip of 4096 elements (every CTA fills its shared tables
+  // first, and the scan over the CTAs' counts is a serial chain)
+  p.G = min((u32)bl_walk_ctas(), (n + 4 * kWalkThreads - 1) / (4 * kWalkThreads));
   p.chunk = ((n + p.G - 1) / p.G + 3) & ~3u;
-  p.samp_m = min(n, kSampMax);
+  p.samp_m = min(n, max(kSampMin, min(kSampMax, n / 4)));
+  p.samp_slots = 2;
+  while (p.samp_slots < 2 * p.samp_m) p.samp_slots <<= 1;
   p.samp_stride = n / p.samp_m;
   // hot: about half an average bucket or more, judged from the sample
   p.hot_thresh = max(4u, p.samp_m / p.NB / 2);
   p.cold_limit = max(32768u, 16u * (n / p.NB));
   p.row_ptr = row_ptr; p.n_rows = n_rows; p.fixed_z = fixed_z; p.vals = vals;
-  const BlLayout L = bl_layout(p.NB, p.G, n);
+  const BlLayout L = bl_layout(p.NB, p.G, n, p.samp_slots);
   unsigned char* sc = (unsigned char*)scratch;
   p.samp_key = (u64*)(sc + L.samp_key); p.samp_cnt = (u32*)(sc + L.samp_cnt);
   p.hot_tab = (u64*)(sc + L.hot_tab); p.hot_idx = (unsigned short*)(sc + L.hot_idx);
@@ -880,11 +908,11 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   p.ukeys = (u64*)ukeys; p.seg_off = seg_off; p.csr_col = csr_col; p.csc_row = csc_row; p.csc_val = csc_val;
   p.flagbits = flagbits; p.wordbase = wordbase; p.n_unique = n_unique; p.status = status;
 
-  cudaMemsetAsync(sc + L.zero_begin, 0, L.zero_end - L.zero_begin, stream);
-  cudaMemsetAsync(sc + L.ff_begin, 0xFF, L.ff_end - L.ff_begin, stream);
-  cudaMemsetAsync(flagbits, 0, sizeof(u32) * ((n + 31) / 32), stream);
+  const u32 zero4 = (u32)((L.zero_end - L.zero_begin) / 16), ones4 = (u32)((L.ff_end - L.ff_begin) / 16);
+  k_bl_clear<<<psb_device_sm_count() * 2, 256, 0, stream>>>(p, (uint4*)(sc + L.zero_begin), zero4, (uint4*)(sc + L.ff_begin),
+                                                            ones4, (n + 31) / 32);
   k_bl_sample<<<(p.samp_m + 255) / 256, 256, 0, stream>>>(p);
-  k_bl_hot<<<kSampSlots / 256, 256, 0, stream>>>(p);
+  k_bl_hot<<<(p.samp_slots + 255) / 256, 256, 0, stream>>>(p);
   const size_t walk_smem = kHotSlots * 8 + kHotSlots * 2 + (size_t)p.NBINS * 4;
   static bool attr_set = false;
   const int remaining = 64 - p.nb_bits - p.lo;      // key bits that distinguish keys inside a bucket
@@ -905,7 +933,7 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   k_bl_scan<<<(p.NBINS + 255) / 256, 256, 0, stream>>>(p);
   k_bl_plan<<<1, 1024, plan_smem, stream>>>(p);
   k_bl_walk<true><<<p.G, kWalkThreads, walk_smem, stream>>>(p);
-  const u32 g11 = min(p.NB, p.G * 6), g12 = min(p.NB, p.G * 4);
+  const u32 sms = (u32)bl_walk_ctas(), g11 = min(p.NB, sms * 6), g12 = min(p.NB, sms * 4);
   if (ck32) {
     k_bl_bucket<u32, 11><<<g11, kBucketThreads, BucketShape<11>::smem_bytes(4), stream>>>(p);
     k_bl_bucket<u32, 12><<<g12, kBucketThreads, BucketShape<12>::smem_bytes(4), stream>>>(p);
@@ -913,9 +941,8 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
     k_bl_bucket<u64, 11><<<g11, kBucketThreads, BucketShape<11>::smem_bytes(8), stream>>>(p);
     k_bl_bucket<u64, 12><<<g12, kBucketThreads, BucketShape<12>::smem_bytes(8), stream>>>(p);
   }
-  k_bl_hot_emit<<<p.G * 8, 256, 0, stream>>>(p);
-  k_bl_gate<<<1, 1, 0, stream>>>(p.ctl, gate_out);
+  k_bl_hot_emit<<<min(sms * 8, (n + 1023) / 1024), 256, 0, stream>>>(p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return -(int)e;
-  return psb_owner_offsets_n(ukeys, n_unique, bounds, S, n, seg_off, own_off, gate_out, stream);
+  return psb_owner_offsets_n(ukeys, n_unique, bounds, S, n, seg_off, own_off, p.ctl + kCtlFallback, gate_out, stream);
 }

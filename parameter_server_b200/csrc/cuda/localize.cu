@@ -20,11 +20,6 @@ static constexpr int kLocThreads = 256;
 static constexpr int kLocItems = 16;
 static constexpr int kLocTile = kLocThreads * kLocItems;  // 4096 = 128 flag words
 
-// Launch gate: with a non-null gate word the kernel runs only when (*gate != 0) == want.
-__device__ __forceinline__ bool gate_skips(const u32* gate, int want) {
-  return gate != nullptr && ((*gate != 0) != (want != 0));
-}
-
 // Loads the warp's 16 x 32 consecutive keys starting at `base` (all requested
 // before the first is used) and returns, per item, the ballot of segment heads.
 // kmask selects the key bits (all ones, or without the packed position bits).
@@ -47,16 +42,10 @@ __device__ __forceinline__ void warp_heads(const u64* __restrict__ keys, u32 n, 
   }
 }
 
-__global__ void __launch_bounds__(kLocThreads) k_uniq_count(const u64* __restrict__ keys_a,
-                                                            const u64* __restrict__ keys_b,
-                                                            const u32* __restrict__ where, u32 n,
-                                                            u32* __restrict__ tile_heads, u64 kmask,
-                                                            const u32* __restrict__ gate) {
+__device__ __forceinline__ void uniq_count_tile(const u64* keys, u32 n, u32 tile, u32* __restrict__ tile_heads, u64 kmask) {
   __shared__ u32 s_w[8];
-  if (gate_skips(gate, 1)) return;
-  const u64* __restrict__ keys = (where && *where) ? keys_b : keys_a;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const u32 base = blockIdx.x * (u32)kLocTile + w * (32 * kLocItems);
+  const u32 base = tile * (u32)kLocTile + w * (32 * kLocItems);
   u64 k[kLocItems];
   u32 bal[kLocItems];
   warp_heads(keys, n, base, lane, kmask, k, bal);
@@ -68,22 +57,26 @@ __global__ void __launch_bounds__(kLocThreads) k_uniq_count(const u64* __restric
   if (threadIdx.x == 0) {
     u32 t = 0;
     for (int i = 0; i < 8; ++i) t += s_w[i];
-    tile_heads[blockIdx.x] = t;
+    tile_heads[tile] = t;
   }
 }
+__global__ void __launch_bounds__(kLocThreads) k_uniq_count(const u64* __restrict__ keys_a,
+                                                            const u64* __restrict__ keys_b,
+                                                            const u32* __restrict__ where, u32 n,
+                                                            u32* __restrict__ tile_heads, u64 kmask) {
+  uniq_count_tile((where && *where) ? keys_b : keys_a, n, blockIdx.x, tile_heads, kmask);
+}
 
-// One block: exclusive scan of tile_heads in place; writes U.
-__global__ void __launch_bounds__(1024) k_uniq_scan(u32* __restrict__ tile_heads, u32 ntiles,
-                                                    u32* __restrict__ n_unique, const u32* __restrict__ gate) {
+// One CTA (any number of whole warps): exclusive scan of tile_heads in place; writes U.
+__device__ __forceinline__ void uniq_scan(u32* tile_heads, u32 ntiles, u32* __restrict__ n_unique) {
   __shared__ u32 s_warp[32];
   __shared__ u32 s_carry;
-  if (gate_skips(gate, 1)) return;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (threadIdx.x == 0) s_carry = 0;
   __syncthreads();
-  for (u32 base = 0; base < ntiles; base += 1024) {
+  for (u32 base = 0; base < ntiles; base += blockDim.x) {
     u32 i = base + threadIdx.x;
-    u32 v = i < ntiles ? tile_heads[i] : 0;
+    u32 v = i < ntiles ? __ldcg(&tile_heads[i]) : 0;
     u32 x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -93,7 +86,7 @@ __global__ void __launch_bounds__(1024) k_uniq_scan(u32* __restrict__ tile_heads
     if (lane == 31) s_warp[w] = x;
     __syncthreads();
     if (w == 0) {
-      u32 t = s_warp[lane];
+      u32 t = lane < nw ? s_warp[lane] : 0u;
       u32 xs = t;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -106,10 +99,13 @@ __global__ void __launch_bounds__(1024) k_uniq_scan(u32* __restrict__ tile_heads
     u32 carry = s_carry;
     if (i < ntiles) tile_heads[i] = carry + s_warp[w] + x - v;
     __syncthreads();
-    if (threadIdx.x == 1023) s_carry = carry + s_warp[w] + x;
+    if (threadIdx.x == blockDim.x - 1) s_carry = carry + s_warp[w] + x;
     __syncthreads();
   }
   if (threadIdx.x == 0) *n_unique = s_carry;
+}
+__global__ void __launch_bounds__(1024) k_uniq_scan(u32* __restrict__ tile_heads, u32 ntiles, u32* __restrict__ n_unique) {
+  uniq_scan(tile_heads, ntiles, n_unique);
 }
 
 // Emits, for the sorted pairs (keys[i], pos[i]) held in buffer A or B (*where):
@@ -120,21 +116,14 @@ __global__ void __launch_bounds__(1024) k_uniq_scan(u32* __restrict__ tile_heads
 //   flagbits[i/32], wordbase[i/32] (head bitmap and heads before each word).
 // Row of a position: pos / fixed_z when row_ptr is null, else the row whose
 // [row_ptr[r], row_ptr[r+1]) contains it.
-__global__ void __launch_bounds__(kLocThreads) k_uniq_emit(
-    const u64* __restrict__ keys_a, const u64* __restrict__ keys_b, const u32* pos_a,
-    const u32* pos_b, const u32* __restrict__ where, u32* csc_row /* may alias pos */, u32 n,
-    const u32* __restrict__ tile_base,
+__device__ __forceinline__ void uniq_emit_tile(
+    const u64* keys, const u32* pos, u32* csc_row /* may alias pos */, u32 n, u32 tile, const u32* tile_base,
     const u32* __restrict__ row_ptr, u32 n_rows, u32 fixed_z, const float* __restrict__ vals,
     u64* __restrict__ ukeys, u32* __restrict__ seg_off, u32* __restrict__ csr_col,
-    float* __restrict__ csc_val, u32* __restrict__ flagbits, u32* __restrict__ wordbase, u64 kmask,
-    const u32* __restrict__ gate) {
+    float* __restrict__ csc_val, u32* __restrict__ flagbits, u32* __restrict__ wordbase, u64 kmask) {
   __shared__ u32 s_w[8];
-  if (gate_skips(gate, 1)) return;
-  const bool in_b = where && *where;
-  const u64* __restrict__ keys = in_b ? keys_b : keys_a;
-  const u32* pos = in_b ? pos_b : pos_a;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const u32 base = blockIdx.x * (u32)kLocTile + w * (32 * kLocItems);
+  const u32 base = tile * (u32)kLocTile + w * (32 * kLocItems);
   u64 key[kLocItems];
   u32 bal[kLocItems];
   warp_heads(keys, n, base, lane, kmask, key, bal);
@@ -143,7 +132,7 @@ __global__ void __launch_bounds__(kLocThreads) k_uniq_emit(
   for (int i = 0; i < kLocItems; ++i) cnt += __popc(bal[i]);
   if (lane == 0) s_w[w] = cnt;
   __syncthreads();
-  u32 run = tile_base[blockIdx.x];
+  u32 run = __ldcg(&tile_base[tile]);
   for (int i = 0; i < w; ++i) run += s_w[i];
   const u32 zinv = fixed_z ? (u32)(0xffffffffu / fixed_z) : 0u;   // umulhi(p, zinv) <= p / fixed_z, short by at most 2
   const u32 le = 0xffffffffu >> (31 - lane);
@@ -180,26 +169,81 @@ __global__ void __launch_bounds__(kLocThreads) k_uniq_emit(
     run += __popc(bal[i]);
   }
 }
+__global__ void __launch_bounds__(kLocThreads) k_uniq_emit(
+    const u64* __restrict__ keys_a, const u64* __restrict__ keys_b, const u32* pos_a,
+    const u32* pos_b, const u32* __restrict__ where, u32* csc_row /* may alias pos */, u32 n,
+    const u32* __restrict__ tile_base,
+    const u32* __restrict__ row_ptr, u32 n_rows, u32 fixed_z, const float* __restrict__ vals,
+    u64* __restrict__ ukeys, u32* __restrict__ seg_off, u32* __restrict__ csr_col,
+    float* __restrict__ csc_val, u32* __restrict__ flagbits, u32* __restrict__ wordbase, u64 kmask) {
+  const bool in_b = where && *where;
+  uniq_emit_tile(in_b ? keys_b : keys_a, in_b ? pos_b : pos_a, csc_row, n, blockIdx.x, tile_base, row_ptr, n_rows, fixed_z,
+                 vals, ukeys, seg_off, csr_col, csc_val, flagbits, wordbase, kmask);
+}
 
 // own_off[s] = lower_bound(ukeys[0..U), bounds[s]) for s in 0..S; own_off[S] = U.
 // Also closes the CSC offsets with seg_off[U] = n.
-__global__ void k_owner_offsets(const u64* __restrict__ ukeys, const u32* __restrict__ n_unique,
-                                const u64* __restrict__ bounds, int S, u32 n,
-                                u32* __restrict__ seg_off, u32* __restrict__ own_off,
-                                const u32* __restrict__ gate, int want) {
-  if (gate_skips(gate, want)) return;
-  const u32 U = *n_unique;
-  int s = threadIdx.x;
-  if (s == 0 && seg_off) seg_off[U] = n;
-  if (s > S) return;
-  if (s == S) { own_off[S] = U; return; }
-  u64 b = bounds[s];
-  u32 lo = 0, hi = U;
-  while (lo < hi) {
-    u32 mid = (lo + hi) >> 1;
-    if (ukeys[mid] < b) lo = mid + 1; else hi = mid;
+// One warp per boundary: 32 probes side by side cut the range by 33 per trip, where a lone thread would wait
+// for log2(U) dependent loads (6 us with 2.7 M keys).
+__device__ __forceinline__ void owner_offsets(const u64* ukeys, u32 U, const u64* __restrict__ bounds, int S, u32 n,
+                                              u32* seg_off, u32* __restrict__ own_off) {
+  const u32 lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    if (seg_off) seg_off[U] = n;
+    own_off[S] = U;
   }
-  own_off[s] = lo;
+  for (int s = threadIdx.x >> 5; s < S; s += blockDim.x >> 5) {
+    const u64 b = bounds[s];
+    u32 lo = 0, hi = U;                            // the answer lies in [lo, hi]
+    while (lo < hi) {
+      const u32 step = (hi - lo + 32) / 33;        // probes at lo + step - 1, lo + 2 * step - 1, ..
+      const u64 at = (u64)lo + (u64)(lane + 1) * step - 1;
+      const bool below = at < hi && __ldcg(&ukeys[at]) < b;
+      const u32 k = (u32)__popc(__ballot_sync(0xffffffffu, below));
+      const u64 end = (u64)lo + (u64)(k + 1) * step - 1;    // the first probe that is not below (k < 32)
+      lo += k * step;
+      if (k < 32 && end < hi) hi = (u32)end;
+    }
+    if (lane == 0) own_off[s] = lo;
+  }
+}
+// Runs only while *skip_when_set is zero (null: always); *gate_out (nullable) receives that word.
+__global__ void __launch_bounds__(256) k_owner_offsets(const u64* __restrict__ ukeys, const u32* __restrict__ n_unique,
+                                                       const u64* __restrict__ bounds, int S, u32 n,
+                                                       u32* __restrict__ seg_off, u32* __restrict__ own_off,
+                                                       const u32* __restrict__ skip_when_set, u32* __restrict__ gate_out) {
+  const u32 skip = skip_when_set ? *skip_when_set : 0u;
+  if (gate_out && threadIdx.x == 0) *gate_out = skip;
+  if (skip) return;
+  owner_offsets(ukeys, *n_unique, bounds, S, n, seg_off, own_off);
+}
+
+// The four steps behind a device word, in one cooperative launch (see k_sort_gated).
+struct GatedLocalize {
+  const u64 *keys_a, *keys_b; const u32 *pos_a, *pos_b; const u32* where; u32* csc_row; u32 n;
+  const u32* row_ptr; u32 n_rows, fixed_z; const float* vals; const u64* bounds; int S;
+  u64* ukeys; u32 *seg_off, *csr_col; float* csc_val; u32 *flagbits, *wordbase, *n_unique, *own_off;
+  u32* tile_heads; u32* bar; u64 kmask; const u32* gate; u32* status;
+};
+__global__ void __launch_bounds__(kLocThreads) k_localize_gated(const GatedLocalize a) {
+  if (*a.gate == 0) return;
+  const u32 ntiles = (a.n + kLocTile - 1) / kLocTile;
+  const bool in_b = a.where && *a.where;
+  const u64* keys = in_b ? a.keys_b : a.keys_a;
+  for (u32 tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    uniq_count_tile(keys, a.n, tile, a.tile_heads, a.kmask);
+    __syncthreads();
+  }
+  if (!grid_barrier(a.bar, a.status)) return;
+  if (blockIdx.x == 0) uniq_scan(a.tile_heads, ntiles, a.n_unique);
+  if (!grid_barrier(a.bar, a.status)) return;
+  for (u32 tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    uniq_emit_tile(keys, in_b ? a.pos_b : a.pos_a, a.csc_row, a.n, tile, a.tile_heads, a.row_ptr, a.n_rows, a.fixed_z, a.vals,
+                   a.ukeys, a.seg_off, a.csr_col, a.csc_val, a.flagbits, a.wordbase, a.kmask);
+    __syncthreads();
+  }
+  if (!grid_barrier(a.bar, a.status)) return;
+  if (blockIdx.x == 0) owner_offsets(a.ukeys, __ldcg(a.n_unique), a.bounds, a.S, a.n, a.seg_off, a.own_off);
 }
 
 }  // namespace psb
@@ -211,7 +255,7 @@ using namespace psb;
 extern "C" int psb_owner_offsets(const psb_u64* ukeys, const uint32_t* n_unique, const psb_u64* bounds, int S,
                                  uint32_t* own_off, cudaStream_t stream) {
   if (S < 1 || S > 64) return -(int)cudaErrorInvalidValue;
-  k_owner_offsets<<<1, 96, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, 0, nullptr, own_off, nullptr, 0);
+  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, 0, nullptr, own_off, nullptr, nullptr);
   return -(int)cudaGetLastError();
 }
 
@@ -229,7 +273,7 @@ static int localize2_impl(const psb_u64* keys_a, const psb_u64* keys_b, const ui
                           uint32_t* seg_off, uint32_t* csr_col, float* csc_val,
                           uint32_t* flagbits, uint32_t* wordbase, uint32_t* n_unique,
                           uint32_t* own_off, void* scratch, int pack_pos_bits, const uint32_t* gate,
-                          cudaStream_t stream) {
+                          uint32_t* status, cudaStream_t stream) {
   if (S < 1 || S > 64) return -(int)cudaErrorInvalidValue;
   if (row_ptr == nullptr && fixed_z == 0) return -(int)cudaErrorInvalidValue;
   if (pack_pos_bits < 0 || pack_pos_bits > 32) return -(int)cudaErrorInvalidValue;
@@ -243,12 +287,28 @@ static int localize2_impl(const psb_u64* keys_a, const psb_u64* keys_b, const ui
     cudaMemsetAsync(seg_off, 0, sizeof(u32), stream);
     return -(int)cudaGetLastError();
   }
-  k_uniq_count<<<ntiles, kLocThreads, 0, stream>>>((const u64*)keys_a, (const u64*)keys_b, where, n, tile_heads, kmask, gate);
-  k_uniq_scan<<<1, 1024, 0, stream>>>(tile_heads, ntiles, n_unique, gate);
+  if (gate != nullptr) {
+    u32* bar = const_cast<u32*>(gate) + 3;             // see psb_sort_pairs_gated
+    static int per_sm = 0;
+    if (per_sm == 0) {
+      int per = 0;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k_localize_gated, kLocThreads, 0);
+      per_sm = per < 1 ? 1 : (per > 4 ? 4 : per);
+    }
+    GatedLocalize a{(const u64*)keys_a, (const u64*)keys_b, pos_a, pos_b, where, csc_row, n, row_ptr, n_rows, fixed_z, vals,
+                    (const u64*)bounds, S, (u64*)ukeys, seg_off, csr_col, csc_val, flagbits, wordbase, n_unique, own_off,
+                    tile_heads, bar, kmask, gate, status};
+    void* args[] = {&a};
+    return -(int)cudaLaunchCooperativeKernel((const void*)k_localize_gated,
+                                             dim3(min(ntiles, (u32)(psb_device_sm_count() * per_sm))), dim3(kLocThreads),
+                                             args, 0, stream);
+  }
+  k_uniq_count<<<ntiles, kLocThreads, 0, stream>>>((const u64*)keys_a, (const u64*)keys_b, where, n, tile_heads, kmask);
+  k_uniq_scan<<<1, 1024, 0, stream>>>(tile_heads, ntiles, n_unique);
   k_uniq_emit<<<ntiles, kLocThreads, 0, stream>>>((const u64*)keys_a, (const u64*)keys_b, pos_a, pos_b, where, csc_row,
                                                   n, tile_heads, row_ptr, n_rows, fixed_z, vals, (u64*)ukeys, seg_off,
-                                                  csr_col, csc_val, flagbits, wordbase, kmask, gate);
-  k_owner_offsets<<<1, 96, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off, own_off, gate, 1);
+                                                  csr_col, csc_val, flagbits, wordbase, kmask);
+  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off, own_off, nullptr, nullptr);
   return -(int)cudaGetLastError();
 }
 
@@ -261,10 +321,10 @@ extern "C" int psb_localize2(const psb_u64* keys_a, const psb_u64* keys_b, const
                              uint32_t* own_off, void* scratch, int pack_pos_bits, cudaStream_t stream) {
   return localize2_impl(keys_a, keys_b, pos_a, pos_b, where, csc_row, n, row_ptr, n_rows, fixed_z, vals, bounds, S,
                         ukeys, seg_off, csr_col, csc_val, flagbits, wordbase, n_unique, own_off, scratch,
-                        pack_pos_bits, nullptr, stream);
+                        pack_pos_bits, nullptr, nullptr, stream);
 }
 
-// Same, but every kernel of the call returns at once unless the device word *gate is non-zero.
+// Same, but nothing happens unless the device word *gate is non-zero (null: always; see k_localize_gated).
 extern "C" int psb_localize2_gated(const psb_u64* keys_a, const psb_u64* keys_b, const uint32_t* pos_a,
                                    const uint32_t* pos_b, const uint32_t* where, uint32_t* csc_row, uint32_t n,
                                    const uint32_t* row_ptr, uint32_t n_rows, uint32_t fixed_z,
@@ -272,20 +332,20 @@ extern "C" int psb_localize2_gated(const psb_u64* keys_a, const psb_u64* keys_b,
                                    uint32_t* seg_off, uint32_t* csr_col, float* csc_val,
                                    uint32_t* flagbits, uint32_t* wordbase, uint32_t* n_unique,
                                    uint32_t* own_off, void* scratch, int pack_pos_bits, const uint32_t* gate,
-                                   cudaStream_t stream) {
+                                   uint32_t* status, cudaStream_t stream) {
   return localize2_impl(keys_a, keys_b, pos_a, pos_b, where, csc_row, n, row_ptr, n_rows, fixed_z, vals, bounds, S,
                         ukeys, seg_off, csr_col, csc_val, flagbits, wordbase, n_unique, own_off, scratch,
-                        pack_pos_bits, gate, stream);
+                        pack_pos_bits, gate, status, stream);
 }
 
-// Owner offsets plus the closing CSC offset seg_off[U] = n; runs only while *skip_when_set is zero
-// (the bucket-based localisation's last step).
+// Owner offsets plus the closing CSC offset seg_off[U] = n; runs only while *skip_when_set is zero, and copies
+// that word to *gate_out (the bucket-based localisation's last step).
 extern "C" int psb_owner_offsets_n(const psb_u64* ukeys, const uint32_t* n_unique, const psb_u64* bounds, int S,
                                    uint32_t n, uint32_t* seg_off, uint32_t* own_off,
-                                   const uint32_t* skip_when_set, cudaStream_t stream) {
+                                   const uint32_t* skip_when_set, uint32_t* gate_out, cudaStream_t stream) {
   if (S < 1 || S > 64) return -(int)cudaErrorInvalidValue;
-  k_owner_offsets<<<1, 96, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off, own_off,
-                                        skip_when_set, 0);
+  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off, own_off,
+                                         skip_when_set, gate_out);
   return -(int)cudaGetLastError();
 }
 
@@ -306,12 +366,12 @@ extern "C" int psb_localize(const psb_u64* sorted_keys, uint32_t* sorted_pos, ui
     cudaMemsetAsync(seg_off, 0, sizeof(u32), stream);
     return -(int)cudaGetLastError();
   }
-  k_uniq_count<<<ntiles, kLocThreads, 0, stream>>>((const u64*)sorted_keys, nullptr, nullptr, n, tile_heads, ~0ull, nullptr);
-  k_uniq_scan<<<1, 1024, 0, stream>>>(tile_heads, ntiles, n_unique, nullptr);
+  k_uniq_count<<<ntiles, kLocThreads, 0, stream>>>((const u64*)sorted_keys, nullptr, nullptr, n, tile_heads, ~0ull);
+  k_uniq_scan<<<1, 1024, 0, stream>>>(tile_heads, ntiles, n_unique);
   k_uniq_emit<<<ntiles, kLocThreads, 0, stream>>>((const u64*)sorted_keys, nullptr, sorted_pos, nullptr, nullptr,
                                                   sorted_pos, n, tile_heads, row_ptr, n_rows, fixed_z, vals,
-                                                  (u64*)ukeys, seg_off, csr_col, csc_val, flagbits, wordbase, ~0ull, nullptr);
-  k_owner_offsets<<<1, 96, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off, own_off, nullptr, 0);
+                                                  (u64*)ukeys, seg_off, csr_col, csc_val, flagbits, wordbase, ~0ull);
+  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off, own_off, nullptr, nullptr);
   return -(int)cudaGetLastError();
 }
 
@@ -371,12 +431,12 @@ extern "C" int psb_localize_static(const psb_u64* sorted_keys, uint32_t* sorted_
   const u32 ntiles = (n + kLocTile - 1) / kLocTile;
   // every tile_heads word that the scan and the emit kernel read is written by
   // k_uniq_count first, so the array needs no clearing between calls
-  k_uniq_count<<<ntiles, kLocThreads, 0, stream>>>((const u64*)sorted_keys, nullptr, nullptr, n, tile_heads, ~0ull, nullptr);
-  k_uniq_scan<<<1, 1024, 0, stream>>>(tile_heads, ntiles, n_unique, nullptr);
+  k_uniq_count<<<ntiles, kLocThreads, 0, stream>>>((const u64*)sorted_keys, nullptr, nullptr, n, tile_heads, ~0ull);
+  k_uniq_scan<<<1, 1024, 0, stream>>>(tile_heads, ntiles, n_unique);
   k_uniq_emit<<<ntiles, kLocThreads, 0, stream>>>((const u64*)sorted_keys, nullptr, sorted_pos, nullptr, nullptr,
                                                   sorted_pos, n, tile_heads, row_ptr, n_rows, fixed_z, vals,
-                                                  (u64*)ukeys, seg_off, csr_col, csc_val, flagbits, wordbase, ~0ull, nullptr);
-  k_owner_offsets<<<1, 96, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off,
-                                        own_off, nullptr, 0);
+                                                  (u64*)ukeys, seg_off, csr_col, csc_val, flagbits, wordbase, ~0ull);
+  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off,
+                                         own_off, nullptr, nullptr);
   return -(int)cudaGetLastError();
 }

@@ -40,10 +40,6 @@ __device__ __forceinline__ u32 ld_status(const u32* p) {
   return v;
 }
 
-// Launch gate: a device word decides whether the kernels of a call run at all (the sort-based
-// localisation is enqueued behind the bucket-based one and only runs when that one gave up).
-__device__ __forceinline__ bool gate_closed(const u32* gate) { return gate != nullptr && *gate == 0; }
-
 __device__ __forceinline__ u32 digit_of(u64 k, int shift, u32 dmask) {
   return (u32)(k >> shift) & dmask;
 }
@@ -53,11 +49,9 @@ __device__ __forceinline__ u32 digit_of(u64 k, int shift, u32 dmask) {
 // pack_bits > 0 (hashed input only): the element index is stored in the low
 // pack_bits bits of the key, which the narrow hash leaves zero, so the pairs
 // travel as single 64-bit words and need no payload array.
-__global__ void __launch_bounds__(256) k_sort_histogram(
+__device__ __forceinline__ void sort_histogram(
     const void* __restrict__ in, int in_kind, u64 seed, u64* __restrict__ keys_out, u32 n,
-    int begin_bit, int end_bit, u32* __restrict__ ghist, int pack_bits, const u32* __restrict__ gate) {
-  __shared__ u32 sh[8 * kRadix];
-  if (gate_closed(gate)) return;
+    int begin_bit, int end_bit, u32* __restrict__ ghist, int pack_bits, u32* sh /* shared, 8 * kRadix words */) {
   const int npass = (end_bit - begin_bit + kRadixBits - 1) / kRadixBits;
   for (int i = threadIdx.x; i < npass * kRadix; i += blockDim.x) sh[i] = 0;
   __syncthreads();
@@ -133,35 +127,39 @@ __global__ void __launch_bounds__(256) k_sort_histogram(
   for (int i = threadIdx.x; i < npass * kRadix; i += blockDim.x)
     if (sh[i]) atomicAdd(&ghist[i], sh[i]);
 }
+__global__ void __launch_bounds__(256) k_sort_histogram(
+    const void* __restrict__ in, int in_kind, u64 seed, u64* __restrict__ keys_out, u32 n,
+    int begin_bit, int end_bit, u32* __restrict__ ghist, int pack_bits) {
+  __shared__ u32 sh[8 * kRadix];
+  sort_histogram(in, in_kind, seed, keys_out, n, begin_bit, end_bit, ghist, pack_bits, sh);
+}
 
 // Pass plan. A digit position whose histogram has a single non-empty bin does
 // not change the order, so its pass is skipped (keys with fewer significant bits
 // than the sorted range, e.g. hashed 40-bit keys, cost proportionally less).
 // plan[p]: bit 0 = skip, bit 1 = source buffer (0 = A, 1 = B), bit 2 = first
 // executed pass (payload defaults to the element index); plan[16] = buffer that
-// holds the result.
-__global__ void __launch_bounds__(kRadix) k_sort_plan(const u32* __restrict__ ghist, int npass, u32 n,
-                                                      u32* __restrict__ plan, u32* __restrict__ gpre,
-                                                      const u32* __restrict__ gate) {
+// holds the result. One CTA of at least kRadix threads.
+__device__ __forceinline__ void sort_plan(const u32* ghist, int npass, u32 n, u32* __restrict__ plan, u32* __restrict__ gpre) {
   __shared__ u32 s_skip[8];
-  if (gate_closed(gate)) return;
   __shared__ u32 s_scan[kRadix];
   const int t = threadIdx.x;
+  const bool mine = t < kRadix;
   if (t < 8) s_skip[t] = 0;
   __syncthreads();
   for (int p = 0; p < npass; ++p) {
     // gpre[p][d] = number of keys whose digit p is below d (global start of digit d)
-    const u32 c = ghist[p * kRadix + t];
-    if (c == n) s_skip[p] = 1;
-    s_scan[t] = c;
+    const u32 c = mine ? __ldcg(&ghist[p * kRadix + t]) : 0u;
+    if (mine && c == n) s_skip[p] = 1;
+    if (mine) s_scan[t] = c;
     __syncthreads();
     for (int o = 1; o < kRadix; o <<= 1) {
-      u32 y = t >= o ? s_scan[t - o] : 0u;
+      u32 y = mine && t >= o ? s_scan[t - o] : 0u;
       __syncthreads();
-      s_scan[t] += y;
+      if (mine) s_scan[t] += y;
       __syncthreads();
     }
-    gpre[p * kRadix + t] = s_scan[t] - c;
+    if (mine) gpre[p * kRadix + t] = s_scan[t] - c;
     __syncthreads();
   }
   if (t == 0) {
@@ -175,12 +173,15 @@ __global__ void __launch_bounds__(kRadix) k_sort_plan(const u32* __restrict__ gh
     plan[17] = first;   // 1: every pass was skipped (the input order is already sorted)
   }
 }
+__global__ void __launch_bounds__(kRadix) k_sort_plan(const u32* __restrict__ ghist, int npass, u32 n,
+                                                      u32* __restrict__ plan, u32* __restrict__ gpre) {
+  sort_plan(ghist, npass, n, plan, gpre);
+}
 
 // When every pass is skipped (the input is already in order) and no payload was
 // given, the payload still has to become the element index.
-__global__ void k_sort_identity_payload(const u32* __restrict__ plan, u32* __restrict__ vals_a, u32 n,
-                                        const u32* __restrict__ gate) {
-  if (gate_closed(gate) || plan[17] == 0) return;
+__global__ void k_sort_identity_payload(const u32* __restrict__ plan, u32* __restrict__ vals_a, u32 n) {
+  if (plan[17] == 0) return;
   for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) vals_a[i] = i;
 }
 
@@ -204,27 +205,23 @@ __global__ void k_sort_identity_payload(const u32* __restrict__ plan, u32* __res
 // aggregate) -> keys scattered to shared memory in digit order -> look-back
 // (the key registers are free by then, so 32 predecessors are fetched per L2
 // round trip) -> coalesced global stores of the digit runs.
-__global__ void __launch_bounds__(kSortThreads, 2) k_sort_onesweep(
-    u64* __restrict__ keys_a, u32* __restrict__ vals_a, u64* __restrict__ keys_b, u32* __restrict__ vals_b,
-    int vals_given, u32 n, int shift, u32 dmask, const u32* __restrict__ gpre,
-    u32* __restrict__ status, u32* __restrict__ err, const u32* __restrict__ plan, int pass,
-    u32* __restrict__ ticket, const u32* __restrict__ gate PSB_TRACE_PARAM) {
+//
+// `pl` is the pass's plan word (not a constant digit). Returns false when no tile is left.
+__device__ __forceinline__ bool sort_onesweep_tile(
+    u64* keys_a, u32* vals_a, u64* keys_b, u32* vals_b,
+    int vals_given, u32 n, int shift, u32 dmask, const u32* gpre,
+    u32* __restrict__ status, u32* __restrict__ err, u32 pl, u32* __restrict__ ticket,
+    u64* s_keys /* shared, kSortTile keys, reused for payloads */ PSB_TRACE_PARAM) {
 #ifdef PSB_SORT_TRACE
   long long ts[12] = {0}; int nts = 0;
 #endif
   PSB_STAMP();
-  if (gate_closed(gate)) return;
-  // the plan word is the same for every tile: keep its line in L1 for the later tiles of this SM
-  u32 pl;
-  asm volatile("ld.global.nc.L1::evict_last.u32 %0, [%1];" : "=r"(pl) : "l"(plan + pass));
-  if (pl & 1u) return;                                   // constant digit: nothing to do
   const bool from_b = (pl >> 1) & 1u;
   const u64* __restrict__ keys_in = from_b ? keys_b : keys_a;
   u64* __restrict__ keys_out = from_b ? keys_a : keys_b;
   const u32* __restrict__ vals_in = from_b ? vals_b : vals_a;
   u32* __restrict__ vals_out = from_b ? vals_a : vals_b;
   if ((pl & 4u) && !vals_given) vals_in = nullptr;       // first executed pass: payload = index
-  __shared__ u64 s_keys[kSortTile];            // 32 KB, reused for payloads
   // per-warp digit counters (<= 256 each), two 16-bit counters per word so that the
   // ranking can use 32-bit shared atomics; read back as 16-bit values afterwards. 8 KB
   __shared__ u32 s_cnt32[kSortWarps * kRadix / 2];
@@ -238,6 +235,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort_onesweep(
   if (t == 0) s_tile = atomicAdd(ticket, 1u);
   __syncthreads();
   const u32 tile = s_tile;
+  if (tile >= (n + kSortTile - 1) / kSortTile) return false;
   const u32 tile_base = tile * (u32)kSortTile;
   const u32 nvalid = min((u32)kSortTile, n - tile_base);
 
@@ -394,7 +392,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort_onesweep(
     for (int q = 0; q < 12; ++q) trace[(size_t)tile * 12 + q] = ts[q];
   }
 #endif
-  if (vals_out == nullptr) return;
+  if (vals_out == nullptr) return true;
   __syncthreads();
   // ---- payloads through the same staging buffer ----
   u32* s_vals = reinterpret_cast<u32*>(s_keys);
@@ -402,7 +400,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort_onesweep(
   for (int i = 0; i < kSortItems; ++i) {
     u32 idx = wbase + i * 32 + lane;
     u32 v = 0;
-    if (idx < nvalid) v = vals_in ? vals_in[tile_base + idx] : tile_base + idx;
+    if (idx < nvalid) v = vals_in ? __ldcg(&vals_in[tile_base + idx]) : tile_base + idx;
     s_vals[off[i]] = v;
   }
   __syncthreads();
@@ -411,6 +409,68 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort_onesweep(
     u32 p = t + j * kSortThreads;
     if (p < nvalid) vals_out[dst[j]] = s_vals[p];
   }
+  return true;
+}
+__global__ void __launch_bounds__(kSortThreads, 2) k_sort_onesweep(
+    u64* __restrict__ keys_a, u32* __restrict__ vals_a, u64* __restrict__ keys_b, u32* __restrict__ vals_b,
+    int vals_given, u32 n, int shift, u32 dmask, const u32* __restrict__ gpre,
+    u32* __restrict__ status, u32* __restrict__ err, const u32* __restrict__ plan, int pass,
+    u32* __restrict__ ticket PSB_TRACE_PARAM) {
+  // the plan word is the same for every tile: keep its line in L1 for the later tiles of this SM
+  u32 pl;
+  asm volatile("ld.global.nc.L1::evict_last.u32 %0, [%1];" : "=r"(pl) : "l"(plan + pass));
+  if (pl & 1u) return;                                   // constant digit: nothing to do
+  __shared__ u64 s_keys[kSortTile];                      // 32 KB
+  sort_onesweep_tile(keys_a, vals_a, keys_b, vals_b, vals_given, n, shift, dmask, gpre, status, err, pl, ticket, s_keys
+#ifdef PSB_SORT_TRACE
+                     , trace
+#endif
+  );
+}
+
+// The whole sort behind a device word: nothing happens unless *gate is set (the bucket-based localisation
+// gave up on its minibatch). One cooperative launch with grid barriers between the steps, because a call
+// that is nearly always skipped costs what its launches cost: the sort and the steps behind it were seventeen of
+// them, 17 us (64,000 nonzeros) to 36 us (13 M) of a localisation that had no use for them.
+struct GatedSort {
+  const void* in; int in_kind; u64 seed;
+  u64* keys_a; u32* vals_a; int vals_given; u64* keys_b; u32* vals_b;
+  u32 n; int begin_bit, end_bit, npass, pack_bits;
+  u32 *ghist, *gpre, *tickets, *plan, *st;               // one array, plus the status words of npass passes
+  u32* bar;                                              // two words behind the gate
+  u32* err; u32* where_out;
+  const u32* gate;
+};
+__global__ void __launch_bounds__(kSortThreads, 2) k_sort_gated(const GatedSort a) {
+  if (*a.gate == 0) return;
+  __shared__ u64 s_keys[kSortTile];
+  u32* bar = a.bar;
+  const u32 ntiles = (a.n + kSortTile - 1) / kSortTile;
+  const u32 gsz = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t words = (size_t)(a.st - a.ghist) + (size_t)a.npass * ntiles * kRadix;
+  for (size_t i = gtid; i < words; i += gsz) a.ghist[i] = 0;
+  if (!grid_barrier(bar, a.err)) return;
+  sort_histogram(a.in, a.in_kind, a.seed, a.keys_a, a.n, a.begin_bit, a.end_bit, a.ghist, a.pack_bits,
+                 reinterpret_cast<u32*>(s_keys));
+  if (!grid_barrier(bar, a.err)) return;
+  if (blockIdx.x == 0) sort_plan(a.ghist, a.npass, a.n, a.plan, a.gpre);
+  if (!grid_barrier(bar, a.err)) return;
+  for (int p = 0; p < a.npass; ++p) {
+    const u32 pl = __ldcg(&a.plan[p]);
+    if (pl & 1u) continue;
+    const int shift = a.begin_bit + p * kRadixBits, bits = min(kRadixBits, a.end_bit - shift);
+    while (sort_onesweep_tile(a.keys_a, a.vals_a, a.keys_b, a.vals_b, a.vals_given, a.n, shift, (1u << bits) - 1,
+                              a.gpre + (size_t)p * kRadix, a.st + (size_t)p * ntiles * kRadix, a.err, pl, a.tickets + p, s_keys
+#ifdef PSB_SORT_TRACE
+                              , nullptr
+#endif
+                              ))
+      __syncthreads();                                   // the tile's shared arrays are used again
+    if (!grid_barrier(bar, a.err)) return;
+  }
+  if (!a.vals_given && a.vals_a && !a.pack_bits && __ldcg(&a.plan[17]) != 0)
+    for (u32 i = gtid; i < a.n; i += gsz) a.vals_a[i] = i;
+  if (gtid == 0) *a.where_out = __ldcg(&a.plan[16]);
 }
 
 }  // namespace psb
@@ -455,23 +515,38 @@ static int sort_pairs_impl(const void* in, int in_kind, psb_u64 seed, psb_u64* k
   u32* tickets = gpre + (size_t)npass * kRadix;   // one zeroed word per pass (16 reserved)
   u32* plan = tickets + 16;
   u32* st = plan + 32;
+  if (gate != nullptr) {
+    static int per_sm = 0;
+    if (per_sm == 0) {
+      int per = 0;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k_sort_gated, kSortThreads, 0);
+      per_sm = per < 1 ? 1 : (per > 2 ? 2 : per);
+    }
+    GatedSort a{in, in_kind, seed, (u64*)keys_a, vals_a, vals_given, (u64*)keys_b, vals_b, n, begin_bit, end_bit, npass,
+                pack_pos_bits, ghist, gpre, tickets, plan, st, const_cast<u32*>(gate) + 1, status, where_out, gate};
+    void* args[] = {&a};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_sort_gated,
+                                                      dim3(min(ntiles, (u32)(psb_device_sm_count() * per_sm))),
+                                                      dim3(kSortThreads), args, 0, stream);
+    return -(int)e;
+  }
   cudaMemsetAsync(scratch, 0, psb_sort_scratch_bytes(n, begin_bit, end_bit), stream);
   int hb = (int)min((u32)(psb_device_sm_count() * 8), (n / 8 + 255) / 256 + 1);
   k_sort_histogram<<<hb, 256, 0, stream>>>(in, in_kind, seed, (u64*)keys_a, n, begin_bit, end_bit, ghist,
-                                           pack_pos_bits, gate);
-  k_sort_plan<<<1, kRadix, 0, stream>>>(ghist, npass, n, plan, gpre, gate);
+                                           pack_pos_bits);
+  k_sort_plan<<<1, kRadix, 0, stream>>>(ghist, npass, n, plan, gpre);
   for (int p = 0; p < npass; ++p) {
     int shift = begin_bit + p * kRadixBits;
     int bits = min(kRadixBits, end_bit - shift);
     k_sort_onesweep<<<ntiles, kSortThreads, 0, stream>>>(
         (u64*)keys_a, vals_a, (u64*)keys_b, vals_b, vals_given, n, shift, (1u << bits) - 1,
-        gpre + (size_t)p * kRadix, st + (size_t)p * ntiles * kRadix, status, plan, p, tickets + p, gate
+        gpre + (size_t)p * kRadix, st + (size_t)p * ntiles * kRadix, status, plan, p, tickets + p
 #ifdef PSB_SORT_TRACE
         , p == trace_pass ? trace : nullptr
 #endif
         );
   }
-  if (!vals_given && vals_a && !pack_pos_bits) k_sort_identity_payload<<<hb, 256, 0, stream>>>(plan, vals_a, n, gate);
+  if (!vals_given && vals_a && !pack_pos_bits) k_sort_identity_payload<<<hb, 256, 0, stream>>>(plan, vals_a, n);
   cudaMemcpyAsync(where_out, plan + 16, sizeof(u32), cudaMemcpyDeviceToDevice, stream);
   return -(int)cudaGetLastError();
 }
@@ -492,7 +567,8 @@ extern "C" int psb_sort_pairs(const void* in, int in_kind, psb_u64 seed, psb_u64
                          );
 }
 
-// Same, but every kernel of the call returns at once unless the device word *gate is non-zero.
+// Same, but nothing happens unless the device word *gate is non-zero (null: always; see k_sort_gated). Four words
+// behind the gate, zero before the first call, belong to the grid barriers of this call and of psb_localize2_gated.
 extern "C" int psb_sort_pairs_gated(const void* in, int in_kind, psb_u64 seed, psb_u64* keys_a,
                                     uint32_t* vals_a, int vals_given, psb_u64* keys_b, uint32_t* vals_b,
                                     uint32_t n, int begin_bit, int end_bit, void* scratch,

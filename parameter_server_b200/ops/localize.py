@@ -8,7 +8,7 @@ key without a full sort (frequent keys by counting, the rest per key-range
 bucket in shared memory); it assumes keys that are spread evenly over the key
 space (hashed keys) and raises a device flag otherwise. ``sort`` is the radix
 sort + head-flag scan. ``auto`` (the default) enqueues ``bucket`` and, behind
-it, the ``sort`` kernels gated on that flag, so the result is right for any
+it, the ``sort`` path gated on that flag (two launches that return at once), so the result is right for any
 input and nothing waits for the host.
 """
 from __future__ import annotations
@@ -63,7 +63,8 @@ class LocalBatch:
         nb = max(L.psb_sort_scratch_bytes(max_nnz, 0, 64), L.psb_localize_scratch_bytes(max_nnz))
         self.scratch = torch.empty(nb, dtype=torch.uint8, device=dev)
         self.bucket_scratch = torch.empty(L.psb_bucket_localize_scratch_bytes(max_nnz), dtype=torch.uint8, device=dev)
-        self.gate = torch.zeros(1, dtype=i32, device=dev)    # 1 = the bucket path gave up on this minibatch
+        # 1 = the bucket path gave up on this minibatch; behind it the barrier words of the gated launches
+        self.gate = torch.zeros(8, dtype=i32, device=dev)[:1]
         self.status = torch.zeros(1, dtype=i32, device=dev)
         self.ukeys = torch.empty(max_nnz, dtype=i64, device=dev)
         self.seg_off = torch.empty(max_nnz + 1, dtype=i32, device=dev)
@@ -167,7 +168,7 @@ class LocalBatch:
                                         ptr(self.csc_row_buf), ptr(self.csc_val), ptr(self.flagbits),
                                         ptr(self.wordbase), ptr(self.n_unique), ptr(self.own_off),
                                         ptr(self.bucket_scratch), ptr(self.status), ptr(self.gate), sp),
-                  "bucket localize", kernels=10)
+                  "bucket localize", kernels=9)
             if method == "bucket":
                 return self
             gate = ptr(self.gate)
@@ -175,13 +176,13 @@ class LocalBatch:
         check(L.psb_sort_pairs_gated(ptr(ids), in_kind, seed, ptr(self.keys_a), 0 if pack else ptr(self.pos_a), 0,
                                      ptr(self.keys_b), 0 if pack else ptr(self.pos_b), n, lo_bit, hi_bit,
                                      ptr(self.scratch), ptr(self.status), ptr(self.where), pack, gate, sp), "sort",
-              kernels=3 + (hi_bit - lo_bit + 7) // 8)
+              kernels=1 if gate else 3 + (hi_bit - lo_bit + 7) // 8)
         check(L.psb_localize2_gated(ptr(self.keys_a), ptr(self.keys_b), ptr(self.pos_a), ptr(self.pos_b),
                                     ptr(self.where), ptr(self.csc_row_buf), n, ptr(row_ptr), self.n_rows,
                                     self.fixed_z, ptr(vals), ptr(bounds), self.S, ptr(self.ukeys), ptr(self.seg_off),
                                     ptr(self.csr_col), ptr(self.csc_val), ptr(self.flagbits), ptr(self.wordbase),
-                                    ptr(self.n_unique), ptr(self.own_off), ptr(self.scratch), pack, gate, sp),
-              "localize", kernels=4)
+                                    ptr(self.n_unique), ptr(self.own_off), ptr(self.scratch), pack, gate, ptr(self.status), sp),
+              "localize", kernels=1 if gate else 4)
         return self
 
     MAX_GRAPHS = 16

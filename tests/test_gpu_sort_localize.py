@@ -289,3 +289,39 @@ def test_bucket_localize_rows_of_all_lengths(cuda_lib, lens):
     torch.cuda.synchronize()
     assert nnz >= b.BUCKET_MIN_NNZ and int(b.gate.item()) == 0 and int(b.status.item()) == 0
     _check_grouped(b, keys, row_ptr, None, bounds_h, rows)
+
+
+@pytest.mark.parametrize("n", [4096, 4097, 16385, 65537, 131071, 262144, 262145, 900001])
+@pytest.mark.parametrize("hash_bits", [40, 0])
+def test_bucket_localize_sizes(cuda_lib, n, hash_bits):
+    """Around the sizes at which the number of buckets, the sample and the walk grid change."""
+    from parameter_server_b200.ops.localize import LocalBatch
+    from parameter_server_b200.utils.oracle import hash_id_to_key
+    rng = np.random.default_rng(n)
+    ids = (rng.zipf(1.3, n) % (1 << 22)).astype(np.int32)
+    keys = hash_id_to_key(ids, 3, hash_bits or 64)
+    bounds_h, bounds = _bounds(3)
+    b = LocalBatch(n, n, 3, "cuda")
+    for _ in range(2):
+        b.localize(torch.from_numpy(ids).cuda(), None, bounds, fixed_z=1, hash_seed=3, hash_bits=hash_bits, method="auto")
+        torch.cuda.synchronize()
+        assert int(b.gate.item()) == 0 and int(b.status.item()) == 0
+        _check_grouped(b, keys, np.arange(n + 1), None, bounds_h, n)
+
+
+@pytest.mark.parametrize("n", [4096, 5001, 70000, 1500001])
+def test_gated_sort_path_sizes(cuda_lib, n):
+    """The sort-based path behind the gate, one launch for the sort and one for the rest, from less than a tile
+    to more tiles than CTAs; the barrier words it shares with the next call are left as they were."""
+    from parameter_server_b200.ops.localize import LocalBatch
+    rng = np.random.default_rng(n)
+    bounds_h, bounds = _bounds(2)
+    b = LocalBatch(n, n, 2, "cuda", real_values=True)
+    for _ in range(3):
+        keys = rng.integers(1, 1 + n // 3, n, dtype=np.int64).astype(np.uint64)
+        vals = rng.random(n, dtype=np.float32)
+        b.localize(torch.from_numpy(keys.view(np.int64)).cuda(), None, bounds, fixed_z=1, hash_seed=None,
+                   vals=torch.from_numpy(vals).cuda(), method="auto")
+        torch.cuda.synchronize()
+        assert int(b.gate.item()) == 1 and int(b.status.item()) == 0
+        _check_grouped(b, keys, np.arange(n + 1), vals, bounds_h, n)
