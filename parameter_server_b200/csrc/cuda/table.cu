@@ -267,6 +267,9 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
   const u32 gsize = gridDim.x * blockDim.x;
   const u32 gtid = blockIdx.x * blockDim.x + threadIdx.x;
   PSB_TSTAMP(0);
+  // The only rank is its own owner: it looks its key list up where it is, without a copy in the request buffer
+  // and without the hand-over by flags (2.7 M keys and 13 M nonzeros: 147 -> 127 us; 1000 keys: 18.5 -> 11.8). With the key-caching filter the buffer keeps its part.
+  const bool alone = S == 1 && (p.phases & 3) == 3 && !p.key_cache;
   // ---- (a) my keys to their owners
   if (p.phases & 1) {
   bool key_hit = false;
@@ -297,13 +300,13 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const u32 j = j0 + q * gsize;
-        k[q] = j < cnt ? p.ukeys[b0 + j] : 0;
+        k[q] = j < cnt && !alone ? p.ukeys[b0 + j] : 0;
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const u32 j = j0 + q * gsize;
         if (j >= cnt) break;
-        if (j < p.req_cap && !key_hit) p.req_keys[s][j] = k[q];
+        if (j < p.req_cap && !key_hit && !alone) p.req_keys[s][j] = k[q];
         if (p.grad_zero) p.grad_zero[b0 + j] = 0.f;
       }
     }
@@ -313,8 +316,11 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
   // (fences are cumulative), and that fence precedes the arrival count.
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence_system();
-    s_last = atomicAdd(&p.done[0], 1u) + 1 == gridDim.x;
+    s_last = 0;
+    if (!alone) {
+      __threadfence_system();
+      s_last = atomicAdd(&p.done[0], 1u) + 1 == gridDim.x;
+    }
   }
   __syncthreads();
   if (s_last && threadIdx.x < S) {
@@ -346,7 +352,11 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
     __syncthreads();
     if (threadIdx.x == 0) {
       u32 n = 0, base = 0;
-      if (wait_flag_ge_sys(p.my_req_ready[r], p.ts1, iters)) {
+      if (alone) {
+        n = s_off[1] - s_off[0];
+        base = s_off[0];
+        if (n > p.req_cap) { set_status(p.status, kInboxOverflow); n = p.req_cap; }
+      } else if (wait_flag_ge_sys(p.my_req_ready[r], p.ts1, iters)) {
         n = *((volatile const u32*)&p.my_req_hdr[r][0]);
         base = *((volatile const u32*)&p.my_req_hdr[r][1]);
       } else {
@@ -358,6 +368,7 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
     __syncthreads();
     PSB_TSTAMP(3);
     const u32 n = s_n & 0x7fffffffu, base = s_base;
+    const u64* req = alone ? p.ukeys + base : p.my_req_keys[r];
     const int kw = p.width > 1 ? p.width : 1;
     if (p.tile_off != nullptr && S > 1) {
       // for the merge in k_apply: where each equal part of my key range starts in this source's list
@@ -397,7 +408,7 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
           if (hit) {
             sc = p.slot_cache_prev[r][j] & 0x7fffffffu;
           } else {
-            const long long sl = table_find<true>(tab, sm, p.my_req_keys[r][j], kMaxProbe);
+            const long long sl = table_find<true>(tab, sm, req[j], kMaxProbe);
             if (sl >= 0) sc = (u32)sl;
             else set_status(p.status, kTableFull);
           }
@@ -460,7 +471,7 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const u32 j = j0 + q * gsize;
-        key[q] = j < n ? p.my_req_keys[r][j] : 0;
+        key[q] = j < n ? req[j] : 0;
         want |= j < n ? 1u << q : 0u;
       }
       const u32 found = find_entries<4>(tab, sm, key, want, kMaxProbe, slot, e);
