@@ -231,11 +231,12 @@ class DataPlane:
 
     def pull_exchange(self, b, ts: int, *, need_applied: int = 0, with_margins: bool = True, loss: int = 0,
                       auc_hist: Optional[torch.Tensor] = None, phases: int = 7, wait_iters: int = 0, channel: int = 0,
-                      stream=None):
+                      out: Optional[torch.Tensor] = None, stream=None):
         """Exchange form of F2 for round ``ts``: keys go to the owners in bulk, the
         owners look them up (inserting absent keys), remember the slots for the push
         of the same round and store the weights into this worker's response buffer.
-        After it, ``push(..., send_keys=False)`` + ``apply`` reuse those slots."""
+        After it, ``push(..., send_keys=False)`` + ``apply`` reuse those slots. ``out`` (one rank, no
+        margins): the weights go there instead of the response buffer."""
         from ..ops._lib import PullExchangeParams
         cfg = self.cfg
         assert cfg.pull_cap >= b.max_nnz, "pull_cap must cover the largest minibatch's unique keys"
@@ -277,6 +278,9 @@ class DataPlane:
         p = self._params("pull_exchange", (ts % (2 * cfg.ring) if ts > 0 else -1, channel), build)
         p.ts1, p.need_applied, p.wait_iters, p.phases = ts + 1, need_applied, wait_iters, phases
         assert self.width == 1 or not with_margins, "margins need scalar values"
+        if out is not None:
+            assert self.S == 1 and not with_margins and out.dtype == torch.float32 and out.is_contiguous()
+            p.resp_w[0] = ptr(out)
         p.ukeys, p.n_unique, p.own_off, p.grad_zero = ptr(b.ukeys), ptr(b.n_unique), ptr(b.own_off), ptr(b.grad)
         # with several ranks this GPU also serves the others' requests, whose lengths the host does not know
         p.work = min(b.n_keys_max * self.width, 0xffffffff) if self.S == 1 else 0
@@ -298,9 +302,11 @@ class DataPlane:
         return v if k == 1 else v.view(n, k)
 
     # ---------------------------------------------------------------- worker: push
-    def push(self, b, ts: int, *, with_gradient: bool = True, send_keys: bool = True, stream=None):
+    def push(self, b, ts: int, *, with_gradient: bool = True, send_keys: bool = True,
+             values: Optional[torch.Tensor] = None, stream=None):
         """F1a: push round ``ts`` of batch ``b``. With ``with_gradient`` the values
-        are X^T gcoef computed in the kernel; otherwise ``b.grad`` is sent as is."""
+        are X^T gcoef computed in the kernel; otherwise ``values`` (contiguous float32; default
+        ``b.grad``) is sent as is."""
         cfg = self.cfg
         q = ts % cfg.ring
 
@@ -328,10 +334,10 @@ class DataPlane:
             p.flagbits, p.wordbase, p.gcoef = ptr(b.flagbits), ptr(b.wordbase), ptr(b.gcoef)
         else:
             p.nnz = 0
-        p.grad = ptr(b.grad)
+        p.grad = ptr(b.grad if values is None else values)
         p.work = min(b.n_keys_max * self.width, 0xffffffff)
         self._round_work[q] = (ts, p.work)
-        assert self.width == 1 or not with_gradient
+        assert (self.width == 1 and values is None) or not with_gradient
         check(_lib.lib().psb_push(C.byref(p), stream_ptr(stream)), "push")
 
     # ---------------------------------------------------------------- server: apply

@@ -143,13 +143,14 @@ class DeviceKVMap:
         with torch.cuda.stream(self.stream):
             b = self._buffer(k)
             n = k.numel()
+            v = None
             if n:
                 v = torch.as_tensor(values, dtype=torch.float32).to(self.dev).flatten()
                 assert v.numel() == n * self.k, f"{n} keys of width {self.k} need {n * self.k} values"
-                b.grad[:n * self.k].copy_(v)
+                v.record_stream(self.stream)          # read by the kernel where it is; its memory stays until then
             rnd = self._round
             self._round += 1
-            self.plane.push(b, rnd, with_gradient=False, stream=self.stream)
+            self.plane.push(b, rnd, with_gradient=False, values=v, stream=self.stream)
         return rnd
 
     def apply_round(self, rnd: int, channel: int = 0):
@@ -197,9 +198,12 @@ class DeviceKVMap:
             if self.plane.cfg.pull_cap:
                 rnd = self._pull_round
                 self._pull_round += 1
+                # one rank: the kernel writes the result; several: the owners write into the response buffer
+                n = k.numel()
+                out = torch.empty((n, self.k) if self.k > 1 else n, dtype=torch.float32, device=self.dev) if self.plane.S == 1 and n else None
                 self.plane.pull_exchange(b, rnd, need_applied=self._round, with_margins=False, channel=channel,
-                                         stream=self.stream)
-                self._results[ts] = self.plane.response_weights(rnd, k.numel()).clone()
+                                         out=out, stream=self.stream)
+                self._results[ts] = out if out is not None else self.plane.response_weights(rnd, n).clone()
             else:
                 self.plane.pull_margin(b, need_applied=self._round, with_margins=False, stream=self.stream)
                 self._results[ts] = b.w_local[:k.numel()].clone()
