@@ -401,66 +401,76 @@ __device__ __forceinline__ bool pass_barrier(u32* word, u32 n, u32* status) {
   return s_ok != 0;
 }
 
-// Column pass of a rank that is alone: the owner's update (darlin_update_body), the broadcast of the new
-// weights and the worker's column state (darlin_dual_p2) of one column by one thread. Leaves the weight
-// change, or 0, per column of the block in p.wnew for the margin pass, and the staging area cleared.
+// Newton step of one column of a rank that is alone (darlin_update_body), from its gradient sums and state.
+struct ColumnStep {
+  float w;       // new weight
+  float d;       // the step to it
+  float vio;     // violation of the optimality condition
+  bool off;      // deactivated (or it was)
+};
+__device__ __forceinline__ ColumnStep column_step(const PsbDarlinUpdate& p, float2 gu, float w, float dl, unsigned char owned) {
+  ColumnStep r{w, 0.f, 0.f, !owned};
+  if (!owned) return r;
+  const float G = gu.x, u = gu.y / p.eta + 1e-10f;
+  const float g_pos = G + p.lambda, g_neg = G - p.lambda;
+  float d = -w;
+  if (w == 0.f) {
+    if (g_pos < 0.f) r.vio = -g_pos;
+    else if (g_neg > 0.f) r.vio = g_neg;
+    else if (g_pos > p.kkt_threshold && g_neg < -p.kkt_threshold) { r.off = true; return r; }
+  }
+  if (g_pos <= u * w) d = -g_pos / u;
+  else if (g_neg >= u * w) d = -g_neg / u;
+  r.d = fminf(dl, fmaxf(-dl, d));
+  r.w = w + r.d;
+  return r;
+}
+
+// Columns of a block whose margins are complete: the owner's update (darlin_update_body), the worker's column
+// state (darlin_dual_p2) and a clean staging area. No other phase that runs beside it touches this block.
 __device__ void darlin_columns_alone(const PsbDarlinGrad& g, const PsbDarlinUpdate& p, const PsbDarlinDual& d, float& vio_max) {
   const u32 gsize = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x;
   float2* stage = reinterpret_cast<float2*>(g.stage);
-  float* change = const_cast<float*>(d.wnew);
   for (u32 c = p.c0 + gtid; c < p.c1; c += gsize) {
     const u32 b = c - p.c0;
     const float2 gu = __ldcg(&stage[b]);
-    stage[b] = make_float2(0.f, 0.f);
     const unsigned char owned = p.active[c], used = d.active[c];
-    float w = p.w[c];
-    const float w_cur = d.w_cur[c], dl = p.delta[c];
-    bool off = !owned;
+    const float w = p.w[c], w_cur = d.w_cur[c], dl = p.delta[c];
+    stage[b] = make_float2(0.f, 0.f);
+    const ColumnStep st = column_step(p, gu, w, dl, owned);
     if (owned) {
-      const float G = gu.x, u = gu.y / p.eta + 1e-10f;
-      const float g_pos = G + p.lambda, g_neg = G - p.lambda;
-      float step = -w, vio = 0.f;
-      if (w == 0.f) {
-        if (g_pos < 0.f) vio = -g_pos;
-        else if (g_neg > 0.f) vio = g_neg;
-        else if (g_pos > p.kkt_threshold && g_neg < -p.kkt_threshold) off = true;
-      }
-      if (off) {
+      if (st.off) {
         p.active[c] = 0;
       } else {
-        vio_max = fmaxf(vio_max, vio);
-        if (g_pos <= u * w) step = -g_pos / u;
-        else if (g_neg >= u * w) step = -g_neg / u;
-        step = fminf(dl, fmaxf(-dl, step));
-        p.delta[c] = fminf(p.delta_max, 2.f * fabsf(step) + 0.1f);
-        w += step;
-        p.w[c] = w;
+        vio_max = fmaxf(vio_max, st.vio);
+        p.delta[c] = fminf(p.delta_max, 2.f * fabsf(st.d) + 0.1f);
+        p.w[c] = st.w;
       }
     }
-    float dw = 0.f;
     if (used) {
-      if (off) {
+      if (st.off) {
         d.active[c] = 0;
         d.w_cur[c] = 0.f;
       } else {
-        dw = w - w_cur;
-        d.delta[c] = fminf(d.delta_max, 2.f * fabsf(dw) + 0.1f);
-        d.w_cur[c] = w;
+        d.delta[c] = fminf(d.delta_max, 2.f * fabsf(st.w - w_cur) + 0.1f);
+        d.w_cur[c] = st.w;
       }
     }
-    change[b] = dw;
   }
 }
 
-// Margin pass of a rank that is alone: margin += change[column] * x over the block's nonzeros.
-__device__ void darlin_margins_alone(const PsbDarlinDual& p, float2* row_state) {
-  if (p.u1 <= p.u0) return;
+// Margins of a rank that is alone: margin += weight change * x over the block's nonzeros. Every nonzero works its
+// column's step out for itself (neighbours share columns, so the loads coalesce): the column pass, and the grid
+// barrier it would need in front of this one, are off the path from one block's gradient to the next.
+__device__ void darlin_margins_alone(const PsbDarlinGrad& g, const PsbDarlinUpdate& p, const PsbDarlinDual& d, float2* row_state) {
+  if (d.u1 <= d.u0) return;
   const u32 gsize = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const u32 gwarp = gtid >> 5, nwarps = gsize >> 5;
-  const u32 nz0 = p.nz0, nz1 = p.nz1;
+  const u32 nz0 = d.nz0, nz1 = d.nz1;
   const u32 w0 = nz0 >> 5, w1 = (nz1 + 31) >> 5;
   const u32 le = 0xffffffffu >> (31 - lane);
+  const float2* stage = reinterpret_cast<const float2*>(g.stage);
   constexpr int kGroup = 4;                 // words whose gathers are in flight together
   for (u32 wa = w0 + gwarp; wa < w1; wa += nwarps * kGroup) {
     u32 col[kGroup], row[kGroup];
@@ -471,35 +481,39 @@ __device__ void darlin_margins_alone(const PsbDarlinDual& p, float2* row_state) 
       const u32 wi = wa + k * nwarps;
       const u32 i = wi * 32 + lane;
       in[k] = wi < w1 && i >= nz0 && i < nz1;
-      if (p.csc_col != nullptr) col[k] = in[k] ? p.csc_col[i] : 0u;
-      else col[k] = in[k] ? p.gcol[p.wordbase[wi] + __popc(p.flagbits[wi] & le) - 1] : 0u;
-      row[k] = in[k] ? p.csc_row[i] : 0u;
-      x[k] = (in[k] && p.csc_val) ? p.csc_val[i] : 1.f;
+      if (d.csc_col != nullptr) col[k] = in[k] ? d.csc_col[i] : 0u;
+      else col[k] = in[k] ? d.gcol[d.wordbase[wi] + __popc(d.flagbits[wi] & le) - 1] : 0u;
+      row[k] = in[k] ? d.csc_row[i] : 0u;
+      x[k] = (in[k] && d.csc_val) ? d.csc_val[i] : 1.f;
     }
 #pragma unroll
     for (int k = 0; k < kGroup; ++k) {
-      const float dw = in[k] ? p.wnew[col[k] - p.c0] : 0.f;
+      if (!in[k]) continue;
+      const u32 c = col[k];
+      const float2 gu = __ldcg(&stage[c - p.c0]);
+      const unsigned char owned = p.active[c], used = d.active[c];
+      const float w = p.w[c], w_cur = d.w_cur[c], dl = p.delta[c];
+      if (!used) continue;
+      const ColumnStep st = column_step(p, gu, w, dl, owned);
+      const float dw = st.off ? 0.f : st.w - w_cur;
       if (dw != 0.f && dw == dw) atomicAdd(&row_state[row[k]].y, dw * x[k]);
     }
   }
 }
 
-__device__ __forceinline__ u64 globaltimer_ns() {
-  u64 t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 // A pass of a rank that is alone (S == 1), without delay. Worker and owner are the same GPU: no slices are
-// exchanged and no flags raised, and a block is three phases with a light barrier behind each: gradient sums ->
-// columns (update and column state in one) -> margins. The general path below needs five grid-wide
-// synchronisations per block, two of them through system-scope flags, and gathers label and margin apart.
-// What bounds it is that chain of phases, not memory: 1.25 M rows, 125 M nonzeros, 256 blocks take 4.3 ms (17 us
-// per block) against 8.4 ms (33 us) in the general path.
+// exchanged and no flags raised, and a block is two phases with a light barrier behind each:
+//
+//   gradient sums of block i, and beside them the column state of block i - 1 (other columns, other staging area)
+//   margins of block i, every nonzero with its column's step worked out on the spot
+//
+// The general path below needs five grid-wide synchronisations per block, two of them through system-scope
+// flags, and gathers label and margin apart: 1.25 M rows, 125 M nonzeros, 256 blocks take 8.4 ms there, 4.33 ms
+// with a barrier between every two of gradient, columns and margins, 4.16 ms here.
 __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const PsbDarlinPass q) {
-  __shared__ PsbDarlinGrad s_g;
-  __shared__ PsbDarlinUpdate s_u;
-  __shared__ PsbDarlinDual s_d;
+  __shared__ PsbDarlinGrad s_g[2];                 // by step parity
+  __shared__ PsbDarlinUpdate s_u[2];
+  __shared__ PsbDarlinDual s_d[2];
   const int R = q.ring;
   const u32 n = q.n_steps;
   if (n == 0) return;
@@ -507,7 +521,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const Psb
   static_assert(WG + WU + WD <= kPassThreads, "one word of the three parameter blocks per thread");
   float2* rows = reinterpret_cast<float2*>(q.row_state);
   const u32 gsize = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x, t = threadIdx.x;
-  auto fetch = [&](u32 i) -> u32 {                // this thread's word of step i's three parameter blocks
+  auto fetch = [&](u32 i) -> u32 {                 // this thread's word of step i's three parameter blocks
     if (i >= n) return 0u;
     const size_t at = (size_t)q.order[i] * R + (q.ts_base + i) % R;
     if (t < WG) return reinterpret_cast<const u32*>(&q.grad[at])[t];
@@ -515,36 +529,46 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const Psb
     if (t < WG + WU + WD) return reinterpret_cast<const u32*>(&q.dual[at])[t - WG - WU];
     return 0u;
   };
+  auto keep = [&](u32 i, u32 word) {               // into the blocks of the step's parity
+    const u32 k = i & 1;
+    if (t < WG) reinterpret_cast<u32*>(&s_g[k])[t] = word;
+    else if (t < WG + WU) reinterpret_cast<u32*>(&s_u[k])[t - WG] = word;
+    else if (t < WG + WU + WD) reinterpret_cast<u32*>(&s_d[k])[t - WG - WU] = word;
+    __syncthreads();
+    if (t == 0) s_u[k].kkt_threshold = q.kkt_threshold;    // read behind the next barrier
+  };
   u32 word = fetch(0), bars = 0;
   float vio_max = 0.f;
-  for (u32 i = 0; i <= n; ++i) {
-    __syncthreads();                             // nobody still reads the previous step's blocks
-    if (i < n) {
-      if (t < WG) reinterpret_cast<u32*>(&s_g)[t] = word;
-      else if (t < WG + WU) reinterpret_cast<u32*>(&s_u)[t - WG] = word;
-      else if (t < WG + WU + WD) reinterpret_cast<u32*>(&s_d)[t - WG - WU] = word;
+  keep(0, word);
+  // labels and margins travel as pairs for the length of the pass
+  for (u32 r = gtid; r < q.n_rows; r += gsize) rows[r] = make_float2(s_g[0].y[r], s_g[0].margin[r]);
+  if (!pass_barrier(q.steps, ++bars, q.status)) return;
+  for (u32 i = 0; i < n; ++i) {
+    const u32 k = i & 1;
+    if (i > 0) {
+      keep(i, word);                               // (the blocks of step i - 2: nobody reads them any more)
+      darlin_columns_alone(s_g[k ^ 1], s_u[k ^ 1], s_d[k ^ 1], vio_max);
+      // a block that comes twice in a row, or shares columns with the one before it, needs their new state
+      if (s_g[k].c0 < s_g[k ^ 1].c1 && s_g[k ^ 1].c0 < s_g[k].c1 && !pass_barrier(q.steps, ++bars, q.status)) return;
     }
-    __syncthreads();
-    if (t == 0) s_u.kkt_threshold = q.kkt_threshold;   // read behind the next barrier
-    if (i == 0) {
-      for (u32 r = gtid; r < q.n_rows; r += gsize) rows[r] = make_float2(s_g.y[r], s_g.margin[r]);
-      if (!pass_barrier(q.steps, ++bars, q.status)) return;
-    }
-    if (i == n) {
-      for (u32 r = gtid; r < q.n_rows; r += gsize) s_d.margin[r] = __ldcg(&rows[r]).y;
-      break;
-    }
+    darlin_grad_p1<true>(s_g[k], rows);
+    if (!pass_barrier(q.steps, ++bars, q.status)) return;
     word = fetch(i + 1);
-    darlin_grad_p1<true>(s_g, rows);
-    if (!pass_barrier(q.steps, ++bars, q.status)) return;
-    darlin_columns_alone(s_g, s_u, s_d, vio_max);
-    if (!pass_barrier(q.steps, ++bars, q.status)) return;
-    darlin_margins_alone(s_d, rows);
+    darlin_margins_alone(s_g[k], s_u[k], s_d[k], rows);
     if (!pass_barrier(q.steps, ++bars, q.status)) return;
   }
+  const u32 k = (n - 1) & 1;
+  darlin_columns_alone(s_g[k], s_u[k], s_d[k], vio_max);
+  for (u32 r = gtid; r < q.n_rows; r += gsize) s_d[k].margin[r] = __ldcg(&rows[r]).y;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) vio_max = fmaxf(vio_max, __shfl_xor_sync(0xffffffffu, vio_max, o));
-  if ((t & 31) == 0 && vio_max > 0.f && s_u.violation) atomicMax((int*)s_u.violation, __float_as_int(vio_max));
+  if ((t & 31) == 0 && vio_max > 0.f && s_u[k].violation) atomicMax((int*)s_u[k].violation, __float_as_int(vio_max));
+}
+
+__device__ __forceinline__ u64 globaltimer_ns() {
+  u64 t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
 }
 
 __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass(const PsbDarlinPass q) {
