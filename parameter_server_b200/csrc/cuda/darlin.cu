@@ -106,7 +106,7 @@ __device__ void darlin_grad_p1(const PsbDarlinGrad& p, const float2* row_state =
         const unsigned char act = in[k] ? p.active[col[k]] : (unsigned char)0;
         float2 ymg = make_float2(0.f, 0.f);
         if (in[k]) {
-          if (kAlone) ymg = __ldcg(&row_state[row[k]]);
+          if (kAlone) ymg = row_state[row[k]];
           else ymg = make_float2(p.y[row[k]], __ldcg(&p.margin[row[k]]));
         }
         const float y = ymg.x, mg = ymg.y;
@@ -490,7 +490,7 @@ __device__ void darlin_margins_alone(const PsbDarlinGrad& g, const PsbDarlinUpda
     for (int k = 0; k < kGroup; ++k) {
       if (!in[k]) continue;
       const u32 c = col[k];
-      const float2 gu = __ldcg(&stage[c - p.c0]);
+      const float2 gu = stage[c - p.c0];
       const unsigned char owned = p.active[c], used = d.active[c];
       const float w = p.w[c], w_cur = d.w_cur[c], dl = p.delta[c];
       if (!used) continue;
@@ -509,7 +509,8 @@ __device__ void darlin_margins_alone(const PsbDarlinGrad& g, const PsbDarlinUpda
 //
 // The general path below needs five grid-wide synchronisations per block, two of them through system-scope
 // flags, and gathers label and margin apart: 1.25 M rows, 125 M nonzeros, 256 blocks take 8.4 ms there, 4.33 ms
-// with a barrier between every two of gradient, columns and margins, 4.16 ms here.
+// with a barrier between every two of gradient, columns and margins, 3.90 ms here (4.16 with the row pairs gathered
+// past L1: a frequent column's rows stand close together, and nothing writes them during a gradient phase).
 __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const PsbDarlinPass q) {
   __shared__ PsbDarlinGrad s_g[2];                 // by step parity
   __shared__ PsbDarlinUpdate s_u[2];
