@@ -33,6 +33,7 @@
 // memory and carries no multicast qualifier.
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <type_traits>
 #include "psb_common.cuh"
 #include "psb_cuda.h"
 
@@ -207,7 +208,8 @@ struct WideXArgs {
 struct WideTileCtx {
   unsigned char* sA;
   unsigned char* sB;
-  u64* bar;        // 2 mbarriers: 0 = TMA, 1 = MMA
+  u64* bar;        // the group's MMA mbarrier
+  int group;       // 128 threads on one tile at a time; its named barrier is 1 + group
   u32 tmem_base;
   u32 idesc;
   u32 phase;
@@ -227,28 +229,31 @@ struct WideTileCtx {
   u32 plong_cap;
 };
 
+// Barrier of the 128 threads of a tile group.
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); }
+
 // One [128 x 64] x [64 x N] tile: `row` holds this thread's 128-byte value row (zeros when
 // absent); the product goes to P[u, :].
 __device__ __forceinline__ bool wide_tile_mma_store(WideTileCtx& c, const uint4 (&row)[8], u32 u, u32 U, int N, float* P,
                                                     u32* status) {
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x & (kTileM - 1), warp = tid >> 5;
 #pragma unroll
   for (int q = 0; q < 8; ++q)   // 16-byte chunk q of row r lands at chunk (q ^ (r & 7))
     *reinterpret_cast<uint4*>(c.sA + tid * 128 + ((q ^ (tid & 7)) << 4)) = row[q];
   fence_async_smem();
-  __syncthreads();
+  group_sync(c.group);
   // ---- MMA: one thread issues K = 64 as four K = 16 steps
   if (tid == 0) {
     tc_fence_after();
     const u64 da = make_smem_desc(smem_u32(c.sA)), db = make_smem_desc(smem_u32(c.sB));
 #pragma unroll
     for (int k = 0; k < 4; ++k) umma_bf16(c.tmem_base, da + (u64)(2 * k), db + (u64)(2 * k), c.idesc, k > 0 ? 1u : 0u);
-    umma_commit(&c.bar[1]);
+    umma_commit(c.bar);
   }
-  if (!mbar_wait(&c.bar[1], c.phase, 1u << 22)) { if (tid == 0) { *c.s_fail = 1; set_status(status, kWaitTimeout); } }
+  if (!mbar_wait(c.bar, c.phase, 1u << 22)) { if (tid == 0) { *c.s_fail = 1; set_status(status, kWaitTimeout); } }
   c.phase ^= 1;
   tc_fence_after();
-  __syncthreads();
+  group_sync(c.group);
   if (*c.s_fail) return false;
   // ---- epilogue: warp w owns TMEM lanes [32w, 32w+32) = rows of the tile
   const int ldp = N + 1;                          // padded: thread = row, so a column is a bank stride apart
@@ -277,7 +282,7 @@ __device__ __forceinline__ bool wide_tile_mma_store(WideTileCtx& c, const uint4 
     const u32 u0 = u - (u32)tid;
     c.s_seg[tid] = c.seg_off[min(u0 + (u32)tid, U)];
     if (tid == 0) c.s_seg[kTileM] = c.seg_off[min(u0 + (u32)kTileM, U)];
-    __syncthreads();
+    group_sync(c.group);
     const u32 i0 = c.s_seg[tid], len = c.s_seg[tid + 1] - i0;
     bool is_long = false;
     if (len > kPullLongSeg && c.plong_cap) {
@@ -299,12 +304,12 @@ __device__ __forceinline__ bool wide_tile_mma_store(WideTileCtx& c, const uint4 
       if ((tid & 31) >= o) inc += v;
     }
     if ((tid & 31) == 31) c.s_wsum[warp] = inc;
-    __syncthreads();
+    group_sync(c.group);
     u32 base = 0;
     for (int w = 0; w < warp; ++w) base += c.s_wsum[w];
     c.s_pre[tid] = base + inc - mine;
     if (tid == kTileM - 1) c.s_pre[kTileM] = base + inc;
-    __syncthreads();
+    group_sync(c.group);
     const u32 total = c.s_pre[kTileM];
     for (u32 t = tid; t < total; t += kTileM) {
       int lo = 0, hi = kTileM - 1;                 // the last key whose share starts at or before t
@@ -317,33 +322,38 @@ __device__ __forceinline__ bool wide_tile_mma_store(WideTileCtx& c, const uint4 
       atomicAdd(&c.margin[row], c.sP[lo * ldp + (int)cx]);
     }
   }
-  __syncthreads();
+  group_sync(c.group);
   return true;
 }
 
-// Common prologue: mbarriers, TMEM allocation, context matrix by TMA. Returns false on a time-out.
-__device__ __forceinline__ bool wide_tile_setup(WideTileCtx& c, const CUtensorMap* ctx_map, int N, u32* s_tmem, u32* status) {
+// Common prologue of all `groups` tile groups: mbarriers (bars[0]: TMA, bars[1 + group]: MMA), TMEM allocation,
+// context matrix by TMA. A time-out is left in the group's s_fail.
+__device__ __forceinline__ void wide_tile_setup(WideTileCtx& c, const CUtensorMap* ctx_map, int N, int groups, u64* bars,
+                                                u32* s_fail, u32* s_tmem, u32* status) {
   const int tid = threadIdx.x, warp = tid >> 5;
   if (tid == 0) {
-    *c.s_fail = 0;
-    mbar_init(&c.bar[0], 1);
-    mbar_init(&c.bar[1], 1);
+    for (int g = 0; g < groups; ++g) s_fail[g] = 0;
+    for (int g = 0; g <= groups; ++g) mbar_init(&bars[g], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) tmem_alloc(s_tmem, (u32)N);
+  if (warp == 0) tmem_alloc(s_tmem, (u32)(groups * N));
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  c.tmem_base = *s_tmem;
+  c.bar = &bars[1 + c.group];
+  c.s_fail = &s_fail[c.group];
+  c.tmem_base = *s_tmem + (u32)(c.group * N);
   if (tid == 0) {
-    mbar_expect_tx(&c.bar[0], (u32)N * 128u);
-    tma_load_2d(c.sB, ctx_map, 0, 0, &c.bar[0]);
+    mbar_expect_tx(&bars[0], (u32)N * 128u);
+    tma_load_2d(c.sB, ctx_map, 0, 0, &bars[0]);
   }
-  if (!mbar_wait(&c.bar[0], 0, 1u << 22)) { if (tid == 0) { *c.s_fail = 1; set_status(status, kWaitTimeout); } }
+  if (!mbar_wait(&bars[0], 0, 1u << 22) && c.group < groups && (tid & (kTileM - 1)) == 0) {
+    *c.s_fail = 1;
+    set_status(status, kWaitTimeout);
+  }
   __syncthreads();
   c.idesc = make_idesc(kTileM, N);
   c.phase = 0;
-  return *c.s_fail == 0;
 }
 
 __global__ void __launch_bounds__(128) k_wide_pull_gemm(const __grid_constant__ CUtensorMap ctx_map, const WidePullArgs p) {
@@ -358,10 +368,10 @@ __global__ void __launch_bounds__(128) k_wide_pull_gemm(const __grid_constant__ 
   const u32 U = *p.n_unique;
   if (tid <= p.S) s_off[tid] = p.own_off[tid];
   __shared__ u32 s_seg[kTileM + 1], s_pre[kTileM + 1], s_wsum[4];
-  WideTileCtx c{smem, smem + kTileM * 128, s_bar, 0, 0, 0, &s_fail,
+  WideTileCtx c{smem, smem + kTileM * 128, nullptr, 0, 0, 0, 0, nullptr,
                 reinterpret_cast<float*>(smem + kTileM * 128 + N * 128), s_seg, s_pre, s_wsum,
                 p.seg_off, p.csc_row, p.row_ctx, p.margin, p.plong_n, p.plong_list, p.plong_rows, p.plong_cap};
-  wide_tile_setup(c, &ctx_map, N, &s_tmem, p.status);
+  wide_tile_setup(c, &ctx_map, N, 1, s_bar, &s_fail, &s_tmem, p.status);
   const u32 ntiles = (U + kTileM - 1) / kTileM;
   for (u32 t = blockIdx.x; t < ntiles && !s_fail; t += gridDim.x) {
     // ---- gather: thread = one key = one 128-byte row
@@ -400,12 +410,18 @@ __global__ void __launch_bounds__(128) k_wide_pull_gemm(const __grid_constant__ 
 // Only bulk stores cross NVLink (keys out, rows back); tiles of an owner that has
 // answered are multiplied while other owners are still sending. `phases` (bit 0: a,
 // bit 1: b, bit 2: c) lets ranks emulated on one GPU run the roles as separate launches.
-__global__ void __launch_bounds__(128) k_wide_pull_xgemm(const __grid_constant__ CUtensorMap ctx_map, const WideXArgs p) {
+//
+// A kernel that allocates TMEM gets one co-resident CTA per SM from a cooperative launch, so the CTA is four groups
+// of 128 threads: the look-up and the rows have sixteen warps of loads in flight, and four tiles (two at N = 128:
+// 256 TMEM columns either way) are multiplied side by side. 140,000 keys, N = 64: 81 us with one group, 53 us.
+static constexpr int kXThreads = 512;
+static constexpr int kXGroups = kXThreads / kTileM;
+__global__ void __launch_bounds__(kXThreads, 1) k_wide_pull_xgemm(const __grid_constant__ CUtensorMap ctx_map, const WideXArgs p) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ u64 s_bar[2];
+  __shared__ u64 s_bar[1 + kXGroups];
   __shared__ u32 s_tmem;
   __shared__ u32 s_off[PSB_MAX_SHARDS + 1];
-  __shared__ u32 s_fail, s_last, s_n, s_base;
+  __shared__ u32 s_fail[kXGroups], s_last, s_n, s_base;
   const int tid = threadIdx.x, warp = tid >> 5;
   const int S = p.S, N = p.N;
   const u32 U = *p.n_unique;
@@ -512,33 +528,37 @@ __global__ void __launch_bounds__(128) k_wide_pull_xgemm(const __grid_constant__
   }
   if (!(p.phases & 4)) return;
   // ---- (c)
-  __shared__ u32 s_seg[kTileM + 1], s_pre[kTileM + 1], s_wsum[4];
-  WideTileCtx c{smem, smem + kTileM * 128, s_bar, 0, 0, 0, &s_fail,
-                reinterpret_cast<float*>(smem + kTileM * 128 + N * 128), s_seg, s_pre, s_wsum,
+  __shared__ u32 s_seg[kXGroups][kTileM + 1], s_pre[kXGroups][kTileM + 1], s_wsum[kXGroups][4];
+  const int groups = 256 / N, group = tid / kTileM, gt = tid % kTileM;
+  unsigned char* sB = smem + groups * kTileM * 128;
+  float* sP = reinterpret_cast<float*>(sB + N * 128) + (size_t)group * kTileM * (N + 1);
+  WideTileCtx c{smem + group * kTileM * 128, sB, nullptr, group, 0, 0, 0, nullptr, sP, s_seg[group], s_pre[group], s_wsum[group],
                 p.seg_off, p.csc_row, p.row_ctx, p.margin, p.plong_n, p.plong_list, p.plong_rows, p.plong_cap};
-  wide_tile_setup(c, &ctx_map, N, &s_tmem, p.status);
+  wide_tile_setup(c, &ctx_map, N, groups, s_bar, s_fail, &s_tmem, p.status);
   const u32 ntiles = (U + kTileM - 1) / kTileM;
-  for (u32 t = blockIdx.x; t < ntiles && !s_fail; t += gridDim.x) {
-    const u32 u0 = t * kTileM, u = u0 + tid;
-    if (tid == 0) {
-      const int sa = owner_of(s_off, S, u0), sb = owner_of(s_off, S, min(u0 + kTileM - 1, U - 1));
-      for (int s = sa; s <= sb; ++s)
-        if (p.alive[s] && !wait_flag_ge_sys(p.my_resp_ready[s], p.ts1, iters)) { s_fail = 1; set_status(p.status, kWaitTimeout); }
-    }
-    __syncthreads();
-    if (s_fail) break;
-    uint4 row[8];
+  if (group < groups)
+    // only the group's own threads write its s_fail, each write in front of one of its barriers
+    for (u32 t = blockIdx.x * groups + group; t < ntiles && !s_fail[group]; t += gridDim.x * groups) {
+      const u32 u0 = t * kTileM, u = u0 + gt;
+      if (gt == 0) {
+        const int sa = owner_of(s_off, S, u0), sb = owner_of(s_off, S, min(u0 + kTileM - 1, U - 1));
+        for (int s = sa; s <= sb; ++s)
+          if (p.alive[s] && !wait_flag_ge_sys(p.my_resp_ready[s], p.ts1, iters)) { s_fail[group] = 1; set_status(p.status, kWaitTimeout); }
+      }
+      group_sync(group);
+      if (s_fail[group]) break;
+      uint4 row[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) row[q] = make_uint4(0, 0, 0, 0);
-    if (u < U) {
-      const uint4* src = reinterpret_cast<const uint4*>(p.my_resp_rows + (size_t)u * kWide);
+      for (int q = 0; q < 8; ++q) row[q] = make_uint4(0, 0, 0, 0);
+      if (u < U) {
+        const uint4* src = reinterpret_cast<const uint4*>(p.my_resp_rows + (size_t)u * kWide);
 #pragma unroll
-      for (int q = 0; q < 8; ++q) row[q] = src[q];
+        for (int q = 0; q < 8; ++q) row[q] = src[q];
+      }
+      if (!wide_tile_mma_store(c, row, u, U, N, p.P, p.status)) break;
     }
-    if (!wide_tile_mma_store(c, row, u, U, N, p.P, p.status)) break;
-  }
   __syncthreads();
-  if (warp == 0) tmem_dealloc(c.tmem_base, (u32)N);
+  if (warp == 0) tmem_dealloc(c.tmem_base, (u32)(groups * N));
 }
 
 // Block sums of three doubles, one atomic per CTA and value: with one per warp the tens of thousands of atomics
@@ -679,9 +699,37 @@ __device__ __forceinline__ u32 tile_size(u32 n, u32 nwarps, u32 most) {
   return t;
 }
 
+// g += sum over the lanes e of [e0, e1) of gc(e) * C[n(e), 2*lane .. 2*lane+1], in order. Eight (then four, then
+// single) elements' broadcasts and shared-memory loads are issued together: one after another they are a chain
+// of 90 cycles per element, and the longest tile of a warp decides the kernel's time (1.3 M nonzeros of 140,000
+// keys: 122 us one by one with segments of up to 256 in a tile, 82 us like this with segments of up to 128).
+__device__ __forceinline__ void wide_run(const __nv_bfloat162* s_ctx, float gc, u32 n, int e0, int e1, int lane, float& g0,
+                                         float& g1) {
+  auto take = [&](auto count, int e) {
+    constexpr int K = decltype(count)::value;
+    float w[K];
+    __nv_bfloat162 c[K];
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+      w[q] = __shfl_sync(0xffffffffu, gc, e + q);
+      c[q] = s_ctx[__shfl_sync(0xffffffffu, n, e + q) * (kWide / 2) + lane];
+    }
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+      g0 += w[q] * __bfloat162float(c[q].x);
+      g1 += w[q] * __bfloat162float(c[q].y);
+    }
+  };
+  int e = e0;
+  for (; e + 8 <= e1; e += 8) take(std::integral_constant<int, 8>(), e);
+  if (e + 4 <= e1) { take(std::integral_constant<int, 4>(), e); e += 4; }
+  for (; e < e1; ++e) take(std::integral_constant<int, 1>(), e);
+}
+
 // Segments longer than this are reduced by many warps (under a Zipf law one key can
 // own a fifth of all nonzeros; a single warp walking it would take milliseconds).
-static constexpr u32 kWideLongSeg = 256;
+static constexpr u32 kWideLongSeg = 128;           // (the caller's list has a place for every 128 nonzeros)
+static constexpr u32 kWideChunk = 256;             // nonzeros of a long segment per warp and trip
 
 // G += sum over the elements [i0, i1) of gcoef[row] * C[ctx(row), 2*lane .. 2*lane+1]; the row ids,
 // coefficients and context ids of 32 elements are fetched by the lanes in parallel and then
@@ -697,14 +745,7 @@ __device__ __forceinline__ void wide_seg_accumulate(const WidePushArgs& p, const
       gc = __ldg(&p.gcoef[r]);
       n = p.row_ctx ? p.row_ctx[r] : r % (u32)p.N;
     }
-    const int cnt = (int)min(32u, i1 - base);
-    for (int e = 0; e < cnt; ++e) {
-      const float gce = __shfl_sync(0xffffffffu, gc, e);
-      const u32 ne = __shfl_sync(0xffffffffu, n, e);
-      const __nv_bfloat162 c2 = s_ctx[ne * (kWide / 2) + lane];
-      g0 += gce * __bfloat162float(c2.x);
-      g1 += gce * __bfloat162float(c2.y);
-    }
+    wide_run(s_ctx, gc, n, 0, (int)min(32u, i1 - base), lane, g0, g1);
   }
 }
 
@@ -746,7 +787,7 @@ __global__ void __launch_bounds__(256) k_wide_push(const WidePushArgs p) {
       i0 = p.seg_off[u];
       len = p.seg_off[u + 1] - i0;
       if (len > kWideLongSeg && p.long_cap) {
-        const u32 nch = (len + kWideLongSeg - 1) / kWideLongSeg;
+        const u32 nch = (len + kWideChunk - 1) / kWideChunk;
         const unsigned long long old = atomicAdd(p.n_long, 1ull | ((unsigned long long)nch << 32));
         const u32 k = (u32)old;
         if (k < p.long_cap) p.long_list[k] = make_uint4(u, (u32)(old >> 32), i0, i0 + len);
@@ -784,17 +825,16 @@ __global__ void __launch_bounds__(256) k_wide_push(const WidePushArgs p) {
       const u32 before = __shfl_up_sync(0xffffffffu, k, 1);
       const u32 heads = __ballot_sync(0xffffffffu, k != (lane ? before : cur));
       const int cnt = (int)min(32u, total - base);
-      for (int e = 0; e < cnt; ++e) {
+      for (int e = 0; e < cnt;) {
         if ((heads >> e) & 1u) {
           if (cur != 32) emit(t0 + cur, g0, g1);
           cur = __shfl_sync(0xffffffffu, k, e);
           g0 = g1 = 0.f;
         }
-        const float gce = __shfl_sync(0xffffffffu, gc, e);
-        const u32 ne = __shfl_sync(0xffffffffu, n, e);
-        const __nv_bfloat162 c2 = s_ctx[ne * (kWide / 2) + lane];
-        g0 += gce * __bfloat162float(c2.x);
-        g1 += gce * __bfloat162float(c2.y);
+        const u32 later = e < 31 ? heads >> (e + 1) : 0u;
+        const int next = later ? min(cnt, e + __ffs(later)) : cnt;     // the end of the run of one key
+        wide_run(s_ctx, gc, n, e, next, lane, g0, g1);
+        e = next;
       }
     }
     if (cur != 32) emit(t0 + cur, g0, g1);
@@ -814,10 +854,10 @@ __global__ void __launch_bounds__(256) k_wide_push(const WidePushArgs p) {
       }
       const uint4 e = __ldcg(&p.long_list[lo]);
       const u32 cc = c - e.y;
-      const u32 b0 = e.z + cc * kWideLongSeg;
+      const u32 b0 = e.z + cc * kWideChunk;
       if (b0 >= e.w) continue;                       // (only if the list overflowed)
       float g0 = 0.f, g1 = 0.f;
-      wide_seg_accumulate(p, s_ctx, b0, min(e.w, b0 + kWideLongSeg), lane, g0, g1);
+      wide_seg_accumulate(p, s_ctx, b0, min(e.w, b0 + kWideChunk), lane, g0, g1);
       atomicAdd(&p.long_acc[(size_t)lo * kWide + 2 * lane], g0);
       atomicAdd(&p.long_acc[(size_t)lo * kWide + 2 * lane + 1], g1);
     }
@@ -1041,25 +1081,17 @@ extern "C" int psb_wide_pull_xgemm(const void* args, const void* ctx, uint32_t m
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return -(int)cudaErrorInvalidValue;
   if ((a.phases & 4) && a.margin == nullptr && a.P == nullptr) return -(int)cudaErrorInvalidValue;
-  size_t smem = (size_t)kTileM * 128 + (size_t)a.N * 128 + 1024 + (a.margin ? (size_t)kTileM * (a.N + 1) * 4 : 0);
+  const size_t groups = 256 / a.N;
+  size_t smem = groups * kTileM * 128 + (size_t)a.N * 128 + 1024 + (a.margin ? groups * kTileM * (a.N + 1) * 4 : 0);
   static bool attr_set = false;
   if (!attr_set) {
-    cudaFuncSetAttribute((const void*)k_wide_pull_xgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
-    // several CTAs per SM must be resident at once: ask for the large shared-memory carve-out
-    cudaFuncSetAttribute((const void*)k_wide_pull_xgemm, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute((const void*)k_wide_pull_xgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
     attr_set = true;
   }
-  // all CTAs must be co-resident: three per SM (each holds N <= 128 of the SM's 512 TMEM columns)
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   (void)max_unique;
-  int per = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)k_wide_pull_xgemm, 128, smem);
-  per = per < 1 ? 1 : (per > 3 ? 3 : per);
   void* params[] = {&map, &a};
-  return -(int)cudaLaunchCooperativeKernel((const void*)k_wide_pull_xgemm, dim3(sms * per), dim3(128), params, smem, stream);
+  return -(int)cudaLaunchCooperativeKernel((const void*)k_wide_pull_xgemm, dim3(psb_device_sm_count()), dim3(kXThreads), params,
+                                           smem, stream);
 }
 
 extern "C" int psb_wide_rowsum(const float* P, int N, const uint32_t* row_ptr, uint32_t n_rows, uint32_t fixed_z,

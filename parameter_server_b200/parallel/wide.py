@@ -137,7 +137,7 @@ class WidePlane:
             self.slot_mult.append(m if m < (1 << 64) else 0)
         self.sync = torch.zeros(16, dtype=torch.int32, device=dev)
         # scratch of the push for keys with very long segments (zeroed once, left zeroed by the kernel)
-        self.long_cap = max(64, cfg.inbox_cap // 256 + 1)
+        self.long_cap = max(64, cfg.inbox_cap // 128 + 1)
         self.long_list = torch.zeros(self.long_cap * 4, dtype=torch.int32, device=dev)   # {key, first chunk, begin, end}
         self.long_acc = torch.zeros(self.long_cap * WIDTH, dtype=torch.float32, device=dev)
         # the fused pull's list of keys with long segments: {count, chunks}, entries, their rows of products
