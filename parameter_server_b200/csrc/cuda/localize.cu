@@ -218,6 +218,24 @@ __global__ void __launch_bounds__(256) k_owner_offsets(const u64* __restrict__ u
   owner_offsets(ukeys, *n_unique, bounds, S, n, seg_off, own_off);
 }
 
+// A key list handed in by the caller: into the request's own buffer, with its length and owner offsets.
+__global__ void __launch_bounds__(256) k_set_keys(const u64* __restrict__ keys, u32 n, u64* __restrict__ ukeys,
+                                                  u32* __restrict__ n_unique, const u64* __restrict__ bounds, int S,
+                                                  u32* __restrict__ own_off) {
+  const u32 gsize = gridDim.x * blockDim.x;
+  for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * gsize) {
+    u64 k[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) k[q] = i + q * gsize < n ? keys[i + q * gsize] : 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i + q * gsize < n) ukeys[i + q * gsize] = k[q];
+  }
+  if (blockIdx.x != gridDim.x - 1) return;
+  if (threadIdx.x == 0) *n_unique = n;
+  owner_offsets(keys, n, bounds, S, n, nullptr, own_off);
+}
+
 // The four steps behind a device word, in one cooperative launch (see k_sort_gated).
 struct GatedLocalize {
   const u64 *keys_a, *keys_b; const u32 *pos_a, *pos_b; const u32* where; u32* csc_row; u32 n;
@@ -256,6 +274,15 @@ extern "C" int psb_owner_offsets(const psb_u64* ukeys, const uint32_t* n_unique,
                                  uint32_t* own_off, cudaStream_t stream) {
   if (S < 1 || S > 64) return -(int)cudaErrorInvalidValue;
   k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, 0, nullptr, own_off, nullptr, nullptr);
+  return -(int)cudaGetLastError();
+}
+
+extern "C" int psb_set_keys(const psb_u64* keys, uint32_t n, psb_u64* ukeys, uint32_t* n_unique, const psb_u64* bounds,
+                            int S, uint32_t* own_off, cudaStream_t stream) {
+  if (S < 1 || S > 64) return -(int)cudaErrorInvalidValue;
+  const u32 blocks = (n + 1023) / 1024, most = (u32)psb_device_sm_count() * 8;
+  k_set_keys<<<min(most, max(1u, blocks)), 256, 0, stream>>>((const u64*)keys, n, (u64*)ukeys, n_unique, (const u64*)bounds, S,
+                                                             own_off);
   return -(int)cudaGetLastError();
 }
 

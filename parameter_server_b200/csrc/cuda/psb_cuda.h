@@ -41,6 +41,9 @@ int psb_localize2_gated(const psb_u64* keys_a, const psb_u64* keys_b, const uint
                         psb_u64* ukeys, uint32_t* seg_off, uint32_t* csr_col, float* csc_val, uint32_t* flagbits,
                         uint32_t* wordbase, uint32_t* n_unique, uint32_t* own_off, void* scratch,
                         int pack_pos_bits, const uint32_t* gate, uint32_t* status, cudaStream_t stream);
+// Copies a sorted unique key list and sets its length and owner offsets (one launch).
+int psb_set_keys(const psb_u64* keys, uint32_t n, psb_u64* ukeys, uint32_t* n_unique, const psb_u64* bounds, int S,
+                 uint32_t* own_off, cudaStream_t stream);
 int psb_owner_offsets_n(const psb_u64* ukeys, const uint32_t* n_unique, const psb_u64* bounds, int S, uint32_t n,
                         uint32_t* seg_off, uint32_t* own_off, const uint32_t* skip_when_set, uint32_t* gate_out,
                         cudaStream_t stream);

@@ -234,10 +234,9 @@ class LocalBatch:
         the device, so nothing here waits for the host."""
         n = ukeys_sorted.numel()
         assert n <= self.max_nnz
-        self.ukeys[:n].copy_(ukeys_sorted)
-        self.n_unique.fill_(n)
-        check(_lib.lib().psb_owner_offsets(ptr(self.ukeys), ptr(self.n_unique), ptr(bounds), self.S,
-                                           ptr(self.own_off), stream_ptr(stream)), "owner offsets")
+        keys = ukeys_sorted.to(self.ukeys.device, torch.int64).contiguous()
+        check(_lib.lib().psb_set_keys(ptr(keys), n, ptr(self.ukeys), ptr(self.n_unique), ptr(bounds), self.S,
+                                      ptr(self.own_off), stream_ptr(stream)), "set keys")
         self.n_rows = 0
         self.nnz = 0
         self.n_keys_max = n
