@@ -13,6 +13,7 @@ once every shard has applied round ``t - tau - 1`` (bounded delay).
 """
 from __future__ import annotations
 
+import contextlib
 from dataclasses import dataclass
 from typing import List, Optional
 
@@ -147,12 +148,14 @@ class SparseLRWorker:
         # stage 2, prep stream: sort + unique + remap (the buffer is free once its push has read it)
         self.prep_stream.wait_event(self._copy_done[k])
         self.prep_stream.wait_event(self._buf_free[k])
-        loc = b.localize_replayed if self.cfg.graph_localize else b.localize
-        with torch.cuda.stream(self.prep_stream):
+        # (localize_replayed enters the stream itself)
+        loc, on = (b.localize_replayed, contextlib.nullcontext()) if self.cfg.graph_localize else \
+            (b.localize, torch.cuda.stream(self.prep_stream))
+        with on:
             loc(ids_d, y_d, self.plane.bounds, fixed_z=fixed_z, row_ptr=rp_d, vals=vals_d,
                 hash_seed=self.cfg.hash_seed, key_bits=self.cfg.key_bits, hash_bits=self.cfg.hash_bits,
                 stream=self.prep_stream)
-            self._prep_done[k].record(self.prep_stream)
+        self._prep_done[k].record(self.prep_stream)
         self.main_stream.wait_event(self._prep_done[k])
         done()
         mark("pull+push+apply")

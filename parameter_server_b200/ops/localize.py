@@ -200,7 +200,7 @@ class LocalBatch:
                 return (t.words.data_ptr(), t.n, t.bits)
             return (0, 0) if t is None else (t.data_ptr(), t.numel())
         key = (addr(ids), None if isinstance(ids, PackedIds) else ids.dtype, addr(y), addr(bounds), addr(row_ptr), addr(vals),
-               tuple(sorted((k, v) for k, v in kw.items())))
+               tuple(kw.items()))
         graphs = self.__dict__.setdefault("_graphs", {})
         ent = graphs.get(key)
         if ent is None or ent == "seen" and sum(1 for v in graphs.values() if v != "seen") >= self.MAX_GRAPHS:

@@ -129,9 +129,10 @@ class DeviceKVMap:
         (values into the owners' inboxes) and this rank's owner half (merge of the round)."""
         ts = self._stamp(ts)
         self._begin(wait)
-        rnd = self.push_only(keys, values)
-        self._push_round_of[ts] = rnd
-        self.apply_round(rnd, channel=channel)
+        k = self._as_keys(keys, self.dev)
+        with torch.cuda.stream(self.stream):
+            rnd = self._push_round_of[ts] = self._push_half(k, values)
+            self._apply_half(rnd, channel)
         self._finish(ts, callback)
         return ts
 
@@ -141,24 +142,31 @@ class DeviceKVMap:
         (``parameter/kv_nodes.py``) let the server node decide when the round is merged."""
         k = self._as_keys(keys, self.dev)
         with torch.cuda.stream(self.stream):
-            b = self._buffer(k)
-            n = k.numel()
-            v = None
-            if n:
-                v = torch.as_tensor(values, dtype=torch.float32).to(self.dev).flatten()
-                assert v.numel() == n * self.k, f"{n} keys of width {self.k} need {n * self.k} values"
-                v.record_stream(self.stream)          # read by the kernel where it is; its memory stays until then
-            rnd = self._round
-            self._round += 1
-            self.plane.push(b, rnd, with_gradient=False, values=v, stream=self.stream)
+            return self._push_half(k, values)
+
+    def _push_half(self, k: torch.Tensor, values) -> int:
+        """:meth:`push_only` on the current stream, which is this container's."""
+        b = self._buffer(k)
+        n = k.numel()
+        v = None
+        if n:
+            v = torch.as_tensor(values, dtype=torch.float32).to(self.dev).flatten()
+            assert v.numel() == n * self.k, f"{n} keys of width {self.k} need {n * self.k} values"
+            v.record_stream(self.stream)              # read by the kernel where it is; its memory stays until then
+        rnd = self._round
+        self._round += 1
+        self.plane.push(b, rnd, with_gradient=False, values=v, stream=self.stream)
         return rnd
 
     def apply_round(self, rnd: int, channel: int = 0):
         """The owner half of push round ``rnd``: merge what every live worker sent (a buffered container
         only consumes the round: its ring slot becomes reusable later, the values stay unmerged)."""
         with torch.cuda.stream(self.stream):
-            self.plane.apply(rnd, channel=channel, stream=self.stream,
-                             opt=OptimizerConfig(algo="keep") if self.buffer_value else None)
+            self._apply_half(rnd, channel)
+
+    def _apply_half(self, rnd: int, channel: int):
+        self.plane.apply(rnd, channel=channel, stream=self.stream,
+                         opt=OptimizerConfig(algo="keep") if self.buffer_value else None)
 
     def buffer(self, ts: int):
         """What this rank, as an owner, received in the push with timestamp ``ts``: one
