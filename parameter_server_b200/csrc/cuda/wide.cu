@@ -23,8 +23,9 @@
 //                     the fused pull has accumulated.
 //   k_wide_push       worker: gradient of every unique key,
 //                     G[u,:] = sum_{rows containing u} gcoef[row] * C[:, ctx(row)],
-//                     one warp per key over the CSC segment, written as bf16
-//                     records into the owner's inbox by peer stores + release flag.
+//                     a warp per 4 to 16 keys over their CSC segments (many warps
+//                     for a long one), written as bf16 records into the owner's
+//                     inbox by peer stores + release flag.
 //   k_wide_apply      owner: bounded wait per source, then AdaGrad on the fp32
 //                     accumulators and bf16 weights, sources applied in rank order
 //                     (grid barrier between sources).
