@@ -48,6 +48,7 @@
 // work instead. Every spin is bounded and reports through the status word.
 #include "psb_common.cuh"
 #include "psb_cuda.h"
+#include <type_traits>
 
 namespace psb {
 
@@ -97,6 +98,7 @@ struct BLP {
   u32 n;
   int lo;                 // low key bits that are always zero (they carry the position when packed)
   int packed;
+  int with_row;           // CSR rows: positions are stored with their row, as {position, row} pairs
   int nb_bits;            // log2(number of buckets)
   u32 NB, NBINS;          // buckets; NB + kHotMax
   u32 G, chunk;           // walk CTAs and elements per CTA
@@ -206,8 +208,9 @@ __global__ void __launch_bounds__(256) k_bl_hot(const BLP p) {
 
 // ---------------------------------------------------------------- 2./4. the two walks
 // Shared-memory layout of a walk CTA: hot table | hot keys | one word per bin.
+// kRow: CSR rows, positions are stored as {position, row} pairs (fixed-length rows do not pay for them).
 // kScatter = false: count. kScatter = true: the words start as this CTA's output cursors.
-template <bool kScatter>
+template <bool kScatter, bool kRow>
 __global__ void __launch_bounds__(kWalkThreads) k_bl_walk(const BLP p) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint4* s_hot = reinterpret_cast<uint4*>(smem);
@@ -264,17 +267,31 @@ __global__ void __launch_bounds__(kWalkThreads) k_bl_walk(const BLP p) {
 #pragma unroll
     for (int q = 0; q < 4; ++q)
       if ((u32)q < nvalid) dst[q] = atomicAdd(&s_bin[bin[q]], 1u);
-    if (!kScatter) return;
+    if constexpr (kScatter) {
+      // The row of a position is found here, where neighbouring threads look at neighbouring rows, and travels
+      // with it: looked up where the nonzeros arrive in key order, it is three dependent random loads each
+      // (3.9 M nonzeros: bucket and hot emit kernels 130 + 51 us that way, 100 + 32 us so, this walk 49 -> 65).
+      u32 row = kRow ? row_of_pos(p, pos, 0) : 0u;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if ((u32)q >= nvalid) break;
-      if (bin[q] >= p.NB) {
-        p.hot_pos[dst[q]] = pos + q;
-      } else if (p.packed) {
-        p.cold_words[dst[q]] = key[q] | (u64)(pos + q);
-      } else {
-        p.cold_words[dst[q]] = key[q];
-        p.cold_pos[dst[q]] = pos + q;
+      for (int q = 0; q < 4; ++q) {
+        if ((u32)q >= nvalid) break;
+        if (kRow) {
+          while (row + 1 < p.n_rows && p.row_ptr[row + 1] <= pos + q) ++row;
+          const uint2 pr = make_uint2(pos + q, row);
+          if (bin[q] >= p.NB) {
+            reinterpret_cast<uint2*>(p.hot_pos)[dst[q]] = pr;
+          } else {
+            p.cold_words[dst[q]] = key[q];
+            reinterpret_cast<uint2*>(p.cold_pos)[dst[q]] = pr;
+          }
+        } else if (bin[q] >= p.NB) {
+          p.hot_pos[dst[q]] = pos + q;
+        } else if (p.packed) {
+          p.cold_words[dst[q]] = key[q] | (u64)(pos + q);
+        } else {
+          p.cold_words[dst[q]] = key[q];
+          p.cold_pos[dst[q]] = pos + q;
+        }
       }
     }
   };
@@ -532,7 +549,7 @@ __device__ __forceinline__ u32 bucket_block_scan(u32 v, u32* s_warp /* 9 words *
   return pre;
 }
 
-template <typename CK, int kBits>
+template <typename CK, int kBits, bool kRow>
 __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
   typedef BucketShape<kBits> Sh;
   constexpr u32 kHsAll = Sh::kHsAll, kHsWords = Sh::kHsWords, kDistinctMax = Sh::kDistinctMax;
@@ -576,12 +593,16 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
   // The first four nonzeros of every thread stay in registers for both passes over the bucket
   // (a bucket of average size has no more), the rest is read again in pass 2.
   u64 w0[4];
-  u32 p0[4];
+  uint2 p0[4];                                     // position, and with kRow its row
+  auto position = [&](u32 j) -> uint2 {
+    if (kRow) return reinterpret_cast<const uint2*>(p.cold_pos)[cb + j];
+    return make_uint2(p.packed ? 0u : p.cold_pos[cb + j], 0u);
+  };
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const u32 j = t + q * kBucketThreads;
     w0[q] = j < nb ? p.cold_words[cb + j] : 0;
-    p0[q] = (j < nb && !p.packed) ? p.cold_pos[cb + j] : 0;
+    p0[q] = j < nb ? position(j) : make_uint2(0u, 0u);
   }
   // hot keys of this bucket enter the table with their total count
   for (u32 i = h0 + t; i < h1; i += kBucketThreads) {
@@ -754,13 +775,13 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
   const u32 zinv = p.fixed_z ? (u32)(0xffffffffu / p.fixed_z) : 0u;
   for (u32 j0 = t; j0 < nb; j0 += 4 * kBucketThreads) {
     u64 wd[4];
-    u32 ps[4];
+    uint2 ps[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const u32 j = j0 + q * kBucketThreads;
       const bool first = j0 == (u32)t;
       wd[q] = first ? w0[q] : (j < nb ? p.cold_words[cb + j] : 0);
-      ps[q] = first ? p0[q] : ((j < nb && !p.packed) ? p.cold_pos[cb + j] : 0);
+      ps[q] = first ? p0[q] : (j < nb ? position(j) : make_uint2(0u, 0u));
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -769,10 +790,10 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
       const CK ck = (CK)((wd[q] << sh_l) >> sh_r);
       const int slot = bucket_find<CK, kBits>(s_key, ck, rem);
       if (slot < 0) continue;                     // cannot happen: the key was inserted in pass 1
-      const u32 pos = p.packed ? (u32)(wd[q] & posmask) : ps[q];
+      const u32 pos = p.packed && !kRow ? (u32)(wd[q] & posmask) : ps[q].x;
       const u32 P = pb + atomicAdd(&s_cnt[slot], 1u);
       const u32 u = ub + s_rank[slot];
-      p.csc_row[P] = row_of_pos(p, pos, zinv);
+      p.csc_row[P] = kRow ? ps[q].y : row_of_pos(p, pos, zinv);
       p.csr_col[pos] = u;
       if (p.csc_val) p.csc_val[P] = p.vals[pos];
     }
@@ -782,6 +803,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
 }
 
 // ---------------------------------------------------------------- 6. hot keys' position lists
+template <bool kRow>
 __global__ void __launch_bounds__(256) k_bl_hot_emit(const BLP p) {
   __shared__ u32 s_base[kHotMax + 1];
   __shared__ u32 s_u[kHotMax], s_seg[kHotMax];
@@ -811,11 +833,16 @@ __global__ void __launch_bounds__(256) k_bl_hot_emit(const BLP p) {
     h = lo;
   }
   for (u32 j0 = begin + lane; j0 < end + lane; j0 += 128) {
-    u32 pos[4];
+    u32 pos[4], row[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const u32 j = j0 + q * 32;
-      pos[q] = j < end ? __ldcs(&p.hot_pos[j]) : 0u;
+      uint2 pr = make_uint2(0u, 0u);
+      if (j < end) {
+        if (kRow) pr = __ldcs(&reinterpret_cast<const uint2*>(p.hot_pos)[j]);
+        else pr.x = __ldcs(&p.hot_pos[j]);
+      }
+      pos[q] = pr.x; row[q] = pr.y;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -824,7 +851,7 @@ __global__ void __launch_bounds__(256) k_bl_hot_emit(const BLP p) {
       while (h + 1 < nh && s_base[h + 1] <= j) ++h;
       const u32 u = s_u[h];
       const u32 P = s_seg[h] + (j - s_base[h]);
-      p.csc_row[P] = row_of_pos(p, pos[q], zinv);
+      p.csc_row[P] = kRow ? row[q] : row_of_pos(p, pos[q], zinv);
       p.csr_col[pos[q]] = u;
       if (p.csc_val) p.csc_val[P] = p.vals[pos[q]];
       if ((P & 31u) == 0) p.wordbase[P >> 5] = (j == s_base[h]) ? u : u + 1;
@@ -900,7 +927,7 @@ extern "C" size_t psb_bucket_localize_scratch_bytes(uint32_t max_n) {
 // low_zero_bits = number of low key bits that are zero in every key (64 - significant bits of a
 // narrow hashed key); when n - 1 fits in them the position rides in the key word (no cold_pos needed).
 // cold_words (n x 8 bytes), cold_pos (n x 4 bytes, may be null when the positions fit) and hot_pos
-// (n x 4 bytes) are work buffers. Outputs as for psb_localize2. *gate_out (device word) is set to 1
+// (n x 4 bytes) are work buffers; with row_ptr cold_pos is always needed and both are n x 8 bytes. Outputs as for psb_localize2. *gate_out (device word) is set to 1
 // when the caller must run the gated sort-based path instead (its outputs then replace these).
 extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, uint32_t n, int low_zero_bits,
                                    const uint32_t* row_ptr, uint32_t n_rows, uint32_t fixed_z,
@@ -924,7 +951,8 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   p.in = in; p.in_kind = in_kind; p.seed = seed; p.n = n;
   p.lo = low_zero_bits;
   p.packed = (low_zero_bits > 0 && (low_zero_bits >= 32 || ((n - 1) >> low_zero_bits) == 0)) ? 1 : 0;
-  if (!p.packed && cold_pos == nullptr) return -(int)cudaErrorInvalidValue;
+  if ((!p.packed || row_ptr != nullptr) && cold_pos == nullptr) return -(int)cudaErrorInvalidValue;
+  p.with_row = row_ptr != nullptr ? 1 : 0;
   p.NB = bl_num_buckets(n);
   p.nb_bits = 0;
   while ((1u << p.nb_bits) < p.NB) ++p.nb_bits;
@@ -968,27 +996,37 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   if (!attr_set) {
     const size_t walk_max = kHotSlots * 4 + kHotMax * 8 + (size_t)(kMaxBuckets + kHotMax) * 4;
     cudaFuncSetAttribute((const void*)k_bl_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((kMaxBuckets + kMaxBuckets / 32) * 8));
-    cudaFuncSetAttribute((const void*)k_bl_walk<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_max);
-    cudaFuncSetAttribute((const void*)k_bl_walk<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_max);
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u32, 11>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<11>::smem_bytes(4));
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u32, 12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<12>::smem_bytes(4));
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u64, 11>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<11>::smem_bytes(8));
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u64, 12>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<12>::smem_bytes(8));
+    cudaFuncSetAttribute((const void*)k_bl_walk<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_max);
+    cudaFuncSetAttribute((const void*)k_bl_walk<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_max);
+    cudaFuncSetAttribute((const void*)k_bl_walk<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_max);
+    cudaFuncSetAttribute((const void*)k_bl_bucket<u32, 11, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<11>::smem_bytes(4));
+    cudaFuncSetAttribute((const void*)k_bl_bucket<u32, 11, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<11>::smem_bytes(4));
+    cudaFuncSetAttribute((const void*)k_bl_bucket<u32, 12, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<12>::smem_bytes(4));
+    cudaFuncSetAttribute((const void*)k_bl_bucket<u32, 12, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<12>::smem_bytes(4));
+    cudaFuncSetAttribute((const void*)k_bl_bucket<u64, 11, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<11>::smem_bytes(8));
+    cudaFuncSetAttribute((const void*)k_bl_bucket<u64, 11, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<11>::smem_bytes(8));
+    cudaFuncSetAttribute((const void*)k_bl_bucket<u64, 12, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<12>::smem_bytes(8));
+    cudaFuncSetAttribute((const void*)k_bl_bucket<u64, 12, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<12>::smem_bytes(8));
     attr_set = true;
   }
-  k_bl_walk<false><<<p.G, kWalkThreads, walk_smem, stream>>>(p);
+  k_bl_walk<false, false><<<p.G, kWalkThreads, walk_smem, stream>>>(p);
   k_bl_scan<<<(p.NBINS + 255) / 256, 256, 0, stream>>>(p);
   k_bl_plan<<<1, 1024, plan_smem, stream>>>(p);
-  k_bl_walk<true><<<p.G, kWalkThreads, walk_smem, stream>>>(p);
+  if (p.with_row) k_bl_walk<true, true><<<p.G, kWalkThreads, walk_smem, stream>>>(p);
+  else k_bl_walk<true, false><<<p.G, kWalkThreads, walk_smem, stream>>>(p);
   const u32 sms = (u32)bl_walk_ctas(), g11 = min(p.NB, sms * 6), g12 = min(p.NB, sms * 4);
-  if (ck32) {
-    k_bl_bucket<u32, 11><<<g11, kBucketThreads, BucketShape<11>::smem_bytes(4), stream>>>(p);
-    k_bl_bucket<u32, 12><<<g12, kBucketThreads, BucketShape<12>::smem_bytes(4), stream>>>(p);
-  } else {
-    k_bl_bucket<u64, 11><<<g11, kBucketThreads, BucketShape<11>::smem_bytes(8), stream>>>(p);
-    k_bl_bucket<u64, 12><<<g12, kBucketThreads, BucketShape<12>::smem_bytes(8), stream>>>(p);
-  }
-  k_bl_hot_emit<<<min(sms * 8, (n + 1023) / 1024), 256, 0, stream>>>(p);
+  auto buckets = [&](auto row) {
+    constexpr bool kRow = decltype(row)::value;
+    if (ck32) {
+      k_bl_bucket<u32, 11, kRow><<<g11, kBucketThreads, BucketShape<11>::smem_bytes(4), stream>>>(p);
+      k_bl_bucket<u32, 12, kRow><<<g12, kBucketThreads, BucketShape<12>::smem_bytes(4), stream>>>(p);
+    } else {
+      k_bl_bucket<u64, 11, kRow><<<g11, kBucketThreads, BucketShape<11>::smem_bytes(8), stream>>>(p);
+      k_bl_bucket<u64, 12, kRow><<<g12, kBucketThreads, BucketShape<12>::smem_bytes(8), stream>>>(p);
+    }
+    k_bl_hot_emit<kRow><<<min(sms * 8, (n + 1023) / 1024), 256, 0, stream>>>(p);
+  };
+  if (p.with_row) buckets(std::true_type()); else buckets(std::false_type());
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return -(int)e;
   return psb_owner_offsets_n(ukeys, n_unique, bounds, S, n, seg_off, own_off, p.ctl + kCtlFallback, gate_out, stream);

@@ -56,8 +56,8 @@ class LocalBatch:
         L = _lib.lib()
         self.keys_a = torch.empty(max_nnz, dtype=i64, device=dev)
         self.keys_b = torch.empty(max_nnz, dtype=i64, device=dev)
-        self.pos_a = torch.empty(max_nnz, dtype=i32, device=dev)
-        self.pos_b = torch.empty(max_nnz, dtype=i32, device=dev)
+        pos = torch.empty(2 * max_nnz, dtype=i32, device=dev)   # the bucket path uses it as one array of pairs
+        self.pos_a, self.pos_b = pos[:max_nnz], pos[max_nnz:]
         self.csc_row_buf = torch.empty(max_nnz, dtype=i32, device=dev)
         self.where = torch.zeros(1, dtype=i32, device=dev)   # which ping-pong buffer holds the sorted pairs
         nb = max(L.psb_sort_scratch_bytes(max_nnz, 0, 64), L.psb_localize_scratch_bytes(max_nnz))

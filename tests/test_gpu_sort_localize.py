@@ -271,21 +271,29 @@ def test_auto_falls_back_to_sort_on_clustered_keys(cuda_lib):
     _check_grouped(b, keys2, np.arange(rows + 1) * z, None, bounds_h, rows)
 
 
+@pytest.mark.parametrize("hash_bits", [None, 40, 0])
 @pytest.mark.parametrize("lens", ["one_row", "empty_rows", "one_each", "last_rows_empty", "long_then_short"])
-def test_bucket_localize_rows_of_all_lengths(cuda_lib, lens):
-    """The row of a nonzero, found between the hints of its block of 32 positions and of the next one."""
+def test_bucket_localize_rows_of_all_lengths(cuda_lib, lens, hash_bits):
+    """The row of a nonzero, found between the hints of its block of 32 positions and of the next one, and carried
+    with its position: raw keys, hashed ids with room for positions in the keys, and without."""
     from parameter_server_b200.ops.localize import LocalBatch
+    from parameter_server_b200.utils.oracle import hash_id_to_key
     rng = np.random.default_rng(5)
     n = {"one_row": [5003], "empty_rows": (rng.random(40000) < 0.13) * rng.integers(1, 3, 40000), "one_each": np.ones(4097, int),
          "last_rows_empty": np.concatenate([rng.integers(0, 9, 1500), np.zeros(700, int)]),
          "long_then_short": np.concatenate([[6000], rng.integers(0, 4, 900)])}[lens]
     row_ptr = np.concatenate([[0], np.cumsum(n)])
     rows, nnz = len(n), int(row_ptr[-1])
-    keys = _rand_keys(nnz, rng, skew=True)
+    if hash_bits is None:
+        keys = _rand_keys(nnz, rng, skew=True)
+        ids = keys.view(np.int64)
+    else:
+        ids = (rng.zipf(1.3, nnz) % (1 << 22)).astype(np.int32)
+        keys = hash_id_to_key(ids, 3, hash_bits or 64)
     bounds_h, bounds = _bounds(2)
     b = LocalBatch(rows, nnz, 2, "cuda")
-    b.localize(torch.from_numpy(keys.view(np.int64)).cuda(), None, bounds,
-               row_ptr=torch.from_numpy(row_ptr.astype(np.int32)).cuda(), hash_seed=None, method="bucket")
+    b.localize(torch.from_numpy(ids).cuda(), None, bounds, row_ptr=torch.from_numpy(row_ptr.astype(np.int32)).cuda(),
+               hash_seed=None if hash_bits is None else 3, hash_bits=hash_bits or 0, method="bucket")
     torch.cuda.synchronize()
     assert nnz >= b.BUCKET_MIN_NNZ and int(b.gate.item()) == 0 and int(b.status.item()) == 0
     _check_grouped(b, keys, row_ptr, None, bounds_h, rows)
