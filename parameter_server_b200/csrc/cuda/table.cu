@@ -845,8 +845,10 @@ __device__ __forceinline__ float4 inbox_value4(const void* vals, int quant, u32 
 }
 
 // kWide: values of width k > 1. An instantiation of its own, so that neither path pays for the other's registers.
+// Four CTAs per SM for the wide one although it spills a little: 262,145 rows of 64 as int8 62 -> 50 us (1 M rows of 8
+// 67 - 68 either way).
 template <bool kWide>
-__global__ void __launch_bounds__(kThreads, 3) k_apply(const PsbApplyParams p) {
+__global__ void __launch_bounds__(kThreads, kWide ? 4 : 3) k_apply(const PsbApplyParams p) {
   __shared__ u32 s_pre[PSB_MAX_SHARDS + 1];
   __shared__ u32 s_cached[PSB_MAX_SHARDS];
   __shared__ u32 s_last;
