@@ -126,8 +126,9 @@ class DeviceKVMap:
              channel: int = 0) -> int:
         """Push sorted unique uint64 keys with one value (``k`` values: an ``(n, k)`` array) each into
         ``channel``; returns the timestamp. ``values`` on this device is read where it is, on the container's
-        stream: leave it unchanged until the request has finished (:meth:`wait`). Both halves of the round are enqueued here: the worker half
-        (values into the owners' inboxes) and this rank's owner half (merge of the round)."""
+        stream: leave it unchanged until the request has finished (:meth:`wait`). Both halves of the round
+        are enqueued here: the worker half (values into the owners' inboxes) and this rank's owner half
+        (merge of the round)."""
         ts = self._stamp(ts)
         self._begin(wait)
         k = self._as_keys(keys, self.dev)
