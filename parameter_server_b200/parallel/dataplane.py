@@ -309,6 +309,9 @@ class DataPlane:
         ``b.grad``) is sent as is."""
         cfg = self.cfg
         q = ts % cfg.ring
+        if values is not None:
+            assert not with_gradient and values.is_cuda and values.dtype == torch.float32 and values.is_contiguous()
+            assert b.nnz or values.numel() >= b.n_keys_max * self.width, "fewer values than the batch has keys"
 
         def build():
             p = PushParams()
@@ -337,7 +340,7 @@ class DataPlane:
         p.grad = ptr(b.grad if values is None else values)
         p.work = min(b.n_keys_max * self.width, 0xffffffff)
         self._round_work[q] = (ts, p.work)
-        assert (self.width == 1 and values is None) or not with_gradient
+        assert self.width == 1 or not with_gradient
         check(_lib.lib().psb_push(C.byref(p), stream_ptr(stream)), "push")
 
     # ---------------------------------------------------------------- server: apply

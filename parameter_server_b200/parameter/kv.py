@@ -152,7 +152,9 @@ class DeviceKVMap:
         n = k.numel()
         v = None
         if n:
-            v = torch.as_tensor(values, dtype=torch.float32).to(self.dev).flatten()
+            # the kernel reads n * k adjacent floats: a column, a step slice or an expanded tensor (which flatten()
+            # returns as the strided view that it is) is copied first
+            v = torch.as_tensor(values, dtype=torch.float32).to(self.dev).flatten().contiguous().resolve_neg()
             assert v.numel() == n * self.k, f"{n} keys of width {self.k} need {n * self.k} values"
             v.record_stream(self.stream)              # read by the kernel where it is; its memory stays until then
         rnd = self._round

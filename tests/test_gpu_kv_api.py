@@ -190,3 +190,22 @@ def test_request_sizes_widths_and_filters(cuda_lib, n, k, quant):
     step = {"none": 0.0, "int8": 1 / 254, "fp16": 2.0 ** -11}[quant]
     bound = (flat.abs().amax(1, keepdim=True) * 2 * step * 1.001 + flat.abs() * 2.0 ** -22).expand_as(flat).flatten()[:n * k].view(n, k)
     assert ((got - 2 * vals).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("exchange", [True, False])
+def test_pushed_values_of_any_stride(cuda_lib, exchange):
+    """A column, a step slice and an expanded tensor are pushed as the numbers they show."""
+    from parameter_server_b200.parameter.kv import DeviceKVVector
+    n = 700
+    keys = np.arange(1, n + 1, dtype=np.uint64) << np.uint64(40)
+    m = torch.randn(2 * n, 5, device="cuda")
+    for vals in (m[:n, 3], m[:n, 3:4], m[::2, 1], m.flatten()[:2 * n:2], torch.full((1,), 2.5, device="cuda").expand(n)):
+        kv = DeviceKVVector.create(table_capacity=1 << 12, max_keys=n, exchange=exchange)
+        kv.wait(kv.push(keys, vals))
+        got = kv.pull(keys)
+        kv.wait(got)
+        assert torch.equal(kv.result(got), vals.flatten())
+    b = kv._bufs[0]
+    for bad in (m[:n, 3], m[:n].double(), m.flatten()[:n - 1]):
+        with pytest.raises(AssertionError):
+            kv.plane.push(b, 100, with_gradient=False, values=bad)

@@ -1,0 +1,55 @@
+"""The values that a device KV container hands to its push kernel, which reads adjacent floats from one address."""
+import numpy as np
+import pytest
+import torch
+
+
+class _Plane:
+    """Stands in for the data plane: reads the values as the kernel does."""
+
+    def __init__(self):
+        self.read = None
+
+    def push(self, b, rnd, *, with_gradient, values, stream):
+        n = b.n
+        self.values = values
+        self.read = values.detach().as_strided((n,), (1,), values.storage_offset()) if n else None
+
+
+class _Buffer:
+    def __init__(self, n):
+        self.n = n
+
+
+def _container(monkeypatch, n, k):
+    from parameter_server_b200.parameter.kv import DeviceKVVector
+    kv = DeviceKVVector.__new__(DeviceKVVector)
+    kv.dev, kv.k, kv.stream, kv._round, kv.plane = torch.device("cpu"), k, None, 0, _Plane()
+    kv._buffer = lambda keys: _Buffer(n * k)
+    monkeypatch.setattr(torch.Tensor, "record_stream", lambda self, stream: None)
+    return kv
+
+
+def _forms(n, k):
+    m = torch.arange(4.0 * n * k).view(n * k, 4)
+    yield "column", m[:, 1]
+    yield "column as a matrix", m[:, 1:2]
+    yield "every second", torch.arange(2.0 * n * k)[::2]
+    yield "expanded scalar", torch.full((1,), 3.0).expand(n * k)
+    yield "expanded row", torch.arange(float(k)).expand(n, k)
+    yield "transposed", torch.arange(float(n * k)).view(k, n).t()
+    yield "part of wider rows", torch.arange(float(n * (k + 3))).view(n, k + 3)[:, 1:1 + k]
+    yield "behind an offset", torch.arange(n * k + 1.0)[1:]
+    yield "double", torch.arange(n * k, dtype=torch.float64)[:]
+    yield "needs a gradient", torch.arange(float(n * k), requires_grad=True)
+    yield "imaginary parts of a conjugate", torch.complex(torch.zeros(n * k), torch.arange(float(n * k))).conj().imag
+    yield "numpy column", np.arange(2.0 * n * k, dtype=np.float32).reshape(n * k, 2)[:, 1]
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (7, 1), (5, 3), (4, 8)])
+def test_push_hands_adjacent_floats_to_the_kernel(monkeypatch, n, k):
+    for name, values in _forms(n, k):
+        kv = _container(monkeypatch, n, k)
+        kv._push_half(torch.arange(n), values)
+        want = torch.as_tensor(values).detach().to(torch.float32).reshape(-1)
+        assert torch.equal(kv.plane.read, want), name
