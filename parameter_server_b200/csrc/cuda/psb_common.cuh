@@ -162,6 +162,10 @@ __device__ __forceinline__ bool grid_barrier(u32* bar, u32* status) {
     __threadfence();
     u32 arrived = atomicAdd(bar, 1u) + 1;
     if (arrived == gridDim.x * gridDim.y * gridDim.z) {
+      // Acquire side of the arrivals: the atomic is relaxed, and the release below is none. Without this fence
+      // nothing orders the last CTA's later loads, nor through its release those of the CTAs that wait, behind
+      // the stores of the CTAs that arrived before it.
+      __threadfence();
       st_relaxed_gpu(bar, 0u);
       st_release_gpu(bar + 1, sense + 1);          // orders the count's reset before the new sense
     } else {
