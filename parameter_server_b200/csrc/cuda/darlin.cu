@@ -501,7 +501,7 @@ __device__ void darlin_margins_alone(const PsbDarlinGrad& g, const PsbDarlinUpda
   }
 }
 
-// A pass of a rank that is alone (S == 1), without delay. Worker and owner are the same GPU: no slices are
+// A pass of a rank that is alone (S == 1) and owns every column, without delay. Worker and owner are the same GPU: no slices are
 // exchanged and no flags raised, and a block is two phases with a light barrier behind each:
 //
 //   gradient sums of block i, and beside them the column state of block i - 1 (other columns, other staging area)

@@ -397,7 +397,7 @@ typedef struct {
   uint32_t* bar;
   uint32_t* status;
   psb_u64* phase_ns;            // optional: 4 accumulators of CTA 0's time per phase (see k_darlin_pass)
-  // One rank and no delay (non-null chooses k_darlin_pass_alone): n_rows pairs {label, margin} of work space, and
+  // One rank that owns every column, and no delay (non-null chooses k_darlin_pass_alone): n_rows pairs {label, margin} of work space, and
   // one word for the pass's grid barriers (cleared by psb_darlin_pass)
   float* row_state;
   uint32_t n_rows;

@@ -303,7 +303,9 @@ class DarlinRank:
         p.kkt_threshold, p.wait_iters = self.kkt_threshold, wait_iters
         p.bar, p.status = ptr(self._pass_bar), ptr(self.status)
         p.phase_ns = ptr(self.phase_ns) if self.phase_ns is not None else None
-        if self.S == 1 and tau == 0:
+        # a pass kernel of its own for one rank without delay, which takes every column of a block for its own: not
+        # when the key range starts above the data's smallest key (no rank owns the columns below it)
+        if self.S == 1 and tau == 0 and self.shard_col[0] == 0:
             if self._row_state is None:
                 self._row_state = torch.empty(2 * max(1, self.n_rows), dtype=torch.float32, device=self.dev)
             p.row_state, p.n_rows, p.steps = ptr(self._row_state), self.n_rows, self._pass_bar.data_ptr() + 8

@@ -202,3 +202,34 @@ def test_pass_of_a_lone_rank_equals_its_blocks_one_by_one(cuda_lib, rows, z, n_f
         assert np.allclose(e[:4], want, rtol=1e-5, atol=1e-5)
         b.violation.zero_()
         a.kkt_threshold = b.kkt_threshold = e[4] / rows * 10
+
+
+def test_pass_of_a_lone_rank_with_columns_that_nobody_owns(cuda_lib):
+    """A key range that starts in the middle of the second block: the first block has no owner, the second one in
+    part. The pass gives what the single-block kernels give, and the columns without an owner keep their weights."""
+    from parameter_server_b200.models.darlin import DarlinConfig, DarlinRank, darlin_heap_bytes
+    from parameter_server_b200.parallel.fabric import Fabric
+    from parameter_server_b200.utils.range import Range
+    rng = np.random.default_rng(3)
+    rows, z = 500, 8
+    keys, y, vals = _data(rng, rows, z, 200, True)
+    gk = np.unique(keys)
+    first = 45
+    cfg = DarlinConfig(lambda_l1=0.5, eta=0.9, block_cols=30, key_range=Range(int(gk[first]), (1 << 64) - 1))
+    a, b = (DarlinRank(Fabric.single(darlin_heap_bytes(cfg, 1)), cfg, torch.from_numpy(keys.view(np.int64)).cuda(),
+                       torch.from_numpy(y).cuda(), fixed_z=z, vals=torch.from_numpy(vals).cuda()) for _ in range(2))
+    assert a.shard_col[0] == first
+    for r in (a, b):
+        r.fabric.view(r.lay["wnew"], (r.R * cfg.block_cols,), torch.float32).zero_()
+    order = list(range(len(a.blocks)))                     # the unowned columns come while the slices are still zero
+    a.run_pass(order, 0, 0)
+    for i, blk in enumerate(order):
+        b.grad(blk, i)
+        b.update(blk, i)
+        b.dual(blk, i)
+    torch.cuda.synchronize()
+    a.check_status(), b.check_status()
+    for name in ("margin", "w_cur", "w_own", "delta_own"):
+        x, w = getattr(a, name).double(), getattr(b, name).double()
+        assert (x - w).norm() <= 1e-4 * w.norm() + 1e-6, name
+    assert not a.w_own[:first].any() and a.w_own[first:].any() and not a.w_cur[:first].any()
