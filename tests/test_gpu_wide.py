@@ -176,3 +176,26 @@ def test_wide_rows_push_and_apply_sizes(cuda_lib, rows, z, N):
     # the gradient travels as bf16 (2^-9 of |G|, whose step is at most 0.1 |G|) and the weight is stored as bf16
     err = (w.lookup(uk).cuda().double() - want).abs()
     assert (err <= 0.1 * G.abs() * 2.0 ** -8 + want.abs() * 2.0 ** -8 + 1e-5).all()
+
+
+@pytest.mark.parametrize("N", [64, 128])
+def test_wide_exchange_pull_reports_rows_that_never_come(cuda_lib, N):
+    """The worker's role alone, for rounds that no owner has answered: every tile group's wait runs out, the kernel
+    returns with a status, and the plane serves the next round."""
+    from parameter_server_b200.ops._lib import PsbCudaError
+    rows, z = 300, 12
+    planes, b, ctx, *_ = _setup(1, N, rows=rows, z=z, seed=5, pull_cap=rows * z)
+    w = planes[0]
+    P = torch.zeros(rows * z, N, device="cuda")
+    for rnd in range(2):
+        w.pull_xgemm(b, ctx, P, rnd, phases=4, wait_iters=1 << 8)
+        torch.cuda.synchronize()
+        with pytest.raises(PsbCudaError):
+            w.check_status()
+    assert not P.any()
+    w.pull_xgemm(b, ctx, P, 2)
+    torch.cuda.synchronize()
+    w.check_status()
+    U = int(b.n_unique.item())
+    want = w.pulled_rows(2, U).float() @ ctx.float().T
+    assert torch.allclose(P[:U], want, rtol=2e-3, atol=2e-3) and P[:U].any()
