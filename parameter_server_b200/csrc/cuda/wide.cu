@@ -537,11 +537,12 @@ __global__ void __launch_bounds__(kXThreads, 1) k_wide_pull_xgemm(const __grid_c
                 p.seg_off, p.csc_row, p.row_ctx, p.margin, p.plong_n, p.plong_list, p.plong_rows, p.plong_cap};
   wide_tile_setup(c, &ctx_map, N, groups, s_bar, s_fail, &s_tmem, p.status);
   const u32 ntiles = (U + kTileM - 1) / kTileM;
-  // s_fail[group] is tested where all threads of the group have passed one of its barriers since the last write, so
-  // that they agree: here (the set-up ended with a block barrier), behind the flag wait and in wide_tile_mma_store.
-  // In the loop's condition thread 0 could run ahead, give up its wait and set it while a slower warp still had to
-  // look: that warp would leave and the others wait at the group's barrier for good.
-  if (group < groups && !s_fail[group])
+  // s_fail[group] is tested only where a barrier of the group lies between every write and the test, and between the
+  // test and the next write (behind the flag wait, which also catches a set-up that failed, and in
+  // wide_tile_mma_store), so that its threads agree. Tested in front of the flag wait, thread 0 could run ahead, give
+  // up and set it while a slower warp still had to look: that warp would leave and the others wait at the group's
+  // barrier for good.
+  if (group < groups)
     for (u32 t = blockIdx.x * groups + group; t < ntiles; t += gridDim.x * groups) {
       const u32 u0 = t * kTileM, u = u0 + gt;
       if (gt == 0) {
