@@ -733,7 +733,7 @@ __device__ __forceinline__ void wide_run(const __nv_bfloat162* s_ctx, float gc, 
 
 // Segments longer than this are reduced by many warps (under a Zipf law one key can
 // own a fifth of all nonzeros; a single warp walking it would take milliseconds).
-static constexpr u32 kWideLongSeg = 128;           // (the caller's list has a place for every 128 nonzeros)
+static constexpr u32 kWideLongSeg = 128;
 static constexpr u32 kWideChunk = 256;             // nonzeros of a long segment per warp and trip
 
 // G += sum over the elements [i0, i1) of gcoef[row] * C[ctx(row), 2*lane .. 2*lane+1]; the row ids,
@@ -799,9 +799,12 @@ __global__ void __launch_bounds__(256) k_wide_push(const WidePushArgs p) {
         const u32 nch = (len + kWideChunk - 1) / kWideChunk;
         const unsigned long long old = atomicAdd(p.n_long, 1ull | ((unsigned long long)nch << 32));
         const u32 k = (u32)old;
-        if (k < p.long_cap) p.long_list[k] = make_uint4(u, (u32)(old >> 32), i0, i0 + len);
-        else set_status(p.status, kInboxOverflow);
-        len = 0;
+        // (the list is sized by the inbox, that is by keys: with fewer keys than nonzeros / 128 it can be full, and
+        // the segment then stays in the tile)
+        if (k < p.long_cap) {
+          p.long_list[k] = make_uint4(u, (u32)(old >> 32), i0, i0 + len);
+          len = 0;
+        }
       } else if (len == 0) {
         emit_zero(u);
       }

@@ -199,3 +199,38 @@ def test_wide_exchange_pull_reports_rows_that_never_come(cuda_lib, N):
     U = int(b.n_unique.item())
     want = w.pulled_rows(2, U).float() @ ctx.float().T
     assert torch.allclose(P[:U], want, rtol=2e-3, atol=2e-3) and P[:U].any()
+
+
+@pytest.mark.parametrize("keys,each", [(100, 200), (100, 129), (70, 1500)])
+def test_wide_push_with_more_long_segments_than_the_list_holds(cuda_lib, keys, each):
+    """An inbox for the keys of a minibatch that repeats them often: the list of long segments is sized by the inbox
+    and fills up, and the rest are summed where they are. Same weights as with an inbox for every nonzero."""
+    from parameter_server_b200.ops.localize import LocalBatch
+    from parameter_server_b200.parallel.fabric import Fabric
+    from parameter_server_b200.parallel.wide import WideConfig, WidePlane, wide_layout
+    g = torch.Generator().manual_seed(keys + each)
+    ids = torch.arange(keys, dtype=torch.int32).repeat(each, 1).cuda()
+    y = torch.where(torch.rand(each, generator=g) < 0.5, 1.0, -1.0).cuda()
+    ctx = (torch.randn(64, 64, generator=g) * 0.3).to(torch.bfloat16).cuda()
+    rows = torch.randn(keys, 64, generator=g) * 0.5
+    got = []
+    for inbox in (keys, keys * each):
+        cfg = WideConfig(table_capacity=1 << 10, inbox_cap=inbox, ring=2)
+        w = WidePlane(Fabric.single(wide_layout(cfg, 1).total()), cfg)
+        assert (w.long_cap < keys) == (inbox == keys)
+        b = LocalBatch(each, keys * each, 1, "cuda")
+        b.localize(ids.flatten(), y, w.bounds, fixed_z=keys, hash_seed=3)
+        uk = b.ukeys[:keys].cpu().numpy().view(np.uint64)
+        w.load(uk, rows)
+        P = torch.zeros(b.max_nnz, 64, device="cuda")
+        for rnd in range(3):                               # the list and its sums are left clean for the next round
+            w.pull_gemm(b, ctx, P)
+            w.rowsum(b, P, 64)
+            w.push(b, ctx, rnd)
+            w.apply(rnd)
+        torch.cuda.synchronize()
+        w.check_status()
+        got.append(w.lookup(uk).float())
+    # 32-bit sums in another order: now and then a weight is rounded to the next bf16 value, three times at most
+    assert (got[0] - got[1]).abs().le(3 * 2.0 ** -8 * got[1].abs() + 1e-4).all()
+    assert not torch.equal(got[0], rows.to(torch.bfloat16).float())
