@@ -141,10 +141,16 @@ class DeviceKVMap:
     def push_only(self, keys, values) -> int:
         """The worker half of a push round: the values go into the owners' inboxes. Returns the round.
         The owner half is :meth:`apply_round`; :meth:`push` does both, the node-level customers
-        (``parameter/kv_nodes.py``) let the server node decide when the round is merged."""
+        (``parameter/kv_nodes.py``) let the server node decide when the round is merged. There is no
+        request to wait for: ``values`` is read in the order of the caller's current stream, which may
+        write to it again right after the call."""
+        v = torch.as_tensor(values, dtype=torch.float32)
+        if v.device.type == torch.device(self.dev).type:
+            v = v.clone()                             # (from the host the copy to the device is a private one)
         k = self._as_keys(keys, self.dev)
+        self._begin(None)
         with torch.cuda.stream(self.stream):
-            return self._push_half(k, values)
+            return self._push_half(k, v)
 
     def _push_half(self, k: torch.Tensor, values) -> int:
         """:meth:`push_only` on the current stream, which is this container's."""
@@ -152,11 +158,12 @@ class DeviceKVMap:
         n = k.numel()
         v = None
         if n:
+            if isinstance(values, torch.Tensor) and values.is_cuda:
+                values.record_stream(self.stream)     # read on this stream: its memory stays until then
             # the kernel reads n * k adjacent floats: a column, a step slice or an expanded tensor (which flatten()
             # returns as the strided view that it is) is copied first
             v = torch.as_tensor(values, dtype=torch.float32).to(self.dev).flatten().contiguous().resolve_neg()
             assert v.numel() == n * self.k, f"{n} keys of width {self.k} need {n * self.k} values"
-            v.record_stream(self.stream)              # read by the kernel where it is; its memory stays until then
         rnd = self._round
         self._round += 1
         self.plane.push(b, rnd, with_gradient=False, values=v, stream=self.stream)

@@ -136,7 +136,8 @@ class KVWorkerCustomer(core.Customer):
 
     def push(self, keys, values, wait: Sequence[int] = (), callback: Optional[Callable] = None) -> int:
         """Send this worker's values of the round to the owners (device) and the push header to every
-        server (host). Returns the executor's timestamp."""
+        server (host). Returns the executor's timestamp. Device values are read in the order of the calling
+        thread's current stream, which may write to them again right after the call."""
         self.backend.push(keys, values)
         return self._header(b"push", wait, callback)
 

@@ -209,3 +209,25 @@ def test_pushed_values_of_any_stride(cuda_lib, exchange):
     for bad in (m[:n, 3], m[:n].double(), m.flatten()[:n - 1]):
         with pytest.raises(AssertionError):
             kv.plane.push(b, 100, with_gradient=False, values=bad)
+
+
+@pytest.mark.parametrize("k", [1, 8])
+def test_push_only_values_may_be_overwritten_after_the_call(cuda_lib, k):
+    """The worker half of a push records no event: values that the caller's stream writes before and after the call,
+    while the container's stream is still busy with something else, are pushed as they were at the call."""
+    from parameter_server_b200.parameter.kv import DeviceKVVector
+    n = 3000
+    kv = DeviceKVVector.create(table_capacity=1 << 13, max_keys=n, k=k)
+    keys = torch.arange(1, n + 1, device="cuda") << 40
+    vals = torch.zeros(n * k, device="cuda")
+    for rnd in range(3):
+        with torch.cuda.stream(kv.stream):
+            torch.cuda._sleep(20_000_000)                  # about ten milliseconds
+        torch.cuda._sleep(2_000_000)
+        vals.fill_(rnd + 1.0)                              # not there yet when push_only is called
+        r = kv.push_only(keys, vals.view(n, k))
+        vals.fill_(100.0)
+        kv.apply_round(r)
+    got = kv.pull(keys)
+    kv.wait(got)
+    assert (kv.result(got) == 6.0).all()

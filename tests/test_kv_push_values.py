@@ -1,4 +1,6 @@
 """The values that a device KV container hands to its push kernel, which reads adjacent floats from one address."""
+import contextlib
+
 import numpy as np
 import pytest
 import torch
@@ -21,12 +23,11 @@ class _Buffer:
         self.n = n
 
 
-def _container(monkeypatch, n, k):
+def _container(n, k):
     from parameter_server_b200.parameter.kv import DeviceKVVector
     kv = DeviceKVVector.__new__(DeviceKVVector)
     kv.dev, kv.k, kv.stream, kv._round, kv.plane = torch.device("cpu"), k, None, 0, _Plane()
     kv._buffer = lambda keys: _Buffer(n * k)
-    monkeypatch.setattr(torch.Tensor, "record_stream", lambda self, stream: None)
     return kv
 
 
@@ -47,9 +48,29 @@ def _forms(n, k):
 
 
 @pytest.mark.parametrize("n,k", [(1, 1), (7, 1), (5, 3), (4, 8)])
-def test_push_hands_adjacent_floats_to_the_kernel(monkeypatch, n, k):
+def test_push_hands_adjacent_floats_to_the_kernel(n, k):
     for name, values in _forms(n, k):
-        kv = _container(monkeypatch, n, k)
+        kv = _container(n, k)
         kv._push_half(torch.arange(n), values)
         want = torch.as_tensor(values).detach().to(torch.float32).reshape(-1)
         assert torch.equal(kv.plane.read, want), name
+
+
+@pytest.mark.parametrize("n,k", [(7, 1), (5, 3)])
+def test_push_only_leaves_the_caller_its_values(monkeypatch, n, k):
+    """Nothing tells the caller of push_only when its values have been read: the kernel gets a copy of its own, made in
+    the order of the caller's stream, and the container's stream starts behind that stream."""
+    kv = _container(n, k)
+    waited = []
+    kv._begin = waited.append
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    for name, values in _forms(n, k):
+        want = torch.as_tensor(values).detach().to(torch.float32).reshape(-1).clone()
+        kv.push_only(torch.arange(n), values)
+        if not isinstance(values, torch.Tensor):
+            values = torch.from_numpy(values)
+        with torch.no_grad():
+            base = values._base if values._base is not None else values
+            base.fill_(77.0)
+        assert torch.equal(kv.plane.values.detach(), want), name
+        assert waited.pop() is None and not waited
