@@ -144,16 +144,15 @@ class DeviceKVMap:
         (``parameter/kv_nodes.py``) let the server node decide when the round is merged. There is no
         request to wait for: ``values`` is read in the order of the caller's current stream, which may
         write to it again right after the call."""
-        v = torch.as_tensor(values, dtype=torch.float32)
-        if v.device.type == torch.device(self.dev).type:
-            v = v.clone()                             # (from the host the copy to the device is a private one)
+        if isinstance(values, torch.Tensor) and values.device.type == torch.device(self.dev).type:
+            values = values.clone()                   # (from the host the copy to the device is a private one)
         k = self._as_keys(keys, self.dev)
         self._begin(None)
         with torch.cuda.stream(self.stream):
-            return self._push_half(k, v)
+            return self._push_half(k, values)
 
     def _push_half(self, k: torch.Tensor, values) -> int:
-        """:meth:`push_only` on the current stream, which is this container's."""
+        """The worker half of a round on the current stream, which is this container's."""
         b = self._buffer(k)
         n = k.numel()
         v = None

@@ -74,3 +74,6 @@ def test_push_only_leaves_the_caller_its_values(monkeypatch, n, k):
             base.fill_(77.0)
         assert torch.equal(kv.plane.values.detach(), want), name
         assert waited.pop() is None and not waited
+    kv = _container(0, k)
+    kv._begin = waited.append
+    assert kv.push_only(torch.arange(0), None) == 0        # a round without keys needs no values
