@@ -38,7 +38,7 @@ def sort_pairs(keys: torch.Tensor, payload: Optional[torch.Tensor] = None, begin
     where = torch.zeros(1, dtype=torch.int32, device=dev)
     check(L.psb_sort_pairs(ptr(ka), 0, 0, ptr(ka), ptr(va), int(payload is not None), ptr(kb), ptr(vb),
                            n, begin_bit, end_bit, ptr(scratch), ptr(status), ptr(where), 0, stream_ptr(stream)), "sort",
-          kernels=3 + (end_bit - begin_bit + 7) // 8)
+          kernels=2 + (payload is None) + (end_bit - begin_bit + 7) // 8)
     _lib.check_status(status, "radix sort")
     in_b = int(where.item()) == 1
     return (kb, vb) if in_b else (ka, va)
@@ -168,7 +168,7 @@ class LocalBatch:
                                         ptr(self.csc_row_buf), ptr(self.csc_val), ptr(self.flagbits),
                                         ptr(self.wordbase), ptr(self.n_unique), ptr(self.own_off),
                                         ptr(self.bucket_scratch), ptr(self.status), ptr(self.gate), sp),
-                  "bucket localize", kernels=9)
+                  "bucket localize", kernels=11)
             if method == "bucket":
                 return self
             gate = ptr(self.gate)
@@ -176,7 +176,7 @@ class LocalBatch:
         check(L.psb_sort_pairs_gated(ptr(ids), in_kind, seed, ptr(self.keys_a), 0 if pack else ptr(self.pos_a), 0,
                                      ptr(self.keys_b), 0 if pack else ptr(self.pos_b), n, lo_bit, hi_bit,
                                      ptr(self.scratch), ptr(self.status), ptr(self.where), pack, gate, sp), "sort",
-              kernels=1 if gate else 3 + (hi_bit - lo_bit + 7) // 8)
+              kernels=1 if gate else 2 + (not pack) + (hi_bit - lo_bit + 7) // 8)
         check(L.psb_localize2_gated(ptr(self.keys_a), ptr(self.keys_b), ptr(self.pos_a), ptr(self.pos_b),
                                     ptr(self.where), ptr(self.csc_row_buf), n, ptr(row_ptr), self.n_rows,
                                     self.fixed_z, ptr(vals), ptr(bounds), self.S, ptr(self.ukeys), ptr(self.seg_off),
@@ -191,7 +191,7 @@ class LocalBatch:
                           row_ptr: Optional[torch.Tensor] = None, vals: Optional[torch.Tensor] = None, **kw):
         """:meth:`localize` on ``stream``, replayed from a CUDA graph once the same call (the same input
         tensors at the same addresses, the same arguments) comes a second time: a training loop that
-        stages its minibatches in fixed buffers then pays one graph launch instead of some twenty
+        stages its minibatches in fixed buffers then pays one graph launch instead of a dozen
         kernel launches. That matters most while host-to-device copies keep PCIe busy, because the
         launch commands of plain kernels are fetched over the same link and queue behind the copies.
         Calls that never repeat (minibatches of varying size) run as plain launches."""

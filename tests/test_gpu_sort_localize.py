@@ -333,3 +333,27 @@ def test_gated_sort_path_sizes(cuda_lib, n):
         torch.cuda.synchronize()
         assert int(b.gate.item()) == 1 and int(b.status.item()) == 0
         _check_grouped(b, keys, np.arange(n + 1), vals, bounds_h, n)
+
+
+@pytest.mark.parametrize("n,method,hash_bits,ragged", [(5000, "auto", 40, False), (5000, "auto", 0, True), (5000, "bucket", 40, True),
+                                                       (5000, "sort", 40, False), (5000, "sort", 0, False), (100, "auto", 40, False)])
+def test_localize_counts_its_launches(cuda_lib, n, method, hash_bits, ragged):
+    """The launch counter grows by the number of kernels that a captured call consists of."""
+    from parameter_server_b200.ops import _lib
+    from parameter_server_b200.ops.localize import LocalBatch
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    ids = torch.randint(0, 1 << 20, (n,), dtype=torch.int32, device="cuda")
+    rows = {"row_ptr": torch.arange(0, n + 1, 10, dtype=torch.int32, device="cuda")} if ragged else {"fixed_z": 10}
+    _, bounds = _bounds(2)
+    b = LocalBatch(n, n, 2, "cuda")
+    b.localize(ids, None, bounds, hash_seed=3, hash_bits=hash_bits, method=method, **rows)
+    torch.cuda.synchronize()
+    before = _lib.LAUNCHES
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        b.localize(ids, None, bounds, hash_seed=3, hash_bits=hash_bits, method=method, **rows)
+    graph = rt.cudaGraph_t(init_value=g.raw_cuda_graph())
+    _, _, count = rt.cudaGraphGetNodes(graph)
+    _, nodes, _ = rt.cudaGraphGetNodes(graph, count)
+    kernels = sum(rt.cudaGraphNodeGetType(x)[1] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel for x in nodes)
+    assert kernels == _lib.LAUNCHES - before
