@@ -276,7 +276,12 @@ __global__ void __launch_bounds__(kWalkThreads) k_bl_walk(const BLP p) {
       for (int q = 0; q < 4; ++q) {
         if ((u32)q >= nvalid) break;
         if (kRow) {
-          while (row + 1 < p.n_rows && p.row_ptr[row + 1] <= pos + q) ++row;
+          if (row + 1 < p.n_rows && p.row_ptr[row + 1] <= pos + q) {
+            ++row;
+            // behind a run of empty rows: searched, since one thread would walk all of it (20,000 nonzeros with
+            // 100,000 empty rows in their midst: 7.0 ms row by row, 0.09 ms like this, as without them)
+            if (row + 1 < p.n_rows && p.row_ptr[row + 1] <= pos + q) row = row_of_pos(p, pos + q, 0);
+          }
           const uint2 pr = make_uint2(pos + q, row);
           if (bin[q] >= p.NB) {
             reinterpret_cast<uint2*>(p.hot_pos)[dst[q]] = pr;

@@ -357,3 +357,29 @@ def test_localize_counts_its_launches(cuda_lib, n, method, hash_bits, ragged):
     _, nodes, _ = rt.cudaGraphGetNodes(graph, count)
     kernels = sum(rt.cudaGraphNodeGetType(x)[1] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel for x in nodes)
     assert kernels == _lib.LAUNCHES - before
+
+
+@pytest.mark.parametrize("split", [0, 1, 2, 3])
+def test_bucket_localize_long_run_of_empty_rows(cuda_lib, split):
+    """300,000 empty rows between two nonzeros, wherever the gap lies among the four nonzeros of a thread: the rows
+    are right, and no thread walks the gap row by row (70 ns a row: 21 ms; all of it takes 0.1 ms)."""
+    from parameter_server_b200.ops.localize import LocalBatch
+    rng = np.random.default_rng(split)
+    n = np.concatenate([np.full(900, 4), [1 + split], np.zeros(300000, int), np.full(900, 4)])
+    row_ptr = np.concatenate([[0], np.cumsum(n)])
+    rows, nnz = len(n), int(row_ptr[-1])
+    keys = _rand_keys(nnz, rng, skew=True)
+    bounds_h, bounds = _bounds(2)
+    b = LocalBatch(rows, nnz, 2, "cuda")
+    ids, rp = torch.from_numpy(keys.view(np.int64)).cuda(), torch.from_numpy(row_ptr.astype(np.int32)).cuda()
+    ms = []
+    for _ in range(5):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        b.localize(ids, None, bounds, row_ptr=rp, hash_seed=None, method="bucket")
+        e1.record()
+        e1.synchronize()
+        ms.append(e0.elapsed_time(e1))
+    assert int(b.gate.item()) == 0 and int(b.status.item()) == 0
+    _check_grouped(b, keys, row_ptr, None, bounds_h, rows)
+    assert min(ms) < 5.0
