@@ -231,3 +231,25 @@ def test_push_only_values_may_be_overwritten_after_the_call(cuda_lib, k):
     got = kv.pull(keys)
     kv.wait(got)
     assert (kv.result(got) == 6.0).all()
+
+
+def test_memory_of_a_key_list_is_not_reused_before_it_is_read(cuda_lib):
+    """Requests run ahead of the container's stream: the device copy of the first one's keys is let go when the
+    second one comes, and the caller's stream allocates and writes tensors of the same size meanwhile."""
+    from parameter_server_b200.parameter.kv import DeviceKVVector
+    n = 5000
+    kv = DeviceKVVector.create(table_capacity=1 << 15, max_keys=n)
+    lists = [np.arange(1 + i * n, 1 + (i + 1) * n, dtype=np.uint64) << np.uint64(32) for i in range(3)]
+    with torch.cuda.stream(kv.stream):
+        torch.cuda._sleep(40_000_000)                      # about twenty milliseconds
+    junk, ts = [], []
+    for i, keys in enumerate(lists):
+        ts.append(kv.push(keys, np.full(n, i + 1, np.float32)))
+        junk += [torch.full((n,), 7, dtype=torch.int64, device="cuda") for _ in range(4)]
+    torch.cuda.current_stream().synchronize()
+    for t in ts:
+        kv.wait(t)
+    for i, keys in enumerate(lists):
+        got = kv.pull(keys)
+        kv.wait(got)
+        assert (kv.result(got) == i + 1.0).all(), i
