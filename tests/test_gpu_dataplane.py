@@ -265,3 +265,54 @@ def test_checkpoint_resume_equals_uninterrupted_run(cuda_lib, tmp_path):
     k_b, w_b = b.plane.dump_nonzero()
     assert torch.equal(k_ref, k_b)
     assert torch.allclose(w_ref, w_b, rtol=1e-6, atol=1e-7)
+
+
+_ROWS = {"one_row": [5000], "three_rows": [1, 0, 600], "empty_rows": [0] * 37 + [3] * 1500 + [0] * 64,
+         "long_among_short": ([3, 0, 17, 512, 5, 513, 0, 39, 8, 600] + [9, 0, 31, 2] * 20) * 12 + [4000, 1, 513],
+         "long_side_by_side": ([700] * 4 + [1] * 60) * 6 + [513, 514, 515], "all_long": [0, 97, 300, 1200, 31] * 9}
+
+
+@pytest.mark.parametrize("exchange", [False, True])
+@pytest.mark.parametrize("vals", [False, True])
+@pytest.mark.parametrize("rows_of", sorted(_ROWS))
+def test_margins_of_rows_of_all_lengths(cuda_lib, rows_of, vals, exchange):
+    """CSR rows without nonzeros, short ones (eight lanes each), long ones among them (the whole warp) and batches
+    of long rows (a warp each), in both pulls: margins, d loss / d margin and statistics against 64 bits."""
+    from parameter_server_b200.ops._lib import LOSS_LOGIT, LOSS_SQUARE_HINGE
+    from parameter_server_b200.ops.localize import LocalBatch
+    from parameter_server_b200.parallel.dataplane import OptimizerConfig
+    from parameter_server_b200.utils.oracle import hash_id_to_key
+    n = np.array(_ROWS[rows_of])
+    row_ptr = np.concatenate([[0], np.cumsum(n)])
+    rows, nnz = len(n), int(row_ptr[-1])
+    rng = np.random.default_rng(rows)
+    plane = _mk(1, OptimizerConfig(), inbox=nnz, pull_cap=nnz if exchange else 0)[0]
+    weight = (rng.normal(size=3000) * 0.1).astype(np.float32)
+    plane.load_state(hash_id_to_key(np.arange(3000), 1), w=torch.from_numpy(weight))
+    ids = np.minimum((rng.pareto(1.05, nnz) * 2).astype(np.int64), 3099).astype(np.int32)     # the last hundred are not in the model
+    y = np.where(rng.random(rows) < 0.5, 1.0, -1.0).astype(np.float32)
+    x = rng.normal(size=nnz).astype(np.float32) if vals else np.ones(nnz, np.float32)
+    b = LocalBatch(rows, nnz, 1, "cuda", real_values=True)
+    b.localize(torch.from_numpy(ids).cuda(), torch.from_numpy(y).cuda(), plane.bounds, hash_seed=1,
+               row_ptr=torch.from_numpy(row_ptr.astype(np.int32)).cuda(), vals=torch.from_numpy(x).cuda() if vals else None)
+    terms = np.where(ids < 3000, weight[np.minimum(ids, 2999)].astype(np.float64), 0.0) * x
+    total = np.concatenate([[0.0], np.cumsum(terms)]), np.concatenate([[0.0], np.cumsum(np.abs(terms))])
+    want, size = (t[row_ptr[1:]] - t[row_ptr[:-1]] for t in total)
+    bound = (n + 2) * 2.0 ** -24 * size + 1e-9           # of any order of 32-bit sums; the rest is the reference's own
+    for rnd, loss in enumerate((LOSS_LOGIT, LOSS_SQUARE_HINGE)):
+        plane.pull_stats.zero_()
+        plane.pull_exchange(b, rnd, loss=loss) if exchange else plane.pull_margin(b, loss=loss)
+        torch.cuda.synchronize()
+        plane.check_status()
+        margin, gcoef = b.margin[:rows].cpu().numpy(), b.gcoef[:rows].cpu().numpy()
+        assert (np.abs(margin - want) <= bound).all()
+        ym = y * want
+        if loss == LOSS_LOGIT:
+            g, l, slope = -y / (1 + np.exp(ym)), np.logaddexp(0, -ym), 0.25
+        else:
+            h = np.maximum(1 - ym, 0)
+            g, l, slope = -2 * y * h, h * h, 2.0
+        assert (np.abs(gcoef - g) <= slope * bound + 1e-6 * (1 + np.abs(g))).all()
+        got = plane.pull_stats.tolist()
+        assert np.isclose(got[0], l.sum(), rtol=1e-5) and got[2] == rows
+        assert abs(got[1] - (ym > 0).sum()) <= (np.abs(ym) <= bound).sum()
