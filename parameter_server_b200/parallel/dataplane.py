@@ -306,7 +306,10 @@ class DataPlane:
              values: Optional[torch.Tensor] = None, stream=None):
         """F1a: push round ``ts`` of batch ``b``. With ``with_gradient`` the values
         are X^T gcoef computed in the kernel; otherwise ``values`` (contiguous float32; default
-        ``b.grad``) is sent as is."""
+        ``b.grad``) is sent as is. A push that reuses a ring slot polls in the kernel until the owners have
+        applied the round that used it; meanwhile its CTAs hold the registers of the SMs (61,440 of 65,536 for
+        a large batch), so a program with streams of its own enqueues this rank's apply of that round in front
+        of it in stream order, by an event or on the same stream."""
         cfg = self.cfg
         q = ts % cfg.ring
         if values is not None:

@@ -57,7 +57,7 @@ class DeviceKVMap:
         self._results: Dict[int, torch.Tensor] = {}
         self._bufs: List[LocalBatch] = [LocalBatch(1, max_keys, plane.S, self.dev) for _ in range(4)]
         if self.k > 1:
-            for b in self._bufs:                      # k values per key, key-major
+            for b in self._bufs:                      # k values per key, key-major, for programs that fill a buffer themselves
                 b.grad = torch.zeros(max_keys * self.k, dtype=torch.float32, device=self.dev)
         self._next_buf = 0
         self.stream = torch.cuda.Stream(device=self.dev)
