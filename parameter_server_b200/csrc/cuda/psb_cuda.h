@@ -269,6 +269,8 @@ int psb_pull_exchange(const PsbPullExchangeParams* p, cudaStream_t stream);
 int psb_table_init(void* table, psb_u64 capacity, cudaStream_t stream);
 int psb_pull_margin(const PsbPullParams* p, cudaStream_t stream);
 int psb_push(const PsbPushParams* p, cudaStream_t stream);
+// CTAs of a push that sums nnz nonzeros and handles up to `work` values.
+int psb_push_grid(uint32_t nnz, uint32_t work);
 int psb_apply(const PsbApplyParams* p, cudaStream_t stream);
 // Compacts (key, w) of every entry with w != 0 into out_keys/out_w; *out_n gets the count.
 int psb_table_dump(const void* table, psb_u64 capacity, psb_u64* out_keys, float* out_w,

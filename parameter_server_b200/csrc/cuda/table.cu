@@ -619,6 +619,8 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
 //   FP16 : float scale[ceil(cap/32)] followed by half  code[cap]
 __device__ __forceinline__ u32 scale_words(u32 cap) { return (cap + 31) / 32; }
 
+static constexpr u32 kPushChunkWords = 16;         // words of 32 nonzeros that a warp sums at a time, at most
+
 __global__ void __launch_bounds__(kThreads) k_push(const PsbPushParams p) {
   __shared__ u32 s_off[PSB_MAX_SHARDS + 1];
   __shared__ u32 s_last;
@@ -646,8 +648,8 @@ __global__ void __launch_bounds__(kThreads) k_push(const PsbPushParams p) {
     // and added to grad once, so a frequent key (a segment of up to millions of
     // nonzeros) costs one atomic per chunk, not one per word: same-address atomics
     // serialise in L2. Four words are loaded per trip (row ids, then the gathers).
-    // chunk length: up to 16 words, but no longer than what keeps every warp busy (small batches)
-    const u32 kChunkWords = max(1u, min(16u, (nwords + nwarps - 1) / nwarps));
+    // chunk length: up to kPushChunkWords, but no longer than what keeps every warp busy (small batches)
+    const u32 kChunkWords = max(1u, min(kPushChunkWords, (nwords + nwarps - 1) / nwarps));
     const u32 nchunks = (nwords + kChunkWords - 1) / kChunkWords;
     for (u32 c = gwarp; c < nchunks; c += nwarps) {
       const u32 wend = min(nwords, (c + 1) * kChunkWords);
@@ -1216,15 +1218,16 @@ extern "C" int psb_device_sm_count(void) {
 }
 
 extern "C" int psb_coop_grid(int which) {
-  static int g[5] = {0, 0, 0, 0, 0};
-  if (which < 0 || which > 4) return 0;
+  static int g[6] = {0, 0, 0, 0, 0, 0};
+  if (which < 0 || which > 5) return 0;
   if (!g[which]) {
     const void* fn = which == 0 ? (const void*)k_pull_margin
-                   : which == 1 ? (const void*)k_push
+                   : which == 1 || which == 5 ? (const void*)k_push
                    : which == 2 ? (const void*)k_apply<false>
                    : which == 3 ? (const void*)k_pull_exchange : (const void*)k_apply<true>;
-    // the push's segmented sum is a chain of loads per chunk of nonzeros: it takes every warp it can get, the
-    // others gain nothing above four CTAs per SM (13 M nonzeros: 82 -> 75 us with six instead of four)
+    // the push's segmented sum is a chain of loads per chunk of nonzeros: it takes every warp it can get (1; 5 is the
+    // smaller grid, see push_grid_of), the others gain nothing above four CTAs per SM (13 M nonzeros: 82 -> 75 us with
+    // six instead of four)
     g[which] = coop_grid_for(fn, which == 1 ? 6 : 4);
   }
   return g[which];
@@ -1266,13 +1269,15 @@ extern "C" int psb_table_load(void* table, psb_u64 mask, psb_u64 key_begin, psb_
 // how many CTAs take part in the arrival counts, flag polls and grid barriers, which is what a small request
 // costs: push, apply and pull of 1000 keys take 53 us on the device with grids by work and one fence per CTA,
 // 68 us with full grids and a fence per thread.
+static int coop_ctas(int which, psb_u64 threads) {
+  const psb_u64 all = (psb_u64)psb_coop_grid(which), want = (threads + kThreads - 1) / kThreads;
+  return (int)(threads == 0 || want > all ? all : want);
+}
 template <typename P>
 static int launch_coop(const void* fn, int which, const P* p, psb_u64 threads, cudaStream_t stream) {
   P local = *p;
   void* args[] = {&local};
-  const psb_u64 all = (psb_u64)psb_coop_grid(which), want = (threads + kThreads - 1) / kThreads;
-  const int grid = (int)(threads == 0 || want > all ? all : want);
-  cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, 0, stream);
+  cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(coop_ctas(which, threads)), dim3(kThreads), args, 0, stream);
   return -(int)e;
 }
 
@@ -1284,9 +1289,18 @@ extern "C" int psb_pull_exchange(const PsbPullExchangeParams* p, cudaStream_t st
   if (p->S < 1 || p->S > PSB_MAX_SHARDS) return -(int)cudaErrorInvalidValue;
   return launch_coop((const void*)k_pull_exchange, 3, p, p->work ? (psb_u64)p->work + 32ull * p->n_rows : 0, stream);
 }
+// Six CTAs per SM where each of their warps gets a whole chunk of 16 words, that is from 3.6 M nonzeros on (or where
+// there is nothing to sum). Below that more warps mean shorter chunks: a frequent key's sum is added up from more
+// parts, one 32-bit atomic after another (390,000 nonzeros: chunks of two words instead of three, and the gradient
+// 1.5 times as far from 64 bits).
+static int push_grid_of(psb_u64 nnz) {
+  const psb_u64 whole = (psb_u64)psb_coop_grid(1) * (kThreads / 32) * kPushChunkWords * 32;
+  return nnz == 0 || nnz >= whole ? 1 : 5;
+}
+extern "C" int psb_push_grid(uint32_t nnz, uint32_t work) { return coop_ctas(push_grid_of(nnz), work); }
 extern "C" int psb_push(const PsbPushParams* p, cudaStream_t stream) {
   if (p->S < 1 || p->S > PSB_MAX_SHARDS) return -(int)cudaErrorInvalidValue;
-  return launch_coop((const void*)k_push, 1, p, p->work, stream);
+  return launch_coop((const void*)k_push, push_grid_of(p->nnz), p, p->work, stream);
 }
 extern "C" int psb_apply(const PsbApplyParams* p, cudaStream_t stream) {
   if (p->S < 1 || p->S > PSB_MAX_SHARDS) return -(int)cudaErrorInvalidValue;

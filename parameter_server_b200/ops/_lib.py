@@ -193,6 +193,7 @@ def _declare(lib):
     lib.psb_table_load.argtypes = [_vp, _u64, _u64, _u64, _vp, _vp, _vp, _vp, _u64, _vp, _vp]
     lib.psb_table_export.argtypes = [_vp, _u64, _vp, _vp, _vp, _vp, _u64, _vp, _vp]
     lib.psb_coop_grid.argtypes = [_i32]
+    lib.psb_push_grid.argtypes = [_u32, _u32]
     lib.psb_darlin_grad.argtypes = [C.POINTER(DarlinGrad), _vp]
     lib.psb_darlin_update.argtypes = [C.POINTER(DarlinUpdate), _vp]
     lib.psb_darlin_dual.argtypes = [C.POINTER(DarlinDual), _vp]

@@ -316,3 +316,13 @@ def test_margins_of_rows_of_all_lengths(cuda_lib, rows_of, vals, exchange):
         got = plane.pull_stats.tolist()
         assert np.isclose(got[0], l.sum(), rtol=1e-5) and got[2] == rows
         assert abs(got[1] - (ym > 0).sum()) <= (np.abs(ym) <= bound).sum()
+
+
+@pytest.mark.parametrize("nnz", [1, 31, 4097, 151552, 390000, 606208, 1000003, 2424832, 2500000, 3637247, 3637248, 13107200])
+def test_push_sums_a_key_from_no_more_parts_than_four_ctas_per_sm_make(cuda_lib, nnz):
+    """Every part of a frequent key's sum is a 32-bit atomic of its own, so the length of a warp's chunk (16 words of
+    32 nonzeros at most) bounds the error of the sum: a larger grid may not shorten it."""
+    def chunk_words(ctas):
+        words, warps = (nnz + 31) // 32, 8 * ctas
+        return max(1, min(16, (words + warps - 1) // warps))
+    assert chunk_words(cuda_lib.psb_push_grid(nnz, nnz)) >= chunk_words(4 * cuda_lib.psb_device_sm_count())
