@@ -59,9 +59,10 @@ __device__ void darlin_grad_p1(const PsbDarlinGrad& p, const float2* row_state =
   const u32 nz0 = p.nz0, nz1 = p.nz1;
   const u32 w0 = nz0 >> 5, w1 = (nz1 + 31) >> 5;
   const u32 le = 0xffffffffu >> (31 - lane);
-  // chunk length: up to 16 words, and such that every warp gets the same number of chunks (16 words each for a
-  // little more than two rounds of chunks would leave the third round nearly empty)
-  const u32 rounds = (w1 - w0 + 16 * nwarps - 1) / (16 * nwarps);
+  // chunk length: 16 words and a little more, such that every warp gets the same number of chunks (16 words each for
+  // a little more than two rounds of chunks would leave the third round nearly empty). Rounds are rounded down: a
+  // shorter chunk would mean more parts, each a 32-bit atomic, in a frequent column's sums.
+  const u32 rounds = max(1u, (w1 - w0) / (16 * nwarps));
   const u32 kChunkWords = max(1u, (w1 - w0 + rounds * nwarps - 1) / (rounds * nwarps));
   const u32 nchunks = (w1 - w0 + kChunkWords - 1) / kChunkWords;
   auto flush = [&](u32 col, float gg, float hh) {

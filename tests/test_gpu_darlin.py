@@ -233,3 +233,8 @@ def test_pass_of_a_lone_rank_with_columns_that_nobody_owns(cuda_lib):
         x, w = getattr(a, name).double(), getattr(b, name).double()
         assert (x - w).norm() <= 1e-4 * w.norm() + 1e-6, name
     assert not a.w_own[:first].any() and a.w_own[first:].any() and not a.w_cur[:first].any()
+
+
+def test_pass_of_a_lone_rank_on_a_block_of_millions_of_nonzeros(cuda_lib):
+    """5.2 M nonzeros of one block: every warp sums two chunks of more than 16 words."""
+    test_pass_of_a_lone_rank_equals_its_blocks_one_by_one(cuda_lib, 130000, 40, 60, 64, True)
