@@ -580,6 +580,7 @@ __device__ __forceinline__ void block_add3(double a, double b, double c, double*
 
 // ---------------------------------------------------------------- rows: prediction, loss, gcoef
 // Eight lanes per row, four nonzeros of each lane in flight: bound by the two dependent gathers (column, product).
+// Trips and lanes are added in 64 bits: eight lanes sum more terms each, one after another, than the 32 of a warp.
 __global__ void __launch_bounds__(256) k_wide_rowsum(const float* __restrict__ P, int N, const u32* __restrict__ row_ptr,
                                                      u32 n_rows, u32 fixed_z, const u32* __restrict__ csr_col,
                                                      const u32* __restrict__ row_ctx, const float* __restrict__ y,
@@ -598,7 +599,7 @@ __global__ void __launch_bounds__(256) k_wide_rowsum(const float* __restrict__ P
       e = row_ptr ? row_ptr[r + 1] : b + fixed_z;
       ctx = row_ctx ? row_ctx[r] : r % (u32)N;
     }
-    float acc = 0.f;
+    double sum = 0;
     for (u32 j0 = b + sub; j0 < e; j0 += 32) {
       u32 col[4];
       float v[4];
@@ -606,10 +607,11 @@ __global__ void __launch_bounds__(256) k_wide_rowsum(const float* __restrict__ P
       for (int q = 0; q < 4; ++q) col[q] = j0 + 8 * q < e ? csr_col[j0 + 8 * q] : 0xffffffffu;
 #pragma unroll
       for (int q = 0; q < 4; ++q) v[q] = col[q] != 0xffffffffu ? P[(size_t)col[q] * N + ctx] : 0.f;
-      acc += (v[0] + v[1]) + (v[2] + v[3]);
+      sum += (double)((v[0] + v[1]) + (v[2] + v[3]));
     }
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float acc = (float)sum;
     if (have && sub == 0) {
       float yy = y[r], ym = yy * acc;
       float en = expf(-fabsf(ym));

@@ -235,3 +235,23 @@ def test_wide_push_with_more_long_segments_than_the_list_holds(cuda_lib, keys, e
     # rounded to the next bf16 value
     assert (got[0] - got[1]).abs().le(3 * 2.0 ** -8 * (got[1].abs() + 0.1)).all()
     assert not torch.equal(got[0], rows.to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("z", [10, 40, 96])
+def test_wide_row_sums_of_eight_lanes_are_as_close_as_those_of_a_warp(cuda_lib, z):
+    """The error of the margins against 64 bits (root mean square over 4000 rows) is no larger than that of a warp per
+    row in 32 bits (32 lanes in sequence, then a tree; emulated here)."""
+    planes, b, ctx, *_ = _setup(1, 64, rows=4000, z=z, seed=z)
+    rows = 4000
+    P = torch.randn(b.max_nnz, 64, device="cuda")
+    planes[0].rowsum(b, P, 64)
+    torch.cuda.synchronize()
+    terms = P[b.csr_col[:rows * z].long(), (torch.arange(rows, device="cuda") % 64).repeat_interleave(z)].view(rows, z).cpu().numpy()
+    want = terms.astype(np.float64).sum(1)
+    lane = np.zeros((rows, 32), np.float32)
+    for j in range(0, z, 32):
+        lane[:, :min(32, z - j)] += terms[:, j:j + 32]
+    while lane.shape[1] > 1:
+        lane = lane[:, :lane.shape[1] // 2] + lane[:, lane.shape[1] // 2:]
+    rms = lambda e: float(np.sqrt(np.mean(np.square(e))))
+    assert rms(b.margin[:rows].cpu().numpy() - want) <= rms(lane[:, 0] - want)
