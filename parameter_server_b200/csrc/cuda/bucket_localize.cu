@@ -17,13 +17,13 @@
 //   2. count      every CTA walks a contiguous slice of the input and counts, in
 //                 shared memory, its nonzeros per hot key and, for all others
 //                 ("cold"), per bucket (bucket = top bits of the key, so buckets
-//                 are ordered by key).
-//   3. scan/plan  prefix sums give every CTA a private output cursor per bin (no
-//                 look-back chain), every bucket its output range, every hot key
-//                 its place in the hot stream.
-//   4. scatter    the same walk again: a cold nonzero goes to its bucket as one
-//                 64-bit word (key | position), a hot nonzero's position goes to
-//                 its key's list.
+//                 are ordered by key). The bin of every nonzero and its place
+//                 among the slice's nonzeros of that bin are kept in one word, so
+//                 that no later step looks a key up or counts again.
+//   3. scan/plan  prefix sums give every slice a private output place per bin (no
+//                 look-back chain) and every bucket its output range.
+//   4. scatter    a cold nonzero goes to its bucket as one 64-bit word (key | row),
+//                 or as key and row.
 //   5. bucket     one CTA per bucket: a shared-memory table de-duplicates the
 //                 bucket's keys and counts them. The table is order preserving
 //                 (home slot = leading bits of the key, linear probing without
@@ -31,12 +31,15 @@
 //                 sorted up to a permutation inside each run of adjacent slots;
 //                 a key's rank is a prefix count plus a look at its own run, and
 //                 nothing is sorted. Hot keys that fall into the bucket are
-//                 merged in, a chained scan over the buckets (decoupled
-//                 look-back, in ticket order) gives the global index of the
-//                 bucket's first unique key, and every nonzero is written to its
-//                 final CSC position.
-//   6. hot emit   the hot keys' position lists are written to the CSC ranges
-//                 that step 5 reserved for them.
+//                 merged in, and every cold nonzero's row goes to its final CSC
+//                 place. What depends on the buckets in front (a key's index in
+//                 the list) stays relative to the bucket: its unique keys are
+//                 left, in order, where its words were, and every cold nonzero
+//                 gets its key's rank. So no bucket waits for another.
+//   6. finish     every CTA adds up the buckets' numbers of keys for itself. The
+//                 key lists close up, and the nonzeros are walked in input order
+//                 once more: a cold one's column is its bucket's first index plus
+//                 its rank, a hot one goes to its CSC place.
 //
 // Inside a key's CSC segment the nonzeros are in no particular order (the sort
 // based path lists them by position).
@@ -67,8 +70,13 @@ static constexpr int kWalkThreads = 1024;         // count / scatter CTAs
 static constexpr int kBucketThreads = 256;
 static constexpr u32 kRunMax = 64;                // longest probe sequence / run of adjacent occupied slots
 static constexpr u32 kMaxBuckets = 8192;
+// The word that the count leaves per nonzero: its bin above its place among its slice's nonzeros of that bin.
+static constexpr int kPlaceBits = 18;
+static constexpr u32 kPlaceMask = (1u << kPlaceBits) - 1;
+static_assert(kMaxBuckets + kHotMax <= 1u << (32 - kPlaceBits), "a bin fits above the place");
+static constexpr u32 kWalkSplit = 2;              // scatter and finish: CTAs that share a slice
 static constexpr int kHintShift = 5;              // one row hint per 32 positions
-// A bucket's table comes in two sizes. 2^11 home slots (35 KB of shared memory, six CTAs per SM) serve
+// A bucket's table comes in two sizes. 2^11 home slots (35 KB of shared memory, five CTAs per SM) serve
 // minibatches in which keys repeat, the usual case; 2^12 (55 KB, four per SM) those in which nearly
 // every nonzero has its own key. The sample decides (k_bl_plan), both kernels are launched and the
 // one that was not chosen returns at once.
@@ -82,13 +90,10 @@ template <int kBits> struct BucketShape {
     return kHsAll * (key_bytes + 4 + 2) + kDistinctMax * (4 + 2) + 2 * kHsWords * 4;
   }
 };
-static constexpr u32 kFlagAgg = 1u << 30;
-static constexpr u32 kFlagIncl = 2u << 30;
-static constexpr u32 kValMask = (1u << 30) - 1;
+static constexpr u32 kHotFlag = 1u << 31;         // segment starts on their way to the finish: a hot key's
 
 // control words
-enum { kCtlNumHot = 0, kCtlTicket = 1, kCtlFallback = 2, kCtlHotElems = 3, kCtlSampleDistinct = 4, kCtlBigTables = 5,
-       kCtlWords = 16 };
+enum { kCtlNumHot = 0, kCtlFallback = 1, kCtlSampleDistinct = 2, kCtlBigTables = 3, kCtlWords = 16 };
 
 struct BLP {
   // input
@@ -96,12 +101,12 @@ struct BLP {
   int in_kind;            // 0 = uint64 keys, 1 = uint32 ids (hashed), 2 = uint64 ids (hashed)
   u64 seed;
   u32 n;
-  int lo;                 // low key bits that are always zero (they carry the position when packed)
+  int lo;                 // low key bits that are always zero (they carry the row when packed)
   int packed;
-  int with_row;           // CSR rows: positions are stored with their row, as {position, row} pairs
+  int pay;                // words that travel beside a cold nonzero's key: row (not packed) and value, 0 to 2
   int nb_bits;            // log2(number of buckets)
   u32 NB, NBINS;          // buckets; NB + kHotMax
-  u32 G, chunk;           // walk CTAs and elements per CTA
+  u32 G, chunk;           // slices of the input and elements per slice
   u32 samp_m, samp_stride, samp_slots, hot_thresh, cold_limit;
   // rows
   const u32* row_ptr; u32 n_rows, fixed_z;
@@ -112,19 +117,22 @@ struct BLP {
   u32* ctl;
   u32* part;              // [G][NBINS]
   u32* bin_total;         // [NBINS]
-  u32* cold_base;         // [NB + 1]
-  u32* pos_base;          // [NB + 1]
-  u32* hot_base;          // [kHotMax + 1]
+  u32* cold_base;         // [NB + 1] where a bucket's cold words start: one place per cold nonzero and per hot key
+  u32* pos_base;          // [NB + 1] where its CSC segments start
   u64* shot_key; u32* shot_h;       // hot keys sorted by key
   u32* bucket_hot_off;    // [NB + 1]
-  u32* hot_u; u32* hot_seg;         // [kHotMax]
-  u32* bstate;            // [NB]
+  u32* hot_seg;           // [kHotMax] where a hot key's segment starts
+  u32* hot_loc;           // [kHotMax] its bucket (above 12 bits) and its rank there
+  u32* bucket_d;          // [NB] unique keys per bucket
   u32* row_hint;          // [n / 32 + 2], with row_ptr only: the row of every 32nd position
-  u64* cold_words; u32* cold_pos; u32* hot_pos;
+  u64* cold_words;        // [n] cold keys by bucket; behind a bucket's CTA its unique keys in order
+  u32* payload;           // [pay * n] beside them; then the unique keys' segment starts
+  u32* place;             // [n] bin and place of every nonzero
+  unsigned short* rank;   // [n] rank of every cold nonzero's key in its bucket, in the order of cold_words
   // outputs
   u64* ukeys; u32* seg_off; u32* csr_col; u32* csc_row; float* csc_val;
   u32* flagbits; u32* wordbase; u32* n_unique;
-  u32* status;
+  const u64* bounds; int S; u32* own_off; u32* gate_out;
 };
 
 __device__ __forceinline__ u64 bl_key_of(const BLP& p, u32 i) {
@@ -164,7 +172,7 @@ __global__ void __launch_bounds__(256) k_bl_clear(const BLP p, uint4* zero, u32 
   for (u32 i = gtid; i < ones4; i += gsize) ones[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
   for (u32 i = gtid; i < flag_words; i += gsize) p.flagbits[i] = 0;
   if (p.row_ptr != nullptr) {
-    // row hints for steps 5 and 6, up to the block behind the last position
+    // row hints for steps 4 and 6, up to the block behind the last position
     const u32 nh = ((p.n - 1) >> kHintShift) + 2;
     for (u32 h = gtid; h < nh; h += gsize) p.row_hint[h] = row_search(p.row_ptr, 0, p.n_rows, h << kHintShift);
   }
@@ -206,27 +214,73 @@ __global__ void __launch_bounds__(256) k_bl_hot(const BLP p) {
   }
 }
 
-// ---------------------------------------------------------------- 2./4. the two walks
-// Shared-memory layout of a walk CTA: hot table | hot keys | one word per bin.
-// kRow: CSR rows, positions are stored as {position, row} pairs (fixed-length rows do not pay for them).
-// kScatter = false: count. kScatter = true: the words start as this CTA's output cursors.
-template <bool kScatter, bool kRow>
-__global__ void __launch_bounds__(kWalkThreads) k_bl_walk(const BLP p) {
+// Four consecutive elements of the input (from element i on; those at or behind `end` are zero), by 16-byte loads
+// where the alignment allows it.
+struct Four { u64 k[4]; };
+__device__ __forceinline__ Four load_input(const BLP& p, u32 i, u32 end) {
+  Four r;
+  const bool wide = i + 3 < end && (((size_t)p.in) & 15) == 0;
+  if (p.in_kind == 1) {
+    u32 id[4] = {0, 0, 0, 0};
+    if (wide) {
+      const uint4 v = *reinterpret_cast<const uint4*>((const u32*)p.in + i);
+      id[0] = v.x; id[1] = v.y; id[2] = v.z; id[3] = v.w;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) if (i + q < end) id[q] = ((const u32*)p.in)[i + q];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) r.k[q] = id[q];
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) r.k[q] = 0;
+    if (wide) {
+      const ulonglong2* v = reinterpret_cast<const ulonglong2*>((const u64*)p.in + i);
+      const ulonglong2 a = v[0], c = v[1];
+      r.k[0] = a.x; r.k[1] = a.y; r.k[2] = c.x; r.k[3] = c.y;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) if (i + q < end) r.k[q] = ((const u64*)p.in)[i + q];
+    }
+  }
+  return r;
+}
+__device__ __forceinline__ u64 to_key(const BLP& p, u64 in) { return p.in_kind == 0 ? in : hash_id_to_key(in, p.seed); }
+
+// Rows of consecutive positions.
+struct RowWalk {
+  u32 row, left;                                   // left (fixed-length rows): positions up to the next row
+  __device__ __forceinline__ RowWalk(const BLP& p, u32 pos, u32 zinv) {
+    row = row_of_pos(p, pos, zinv);
+    left = p.row_ptr == nullptr ? (row + 1) * p.fixed_z - pos : 0u;
+  }
+  // to position pos + 1, which has a row
+  __device__ __forceinline__ void next(const BLP& p, u32 pos) {
+    if (p.row_ptr == nullptr) {
+      if (--left == 0) { ++row; left = p.fixed_z; }
+    } else if (row + 1 < p.n_rows && p.row_ptr[row + 1] <= pos + 1) {
+      ++row;
+      // behind a run of empty rows: searched, since one thread would walk all of it (20,000 nonzeros with
+      // 100,000 empty rows in their midst: 7.0 ms row by row, 0.09 ms like this, as without them)
+      if (row + 1 < p.n_rows && p.row_ptr[row + 1] <= pos + 1) row = row_of_pos(p, pos + 1, 0);
+    }
+  }
+};
+
+// ---------------------------------------------------------------- 2. count
+// Shared memory: hot table | hot keys | one counter per bin. Bound by instruction issue (hash, look-up) and the
+// shared-memory accesses. Keeping each nonzero's bin and place (the counter's old value, which a reduction would not
+// return) takes 14 us of 72 for 13.1 M nonzeros, and saves the scatter its look-ups and counters and the finish all of it.
+__global__ void __launch_bounds__(kWalkThreads) k_bl_count(const BLP p) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint4* s_hot = reinterpret_cast<uint4*>(smem);
   u64* s_hkey = reinterpret_cast<u64*>(smem + kHotSlots * 4);
   u32* s_bin = reinterpret_cast<u32*>(smem + kHotSlots * 4 + kHotMax * 8);
-  if (kScatter && p.ctl[kCtlFallback]) return;
   const u32 nh = min(p.ctl[kCtlNumHot], kHotMax);
   const int t = threadIdx.x;
   for (u32 i = t; i < kHotBuckets; i += kWalkThreads) s_hot[i] = reinterpret_cast<const uint4*>(p.hot_tab)[i];
   for (u32 i = t; i < nh; i += kWalkThreads) s_hkey[i] = p.hot_key[i];
-  u32* my_part = p.part + (size_t)blockIdx.x * p.NBINS;
-  for (u32 i = t; i < p.NBINS; i += kWalkThreads) {
-    u32 v = 0;
-    if (kScatter) v = my_part[i] + (i < p.NB ? p.cold_base[i] : p.hot_base[i - p.NB]);
-    s_bin[i] = v;
-  }
+  for (u32 i = t; i < p.NBINS; i += kWalkThreads) s_bin[i] = 0;
   __syncthreads();
   const u32 begin = blockIdx.x * p.chunk;
   const u32 end = min(p.n, begin + p.chunk);
@@ -256,122 +310,139 @@ __global__ void __launch_bounds__(kWalkThreads) k_bl_walk(const BLP p) {
     }
     return (u32)(key >> bshift);
   };
-  // Four elements: all look-ups, then all counts (when scattering: output places from the bins' cursors), then
-  // all stores, so that no element waits for another's chain. Plain shared-memory atomics, also for the hot
-  // keys: lanes that hit one address serialise inside the instruction, which costs far less than finding the
-  // groups first.
-  auto handle = [&](const u64 (&key)[4], u32 pos, u32 nvalid) {
-    u32 bin[4], dst[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) bin[q] = (u32)q < nvalid ? bin_of(key[q]) : 0u;
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if ((u32)q < nvalid) dst[q] = atomicAdd(&s_bin[bin[q]], 1u);
-    if constexpr (kScatter) {
-      // The row of a position is found here, where neighbouring threads look at neighbouring rows, and travels
-      // with it: looked up where the nonzeros arrive in key order, it is three dependent random loads each
-      // (3.9 M nonzeros: bucket and hot emit kernels 130 + 51 us that way, 100 + 32 us so, this walk 49 -> 65).
-      u32 row = kRow ? row_of_pos(p, pos, 0) : 0u;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if ((u32)q >= nvalid) break;
-        if (kRow) {
-          if (row + 1 < p.n_rows && p.row_ptr[row + 1] <= pos + q) {
-            ++row;
-            // behind a run of empty rows: searched, since one thread would walk all of it (20,000 nonzeros with
-            // 100,000 empty rows in their midst: 7.0 ms row by row, 0.09 ms like this, as without them)
-            if (row + 1 < p.n_rows && p.row_ptr[row + 1] <= pos + q) row = row_of_pos(p, pos + q, 0);
-          }
-          const uint2 pr = make_uint2(pos + q, row);
-          if (bin[q] >= p.NB) {
-            reinterpret_cast<uint2*>(p.hot_pos)[dst[q]] = pr;
-          } else {
-            p.cold_words[dst[q]] = key[q];
-            reinterpret_cast<uint2*>(p.cold_pos)[dst[q]] = pr;
-          }
-        } else if (bin[q] >= p.NB) {
-          p.hot_pos[dst[q]] = pos + q;
-        } else if (p.packed) {
-          p.cold_words[dst[q]] = key[q] | (u64)(pos + q);
-        } else {
-          p.cold_words[dst[q]] = key[q];
-          p.cold_pos[dst[q]] = pos + q;
-        }
-      }
-    }
-  };
-  // Four consecutive elements per thread and trip, the next trip's loads in flight while these are handled.
+  // Four consecutive elements per thread and trip, the next trip's loads in flight while these are handled: all
+  // look-ups, then all counts, then the store, so that no element waits for another's chain. Plain shared-memory
+  // atomics, also for the hot keys: lanes that hit one address serialise inside the instruction, which costs far
+  // less than finding the groups first.
   const u32 step = 4u * kWalkThreads;
-  if (p.in_kind == 1 && (((size_t)p.in) & 15) == 0) {
-    // 32-bit ids: one 16-byte load per trip
-    const u32* ids = (const u32*)p.in;
-    u32 i = begin + 4u * t;
-    uint4 cur = make_uint4(0, 0, 0, 0);
-    if (i + 3 < end) cur = *reinterpret_cast<const uint4*>(ids + i);
-    for (; i < end; i += step) {
-      uint4 nxt = make_uint4(0, 0, 0, 0);
-      if (i + step + 3 < end) nxt = *reinterpret_cast<const uint4*>(ids + i + step);
-      u32 id[4] = {cur.x, cur.y, cur.z, cur.w};
-      const u32 nvalid = min(4u, end - i);
-      if (nvalid < 4) {
+  u32 i = begin + 4u * t;
+  Four nxt = load_input(p, i, end);
+  for (; i < end; i += step) {
+    const Four cur = nxt;
+    nxt = load_input(p, i + step < end ? i + step : end, end);
+    const u32 nvalid = min(4u, end - i);
+    u32 bin[4], at[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) id[q] = (u32)q < nvalid ? ids[i + q] : 0u;
-      }
-      u64 key[4];
+    for (int q = 0; q < 4; ++q) bin[q] = (u32)q < nvalid ? bin_of(to_key(p, cur.k[q])) : 0u;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) key[q] = hash_id_to_key(id[q], p.seed);
-      handle(key, i, nvalid);
-      cur = nxt;
-    }
-  } else {
-    u64 nxt[4];
-    auto fetch = [&](u32 i) {
-      if (p.in_kind == 0 && i + 3 < end && (((size_t)p.in) & 15) == 0) {
-        const ulonglong2* v = reinterpret_cast<const ulonglong2*>((const u64*)p.in + i);
-        const ulonglong2 a = v[0], c = v[1];
-        nxt[0] = a.x; nxt[1] = a.y; nxt[2] = c.x; nxt[3] = c.y;
-      } else {
+    for (int q = 0; q < 4; ++q) at[q] = (u32)q < nvalid ? atomicAdd(&s_bin[bin[q]], 1u) : 0u;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) nxt[q] = (i + q < end) ? bl_key_of(p, i + q) : 0;
-      }
-    };
-    u32 i = begin + 4u * t;
-    fetch(i);
-    for (; i < end; i += step) {
-      const u64 key[4] = {nxt[0], nxt[1], nxt[2], nxt[3]};
-      fetch(i + step);
-      handle(key, i, min(4u, end - i));
+    for (int q = 0; q < 4; ++q) at[q] |= bin[q] << kPlaceBits;
+    if (nvalid == 4) {
+      *reinterpret_cast<uint4*>(p.place + i) = make_uint4(at[0], at[1], at[2], at[3]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) if ((u32)q < nvalid) p.place[i + q] = at[q];
     }
   }
-  if (!kScatter) {
-    __syncthreads();
-    for (u32 i = t; i < p.NBINS; i += kWalkThreads) my_part[i] = s_bin[i];
+  __syncthreads();
+  u32* my_part = p.part + (size_t)blockIdx.x * p.NBINS;
+  for (u32 k = t; k < p.NBINS; k += kWalkThreads) my_part[k] = s_bin[k];
+}
+
+// What a CTA of the scatter or the finish has of the input: a share of one slice.
+struct Share {
+  u32 slice, begin, end;
+  __device__ __forceinline__ Share(const BLP& p) {
+    slice = blockIdx.x / kWalkSplit;
+    const u32 part = (p.chunk / kWalkSplit + 3) & ~3u, b = slice * p.chunk, e = min(p.n, b + p.chunk);
+    begin = min(e, b + (blockIdx.x % kWalkSplit) * part);
+    end = blockIdx.x % kWalkSplit == kWalkSplit - 1 ? e : min(e, begin + part);
+  }
+};
+__device__ __forceinline__ uint4 load_places(const BLP& p, u32 i, u32 end) {
+  if (i + 3 < end) return __ldcs(reinterpret_cast<const uint4*>(p.place + i));
+  uint4 v = make_uint4(0, 0, 0, 0);
+  if (i < end) v.x = p.place[i];
+  if (i + 1 < end) v.y = p.place[i + 1];
+  if (i + 2 < end) v.z = p.place[i + 2];
+  return v;
+}
+
+// ---------------------------------------------------------------- 4. scatter
+// Cold nonzeros to their buckets. Bound by the stores, each a sector of its own (a slice has five words for a bucket):
+// 13.1 M nonzeros, 6 M of them cold: 106 us, 56 us without the stores (149 us with the keys looked up and counted again).
+__global__ void __launch_bounds__(kWalkThreads, 2) k_bl_scatter(const BLP p) {
+  extern __shared__ __align__(16) u32 s_base[];
+  if (p.ctl[kCtlFallback]) return;
+  const Share sh(p);
+  const int t = threadIdx.x;
+  const u32* part = p.part + (size_t)sh.slice * p.NBINS;
+  for (u32 i = t; i < p.NB; i += kWalkThreads) s_base[i] = part[i] + p.cold_base[i];
+  __syncthreads();
+  const u32 zinv = p.fixed_z ? (u32)(0xffffffffu / p.fixed_z) : 0u;
+  const u32 step = 4u * kWalkThreads;
+  u32 i = sh.begin + 4u * t;
+  Four nk = load_input(p, i, sh.end);
+  uint4 np = load_places(p, i, sh.end);
+  for (; i < sh.end; i += step) {
+    const Four cur = nk;
+    const u32 at[4] = {np.x, np.y, np.z, np.w};
+    const u32 j = i + step < sh.end ? i + step : sh.end;
+    nk = load_input(p, j, sh.end);
+    np = load_places(p, j, sh.end);
+    // the row of a position is found here, where neighbouring threads look at neighbouring rows, and travels with
+    // the key: looked up where the nonzeros arrive in key order, it is three dependent random loads each
+    RowWalk r(p, i, zinv);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (i + q >= sh.end) break;
+      if (q > 0) r.next(p, i + q - 1);
+      const u32 bin = at[q] >> kPlaceBits;
+      if (bin >= p.NB) continue;
+      const u32 dst = s_base[bin] + (at[q] & kPlaceMask);
+      p.cold_words[dst] = to_key(p, cur.k[q]) | (p.packed ? (u64)r.row : 0ull);
+      if (p.pay == 2) reinterpret_cast<uint2*>(p.payload)[dst] = make_uint2(r.row, __float_as_uint(p.vals[i + q]));
+      else if (p.pay == 1) p.payload[dst] = p.packed ? __float_as_uint(p.vals[i + q]) : r.row;
+    }
   }
 }
 
 // ---------------------------------------------------------------- 3. scan + plan
-// Per bin: exclusive prefix over the walk CTAs (in place) and the bin's total.
-__global__ void __launch_bounds__(256) k_bl_scan(const BLP p) {
-  const u32 bin = blockIdx.x * blockDim.x + threadIdx.x;
-  if (bin >= p.NBINS) return;
-  u32 run = 0;
-  // sixteen CTAs' counts are fetched before the first prefix is stored
-  for (u32 c0 = 0; c0 < p.G; c0 += 16) {
-    u32 v[16];
+// Per bin: exclusive prefix over the slices (in place) and the bin's total. A CTA takes 32 bins, each of its warps
+// an eighth of the slices, all of them fetched at once. (148 slices x 10,240 bins: 3.4 us; 7.7 us with one thread per
+// bin, sixteen slices at a time.)
+static constexpr int kScanWarps = 8, kScanKeep = 20;
+__global__ void __launch_bounds__(32 * kScanWarps) k_bl_scan(const BLP p) {
+  __shared__ u32 s_sum[kScanWarps][32];
+  const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5, bin = blockIdx.x * 32 + lane;
+  const u32 per = (p.G + kScanWarps - 1) / kScanWarps, c0 = min(p.G, w * per), c1 = min(p.G, c0 + per);
+  const bool have = bin < p.NBINS;
+  u32* col = p.part + bin;
+  u32 v[kScanKeep], sum = 0;
+  if (have) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k) v[k] = (c0 + k < p.G) ? p.part[(size_t)(c0 + k) * p.NBINS + bin] : 0u;
+    for (u32 k = 0; k < kScanKeep; ++k) v[k] = c0 + k < c1 ? col[(size_t)(c0 + k) * p.NBINS] : 0u;
 #pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      if (c0 + k < p.G) p.part[(size_t)(c0 + k) * p.NBINS + bin] = run;
-      run += v[k];
-    }
+    for (u32 k = 0; k < kScanKeep; ++k) sum += v[k];
+    for (u32 c = c0 + kScanKeep; c < c1; ++c) sum += col[(size_t)c * p.NBINS];
   }
-  p.bin_total[bin] = run;
+  s_sum[w][lane] = sum;
+  __syncthreads();
+  if (!have) return;
+  u32 run = 0, total = 0;
+#pragma unroll
+  for (u32 k = 0; k < kScanWarps; ++k) {
+    const u32 x = s_sum[k][lane];
+    if (k < w) run += x;
+    total += x;
+  }
+#pragma unroll
+  for (u32 k = 0; k < kScanKeep; ++k) {
+    if (c0 + k < c1) col[(size_t)(c0 + k) * p.NBINS] = run;
+    run += v[k];
+  }
+  for (u32 c = c0 + kScanKeep; c < c1; ++c) {
+    const u32 x = col[(size_t)c * p.NBINS];
+    col[(size_t)c * p.NBINS] = run;
+    run += x;
+  }
+  if (w == 0) p.bin_total[bin] = total;
 }
 
-// One CTA: the hot keys grouped by bucket, the hot stream's offsets, and per bucket the cold stream
-// offset, the final output offset and its first hot key. Every thread owns adjacent buckets and two adjacent hot
-// keys, kept in registers; the four prefix sums go through one block scan, and four buckets go out in one store:
+// One CTA: the hot keys grouped by bucket, and per bucket the offset of its cold words, the final output offset and
+// its first hot key. Every thread owns adjacent buckets and two adjacent hot
+// keys, kept in registers; the three prefix sums go through one block scan, and four buckets go out in one store:
 // a lone SM is bound by the number of sectors it asks for. 8192 buckets: 9 us (18 us as four scans of arrays in
 // shared memory, and as long with one scan and a store per bucket), all of it on the critical path.
 static constexpr int kPlanPer = kMaxBuckets / 1024;               // buckets per thread at most
@@ -380,7 +451,7 @@ __global__ void __launch_bounds__(1024) k_bl_plan(const BLP p) {
   extern __shared__ __align__(16) unsigned char smem[];
   u32* s_hn = reinterpret_cast<u32*>(smem);         // [NB, padded] hot nonzeros per bucket
   u32* s_hc = s_hn + plan_pad(p.NB);                // [NB, padded] hot keys per bucket, then the place of the next one
-  __shared__ u32 s_tot[4][32];
+  __shared__ u32 s_tot[3][32];
   __shared__ u32 s_max;
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const u32 nh = min(p.ctl[kCtlNumHot], kHotMax);
@@ -417,19 +488,20 @@ __global__ void __launch_bounds__(1024) k_bl_plan(const BLP p) {
       atomicAdd(&s_hc[b], 1u);
     }
   __syncthreads();
-  // {cold nonzeros, all nonzeros, hot keys, nonzeros of hot keys} before this thread's buckets and hot keys
-  u32 v[4] = {0, 0, 0, ht[0] + ht[1]}, mx = 0;
+  // {cold words, all nonzeros, hot keys} before this thread's buckets. A bucket has room among the cold words for its
+  // hot keys too (every one of them stands for nonzeros that are not there): its unique keys go there in the end.
+  u32 v[3] = {0, 0, 0}, mx = 0;
 #pragma unroll
   for (int k = 0; k < kPlanPer; ++k)
     if ((u32)k < per && b0 + k < p.NB) {
       const u32 b = plan_pad(b0 + k);
-      v[0] += cold[k]; v[1] += cold[k] + s_hn[b]; v[2] += s_hc[b];
+      v[0] += cold[k] + s_hc[b]; v[1] += cold[k] + s_hn[b]; v[2] += s_hc[b];
       mx = max(mx, cold[k]);
     }
   atomicMax(&s_max, mx);
-  u32 x[4];
+  u32 x[3];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < 3; ++q) {
     x[q] = v[q];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -439,7 +511,7 @@ __global__ void __launch_bounds__(1024) k_bl_plan(const BLP p) {
     if (lane == 31) s_tot[q][w] = x[q];
   }
   __syncthreads();
-  if (w < 4) {                                      // warp q turns the 32 totals of value q into prefixes
+  if (w < 3) {                                      // warp q turns the 32 totals of value q into prefixes
     u32 y = s_tot[w][lane];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -449,16 +521,16 @@ __global__ void __launch_bounds__(1024) k_bl_plan(const BLP p) {
     s_tot[w][lane] = y;
   }
   __syncthreads();
-  u32 run[4];
+  u32 run[3];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) run[q] = (w ? s_tot[q][w - 1] : 0u) + x[q] - v[q];
+  for (int q = 0; q < 3; ++q) run[q] = (w ? s_tot[q][w - 1] : 0u) + x[q] - v[q];
   __align__(16) u32 out[3][kPlanPer];
 #pragma unroll
   for (int k = 0; k < kPlanPer; ++k)
     if ((u32)k < per && b0 + k < p.NB) {
       const u32 b = plan_pad(b0 + k), c = s_hc[b];
       out[0][k] = run[0]; out[1][k] = run[1]; out[2][k] = run[2];
-      run[0] += cold[k]; run[1] += cold[k] + s_hn[b];
+      run[0] += cold[k] + c; run[1] += cold[k] + s_hn[b];
       s_hc[b] = run[2];
       run[2] += c;
     }
@@ -475,7 +547,6 @@ __global__ void __launch_bounds__(1024) k_bl_plan(const BLP p) {
         if ((u32)k < per && b0 + k < p.NB) dst[q][b0 + k] = out[q][k];
     }
   }
-  *reinterpret_cast<uint2*>(p.hot_base + 2 * t) = make_uint2(run[3], run[3] + ht[0]);
   __syncthreads();
   // hot keys grouped by bucket (any order inside a bucket: the bucket kernel puts them into its table)
 #pragma unroll
@@ -487,8 +558,6 @@ __global__ void __launch_bounds__(1024) k_bl_plan(const BLP p) {
     }
   if (t == 0) {
     p.cold_base[p.NB] = s_tot[0][31]; p.pos_base[p.NB] = s_tot[1][31]; p.bucket_hot_off[p.NB] = s_tot[2][31];
-    p.hot_base[kHotMax] = s_tot[3][31];
-    p.ctl[kCtlHotElems] = s_tot[3][31];
     if (s_max > p.cold_limit) p.ctl[kCtlFallback] = 1;   // keys are not spread evenly: use the sort
     // more than three quarters of the sampled nonzeros have a key of their own: the big tables
     p.ctl[kCtlBigTables] = (4ull * p.ctl[kCtlSampleDistinct] > 3ull * p.samp_m) ? 1u : 0u;
@@ -554,7 +623,11 @@ __device__ __forceinline__ u32 bucket_block_scan(u32 v, u32* s_warp /* 9 words *
   return pre;
 }
 
-template <typename CK, int kBits, bool kRow>
+// kPay: something travels beside the keys' words (BLP::pay is not 0). Bound by the latencies of its short phases, which
+// five CTAs per SM overlap. 13.1 M nonzeros, 8192 buckets: 117 us, and 222 us with the index of the bucket's first
+// key fetched by a look-back over the buckets in front (42 us) and every nonzero's column stored where the nonzero came
+// from (50 us).
+template <typename CK, int kBits, bool kPay>
 __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
   typedef BucketShape<kBits> Sh;
   constexpr u32 kHsAll = Sh::kHsAll, kHsWords = Sh::kHsWords, kDistinctMax = Sh::kDistinctMax;
@@ -567,18 +640,20 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
   u32* s_hbits = s_bits + kHsWords;                                            // slots that hold a hot key
   unsigned short* s_rank = reinterpret_cast<unsigned short*>(s_hbits + kHsWords);  // per slot: hot index, then rank
   unsigned short* s_dense = s_rank + kHsAll;                                   // occupied slots in slot order
-  __shared__ u32 s_ovf, s_b, s_ubase, s_warp[kBucketThreads / 32 + 1];
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  // A CTA takes buckets by ticket until none is left (a few CTAs per SM are launched, not one per bucket).
-  for (;;) {
-  if (t == 0) {
-    // one thread reads the flags for the whole CTA: other CTAs may raise the fallback flag at any moment
-    const bool mine = (p.ctl[kCtlBigTables] != 0) == (kBits == 12);
-    s_b = (!mine || ld_relaxed_gpu(&p.ctl[kCtlFallback])) ? 0xFFFFFFFFu : atomicAdd(&p.ctl[kCtlTicket], 1u);
-    s_ovf = 0;
-  }
+  __shared__ u32 s_ovf, s_stop, s_warp[kBucketThreads / 32 + 1];
+  const int t = threadIdx.x;
+  if ((p.ctl[kCtlBigTables] != 0) != (kBits == 12)) return;
+  const int sh_l = p.nb_bits, sh_r = p.nb_bits + p.lo;
+  const int rem = 64 - sh_r;                    // significant bits of a compact key
+  const u64 rowmask = p.packed ? ((1ull << p.lo) - 1) : 0ull;
+  const bool row_beside = kPay && !p.packed, val_beside = kPay && p.vals != nullptr;
+  for (u32 b = blockIdx.x; b < p.NB; b += gridDim.x) {
+  const u32 cb = p.cold_base[b], ce = p.cold_base[b + 1], pb = p.pos_base[b];
+  const u32 h0 = p.bucket_hot_off[b], h1 = p.bucket_hot_off[b + 1];
+  // one thread reads the flag for the whole CTA: other CTAs may raise it at any moment
+  if (t == 0) { s_stop = ld_relaxed_gpu(&p.ctl[kCtlFallback]); s_ovf = 0; }
   {
-    // keys = all ones, counts = 0, bitmaps = 0, with 16-byte stores (while the ticket is on its way)
+    // keys = all ones, counts = 0, bitmaps = 0, with 16-byte stores (while the loads are on their way)
     uint4* k4 = reinterpret_cast<uint4*>(s_key);
     const u32 nk4 = kHsAll * sizeof(CK) / 16;
     for (u32 i = t; i < nk4; i += kBucketThreads) k4[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
@@ -586,29 +661,25 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
     for (u32 i = t; i < kHsAll / 4; i += kBucketThreads) c4[i] = make_uint4(0, 0, 0, 0);
     for (u32 i = t; i < 2 * kHsWords; i += kBucketThreads) s_bits[i] = 0;
   }
-  __syncthreads();
-  const u32 b = s_b;
-  if (b >= p.NB) return;
-  const u32 cb = p.cold_base[b], nb = p.cold_base[b + 1] - cb;
-  const u32 pb = p.pos_base[b];
-  const u32 h0 = p.bucket_hot_off[b], h1 = p.bucket_hot_off[b + 1];
-  const int sh_l = p.nb_bits, sh_r = p.nb_bits + p.lo;
-  const int rem = 64 - sh_r;                    // significant bits of a compact key
-  const u64 posmask = p.packed ? ((1ull << p.lo) - 1) : 0ull;
+  const u32 nb = ce - cb - (h1 - h0);
   // The first four nonzeros of every thread stay in registers for both passes over the bucket
   // (a bucket of average size has no more), the rest is read again in pass 2.
   u64 w0[4];
-  uint2 p0[4];                                     // position, and with kRow its row
-  auto position = [&](u32 j) -> uint2 {
-    if (kRow) return reinterpret_cast<const uint2*>(p.cold_pos)[cb + j];
-    return make_uint2(p.packed ? 0u : p.cold_pos[cb + j], 0u);
+  uint2 p0[4];                                     // row and value, as far as they travel beside the key
+  auto beside = [&](u32 j) -> uint2 {
+    if (!kPay) return make_uint2(0u, 0u);
+    if (p.pay == 2) return reinterpret_cast<const uint2*>(p.payload)[cb + j];
+    const u32 x = p.payload[cb + j];
+    return make_uint2(x, x);
   };
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const u32 j = t + q * kBucketThreads;
     w0[q] = j < nb ? p.cold_words[cb + j] : 0;
-    p0[q] = j < nb ? position(j) : make_uint2(0u, 0u);
+    p0[q] = j < nb ? beside(j) : make_uint2(0u, 0u);
   }
+  __syncthreads();
+  if (s_stop) return;
   // hot keys of this bucket enter the table with their total count
   for (u32 i = h0 + t; i < h1; i += kBucketThreads) {
     const u32 h = p.shot_h[i];
@@ -646,11 +717,10 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
   __syncthreads();
   if (s_ovf) {
     // keys bunched inside the bucket (or too many of them): hand the whole minibatch to the sort-based path
-    if (t == 0) { st_relaxed_gpu(&p.ctl[kCtlFallback], 1u); st_relaxed_gpu(&p.bstate[b], kFlagIncl); }
+    if (t == 0) st_relaxed_gpu(&p.ctl[kCtlFallback], 1u);
     return;
   }
-  // the bucket's number of unique keys is known: publish it for the buckets behind
-  if (t == 0) st_relaxed_gpu(&p.bstate[b], (b == 0 ? kFlagIncl : kFlagAgg) | d);
+  if (t == 0) p.bucket_d[b] = d;
   {
     u32 wbits = myw, k = wpre;
     while (wbits) {
@@ -695,89 +765,27 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
     my_rank[k] = r; my_start[k] = st;
   }
   if (bad) s_ovf = 1;
-  // unique keys in all buckets before this one: look back over the published counts
-  if (w == 0) {
-    u32 ex = 0;
-    if (b > 0) {
-      long long q = (long long)b - 1;
-      u32 spins = 0;
-      bool done = false;
-      while (!done && q >= 0) {
-        // 4 x 32 buckets are fetched per round trip to L2 and consumed from the nearest on
-        u32 v[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const long long idx = q - 32 * k - lane;
-          v[k] = kFlagIncl;
-          if (idx >= 0) v[k] = ld_relaxed_gpu(p.bstate + idx);
-        }
-        u32 add = 0;
-        int taken = 0;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (done || taken < 32 * k) continue;    // warp-uniform
-          const u32 f = v[k] & ~kValMask;
-          const u32 empty = __ballot_sync(0xffffffffu, f == 0);
-          const u32 incl = __ballot_sync(0xffffffffu, f == kFlagIncl);
-          const int first_empty = empty ? __ffs(empty) - 1 : 32;
-          const int first_incl = incl ? __ffs(incl) - 1 : 32;
-          const int upto = first_incl < first_empty ? first_incl + 1 : first_empty;   // lanes [0, upto) are usable
-          if (lane < upto) add += v[k] & kValMask;
-          taken += upto;
-          if (first_incl < first_empty) done = true;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
-        ex += add;
-        if (!done) {
-          q -= taken;
-          if (taken == 0) {
-            // a bucket that gave up (or never started because of that) publishes nothing: stop waiting
-            if (ld_relaxed_gpu(&p.ctl[kCtlFallback])) break;
-            if (++spins > kGridWaitIters) { if (lane == 0) set_status(p.status, kLookbackTimeout); break; }
-            __nanosleep(40);
-          }
-        }
-      }
-      if (lane == 0) st_relaxed_gpu(&p.bstate[b], kFlagIncl | ((ex + d) & kValMask));
-    }
-    if (lane == 0) {
-      s_ubase = ex;
-      if (b == p.NB - 1) *p.n_unique = ex + d;
-    }
-  }
   __syncthreads();
   if (s_ovf) {
     if (t == 0) st_relaxed_gpu(&p.ctl[kCtlFallback], 1u);
     return;
   }
-  const u32 ub = s_ubase;
-  const u64 bucket_bits = (u64)b << (64 - p.nb_bits);
 #pragma unroll
   for (int k = 0; k < kEntriesPerThread; ++k) {
     if (my_rank[k] == 0xFFFFFFFFu) continue;
-    const u32 slot = s_dense[t + k * kBucketThreads];
-    const u32 c = s_cnt[slot];
+    const u32 i = t + k * kBucketThreads, slot = s_dense[i];
     const bool is_hot = (s_hbits[slot >> 5] >> (slot & 31)) & 1u;
     const u32 hh = is_hot ? s_rank[slot] : 0u;
-    const u32 start = my_start[k];
-    s_cnt[slot] = start;
+    s_cnt[slot] = my_start[k];
     s_rank[slot] = (unsigned short)my_rank[k];
-    const u32 u = ub + my_rank[k], P = pb + start;
-    p.ukeys[u] = bucket_bits | ((u64)s_key[slot] << p.lo);
-    p.seg_off[u] = P;
-    atomicOr(&p.flagbits[P >> 5], 1u << (P & 31));
-    if (is_hot) {
-      p.hot_u[hh] = u;          // the hot emit kernel fills this segment (and its wordbase words)
-      p.hot_seg[hh] = P;
-    } else {
-      // number of segment heads before every 32-aligned position inside the segment
-      for (u32 wd = (P + 31) >> 5; (wd << 5) < P + c; ++wd) p.wordbase[wd] = ((wd << 5) == P) ? u : u + 1;
+    s_start[i] = my_start[k] | (is_hot ? kHotFlag : 0u);
+    if (is_hot) {                                  // for the finish, which places this key's nonzeros
+      p.hot_seg[hh] = pb + my_start[k];
+      p.hot_loc[hh] = (b << 12) | my_rank[k];
     }
   }
   __syncthreads();
-  // pass 2: every nonzero to its place
-  const u32 zinv = p.fixed_z ? (u32)(0xffffffffu / p.fixed_z) : 0u;
+  // pass 2: every nonzero's row to its place, and the rank of its key
   for (u32 j0 = t; j0 < nb; j0 += 4 * kBucketThreads) {
     u64 wd[4];
     uint2 ps[4];
@@ -786,7 +794,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
       const u32 j = j0 + q * kBucketThreads;
       const bool first = j0 == (u32)t;
       wd[q] = first ? w0[q] : (j < nb ? p.cold_words[cb + j] : 0);
-      ps[q] = first ? p0[q] : (j < nb ? position(j) : make_uint2(0u, 0u));
+      ps[q] = first ? p0[q] : (j < nb ? beside(j) : make_uint2(0u, 0u));
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -795,81 +803,185 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
       const CK ck = (CK)((wd[q] << sh_l) >> sh_r);
       const int slot = bucket_find<CK, kBits>(s_key, ck, rem);
       if (slot < 0) continue;                     // cannot happen: the key was inserted in pass 1
-      const u32 pos = p.packed && !kRow ? (u32)(wd[q] & posmask) : ps[q].x;
       const u32 P = pb + atomicAdd(&s_cnt[slot], 1u);
-      const u32 u = ub + s_rank[slot];
-      p.csc_row[P] = kRow ? ps[q].y : row_of_pos(p, pos, zinv);
-      p.csr_col[pos] = u;
-      if (p.csc_val) p.csc_val[P] = p.vals[pos];
+      p.csc_row[P] = row_beside ? ps[q].x : (u32)(wd[q] & rowmask);
+      if (val_beside) p.csc_val[P] = __uint_as_float(ps[q].y);
+      p.rank[cb + j] = s_rank[slot];
     }
+  }
+  __syncthreads();
+  // the unique keys and their segment starts, in order, over the words and what travelled beside them
+  u32* seg = p.payload + (size_t)cb * max(1, p.pay);
+  const u64 bucket_bits = (u64)b << (64 - p.nb_bits);
+  for (u32 i = t; i < d; i += kBucketThreads) {
+    const u32 slot = s_dense[i], r = s_rank[slot];
+    p.cold_words[cb + r] = bucket_bits | ((u64)s_key[slot] << p.lo);
+    seg[r] = s_start[i];
   }
   __syncthreads();       // the tables are rebuilt for the next bucket
   }
 }
 
-// ---------------------------------------------------------------- 6. hot keys' position lists
-template <bool kRow>
-__global__ void __launch_bounds__(256) k_bl_hot_emit(const BLP p) {
-  __shared__ u32 s_base[kHotMax + 1];
-  __shared__ u32 s_u[kHotMax], s_seg[kHotMax];
-  if (p.ctl[kCtlFallback]) return;
+// ---------------------------------------------------------------- 6. finish
+// Shared memory: per bucket the index of its first unique key and the place of this slice's first cold word; per hot
+// key its index and the place of this slice's first nonzero. Bound by memory: a place read and a column written per
+// nonzero, a 2-byte gather per cold and a 4-byte store of its own per hot one (13.1 M nonzeros: 110 us).
+__global__ void __launch_bounds__(kWalkThreads, 2) k_bl_finish(const BLP p) {
+  extern __shared__ __align__(16) u32 s_first[];   // [NB + 4] [NB] [kHotMax] [kHotMax]
+  __shared__ u32 s_tot[32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const u32 skip = p.ctl[kCtlFallback];
+  if (blockIdx.x == 0 && t == 0) *p.gate_out = skip;
+  if (skip) return;
+  u32* s_base = s_first + p.NB + 4;
+  u32* s_hot_u = s_base + p.NB;
+  u32* s_hot_at = s_hot_u + kHotMax;
+  const Share sh(p);
+  const u32* part = p.part + (size_t)sh.slice * p.NBINS;
   const u32 nh = min(p.ctl[kCtlNumHot], kHotMax);
-  if (nh == 0) return;
-  for (u32 i = threadIdx.x; i <= nh; i += blockDim.x) s_base[i] = p.hot_base[i];
-  for (u32 i = threadIdx.x; i < nh; i += blockDim.x) { s_u[i] = p.hot_u[i]; s_seg[i] = p.hot_seg[i]; }
-  __syncthreads();
-  const u32 total = s_base[nh];
-  const u32 zinv = p.fixed_z ? (u32)(0xffffffffu / p.fixed_z) : 0u;
-  // A warp walks one contiguous piece of the hot stream, 4 x 32 positions per trip. The stream is
-  // grouped by hot key, so the key index only ever moves forward: one binary search at the start.
-  const int lane = threadIdx.x & 31;
-  const u32 nwarps = gridDim.x * (blockDim.x >> 5);
-  const u32 gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const u32 piece = ((total + nwarps - 1) / nwarps + 127) & ~127u;
-  const u32 begin = min(total, gw * piece), end = min(total, begin + piece);
-  if (begin >= end) return;
-  u32 h;
-  {
-    u32 lo = 0, hi = nh;                            // largest h with s_base[h] <= begin
-    while (hi - lo > 1) {
-      u32 mid = (lo + hi) >> 1;
-      if (s_base[mid] <= begin) lo = mid; else hi = mid;
-    }
-    h = lo;
+  // a thread adds up adjacent buckets
+  const u32 per = (p.NB + kWalkThreads - 1) / kWalkThreads, b0 = min(p.NB, t * per), b1 = min(p.NB, b0 + per);
+  u32 cnt[kPlanPer], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kPlanPer; ++k) {
+    cnt[k] = b0 + k < b1 ? p.bucket_d[b0 + k] : 0u;
+    sum += cnt[k];
   }
-  for (u32 j0 = begin + lane; j0 < end + lane; j0 += 128) {
-    u32 pos[4], row[4];
+  for (u32 i = t; i < p.NB; i += kWalkThreads) s_base[i] = part[i] + p.cold_base[i];
+  for (u32 h = t; h < nh; h += kWalkThreads) {
+    s_hot_u[h] = p.hot_loc[h];
+    s_hot_at[h] = p.hot_seg[h] + part[p.NB + h];
+  }
+  u32 x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u32 y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) s_tot[w] = x;
+  __syncthreads();
+  u32 run = x - sum, total = 0;
+#pragma unroll
+  for (int k = 0; k < kWalkThreads / 32; ++k) {
+    const u32 y = s_tot[k];
+    if (k < w) run += y;
+    total += y;
+  }
+#pragma unroll
+  for (int k = 0; k < kPlanPer; ++k) {
+    if (b0 + k < b1) s_first[b0 + k] = run;
+    run += cnt[k];
+  }
+  if (t == 0) s_first[p.NB] = total;
+  __syncthreads();
+  for (u32 h = t; h < nh; h += kWalkThreads) {
+    const u32 loc = s_hot_u[h];
+    s_hot_u[h] = s_first[loc >> 12] + (loc & 0xFFFu);
+  }
+  __syncthreads();
+  // (a) the unique keys close up: a warp per bucket
+  const u32 pw = p.pay > 1 ? 2u : 1u;
+  for (u32 b = blockIdx.x * (kWalkThreads / 32) + w; b < p.NB; b += gridDim.x * (kWalkThreads / 32)) {
+    const u32 first = s_first[b], d = s_first[b + 1] - first;
+    const u64* keys = p.cold_words + p.cold_base[b];
+    const u32* seg = p.payload + (size_t)p.cold_base[b] * pw;
+    const u32 pb = p.pos_base[b], pe = p.pos_base[b + 1];
+    for (u32 r0 = lane; r0 < d; r0 += 128) {
+      u64 key[4];
+      u32 st[4], nx[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const u32 r = r0 + 32 * q;
+        key[q] = r < d ? keys[r] : 0;
+        st[q] = r < d ? seg[r] : 0u;
+        nx[q] = r + 1 < d ? seg[r + 1] : 0u;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const u32 r = r0 + 32 * q;
+        if (r >= d) break;
+        const u32 u = first + r, P = pb + (st[q] & ~kHotFlag), e = r + 1 < d ? pb + (nx[q] & ~kHotFlag) : pe;
+        p.ukeys[u] = key[q];
+        p.seg_off[u] = P;
+        atomicOr(&p.flagbits[P >> 5], 1u << (P & 31));
+        // number of segment heads before every 32-aligned position inside the segment (a hot key's: below)
+        if (!(st[q] & kHotFlag))
+          for (u32 wd = (P + 31) >> 5; (wd << 5) < e; ++wd) p.wordbase[wd] = ((wd << 5) == P) ? u : u + 1;
+      }
+    }
+  }
+  // (b) the number of keys and the owners' shares of them
+  if (blockIdx.x == 0) {
+    for (u32 s = w; s < (u32)p.S; s += kWalkThreads / 32) {
+      const u64 bound = p.bounds[s];
+      const u32 b = (u32)(bound >> (64 - p.nb_bits));
+      const u32 first = s_first[b], d = s_first[b + 1] - first;
+      const u64* keys = p.cold_words + p.cold_base[b];
+      u32 below = 0;
+      if (bound << p.nb_bits)                      // (no key of a bucket lies below its first)
+        for (u32 r = lane; r < d; r += 32) below += keys[r] < bound ? 1u : 0u;
+      below = __reduce_add_sync(0xffffffffu, below);
+      if (lane == 0) p.own_off[s] = first + below;
+    }
+    if (t == 0) {
+      p.own_off[p.S] = total;
+      p.seg_off[total] = p.n;
+      *p.n_unique = total;
+    }
+  }
+  // (c) the nonzeros in input order
+  const u32 zinv = p.fixed_z ? (u32)(0xffffffffu / p.fixed_z) : 0u;
+  const u32 step = 4u * kWalkThreads;
+  u32 i = sh.begin + 4u * t;
+  uint4 np = load_places(p, i, sh.end);
+  for (; i < sh.end; i += step) {
+    const u32 at[4] = {np.x, np.y, np.z, np.w};
+    np = load_places(p, i + step < sh.end ? i + step : sh.end, sh.end);
+    u32 u[4];
+    bool any_hot = false;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const u32 j = j0 + q * 32;
-      uint2 pr = make_uint2(0u, 0u);
-      if (j < end) {
-        if (kRow) pr = __ldcs(&reinterpret_cast<const uint2*>(p.hot_pos)[j]);
-        else pr.x = __ldcs(&p.hot_pos[j]);
+      const u32 bin = at[q] >> kPlaceBits;
+      u[q] = 0;
+      if (i + q >= sh.end) continue;
+      if (bin < p.NB) u[q] = p.rank[s_base[bin] + (at[q] & kPlaceMask)];
+      else any_hot = true;
+    }
+    if (any_hot) {
+      RowWalk r(p, i, zinv);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (i + q >= sh.end) break;
+        if (q > 0) r.next(p, i + q - 1);
+        const u32 bin = at[q] >> kPlaceBits;
+        if (bin < p.NB) continue;
+        const u32 h = bin - p.NB, P = s_hot_at[h] + (at[q] & kPlaceMask);
+        u[q] = s_hot_u[h];
+        p.csc_row[P] = r.row;
+        if (p.csc_val) p.csc_val[P] = p.vals[i + q];
+        if ((P & 31u) == 0) p.wordbase[P >> 5] = P == p.hot_seg[h] ? u[q] : u[q] + 1;
       }
-      pos[q] = pr.x; row[q] = pr.y;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const u32 j = j0 + q * 32;
-      if (j >= end) break;
-      while (h + 1 < nh && s_base[h + 1] <= j) ++h;
-      const u32 u = s_u[h];
-      const u32 P = s_seg[h] + (j - s_base[h]);
-      p.csc_row[P] = kRow ? row[q] : row_of_pos(p, pos[q], zinv);
-      p.csr_col[pos[q]] = u;
-      if (p.csc_val) p.csc_val[P] = p.vals[pos[q]];
-      if ((P & 31u) == 0) p.wordbase[P >> 5] = (j == s_base[h]) ? u : u + 1;
+      const u32 bin = at[q] >> kPlaceBits;
+      if (i + q < sh.end && bin < p.NB) u[q] += s_first[bin];
+    }
+    if (i + 3 < sh.end) {
+      *reinterpret_cast<uint4*>(p.csr_col + i) = make_uint4(u[0], u[1], u[2], u[3]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) if (i + q < sh.end) p.csr_col[i + q] = u[q];
     }
   }
 }
 
 // scratch layout (bytes), shared by the size query and the launcher
 struct BlLayout {
-  size_t zero_begin, samp_cnt, ctl, bstate, zero_end;
+  size_t zero_begin, samp_cnt, ctl, zero_end;
   size_t ff_begin, samp_key, hot_tab, ff_end;
-  size_t hot_key, part, bin_total, cold_base, pos_base, hot_base, shot_key, shot_h, bucket_hot_off,
-      hot_u, hot_seg, row_hint, total;
+  size_t hot_key, part, bin_total, cold_base, pos_base, shot_key, shot_h, bucket_hot_off,
+      hot_seg, hot_loc, bucket_d, row_hint, total;
 };
 static size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 static BlLayout bl_layout(u32 NB, u32 G, u32 n, u32 samp_slots) {
@@ -879,7 +991,6 @@ static BlLayout bl_layout(u32 NB, u32 G, u32 n, u32 samp_slots) {
   L.zero_begin = o;
   L.samp_cnt = o; o = al(o + (size_t)samp_slots * 4);
   L.ctl = o; o = al(o + kCtlWords * 4);
-  L.bstate = o; o = al(o + (size_t)NB * 4);
   L.zero_end = o;
   L.ff_begin = o;
   L.samp_key = o; o = al(o + (size_t)samp_slots * 8);
@@ -890,12 +1001,12 @@ static BlLayout bl_layout(u32 NB, u32 G, u32 n, u32 samp_slots) {
   L.bin_total = o; o = al(o + (size_t)NBINS * 4);
   L.cold_base = o; o = al(o + (size_t)(NB + 1) * 4);
   L.pos_base = o; o = al(o + (size_t)(NB + 1) * 4);
-  L.hot_base = o; o = al(o + (kHotMax + 1) * 4);
   L.shot_key = o; o = al(o + kHotMax * 8);
   L.shot_h = o; o = al(o + kHotMax * 4);
   L.bucket_hot_off = o; o = al(o + (size_t)(NB + 1) * 4);
-  L.hot_u = o; o = al(o + kHotMax * 4);
   L.hot_seg = o; o = al(o + kHotMax * 4);
+  L.hot_loc = o; o = al(o + kHotMax * 4);
+  L.bucket_d = o; o = al(o + (size_t)NB * 4);
   L.row_hint = o; o = al(o + ((size_t)(n >> kHintShift) + 2) * 4);
   L.total = o;
   return L;
@@ -912,11 +1023,13 @@ static u32 bl_num_buckets(u32 n) {
   while (nb < 512 && (size_t)nb * 512 <= n) nb <<= 1;
   return nb;
 }
-static int bl_walk_ctas() {
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms > 0 ? sms : 1;
+// Slices of the input: one per SM, and as many as keep a nonzero's place in its bits.
+static u32 bl_most_slices(u32 n) { return max((u32)max(1, psb_device_sm_count()), (u32)(((size_t)n + kPlaceMask) >> kPlaceBits)); }
+// Resident CTAs of a bucket kernel.
+static u32 bl_bucket_ctas(const void* fn, size_t smem) {
+  int per = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, kBucketThreads, smem);
+  return (u32)max(1, per) * (u32)max(1, psb_device_sm_count());
 }
 
 }  // namespace psb
@@ -925,15 +1038,15 @@ using namespace psb;
 
 extern "C" size_t psb_bucket_localize_scratch_bytes(uint32_t max_n) {
   // sized for the largest bucket count; the per-nonzero buffers are the caller's
-  return bl_layout(kMaxBuckets, (u32)bl_walk_ctas(), max_n, kSampSlots).total;
+  return bl_layout(kMaxBuckets, bl_most_slices(max_n), max_n, kSampSlots).total;
 }
 
 // Groups the n nonzeros of a minibatch by key. Inputs as for psb_sort_pairs (in, in_kind, seed);
 // low_zero_bits = number of low key bits that are zero in every key (64 - significant bits of a
-// narrow hashed key); when n - 1 fits in them the position rides in the key word (no cold_pos needed).
-// cold_words (n x 8 bytes), cold_pos (n x 4 bytes, may be null when the positions fit) and hot_pos
-// (n x 4 bytes) are work buffers; with row_ptr cold_pos is always needed and both are n x 8 bytes. Outputs as for psb_localize2. *gate_out (device word) is set to 1
-// when the caller must run the gated sort-based path instead (its outputs then replace these).
+// narrow hashed key); when n_rows - 1 fits in them the row rides in the key word. Work buffers of n x 8 bytes each,
+// 16-byte aligned like csr_col: cold_words (cold keys by bucket), cold_pos (what travels beside them) and hot_pos
+// (places and ranks of the nonzeros). Outputs as for psb_localize2. *gate_out (device word) is
+// set to 1 when the caller must run the gated sort-based path instead (its outputs then replace these).
 extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, uint32_t n, int low_zero_bits,
                                    const uint32_t* row_ptr, uint32_t n_rows, uint32_t fixed_z,
                                    const float* vals, const psb_u64* bounds, int S,
@@ -955,16 +1068,17 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   BLP p{};
   p.in = in; p.in_kind = in_kind; p.seed = seed; p.n = n;
   p.lo = low_zero_bits;
-  p.packed = (low_zero_bits > 0 && (low_zero_bits >= 32 || ((n - 1) >> low_zero_bits) == 0)) ? 1 : 0;
-  if ((!p.packed || row_ptr != nullptr) && cold_pos == nullptr) return -(int)cudaErrorInvalidValue;
-  p.with_row = row_ptr != nullptr ? 1 : 0;
+  if (row_ptr == nullptr) n_rows = (n + fixed_z - 1) / fixed_z;
+  p.packed = (low_zero_bits > 0 && n_rows > 0 && (low_zero_bits >= 32 || ((n_rows - 1) >> low_zero_bits) == 0)) ? 1 : 0;
+  p.pay = (p.packed ? 0 : 1) + (vals != nullptr ? 1 : 0);
+  if (cold_pos == nullptr || ((((size_t)cold_words) | ((size_t)cold_pos) | ((size_t)hot_pos) | ((size_t)csr_col)) & 15) != 0)
+    return -(int)cudaErrorInvalidValue;
   p.NB = bl_num_buckets(n);
   p.nb_bits = 0;
   while ((1u << p.nb_bits) < p.NB) ++p.nb_bits;
   p.NBINS = p.NB + kHotMax;
-  // walk CTAs: one per SM, and no more than get a full trip of 4096 elements (every CTA fills its shared tables
-  // first, and the scan over the CTAs' counts is a serial chain)
-  p.G = min((u32)bl_walk_ctas(), (n + 4 * kWalkThreads - 1) / (4 * kWalkThreads));
+  // no more slices than get a full trip of 4096 elements (every CTA fills its shared tables first)
+  p.G = min(bl_most_slices(n), (n + 4 * kWalkThreads - 1) / (4 * kWalkThreads));
   p.chunk = ((n + p.G - 1) / p.G + 3) & ~3u;
   p.samp_m = min(n, max(kSampMin, min(kSampMax, n / 4)));
   p.samp_slots = 2;
@@ -981,58 +1095,57 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   p.hot_key = (u64*)(sc + L.hot_key);
   p.ctl = (u32*)(sc + L.ctl); p.part = (u32*)(sc + L.part); p.bin_total = (u32*)(sc + L.bin_total);
   p.cold_base = (u32*)(sc + L.cold_base); p.pos_base = (u32*)(sc + L.pos_base);
-  p.hot_base = (u32*)(sc + L.hot_base); p.shot_key = (u64*)(sc + L.shot_key); p.shot_h = (u32*)(sc + L.shot_h);
-  p.bucket_hot_off = (u32*)(sc + L.bucket_hot_off); p.hot_u = (u32*)(sc + L.hot_u);
-  p.hot_seg = (u32*)(sc + L.hot_seg); p.row_hint = (u32*)(sc + L.row_hint); p.bstate = (u32*)(sc + L.bstate);
-  p.cold_words = (u64*)cold_words; p.cold_pos = cold_pos; p.hot_pos = hot_pos;
+  p.shot_key = (u64*)(sc + L.shot_key); p.shot_h = (u32*)(sc + L.shot_h);
+  p.bucket_hot_off = (u32*)(sc + L.bucket_hot_off); p.hot_seg = (u32*)(sc + L.hot_seg);
+  p.hot_loc = (u32*)(sc + L.hot_loc); p.bucket_d = (u32*)(sc + L.bucket_d); p.row_hint = (u32*)(sc + L.row_hint);
+  p.cold_words = (u64*)cold_words; p.payload = cold_pos; p.place = hot_pos; p.rank = (unsigned short*)(hot_pos + n);
   p.ukeys = (u64*)ukeys; p.seg_off = seg_off; p.csr_col = csr_col; p.csc_row = csc_row; p.csc_val = csc_val;
-  p.flagbits = flagbits; p.wordbase = wordbase; p.n_unique = n_unique; p.status = status;
+  p.flagbits = flagbits; p.wordbase = wordbase; p.n_unique = n_unique;
+  p.bounds = (const u64*)bounds; p.S = S; p.own_off = own_off; p.gate_out = gate_out;
 
   const u32 zero4 = (u32)((L.zero_end - L.zero_begin) / 16), ones4 = (u32)((L.ff_end - L.ff_begin) / 16);
   k_bl_clear<<<psb_device_sm_count() * 2, 256, 0, stream>>>(p, (uint4*)(sc + L.zero_begin), zero4, (uint4*)(sc + L.ff_begin),
                                                             ones4, (n + 31) / 32);
   k_bl_sample<<<(p.samp_m + 255) / 256, 256, 0, stream>>>(p);
   k_bl_hot<<<(p.samp_slots + 255) / 256, 256, 0, stream>>>(p);
-  const size_t walk_smem = kHotSlots * 4 + kHotMax * 8 + (size_t)p.NBINS * 4;
-  static bool attr_set = false;
+  const size_t count_smem = kHotSlots * 4 + kHotMax * 8 + (size_t)p.NBINS * 4;
+  const size_t scatter_smem = (size_t)p.NB * 4, finish_smem = (size_t)(2 * p.NB + 4 + 2 * kHotMax) * 4;
   const int remaining = 64 - p.nb_bits - p.lo;      // key bits that distinguish keys inside a bucket
   const bool ck32 = remaining <= 31;
   const size_t plan_smem = (size_t)(p.NB + p.NB / 32) * 8;
-  if (!attr_set) {
-    const size_t walk_max = kHotSlots * 4 + kHotMax * 8 + (size_t)(kMaxBuckets + kHotMax) * 4;
-    cudaFuncSetAttribute((const void*)k_bl_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)((kMaxBuckets + kMaxBuckets / 32) * 8));
-    cudaFuncSetAttribute((const void*)k_bl_walk<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_max);
-    cudaFuncSetAttribute((const void*)k_bl_walk<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_max);
-    cudaFuncSetAttribute((const void*)k_bl_walk<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_max);
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u32, 11, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<11>::smem_bytes(4));
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u32, 11, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<11>::smem_bytes(4));
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u32, 12, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<12>::smem_bytes(4));
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u32, 12, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<12>::smem_bytes(4));
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u64, 11, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<11>::smem_bytes(8));
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u64, 11, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<11>::smem_bytes(8));
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u64, 12, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<12>::smem_bytes(8));
-    cudaFuncSetAttribute((const void*)k_bl_bucket<u64, 12, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BucketShape<12>::smem_bytes(8));
-    attr_set = true;
-  }
-  k_bl_walk<false, false><<<p.G, kWalkThreads, walk_smem, stream>>>(p);
-  k_bl_scan<<<(p.NBINS + 255) / 256, 256, 0, stream>>>(p);
+  static const bool attr_set = [] {
+    auto most = [](const void* fn, size_t bytes) { cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
+    most((const void*)k_bl_count, kHotSlots * 4 + kHotMax * 8 + (size_t)(kMaxBuckets + kHotMax) * 4);
+    most((const void*)k_bl_plan, (size_t)(kMaxBuckets + kMaxBuckets / 32) * 8);
+    most((const void*)k_bl_scatter, (size_t)kMaxBuckets * 4);
+    most((const void*)k_bl_finish, (size_t)(2 * kMaxBuckets + 4 + 2 * kHotMax) * 4);
+    return true;
+  }();
+  (void)attr_set;
+  k_bl_count<<<p.G, kWalkThreads, count_smem, stream>>>(p);
+  k_bl_scan<<<(p.NBINS + 31) / 32, 32 * kScanWarps, 0, stream>>>(p);
   k_bl_plan<<<1, 1024, plan_smem, stream>>>(p);
-  if (p.with_row) k_bl_walk<true, true><<<p.G, kWalkThreads, walk_smem, stream>>>(p);
-  else k_bl_walk<true, false><<<p.G, kWalkThreads, walk_smem, stream>>>(p);
-  const u32 sms = (u32)bl_walk_ctas(), g11 = min(p.NB, sms * 6), g12 = min(p.NB, sms * 4);
-  auto buckets = [&](auto row) {
-    constexpr bool kRow = decltype(row)::value;
-    if (ck32) {
-      k_bl_bucket<u32, 11, kRow><<<g11, kBucketThreads, BucketShape<11>::smem_bytes(4), stream>>>(p);
-      k_bl_bucket<u32, 12, kRow><<<g12, kBucketThreads, BucketShape<12>::smem_bytes(4), stream>>>(p);
-    } else {
-      k_bl_bucket<u64, 11, kRow><<<g11, kBucketThreads, BucketShape<11>::smem_bytes(8), stream>>>(p);
-      k_bl_bucket<u64, 12, kRow><<<g12, kBucketThreads, BucketShape<12>::smem_bytes(8), stream>>>(p);
-    }
-    k_bl_hot_emit<kRow><<<min(sms * 8, (n + 1023) / 1024), 256, 0, stream>>>(p);
+  k_bl_scatter<<<p.G * kWalkSplit, kWalkThreads, scatter_smem, stream>>>(p);
+  auto bucket = [&](auto key, auto bits, auto pay) {
+    typedef decltype(key) CK;
+    constexpr int kBits = decltype(bits)::value;
+    constexpr size_t smem = BucketShape<kBits>::smem_bytes(sizeof(CK));
+    const auto fn = k_bl_bucket<CK, kBits, decltype(pay)::value>;
+    static const u32 ctas = [fn] {
+      cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      return bl_bucket_ctas((const void*)fn, smem);
+    }();
+    fn<<<min(p.NB, ctas), kBucketThreads, smem, stream>>>(p);
   };
-  if (p.with_row) buckets(std::true_type()); else buckets(std::false_type());
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return -(int)e;
-  return psb_owner_offsets_n(ukeys, n_unique, bounds, S, n, seg_off, own_off, p.ctl + kCtlFallback, gate_out, stream);
+  auto buckets = [&](auto key, auto pay) {
+    bucket(key, std::integral_constant<int, 11>(), pay);
+    bucket(key, std::integral_constant<int, 12>(), pay);
+  };
+  if (p.pay) {
+    if (ck32) buckets(u32(), std::true_type()); else buckets(u64(), std::true_type());
+  } else {
+    if (ck32) buckets(u32(), std::false_type()); else buckets(u64(), std::false_type());
+  }
+  k_bl_finish<<<p.G * kWalkSplit, kWalkThreads, finish_smem, stream>>>(p);
+  return -(int)cudaGetLastError();
 }

@@ -168,7 +168,7 @@ class LocalBatch:
                                         ptr(self.csc_row_buf), ptr(self.csc_val), ptr(self.flagbits),
                                         ptr(self.wordbase), ptr(self.n_unique), ptr(self.own_off),
                                         ptr(self.bucket_scratch), ptr(self.status), ptr(self.gate), sp),
-                  "bucket localize", kernels=11)
+                  "bucket localize", kernels=10)
             if method == "bucket":
                 return self
             gate = ptr(self.gate)

@@ -383,3 +383,56 @@ def test_bucket_localize_long_run_of_empty_rows(cuda_lib, split):
     assert int(b.gate.item()) == 0 and int(b.status.item()) == 0
     _check_grouped(b, keys, row_ptr, None, bounds_h, rows)
     assert min(ms) < 5.0
+
+
+@pytest.mark.parametrize("values", [False, True])
+@pytest.mark.parametrize("hash_bits,rows", [(40, 3000), (52, 4096), (52, 4097), (24, 3001), (0, 3000)])
+@pytest.mark.parametrize("ragged", [False, True])
+def test_bucket_localize_what_travels_beside_a_key(cuda_lib, ragged, hash_bits, rows, values):
+    """A row rides in the zero bits of its key as long as every row fits (4096 rows in 12 bits, 4097 do not), else
+    beside it; a value always beside it."""
+    from parameter_server_b200.ops.localize import LocalBatch
+    from parameter_server_b200.utils.oracle import hash_id_to_key
+    rng = np.random.default_rng(rows + values)
+    n = rng.integers(0, 17, rows) if ragged else np.full(rows, 7)
+    row_ptr = np.concatenate([[0], np.cumsum(n)])
+    nnz = int(row_ptr[-1])
+    ids = (rng.zipf(1.3, nnz) % (1 << 22)).astype(np.int32)
+    keys = hash_id_to_key(ids, 3, hash_bits or 64)
+    vals = rng.random(nnz, dtype=np.float32) if values else None
+    bounds_h, bounds = _bounds(5)
+    b = LocalBatch(rows, nnz, 5, "cuda", real_values=values)
+    kw = dict(row_ptr=torch.from_numpy(row_ptr.astype(np.int32)).cuda()) if ragged else dict(fixed_z=7)
+    b.localize(torch.from_numpy(ids).cuda(), None, bounds, vals=torch.from_numpy(vals).cuda() if values else None, hash_seed=3,
+               hash_bits=hash_bits, method="bucket", **kw)
+    torch.cuda.synchronize()
+    assert int(b.gate.item()) == 0 and int(b.status.item()) == 0
+    _check_grouped(b, keys, row_ptr, vals, bounds_h, rows)
+
+
+@pytest.mark.parametrize("z", [1, 3, 5000])
+def test_bucket_localize_more_slices_than_sms(cuda_lib, z):
+    """A slice of the input is at most as long as a nonzero's place in it has bits: from 148 x 2^18 nonzeros on there are
+    more slices than SMs."""
+    from parameter_server_b200.ops import _lib
+    from parameter_server_b200.ops.localize import LocalBatch
+    n = ((_lib.lib().psb_device_sm_count() << 18) // 15000 + 1) * 15000
+    g = torch.Generator(device="cuda").manual_seed(z)
+    # half of the nonzeros on a thousand ids, the rest on half a million
+    ids = torch.where(torch.rand(n, device="cuda", generator=g) < 0.5, torch.randint(0, 1000, (n,), device="cuda", generator=g),
+                      torch.randint(0, 1 << 19, (n,), device="cuda", generator=g)).to(torch.int32)
+    b = LocalBatch(n // z, n, 1, "cuda")
+    b.localize(ids, None, _bounds(1)[1], fixed_z=z, hash_seed=0, hash_bits=40, method="bucket")
+    torch.cuda.synchronize()
+    assert int(b.gate.item()) == 0 and int(b.status.item()) == 0
+    U = int(b.n_unique.item())
+    wide, keys = ids.long(), torch.empty(n, dtype=torch.int64, device="cuda")
+    _lib.check(_lib.lib().psb_hash_ids(0, _lib.ptr(wide), _lib.ptr(keys), n, 40 << 56, _lib.stream_ptr()), "hash")
+    sign = -(1 << 63)
+    u, inv, count = torch.unique(keys ^ sign, return_inverse=True, return_counts=True)
+    assert U == u.numel() and torch.equal(b.ukeys[:U], u ^ sign) and torch.equal(b.csr_col[:n].long(), inv)
+    assert torch.equal((b.seg_off[1:U + 1] - b.seg_off[:U]).long(), count)
+    segment = torch.repeat_interleave(torch.arange(U, device="cuda"), count)
+    rows = torch.arange(n, device="cuda") // z
+    got = torch.sort(segment * (n // z + 1) + b.csc_row[:n].long())[0]
+    assert torch.equal(got, torch.sort(inv * (n // z + 1) + rows)[0])
