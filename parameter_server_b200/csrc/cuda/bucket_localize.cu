@@ -161,7 +161,9 @@ __device__ __forceinline__ u32 row_of_pos(const BLP& p, u32 pos, u32 zinv) {
   // search takes a step or two instead of log2(n_rows) dependent loads per nonzero (3.9 M nonzeros in 100,000
   // rows: localisation and margins 579 -> 466 us).
   const u32 b = pos >> kHintShift;
-  return row_search(p.row_ptr, p.row_hint[b], min(p.row_hint[b + 1] + 1, p.n_rows), pos);
+  // (clamped: row offsets that do not ascend from 0 to n leave hints unwritten)
+  const u32 lo = min(p.row_hint[b], p.n_rows - 1), hi = min(p.row_hint[b + 1], p.n_rows - 1) + 1;
+  return row_search(p.row_ptr, lo, max(lo + 1, hi), pos);
 }
 
 // ---------------------------------------------------------------- 0. clean scratch
@@ -172,38 +174,85 @@ __global__ void __launch_bounds__(256) k_bl_clear(const BLP p, uint4* zero, u32 
   for (u32 i = gtid; i < ones4; i += gsize) ones[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
   for (u32 i = gtid; i < flag_words; i += gsize) p.flagbits[i] = 0;
   if (p.row_ptr != nullptr) {
-    // row hints for steps 4 and 6, up to the block behind the last position
-    const u32 nh = ((p.n - 1) >> kHintShift) + 2;
-    for (u32 h = gtid; h < nh; h += gsize) p.row_hint[h] = row_search(p.row_ptr, 0, p.n_rows, h << kHintShift);
+    // Row hints for steps 4 and 6, up to the block behind the last position: every row writes those of the blocks that
+    // start in it, a long one with its whole warp. (A search per hint waited for log2(rows) dependent loads.)
+    const u32 lane = threadIdx.x & 31;
+    for (u32 r0 = gtid - lane; r0 < p.n_rows; r0 += gsize) {
+      const u32 r = r0 + lane;
+      u32 h0 = 0, h1 = 0;
+      if (r < p.n_rows) {
+        const u32 b = r == 0 ? 0u : p.row_ptr[r], e = r + 1 == p.n_rows ? p.n : min(p.n, p.row_ptr[r + 1]);
+        h0 = (b + 31) >> kHintShift;
+        h1 = e > b ? (e + 31) >> kHintShift : h0;
+      }
+      const bool longer = h1 > h0 + 16;
+      if (!longer) for (u32 h = h0; h < h1; ++h) p.row_hint[h] = r;
+      for (u32 m = __ballot_sync(0xffffffffu, longer); m; m &= m - 1) {
+        const int first = __ffs(m) - 1;
+        const u32 a0 = __shfl_sync(0xffffffffu, h0, first), a1 = __shfl_sync(0xffffffffu, h1, first);
+        for (u32 h = a0 + lane; h < a1; h += 32) p.row_hint[h] = r0 + first;
+      }
+    }
+    if (gtid == 0) p.row_hint[((p.n - 1) >> kHintShift) + 1] = p.n_rows - 1;
   }
 }
 
 // ---------------------------------------------------------------- 1. sample
-__global__ void __launch_bounds__(256) k_bl_sample(const BLP p) {
-  const u32 j = blockIdx.x * blockDim.x + threadIdx.x;
+// A CTA counts its share of the sample in shared memory first: added one by one, the most frequent keys would each
+// take thousands of atomics on one address.
+static constexpr int kSampThreads = 1024;
+static constexpr u32 kSampLocal = 2 * kSampThreads;
+__global__ void __launch_bounds__(kSampThreads) k_bl_sample(const BLP p) {
+  __shared__ u64 s_key[kSampLocal];
+  __shared__ u32 s_cnt[kSampLocal];
+  const u32 t = threadIdx.x, j = blockIdx.x * kSampThreads + t;
   const bool valid = j < p.samp_m;
   const u64 key = valid ? bl_key_of(p, j * p.samp_stride) : kEmptyKey;
-  // equal keys of a warp count once (the most frequent key would otherwise take thousands of
-  // atomics on one address)
-  const u32 m = __match_any_sync(0xffffffffu, key);
-  if (!valid || (int)(threadIdx.x & 31) != __ffs(m) - 1) return;
-  u32 slot = (u32)(fmix64(key) & (p.samp_slots - 1));
-  for (u32 probe = 0; probe < p.samp_slots; ++probe) {
-    u64 old = atomicCAS(&p.samp_key[slot], kEmptyKey, key);
-    if (old == kEmptyKey || old == key) { atomicAdd(&p.samp_cnt[slot], (u32)__popc(m)); return; }
-    slot = (slot + 1) & (p.samp_slots - 1);
+  for (u32 i = t; i < kSampLocal; i += kSampThreads) { s_key[i] = kEmptyKey; s_cnt[i] = 0; }
+  __syncthreads();
+  if (valid) {
+    u32 slot = (u32)(fmix64(key) & (kSampLocal - 1));
+    for (u32 probe = 0; probe < kSampLocal; ++probe) {
+      const u64 old = atomicCAS(&s_key[slot], kEmptyKey, key);
+      if (old == kEmptyKey || old == key) { atomicAdd(&s_cnt[slot], 1u); break; }
+      slot = (slot + 1) & (kSampLocal - 1);
+    }
+  }
+  __syncthreads();
+  for (u32 i = t; i < kSampLocal; i += kSampThreads) {
+    const u32 c = s_cnt[i];
+    if (c == 0) continue;
+    const u64 k = s_key[i];
+    u32 slot = (u32)(fmix64(k) & (p.samp_slots - 1));
+    for (u32 probe = 0; probe < p.samp_slots; ++probe) {
+      const u64 old = atomicCAS(&p.samp_key[slot], kEmptyKey, k);
+      if (old == kEmptyKey || old == k) { atomicAdd(&p.samp_cnt[slot], c); break; }
+      slot = (slot + 1) & (p.samp_slots - 1);
+    }
   }
 }
 
-__global__ void __launch_bounds__(256) k_bl_hot(const BLP p) {
-  const u32 s = blockIdx.x * blockDim.x + threadIdx.x;
+// Keys counted often enough become hot. One atomic per CTA on each of the two counters: with one per warp and per key they
+// queue up on the two addresses.
+static constexpr int kHotThreads = 1024;
+__global__ void __launch_bounds__(kHotThreads) k_bl_hot(const BLP p) {
+  __shared__ u32 s_n, s_base;
+  const u32 s = blockIdx.x * kHotThreads + threadIdx.x;
   const u32 c = s < p.samp_slots ? p.samp_cnt[s] : 0u;
+  if (threadIdx.x == 0) s_n = 0;
   // distinct keys of the sample (how much keys repeat decides the size of the buckets' tables)
-  const u32 occ = __ballot_sync(0xffffffffu, c > 0);
-  if ((threadIdx.x & 31) == 0 && occ) atomicAdd(&p.ctl[kCtlSampleDistinct], (u32)__popc(occ));
-  if (c < p.hot_thresh) return;
+  const u32 occ = (u32)__syncthreads_count(c > 0);
+  const bool hot = c >= p.hot_thresh;
+  const u32 mine = hot ? atomicAdd(&s_n, 1u) : 0u;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (occ) atomicAdd(&p.ctl[kCtlSampleDistinct], occ);
+    s_base = s_n ? atomicAdd(&p.ctl[kCtlNumHot], s_n) : 0u;
+  }
+  __syncthreads();
+  if (!hot) return;
   const u64 key = p.samp_key[s];
-  const u32 h = atomicAdd(&p.ctl[kCtlNumHot], 1u);
+  const u32 h = s_base + mine;
   if (h >= kHotMax) return;                                    // more candidates than places: the rest stay cold
   p.hot_key[h] = key;
   const u32 hash = hot_hash(key), entry = ((hash & 0xFFFFFu) << 11) | h;
@@ -1106,8 +1155,8 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   const u32 zero4 = (u32)((L.zero_end - L.zero_begin) / 16), ones4 = (u32)((L.ff_end - L.ff_begin) / 16);
   k_bl_clear<<<psb_device_sm_count() * 2, 256, 0, stream>>>(p, (uint4*)(sc + L.zero_begin), zero4, (uint4*)(sc + L.ff_begin),
                                                             ones4, (n + 31) / 32);
-  k_bl_sample<<<(p.samp_m + 255) / 256, 256, 0, stream>>>(p);
-  k_bl_hot<<<(p.samp_slots + 255) / 256, 256, 0, stream>>>(p);
+  k_bl_sample<<<(p.samp_m + kSampThreads - 1) / kSampThreads, kSampThreads, 0, stream>>>(p);
+  k_bl_hot<<<(p.samp_slots + kHotThreads - 1) / kHotThreads, kHotThreads, 0, stream>>>(p);
   const size_t count_smem = kHotSlots * 4 + kHotMax * 8 + (size_t)p.NBINS * 4;
   const size_t scatter_smem = (size_t)p.NB * 4, finish_smem = (size_t)(2 * p.NB + 4 + 2 * kHotMax) * 4;
   const int remaining = 64 - p.nb_bits - p.lo;      // key bits that distinguish keys inside a bucket
