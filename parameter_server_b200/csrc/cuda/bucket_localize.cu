@@ -135,6 +135,14 @@ struct BLP {
   const u64* bounds; int S; u32* own_off; u32* gate_out;
 };
 
+// The steps are launched with programmatic stream serialisation: a step's CTAs come in while the step before it drains, and
+// wait here, before they read anything, until it has ended and its stores are visible (so all the steps before it
+// have, too). The next step may come in from here on.
+__device__ __forceinline__ void behind_the_step_before() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ u64 bl_key_of(const BLP& p, u32 i) {
   if (p.in_kind == 0) return ((const u64*)p.in)[i];
   u64 id = p.in_kind == 1 ? (u64)((const u32*)p.in)[i] : ((const u64*)p.in)[i];
@@ -169,6 +177,7 @@ __device__ __forceinline__ u32 row_of_pos(const BLP& p, u32 pos, u32 zinv) {
 // ---------------------------------------------------------------- 0. clean scratch
 // Everything that starts as zeros or ones, and the row hints, in one launch instead of one per region.
 __global__ void __launch_bounds__(256) k_bl_clear(const BLP p, uint4* zero, u32 zero4, uint4* ones, u32 ones4, u32 flag_words) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const u32 gsize = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x;
   for (u32 i = gtid; i < zero4; i += gsize) zero[i] = make_uint4(0, 0, 0, 0);
   for (u32 i = gtid; i < ones4; i += gsize) ones[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
@@ -203,6 +212,7 @@ __global__ void __launch_bounds__(256) k_bl_clear(const BLP p, uint4* zero, u32 
 static constexpr int kSampThreads = 1024;
 static constexpr u32 kSampLocal = 2 * kSampThreads;
 __global__ void __launch_bounds__(kSampThreads) k_bl_sample(const BLP p) {
+  behind_the_step_before();
   __shared__ u64 s_key[kSampLocal];
   __shared__ u32 s_cnt[kSampLocal];
   const u32 t = threadIdx.x, j = blockIdx.x * kSampThreads + t;
@@ -236,6 +246,7 @@ __global__ void __launch_bounds__(kSampThreads) k_bl_sample(const BLP p) {
 // queue up on the two addresses.
 static constexpr int kHotThreads = 1024;
 __global__ void __launch_bounds__(kHotThreads) k_bl_hot(const BLP p) {
+  behind_the_step_before();
   __shared__ u32 s_n, s_base;
   const u32 s = blockIdx.x * kHotThreads + threadIdx.x;
   const u32 c = s < p.samp_slots ? p.samp_cnt[s] : 0u;
@@ -321,6 +332,7 @@ struct RowWalk {
 // shared-memory accesses. Keeping each nonzero's bin and place (the counter's old value, which a reduction would not
 // return) takes 14 us of 72 for 13.1 M nonzeros, and saves the scatter its look-ups and counters and the finish all of it.
 __global__ void __launch_bounds__(kWalkThreads) k_bl_count(const BLP p) {
+  behind_the_step_before();
   extern __shared__ __align__(16) unsigned char smem[];
   uint4* s_hot = reinterpret_cast<uint4*>(smem);
   u64* s_hkey = reinterpret_cast<u64*>(smem + kHotSlots * 4);
@@ -412,6 +424,7 @@ __device__ __forceinline__ uint4 load_places(const BLP& p, u32 i, u32 end) {
 // Cold nonzeros to their buckets. Bound by the stores, each a sector of its own (a slice has five words for a bucket):
 // 13.1 M nonzeros, 6 M of them cold: 106 us, 56 us without the stores (149 us with the keys looked up and counted again).
 __global__ void __launch_bounds__(kWalkThreads, 2) k_bl_scatter(const BLP p) {
+  behind_the_step_before();
   extern __shared__ __align__(16) u32 s_base[];
   if (p.ctl[kCtlFallback]) return;
   const Share sh(p);
@@ -453,6 +466,7 @@ __global__ void __launch_bounds__(kWalkThreads, 2) k_bl_scatter(const BLP p) {
 // bin, sixteen slices at a time.)
 static constexpr int kScanWarps = 8, kScanKeep = 20;
 __global__ void __launch_bounds__(32 * kScanWarps) k_bl_scan(const BLP p) {
+  behind_the_step_before();
   __shared__ u32 s_sum[kScanWarps][32];
   const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5, bin = blockIdx.x * 32 + lane;
   const u32 per = (p.G + kScanWarps - 1) / kScanWarps, c0 = min(p.G, w * per), c1 = min(p.G, c0 + per);
@@ -497,6 +511,7 @@ __global__ void __launch_bounds__(32 * kScanWarps) k_bl_scan(const BLP p) {
 static constexpr int kPlanPer = kMaxBuckets / 1024;               // buckets per thread at most
 __device__ __forceinline__ u32 plan_pad(u32 i) { return i + (i >> 5); }   // adjacent entries of a thread: no bank conflicts
 __global__ void __launch_bounds__(1024) k_bl_plan(const BLP p) {
+  behind_the_step_before();
   extern __shared__ __align__(16) unsigned char smem[];
   u32* s_hn = reinterpret_cast<u32*>(smem);         // [NB, padded] hot nonzeros per bucket
   u32* s_hc = s_hn + plan_pad(p.NB);                // [NB, padded] hot keys per bucket, then the place of the next one
@@ -678,6 +693,7 @@ __device__ __forceinline__ u32 bucket_block_scan(u32 v, u32* s_warp /* 9 words *
 // from (50 us).
 template <typename CK, int kBits, bool kPay>
 __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
+  behind_the_step_before();
   typedef BucketShape<kBits> Sh;
   constexpr u32 kHsAll = Sh::kHsAll, kHsWords = Sh::kHsWords, kDistinctMax = Sh::kDistinctMax;
   constexpr int kEntriesPerThread = Sh::kEntriesPerThread;
@@ -876,6 +892,7 @@ __global__ void __launch_bounds__(kBucketThreads) k_bl_bucket(const BLP p) {
 // key its index and the place of this slice's first nonzero. Bound by memory: a place read and a column written per
 // nonzero, a 2-byte gather per cold and a 4-byte store of its own per hot one (13.1 M nonzeros: 110 us).
 __global__ void __launch_bounds__(kWalkThreads, 2) k_bl_finish(const BLP p) {
+  behind_the_step_before();
   extern __shared__ __align__(16) u32 s_first[];   // [NB + 4] [NB] [kHotMax] [kHotMax]
   __shared__ u32 s_tot[32];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -1025,6 +1042,17 @@ __global__ void __launch_bounds__(kWalkThreads, 2) k_bl_finish(const BLP p) {
   }
 }
 
+template <typename... A>
+static void launch_step(void (*fn)(A...), u32 grid, u32 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid); c.blockDim = dim3(block); c.dynamicSmemBytes = smem; c.stream = stream;
+  cudaLaunchAttribute a = {};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &a; c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, fn, args...);
+}
+
 // scratch layout (bytes), shared by the size query and the launcher
 struct BlLayout {
   size_t zero_begin, samp_cnt, ctl, zero_end;
@@ -1155,8 +1183,8 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   const u32 zero4 = (u32)((L.zero_end - L.zero_begin) / 16), ones4 = (u32)((L.ff_end - L.ff_begin) / 16);
   k_bl_clear<<<psb_device_sm_count() * 2, 256, 0, stream>>>(p, (uint4*)(sc + L.zero_begin), zero4, (uint4*)(sc + L.ff_begin),
                                                             ones4, (n + 31) / 32);
-  k_bl_sample<<<(p.samp_m + kSampThreads - 1) / kSampThreads, kSampThreads, 0, stream>>>(p);
-  k_bl_hot<<<(p.samp_slots + kHotThreads - 1) / kHotThreads, kHotThreads, 0, stream>>>(p);
+  launch_step(k_bl_sample, (p.samp_m + kSampThreads - 1) / kSampThreads, kSampThreads, 0, stream, p);
+  launch_step(k_bl_hot, (p.samp_slots + kHotThreads - 1) / kHotThreads, kHotThreads, 0, stream, p);
   const size_t count_smem = kHotSlots * 4 + kHotMax * 8 + (size_t)p.NBINS * 4;
   const size_t scatter_smem = (size_t)p.NB * 4, finish_smem = (size_t)(2 * p.NB + 4 + 2 * kHotMax) * 4;
   const int remaining = 64 - p.nb_bits - p.lo;      // key bits that distinguish keys inside a bucket
@@ -1171,10 +1199,10 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
     return true;
   }();
   (void)attr_set;
-  k_bl_count<<<p.G, kWalkThreads, count_smem, stream>>>(p);
-  k_bl_scan<<<(p.NBINS + 31) / 32, 32 * kScanWarps, 0, stream>>>(p);
-  k_bl_plan<<<1, 1024, plan_smem, stream>>>(p);
-  k_bl_scatter<<<p.G * kWalkSplit, kWalkThreads, scatter_smem, stream>>>(p);
+  launch_step(k_bl_count, p.G, kWalkThreads, count_smem, stream, p);
+  launch_step(k_bl_scan, (p.NBINS + 31) / 32, 32 * kScanWarps, 0, stream, p);
+  launch_step(k_bl_plan, 1, 1024, plan_smem, stream, p);
+  launch_step(k_bl_scatter, p.G * kWalkSplit, kWalkThreads, scatter_smem, stream, p);
   auto bucket = [&](auto key, auto bits, auto pay) {
     typedef decltype(key) CK;
     constexpr int kBits = decltype(bits)::value;
@@ -1184,7 +1212,7 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
       cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       return bl_bucket_ctas((const void*)fn, smem);
     }();
-    fn<<<min(p.NB, ctas), kBucketThreads, smem, stream>>>(p);
+    launch_step(fn, min(p.NB, ctas), kBucketThreads, smem, stream, p);
   };
   auto buckets = [&](auto key, auto pay) {
     bucket(key, std::integral_constant<int, 11>(), pay);
@@ -1195,6 +1223,6 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   } else {
     if (ck32) buckets(u32(), std::false_type()); else buckets(u64(), std::false_type());
   }
-  k_bl_finish<<<p.G * kWalkSplit, kWalkThreads, finish_smem, stream>>>(p);
+  launch_step(k_bl_finish, p.G * kWalkSplit, kWalkThreads, finish_smem, stream, p);
   return -(int)cudaGetLastError();
 }
