@@ -357,6 +357,12 @@ struct WarpTile {
   }
 };
 
+// The fence between a CTA's stores and its arrival, and between the arrivals and the flag: this GPU is the only reader
+// where there is one rank.
+__device__ __forceinline__ void fence_readers(int S) {
+  if (S == 1) __threadfence(); else __threadfence_system();
+}
+
 // ------------------------------------------------------------------ F2 (exchange form)
 __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchangeParams p) {
   __shared__ u32 s_off[PSB_MAX_SHARDS + 1];
@@ -421,7 +427,7 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
   if (threadIdx.x == 0) {
     s_last = 0;
     if (!alone) {
-      __threadfence_system();
+      fence_readers(S);
       s_last = atomicAdd(&p.done[0], 1u) + 1 == gridDim.x;
     }
   }
@@ -430,11 +436,10 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
     int s = threadIdx.x;
     u32 c = s_off[s + 1] - s_off[s];
     if (c > p.req_cap) { set_status(p.status, kInboxOverflow); c = p.req_cap; }
-    __threadfence_system();
+    fence_readers(S);
     p.req_hdr[s][0] = c | (key_hit ? 0x80000000u : 0u);     // top bit: no keys, answer from the remembered slots
     p.req_hdr[s][1] = s_off[s];
-    __threadfence_system();
-    st_release_sys(p.req_ready[s], p.ts1);
+    st_release_sys(p.req_ready[s], p.ts1);         // (orders this thread's header words, and with the fence all keys)
     if (s == 0) {
       atomicExch(&p.done[0], 0u);
       // every CTA has read the other parity's fingerprint by now: clear it for the next round
@@ -590,14 +595,16 @@ __global__ void __launch_bounds__(kThreads) k_pull_exchange(const PsbPullExchang
     }
   }
   PSB_TSTAMP(4);
+  // The only rank's answers to itself, without margins: the end of the launch is what their reader waits for.
+  if (alone && p.phases == 7 && p.n_rows == 0) return;
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence_system();                        // one per CTA, as in (a)
+    fence_readers(S);                              // one per CTA, as in (a)
     s_last = atomicAdd(&p.done[1], 1u) + 1 == gridDim.x;
   }
   __syncthreads();
   if (s_last && threadIdx.x < S && p.alive[threadIdx.x]) {
-    __threadfence_system();
+    fence_readers(S);
     st_release_sys(p.resp_ready[threadIdx.x], p.ts1);
   }
   if (s_last && threadIdx.x == 0) atomicExch(&p.done[1], 0u);
@@ -812,16 +819,15 @@ __global__ void __launch_bounds__(kThreads) k_push(const PsbPushParams p) {
   PSB_TSTAMP(3);
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence_system();                        // one per CTA (see k_pull_exchange)
+    fence_readers(S);                              // one per CTA (see k_pull_exchange)
     s_last = atomicAdd(p.done, 1u) + 1 == gridDim.x;
   }
   __syncthreads();
   if (s_last && threadIdx.x < S) {
     int s = threadIdx.x;
-    __threadfence_system();
+    fence_readers(S);
     *p.count[s] = min(s_off[s + 1] - s_off[s], p.inbox_cap);
     if (p.mode[s]) *p.mode[s] = omit_keys ? 1u : 0u;
-    __threadfence_system();
     st_release_sys(p.ready[s], p.ts1);
     if (s == 0) atomicExch(p.done, 0u);
   }
@@ -1196,7 +1202,7 @@ __global__ void __launch_bounds__(kThreads, kWide ? 4 : 3) k_apply(const PsbAppl
   __syncthreads();
   if (s_last && threadIdx.x == 0) {
     if (p.slow) atomicExch(p.slow, 0u);
-    __threadfence_system();
+    fence_readers(S);
     st_release_sys(p.applied, p.ts1);
     atomicExch(p.done, 0u);
   }
