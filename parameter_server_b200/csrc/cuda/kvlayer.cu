@@ -151,8 +151,12 @@ __global__ void __launch_bounds__(256, kLayerCtas) k_layer_apply(const LayerAppl
   for (int r = 0; r < p.S; ++r) aligned = aligned && ((((size_t)p.inbox[r]) & 15) == 0);
   const u64 n4 = aligned ? p.n / 4 : 0;
   const bool stream = p.n > kStreamElems;
-  // two groups of four per thread and trip, all their loads first; what the inbox held is not read again
-  for (u64 i = gtid; i < n4; i += 2 * gsize) {
+  // two groups of four per thread and trip, all their loads first; what the inbox held is not read again. From the back to
+  // the front: the end of the inbox is what the push wrote last and L2 still has, and the front of the segment is what the
+  // pull reads first.
+  for (u64 trip = (n4 + 2 * gsize - 1) / (2 * gsize); trip-- > 0;) {
+    const u64 i = gtid + trip * 2 * gsize;
+    if (i >= n4) continue;
     const bool two = i + gsize < n4;
     float4 s[2], d[2];
 #pragma unroll
