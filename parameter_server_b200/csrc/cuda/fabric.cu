@@ -31,6 +31,23 @@ extern "C" int psb_ipc_open(const void* handle, void** ptr) {
 extern "C" int psb_ipc_close(void* ptr) { return -(int)cudaIpcCloseMemHandle(ptr); }
 extern "C" int psb_ipc_handle_bytes(void) { return (int)sizeof(cudaIpcMemHandle_t); }
 
+// What `later` is given from now on runs behind what `earlier` has been given so far. An event of the call's own, so that
+// threads with streams of their own cannot get in each other's way; both streams belong to the current device.
+extern "C" int psb_stream_after(cudaStream_t later, cudaStream_t earlier) {
+  if (later == earlier) return 0;
+  cudaEvent_t ev;
+  cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  if (e != cudaSuccess) return -(int)e;
+  e = cudaEventRecord(ev, earlier);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(later, ev, 0);
+  const cudaError_t d = cudaEventDestroy(ev);      // (released by the runtime when the wait is over)
+  return -(int)(e != cudaSuccess ? e : d);
+}
+// One word of device memory to pinned host memory, in stream order.
+extern "C" int psb_read_word(uint32_t* host, const uint32_t* device, cudaStream_t stream) {
+  return -(int)cudaMemcpyAsync(host, device, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
+}
+
 extern "C" int psb_set_device(int dev) { return -(int)cudaSetDevice(dev); }
 extern "C" int psb_can_access_peer(int dev, int peer) {
   int ok = 0;

@@ -431,6 +431,8 @@ int psb_ipc_export(void* ptr, void* handle_out /*64 host bytes*/);
 int psb_ipc_open(const void* handle, void** ptr);
 int psb_ipc_close(void* ptr);
 int psb_ipc_handle_bytes(void);
+int psb_stream_after(cudaStream_t later, cudaStream_t earlier);
+int psb_read_word(uint32_t* host /*pinned*/, const uint32_t* device, cudaStream_t stream);
 int psb_set_device(int dev);
 int psb_can_access_peer(int dev, int peer);
 const char* psb_error_string(int neg_code);

@@ -109,16 +109,16 @@ class SparseLRWorker:
         k = self.step_no % len(self.bufs)
         b = self.bufs[k]
         dev = self.plane.device
-        cur = torch.cuda.current_stream(dev)
+        cur = torch.cuda.current_stream(self.copy_stream.device.index)
         mark = torch.cuda.nvtx.range_push if self.cfg.nvtx else (lambda name: None)
         done = torch.cuda.nvtx.range_pop if self.cfg.nvtx else (lambda: None)
         mark(f"submit {self.step_no}: copy")
         # stage 1, copy stream: host -> device into this buffer's staging area (reusable once the
         # localise that last read it has finished)
-        self.copy_stream.wait_stream(cur)
+        _lib.run_behind(self.copy_stream, cur)
         self.copy_stream.wait_event(self._prep_done[k])
         self.copy_stream.wait_event(self._buf_free[k])   # labels / row offsets / values are read until the push
-        with torch.cuda.stream(self.copy_stream):
+        with _lib.on_stream(self.copy_stream):
             def to_dev(t, name):
                 if isinstance(t, PackedIds):                # ids as a bit stream: copy the words, keep width and count
                     return t if t.is_cuda else PackedIds(to_dev(t.words, name), t.bits, t.n)
@@ -150,7 +150,7 @@ class SparseLRWorker:
         self.prep_stream.wait_event(self._buf_free[k])
         # (localize_replayed enters the stream itself)
         loc, on = (b.localize_replayed, contextlib.nullcontext()) if self.cfg.graph_localize else \
-            (b.localize, torch.cuda.stream(self.prep_stream))
+            (b.localize, _lib.on_stream(self.prep_stream))
         with on:
             loc(ids_d, y_d, self.plane.bounds, fixed_z=fixed_z, row_ptr=rp_d, vals=vals_d,
                 hash_seed=self.cfg.hash_seed, key_bits=self.cfg.key_bits, hash_bits=self.cfg.hash_bits,
@@ -188,11 +188,9 @@ class SparseLRWorker:
 
     def wait(self):
         """Make the current stream wait for everything submitted so far."""
-        cur = torch.cuda.current_stream(self.plane.device)
-        cur.wait_stream(self.main_stream)
-        cur.wait_stream(self.server_stream)
-        cur.wait_stream(self.prep_stream)
-        cur.wait_stream(self.copy_stream)
+        cur = torch.cuda.current_stream(self.copy_stream.device.index)
+        for stream in (self.main_stream, self.server_stream, self.prep_stream, self.copy_stream):
+            _lib.run_behind(cur, stream)
 
     def read_progress(self, reset: bool = True):
         """Device -> host read of the progress counters: dict with the summed

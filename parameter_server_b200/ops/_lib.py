@@ -176,6 +176,8 @@ def _declare(lib):
                                          _vp, _vp]
     lib.psb_localize2_gated.argtypes = [_vp, _vp, _vp, _vp, _vp, _vp, _u32, _vp, _u32, _u32, _vp, _vp, _i32, _vp, _vp, _vp,
                                         _vp, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _vp, _vp]
+    lib.psb_stream_after.argtypes = [_vp, _vp]
+    lib.psb_read_word.argtypes = [_vp, _vp, _vp]
     lib.psb_bucket_localize_scratch_bytes.restype = sz
     lib.psb_bucket_localize_scratch_bytes.argtypes = [_u32]
     lib.psb_bucket_localize.argtypes = [_vp, _i32, _u64, _u32, _i32, _vp, _u32, _u32, _vp, _vp, _i32, _vp, _vp, _vp,
@@ -286,6 +288,43 @@ def stream_ptr(stream=None) -> int:
     if stream is None:
         stream = torch.cuda.current_stream()
     return stream.cuda_stream
+
+
+class on_stream:
+    """``with torch.cuda.stream(stream)`` for the calls of a training step or a request: where ``stream`` is on the current
+    device, as it is in a process per GPU, without the look-ups of devices that cost it most of its time. ``None``:
+    nothing changes."""
+    __slots__ = ("stream", "before", "general")
+
+    def __init__(self, stream):
+        self.stream = stream
+
+    def __enter__(self):
+        self.before = self.general = None
+        if self.stream is None:
+            return
+        index = self.stream.device.index
+        if torch.cuda.current_device() != index:
+            self.general = torch.cuda.stream(self.stream)
+            self.general.__enter__()
+            return
+        self.before = torch.cuda.current_stream(index)
+        torch.cuda.set_stream(self.stream)
+
+    def __exit__(self, *error):
+        if self.general is not None:
+            self.general.__exit__(*error)
+        elif self.before is not None:
+            torch.cuda.set_stream(self.before)
+
+
+def run_behind(later, earlier):
+    """What ``later`` is given from now on runs behind what ``earlier`` has been given so far (``later.wait_stream(earlier)``
+    in one call into the library)."""
+    if torch.cuda.current_device() != earlier.device.index:
+        later.wait_stream(earlier)                     # (the library's event belongs to the current device)
+        return
+    check(lib().psb_stream_after(later.cuda_stream, earlier.cuda_stream), "stream order", kernels=0)
 
 
 def check_status(status: torch.Tensor, what: str = "", reset=()):

@@ -208,7 +208,7 @@ class LocalBatch:
                 for k in [k for k, v in graphs.items() if v == "seen"]:
                     del graphs[k]
             graphs[key] = "seen"
-            with torch.cuda.stream(stream):
+            with _lib.on_stream(stream):
                 return self.localize(ids, y, bounds, row_ptr=row_ptr, vals=vals, stream=stream, **kw)
         if ent == "seen":
             g = torch.cuda.CUDAGraph()
@@ -223,7 +223,7 @@ class LocalBatch:
         g, state, kernels, _ = ent
         for a, v in state.items():
             setattr(self, a, v)
-        with torch.cuda.stream(stream):
+        with _lib.on_stream(stream):
             g.replay()
         _lib.LAUNCHES += kernels
         return self

@@ -36,6 +36,7 @@ from typing import Callable, Dict, List, Optional
 import numpy as np
 import torch
 
+from ..ops import _lib
 from ..ops.localize import LocalBatch
 from ..parallel.dataplane import DataPlane, OptimizerConfig, PlaneConfig, heap_layout
 from ..parallel.fabric import Fabric
@@ -61,6 +62,11 @@ class DeviceKVMap:
                 b.grad = torch.zeros(max_keys * self.k, dtype=torch.float32, device=self.dev)
         self._next_buf = 0
         self.stream = torch.cuda.Stream(device=self.dev)
+        # The plane's status word as a pull leaves it, copied behind the pull: its wait() then needs no blocking transfer of
+        # its own.
+        self._status_host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        self._status_seen = self._status_host.numpy()
+        self._status_read: set = set()                # timestamps of the requests behind which it was copied
 
     @classmethod
     def create(cls, fabric_or_none=None, *, table_capacity: int = 1 << 20, max_keys: int = 1 << 18,
@@ -89,7 +95,7 @@ class DeviceKVMap:
         return ts
 
     def _begin(self, wait: Optional[List[int]]):
-        self.stream.wait_stream(torch.cuda.current_stream(self.dev))
+        _lib.run_behind(self.stream, torch.cuda.current_stream(self.stream.device.index))
         for t in wait or []:
             ev = self._events.get(t)
             if ev is not None:
@@ -111,9 +117,14 @@ class DeviceKVMap:
         b = self._bufs[self._next_buf]
         self._next_buf = (self._next_buf + 1) % len(self._bufs)
         keys.record_stream(self.stream)               # read on this stream: its memory stays until then
-        b.set_keys(keys, self.plane.bounds)
+        b.set_keys(keys, self.plane.bounds, stream=self.stream)
         self._last_keys_tag, self._last_buf, self._last_keys = tag, b, keys      # (keeps the tensor, and so its id, alive)
         return b
+
+    def _in_place(self, values) -> bool:
+        """Whether the push kernel, which reads adjacent floats from one address, can read ``values`` where it is."""
+        return (isinstance(values, torch.Tensor) and values.is_cuda and values.dtype == torch.float32
+                and values.is_contiguous() and not values.is_neg() and values.device == self.stream.device)
 
     @staticmethod
     def _as_keys(keys, dev) -> torch.Tensor:
@@ -133,7 +144,9 @@ class DeviceKVMap:
         ts = self._stamp(ts)
         self._begin(wait)
         k = self._as_keys(keys, self.dev)
-        with torch.cuda.stream(self.stream):
+        # conversions run on the container's stream; without any the stream need not be entered
+        ready = self._in_place(values) and k.dtype == torch.int64 and k.is_contiguous() and k.device == values.device
+        with _lib.on_stream(None if ready else self.stream):
             rnd = self._push_round_of[ts] = self._push_half(k, values)
             self._apply_half(rnd, channel)
         self._finish(ts, callback)
@@ -153,7 +166,8 @@ class DeviceKVMap:
             return self._push_half(k, values)
 
     def _push_half(self, k: torch.Tensor, values) -> int:
-        """The worker half of a round on the current stream, which is this container's."""
+        """The worker half of a round, on this container's stream (which is the current one where ``values`` or ``k`` are
+        still to be converted)."""
         b = self._buffer(k)
         n = k.numel()
         v = None
@@ -162,7 +176,8 @@ class DeviceKVMap:
                 values.record_stream(self.stream)     # read on this stream: its memory stays until then
             # the kernel reads n * k adjacent floats: a column, a step slice or an expanded tensor (which flatten()
             # returns as the strided view that it is) is copied first
-            v = torch.as_tensor(values, dtype=torch.float32).to(self.dev).flatten().contiguous().resolve_neg()
+            v = values if self._in_place(values) else \
+                torch.as_tensor(values, dtype=torch.float32).to(self.dev).flatten().contiguous().resolve_neg()
             assert v.numel() == n * self.k, f"{n} keys of width {self.k} need {n * self.k} values"
         rnd = self._round
         self._round += 1
@@ -211,7 +226,7 @@ class DeviceKVMap:
         ts = self._stamp(ts)
         k = self._as_keys(keys, self.dev)
         self._begin(wait)
-        with torch.cuda.stream(self.stream):
+        with _lib.on_stream(self.stream):
             b = self._buffer(k)
             # the owners must have applied every round pushed so far
             if self.plane.cfg.pull_cap:
@@ -226,6 +241,9 @@ class DeviceKVMap:
             else:
                 self.plane.pull_margin(b, need_applied=self._round, with_margins=False, stream=self.stream)
                 self._results[ts] = b.w_local[:k.numel()].clone()
+        _lib.check(_lib.lib().psb_read_word(self._status_host.data_ptr(), self.plane.status.data_ptr(), self.stream.cuda_stream),
+                   "status", kernels=0)
+        self._status_read.add(ts)
         self._finish(ts, callback)
         return ts
 
@@ -233,7 +251,12 @@ class DeviceKVMap:
         ev = self._events.pop(ts, None)
         if ev is not None:
             ev.synchronize()
-        self.plane.check_status("kv")
+        if ev is None or ts not in self._status_read or self._status_seen[0] != 0:
+            try:
+                self.plane.check_status("kv")
+            finally:
+                self._status_seen[0] = 0
+        self._status_read.discard(ts)
         cb = self._callbacks.pop(ts, None)
         if cb is not None:
             cb()
@@ -246,6 +269,7 @@ class DeviceKVMap:
         self._events.pop(ts, None)
         self._callbacks.pop(ts, None)
         self._results.pop(ts, None)
+        self._status_read.discard(ts)
 
     def write_to_file(self, path: str):
         """``key<TAB>value`` per non-zero entry of this shard."""

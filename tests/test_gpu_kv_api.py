@@ -253,3 +253,45 @@ def test_memory_of_a_key_list_is_not_reused_before_it_is_read(cuda_lib):
         got = kv.pull(keys)
         kv.wait(got)
         assert (kv.result(got) == i + 1.0).all(), i
+
+
+def test_wait_reports_the_status_that_a_pull_left(cuda_lib):
+    """The status word travels with the pull; an error in it is raised once and cleared, as when wait() reads the word itself."""
+    from parameter_server_b200.ops._lib import PsbCudaError
+    from parameter_server_b200.parameter.kv import DeviceKVVector
+    kv = DeviceKVVector.create(table_capacity=1 << 12, max_keys=1 << 10)
+    keys = torch.arange(1, 6, dtype=torch.int64, device="cuda")
+    pushed = kv.push(keys, torch.ones(5, device="cuda"))
+    kv.plane.status.fill_(1)
+    first, second = kv.pull(keys), kv.pull(keys, wait=[pushed])
+    with pytest.raises(PsbCudaError):
+        kv.wait(first)
+    kv.wait(second)
+    kv.wait(pushed)
+    assert kv.result(second).tolist() == [1.0] * 5
+    kv.plane.status.fill_(1)
+    again = kv.push(keys, torch.ones(5, device="cuda"))
+    with pytest.raises(PsbCudaError):
+        kv.wait(again)                                 # (behind a push the word is read by wait())
+
+
+def test_on_stream_is_left_as_it_was_entered(cuda_lib):
+    from parameter_server_b200.ops._lib import on_stream, run_behind
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    before = torch.cuda.current_stream()
+    with on_stream(a):
+        assert torch.cuda.current_stream() == a
+        with pytest.raises(ZeroDivisionError), on_stream(b):
+            assert torch.cuda.current_stream() == b
+            1 / 0
+        assert torch.cuda.current_stream() == a
+        with on_stream(None):
+            assert torch.cuda.current_stream() == a
+    assert torch.cuda.current_stream() == before
+    x = torch.zeros(1 << 24, device="cuda")
+    run_behind(a, before)
+    with on_stream(a):
+        for _ in range(50):
+            x += 1
+    run_behind(before, a)
+    assert float(x.sum()) == 50.0 * x.numel()
