@@ -137,7 +137,8 @@ struct BLP {
 
 // The steps are launched with programmatic stream serialisation: a step's CTAs come in while the step before it drains, and
 // wait here, before they read anything, until it has ended and its stores are visible (so all the steps before it
-// have, too). The next step may come in from here on.
+// have, too). The next step may come in from here on. Launched one by one, 64,000 nonzeros take 53 us instead of 70 and
+// 3.9 M 202 instead of 216; replayed from a graph, 49 and 50, 197 and 194.
 __device__ __forceinline__ void behind_the_step_before() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -184,7 +185,8 @@ __global__ void __launch_bounds__(256) k_bl_clear(const BLP p, uint4* zero, u32 
   for (u32 i = gtid; i < flag_words; i += gsize) p.flagbits[i] = 0;
   if (p.row_ptr != nullptr) {
     // Row hints for steps 4 and 6, up to the block behind the last position: every row writes those of the blocks that
-    // start in it, a long one with its whole warp. (A search per hint waited for log2(rows) dependent loads.)
+    // start in it, a long one with its whole warp. (3.9 M nonzeros in 100,000 rows: this kernel 3.2 us; 9.4 with a search
+    // of log2(rows) dependent loads per hint.)
     const u32 lane = threadIdx.x & 31;
     for (u32 r0 = gtid - lane; r0 < p.n_rows; r0 += gsize) {
       const u32 r = r0 + lane;
@@ -207,43 +209,26 @@ __global__ void __launch_bounds__(256) k_bl_clear(const BLP p, uint4* zero, u32 
 }
 
 // ---------------------------------------------------------------- 1. sample
-// A CTA counts its share of the sample in shared memory first: added one by one, the most frequent keys would each
-// take thousands of atomics on one address.
-static constexpr int kSampThreads = 1024;
-static constexpr u32 kSampLocal = 2 * kSampThreads;
-__global__ void __launch_bounds__(kSampThreads) k_bl_sample(const BLP p) {
+// (Counted in shared memory per CTA first, it takes as long: 65,536 elements 9 us like this, 10 that way; 16,384 5 and 6.)
+__global__ void __launch_bounds__(256) k_bl_sample(const BLP p) {
   behind_the_step_before();
-  __shared__ u64 s_key[kSampLocal];
-  __shared__ u32 s_cnt[kSampLocal];
-  const u32 t = threadIdx.x, j = blockIdx.x * kSampThreads + t;
+  const u32 j = blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = j < p.samp_m;
   const u64 key = valid ? bl_key_of(p, j * p.samp_stride) : kEmptyKey;
-  for (u32 i = t; i < kSampLocal; i += kSampThreads) { s_key[i] = kEmptyKey; s_cnt[i] = 0; }
-  __syncthreads();
-  if (valid) {
-    u32 slot = (u32)(fmix64(key) & (kSampLocal - 1));
-    for (u32 probe = 0; probe < kSampLocal; ++probe) {
-      const u64 old = atomicCAS(&s_key[slot], kEmptyKey, key);
-      if (old == kEmptyKey || old == key) { atomicAdd(&s_cnt[slot], 1u); break; }
-      slot = (slot + 1) & (kSampLocal - 1);
-    }
-  }
-  __syncthreads();
-  for (u32 i = t; i < kSampLocal; i += kSampThreads) {
-    const u32 c = s_cnt[i];
-    if (c == 0) continue;
-    const u64 k = s_key[i];
-    u32 slot = (u32)(fmix64(k) & (p.samp_slots - 1));
-    for (u32 probe = 0; probe < p.samp_slots; ++probe) {
-      const u64 old = atomicCAS(&p.samp_key[slot], kEmptyKey, k);
-      if (old == kEmptyKey || old == k) { atomicAdd(&p.samp_cnt[slot], c); break; }
-      slot = (slot + 1) & (p.samp_slots - 1);
-    }
+  // equal keys of a warp count once (the most frequent key would otherwise take thousands of
+  // atomics on one address)
+  const u32 m = __match_any_sync(0xffffffffu, key);
+  if (!valid || (int)(threadIdx.x & 31) != __ffs(m) - 1) return;
+  u32 slot = (u32)(fmix64(key) & (p.samp_slots - 1));
+  for (u32 probe = 0; probe < p.samp_slots; ++probe) {
+    u64 old = atomicCAS(&p.samp_key[slot], kEmptyKey, key);
+    if (old == kEmptyKey || old == key) { atomicAdd(&p.samp_cnt[slot], (u32)__popc(m)); return; }
+    slot = (slot + 1) & (p.samp_slots - 1);
   }
 }
 
-// Keys counted often enough become hot. One atomic per CTA on each of the two counters: with one per warp and per key they
-// queue up on the two addresses.
+// Keys counted often enough become hot. One atomic per CTA on each of the two counters (131,072 places: 4.1 us; 7.1 with one
+// per warp and per key, which queue up on the two addresses).
 static constexpr int kHotThreads = 1024;
 __global__ void __launch_bounds__(kHotThreads) k_bl_hot(const BLP p) {
   behind_the_step_before();
@@ -1183,7 +1168,7 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   const u32 zero4 = (u32)((L.zero_end - L.zero_begin) / 16), ones4 = (u32)((L.ff_end - L.ff_begin) / 16);
   k_bl_clear<<<psb_device_sm_count() * 2, 256, 0, stream>>>(p, (uint4*)(sc + L.zero_begin), zero4, (uint4*)(sc + L.ff_begin),
                                                             ones4, (n + 31) / 32);
-  launch_step(k_bl_sample, (p.samp_m + kSampThreads - 1) / kSampThreads, kSampThreads, 0, stream, p);
+  launch_step(k_bl_sample, (p.samp_m + 255) / 256, 256, 0, stream, p);
   launch_step(k_bl_hot, (p.samp_slots + kHotThreads - 1) / kHotThreads, kHotThreads, 0, stream, p);
   const size_t count_smem = kHotSlots * 4 + kHotMax * 8 + (size_t)p.NBINS * 4;
   const size_t scatter_smem = (size_t)p.NB * 4, finish_smem = (size_t)(2 * p.NB + 4 + 2 * kHotMax) * 4;
