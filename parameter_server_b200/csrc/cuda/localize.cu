@@ -207,14 +207,9 @@ __device__ __forceinline__ void owner_offsets(const u64* ukeys, u32 U, const u64
     if (lane == 0) own_off[s] = lo;
   }
 }
-// Runs only while *skip_when_set is zero (null: always); *gate_out (nullable) receives that word.
 __global__ void __launch_bounds__(256) k_owner_offsets(const u64* __restrict__ ukeys, const u32* __restrict__ n_unique,
                                                        const u64* __restrict__ bounds, int S, u32 n,
-                                                       u32* __restrict__ seg_off, u32* __restrict__ own_off,
-                                                       const u32* __restrict__ skip_when_set, u32* __restrict__ gate_out) {
-  const u32 skip = skip_when_set ? *skip_when_set : 0u;
-  if (gate_out && threadIdx.x == 0) *gate_out = skip;
-  if (skip) return;
+                                                       u32* __restrict__ seg_off, u32* __restrict__ own_off) {
   owner_offsets(ukeys, *n_unique, bounds, S, n, seg_off, own_off);
 }
 
@@ -273,7 +268,7 @@ using namespace psb;
 extern "C" int psb_owner_offsets(const psb_u64* ukeys, const uint32_t* n_unique, const psb_u64* bounds, int S,
                                  uint32_t* own_off, cudaStream_t stream) {
   if (S < 1 || S > 64) return -(int)cudaErrorInvalidValue;
-  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, 0, nullptr, own_off, nullptr, nullptr);
+  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, 0, nullptr, own_off);
   return -(int)cudaGetLastError();
 }
 
@@ -335,7 +330,7 @@ static int localize2_impl(const psb_u64* keys_a, const psb_u64* keys_b, const ui
   k_uniq_emit<<<ntiles, kLocThreads, 0, stream>>>((const u64*)keys_a, (const u64*)keys_b, pos_a, pos_b, where, csc_row,
                                                   n, tile_heads, row_ptr, n_rows, fixed_z, vals, (u64*)ukeys, seg_off,
                                                   csr_col, csc_val, flagbits, wordbase, kmask);
-  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off, own_off, nullptr, nullptr);
+  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off, own_off);
   return -(int)cudaGetLastError();
 }
 
@@ -365,17 +360,6 @@ extern "C" int psb_localize2_gated(const psb_u64* keys_a, const psb_u64* keys_b,
                         pack_pos_bits, gate, status, stream);
 }
 
-// Owner offsets plus the closing CSC offset seg_off[U] = n; runs only while *skip_when_set is zero, and copies
-// that word to *gate_out (the bucket-based localisation's last step).
-extern "C" int psb_owner_offsets_n(const psb_u64* ukeys, const uint32_t* n_unique, const psb_u64* bounds, int S,
-                                   uint32_t n, uint32_t* seg_off, uint32_t* own_off,
-                                   const uint32_t* skip_when_set, uint32_t* gate_out, cudaStream_t stream) {
-  if (S < 1 || S > 64) return -(int)cudaErrorInvalidValue;
-  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off, own_off,
-                                         skip_when_set, gate_out);
-  return -(int)cudaGetLastError();
-}
-
 // Sorted pairs in one buffer; sorted_pos is rewritten in place with the CSC row index.
 extern "C" int psb_localize(const psb_u64* sorted_keys, uint32_t* sorted_pos, uint32_t n,
                             const uint32_t* row_ptr, uint32_t n_rows, uint32_t fixed_z,
@@ -398,7 +382,7 @@ extern "C" int psb_localize(const psb_u64* sorted_keys, uint32_t* sorted_pos, ui
   k_uniq_emit<<<ntiles, kLocThreads, 0, stream>>>((const u64*)sorted_keys, nullptr, sorted_pos, nullptr, nullptr,
                                                   sorted_pos, n, tile_heads, row_ptr, n_rows, fixed_z, vals,
                                                   (u64*)ukeys, seg_off, csr_col, csc_val, flagbits, wordbase, ~0ull);
-  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off, own_off, nullptr, nullptr);
+  k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off, own_off);
   return -(int)cudaGetLastError();
 }
 
@@ -464,6 +448,6 @@ extern "C" int psb_localize_static(const psb_u64* sorted_keys, uint32_t* sorted_
                                                   sorted_pos, n, tile_heads, row_ptr, n_rows, fixed_z, vals,
                                                   (u64*)ukeys, seg_off, csr_col, csc_val, flagbits, wordbase, ~0ull);
   k_owner_offsets<<<1, 256, 0, stream>>>((const u64*)ukeys, n_unique, (const u64*)bounds, S, n, seg_off,
-                                         own_off, nullptr, nullptr);
+                                         own_off);
   return -(int)cudaGetLastError();
 }

@@ -44,9 +44,6 @@ int psb_localize2_gated(const psb_u64* keys_a, const psb_u64* keys_b, const uint
 // Copies a sorted unique key list and sets its length and owner offsets (one launch).
 int psb_set_keys(const psb_u64* keys, uint32_t n, psb_u64* ukeys, uint32_t* n_unique, const psb_u64* bounds, int S,
                  uint32_t* own_off, cudaStream_t stream);
-int psb_owner_offsets_n(const psb_u64* ukeys, const uint32_t* n_unique, const psb_u64* bounds, int S, uint32_t n,
-                        uint32_t* seg_off, uint32_t* own_off, const uint32_t* skip_when_set, uint32_t* gate_out,
-                        cudaStream_t stream);
 // Bucket-based localisation (bucket_localize.cu): groups the nonzeros by key without a full sort.
 size_t psb_bucket_localize_scratch_bytes(uint32_t max_n);
 int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, uint32_t n, int low_zero_bits,
