@@ -48,6 +48,9 @@ static constexpr int kGradGroup = 4;
 // by side (k_darlin_pass). index: this CTA's place among them.
 struct Part { u32 index, count; };
 __device__ __forceinline__ Part whole_grid() { return Part{blockIdx.x, gridDim.x}; }
+// Words of 32 nonzeros per CTA of k_darlin_pass_alone: each takes an adjacent part of the block.
+static constexpr u32 kAloneWarps = 32;
+__device__ __forceinline__ u32 part_words(u32 words) { return (words + gridDim.x - 1) / gridDim.x; }
 // kAlone (k_darlin_pass_alone): label and margin of a row are one pair in row_state (one gather instead of
 // two) and the staging area holds (G, U) pairs (one vector atomic per column piece instead of two).
 template <bool kAlone>
@@ -65,6 +68,10 @@ __device__ void darlin_grad_p1(const PsbDarlinGrad& p, const float2* row_state =
   const u32 rounds = max(1u, (w1 - w0) / (16 * nwarps));
   const u32 kChunkWords = max(1u, (w1 - w0 + rounds * nwarps - 1) / (rounds * nwarps));
   const u32 nchunks = (w1 - w0 + kChunkWords - 1) / kChunkWords;
+  // kAlone: the chunks of a CTA are adjacent (see part_words), so that the margin pass finds its nonzeros in this SM's L1
+  const u32 part = kAlone ? part_words(w1 - w0) : 0u;
+  const u32 part0 = w0 + blockIdx.x * part, part1 = min(w1, part0 + part);
+  const u32 part_rounds = max(1u, part / (16 * kAloneWarps)), part_chunk = max(1u, (part + part_rounds * kAloneWarps - 1) / (part_rounds * kAloneWarps));
   auto flush = [&](u32 col, float gg, float hh) {
     const u32 c = col - p.c0;
     if (kAlone) {
@@ -75,8 +82,9 @@ __device__ void darlin_grad_p1(const PsbDarlinGrad& p, const float2* row_state =
       atomicAdd(&p.stage[p.block_cap + c], hh);
     }
   };
-  for (u32 ch = gwarp; ch < nchunks; ch += nwarps) {
-    const u32 wb = w0 + ch * kChunkWords, we = min(w1, wb + kChunkWords);
+  for (u32 ch = kAlone ? threadIdx.x >> 5 : gwarp;; ch += kAlone ? kAloneWarps : nwarps) {
+    const u32 wb = kAlone ? part0 + ch * part_chunk : w0 + ch * kChunkWords, we = min(kAlone ? part1 : w1, wb + (kAlone ? part_chunk : kChunkWords));
+    if (kAlone ? wb >= part1 : ch >= nchunks) break;
     float cg = 0.f, chh = 0.f;   // sums so far of the column that is open at the word boundary
     u32 ccol = 0;                // that column
     bool open = false;
@@ -92,13 +100,13 @@ __device__ void darlin_grad_p1(const PsbDarlinGrad& p, const float2* row_state =
         const u32 i = wi * 32 + lane;
         in[k] = valid && i >= nz0 && i < nz1;
         if (p.csc_col != nullptr) {
-          col[k] = in[k] ? p.csc_col[i] : 0u;                         // the column of every nonzero is at hand
+          col[k] = in[k] ? __ldg(&p.csc_col[i]) : 0u;                 // the column of every nonzero is at hand
         } else {
           const u32 base = valid ? p.wordbase[wi] : 0u;
           col[k] = in[k] ? p.gcol[base + __popc(f[k] & le) - 1] : 0u;   // local unique key -> global column
         }
-        row[k] = in[k] ? p.csc_row[i] : 0u;
-        val[k] = (in[k] && p.csc_val) ? p.csc_val[i] : 1.f;
+        row[k] = in[k] ? __ldg(&p.csc_row[i]) : 0u;
+        val[k] = (in[k] && p.csc_val) ? __ldg(&p.csc_val[i]) : 1.f;
       }
 #pragma unroll
       for (int k = 0; k < kGradGroup; ++k) {
@@ -384,13 +392,16 @@ static constexpr int kPassThreads = 1024;
 
 // Grid barrier number `n` (1, 2, ...) of a launch on a word that was zero at its start: one fire-and-forget
 // arrival, then polls until everybody's has landed. Against grid_barrier it saves the sense load and the
-// release by the last to arrive: one trip to L2 instead of three. Bounded like grid_barrier.
-__device__ __forceinline__ bool pass_barrier(u32* word, u32 n, u32* status) {
-  __shared__ u32 s_ok;
+// release by the last to arrive: one trip to L2 instead of three. Bounded like grid_barrier. Between the two halves a
+// CTA does what nobody waits for at this barrier.
+__device__ __forceinline__ void pass_arrive(u32* word) {
   __syncthreads();
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
+}
+__device__ __forceinline__ bool pass_wait(u32* word, u32 n, u32* status) {
+  __shared__ u32 s_ok;
   if (threadIdx.x == 0) {
     const u32 target = n * gridDim.x;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
     u32 ok = 1;
     for (u32 it = 0; ld_acquire_gpu(word) < target;) {
       if (++it > kGridWaitIters) { ok = 0; set_status(status, kBarrierTimeout); break; }
@@ -400,6 +411,10 @@ __device__ __forceinline__ bool pass_barrier(u32* word, u32 n, u32* status) {
   }
   __syncthreads();
   return s_ok != 0;
+}
+__device__ __forceinline__ bool pass_barrier(u32* word, u32 n, u32* status) {
+  pass_arrive(word);
+  return pass_wait(word, n, status);
 }
 
 // Newton step of one column of a rank that is alone (darlin_update_body), from its gradient sums and state.
@@ -465,27 +480,26 @@ __device__ void darlin_columns_alone(const PsbDarlinGrad& g, const PsbDarlinUpda
 // barrier it would need in front of this one, are off the path from one block's gradient to the next.
 __device__ void darlin_margins_alone(const PsbDarlinGrad& g, const PsbDarlinUpdate& p, const PsbDarlinDual& d, float2* row_state) {
   if (d.u1 <= d.u0) return;
-  const u32 gsize = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
-  const u32 gwarp = gtid >> 5, nwarps = gsize >> 5;
   const u32 nz0 = d.nz0, nz1 = d.nz1;
   const u32 w0 = nz0 >> 5, w1 = (nz1 + 31) >> 5;
   const u32 le = 0xffffffffu >> (31 - lane);
   const float2* stage = reinterpret_cast<const float2*>(g.stage);
   constexpr int kGroup = 4;                 // words whose gathers are in flight together
-  for (u32 wa = w0 + gwarp; wa < w1; wa += nwarps * kGroup) {
+  const u32 part = part_words(w1 - w0), part0 = w0 + blockIdx.x * part, part1 = min(w1, part0 + part);
+  for (u32 wa = part0 + (threadIdx.x >> 5); wa < part1; wa += kAloneWarps * kGroup) {
     u32 col[kGroup], row[kGroup];
     float x[kGroup];
     bool in[kGroup];
 #pragma unroll
     for (int k = 0; k < kGroup; ++k) {
-      const u32 wi = wa + k * nwarps;
+      const u32 wi = wa + k * kAloneWarps;
       const u32 i = wi * 32 + lane;
-      in[k] = wi < w1 && i >= nz0 && i < nz1;
-      if (d.csc_col != nullptr) col[k] = in[k] ? d.csc_col[i] : 0u;
+      in[k] = wi < part1 && i >= nz0 && i < nz1;
+      if (d.csc_col != nullptr) col[k] = in[k] ? __ldg(&d.csc_col[i]) : 0u;
       else col[k] = in[k] ? d.gcol[d.wordbase[wi] + __popc(d.flagbits[wi] & le) - 1] : 0u;
-      row[k] = in[k] ? d.csc_row[i] : 0u;
-      x[k] = (in[k] && d.csc_val) ? d.csc_val[i] : 1.f;
+      row[k] = in[k] ? __ldg(&d.csc_row[i]) : 0u;
+      x[k] = (in[k] && d.csc_val) ? __ldg(&d.csc_val[i]) : 1.f;
     }
 #pragma unroll
     for (int k = 0; k < kGroup; ++k) {
@@ -502,16 +516,28 @@ __device__ void darlin_margins_alone(const PsbDarlinGrad& g, const PsbDarlinUpda
   }
 }
 
+// The lines of an array's elements [b, e) on their way to L2.
+template <typename T>
+__device__ __forceinline__ void prefetch_range(const T* a, u32 b, u32 e) {
+  constexpr u32 kPer = 128 / sizeof(T);
+  for (u32 i = b + kPer * (blockIdx.x * kPassThreads + threadIdx.x); i < e; i += kPer * gridDim.x * kPassThreads)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(a + i));
+}
+
 // A pass of a rank that is alone (S == 1) and owns every column, without delay. Worker and owner are the same GPU: no slices are
 // exchanged and no flags raised, and a block is two phases with a light barrier behind each:
 //
-//   gradient sums of block i, and beside them the column state of block i - 1 (other columns, other staging area)
+//   gradient sums of block i
 //   margins of block i, every nonzero with its column's step worked out on the spot
 //
-// The general path below needs five grid-wide synchronisations per block, two of them through system-scope
-// flags, and gathers label and margin apart: 1.25 M rows, 125 M nonzeros, 256 blocks take 8.4 ms there, 4.33 ms
-// with a barrier between every two of gradient, columns and margins, 3.90 ms here (4.16 with the row pairs gathered
-// past L1: a frequent column's rows stand close together, and nothing writes them during a gradient phase).
+// Between arriving at a barrier and waiting for it a CTA sees to what is not on that path: the column state of block
+// i - 1 (other columns, other staging area), and the state of block i + 1's columns on its way to L2, of which a block
+// reads 1.2 MB that were last touched a pass ago. The general path below needs five grid-wide synchronisations per block,
+// two of them through system-scope flags, and gathers label and margin apart. 1.25 M rows, 125 M nonzeros, 256 blocks:
+// 8.4 ms there, 3.91 ms here without the prefetch, 3.70 with it, 3.61 with a CTA's nonzeros adjacent and the same
+// in both phases. Bound by latency: a block of 0.3 M nonzeros is 14 us, two phases of dependent gathers (3 us on average,
+// 5 for the slowest CTA) and two barriers of 1.2 us. (Not faster: the next block's nonzeros in shared memory beforehand,
+// 5.4 ms, since the row gathers then lack L1; in L2 beforehand.)
 __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const PsbDarlinPass q) {
   __shared__ PsbDarlinGrad s_g[2];                 // by step parity
   __shared__ PsbDarlinUpdate s_u[2];
@@ -523,9 +549,10 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const Psb
   static_assert(WG + WU + WD <= kPassThreads, "one word of the three parameter blocks per thread");
   float2* rows = reinterpret_cast<float2*>(q.row_state);
   const u32 gsize = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x, t = threadIdx.x;
+  auto place = [&](u32 i) -> size_t { return (size_t)q.order[i] * R + (q.ts_base + i) % R; };
   auto fetch = [&](u32 i) -> u32 {                 // this thread's word of step i's three parameter blocks
     if (i >= n) return 0u;
-    const size_t at = (size_t)q.order[i] * R + (q.ts_base + i) % R;
+    const size_t at = place(i);
     if (t < WG) return reinterpret_cast<const u32*>(&q.grad[at])[t];
     if (t < WG + WU) return reinterpret_cast<const u32*>(&q.update[at])[t - WG];
     if (t < WG + WU + WD) return reinterpret_cast<const u32*>(&q.dual[at])[t - WG - WU];
@@ -547,17 +574,34 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const Psb
   if (!pass_barrier(q.steps, ++bars, q.status)) return;
   for (u32 i = 0; i < n; ++i) {
     const u32 k = i & 1;
+    bool columns_left = i > 0;
     if (i > 0) {
       keep(i, word);                               // (the blocks of step i - 2: nobody reads them any more)
-      darlin_columns_alone(s_g[k ^ 1], s_u[k ^ 1], s_d[k ^ 1], vio_max);
       // a block that comes twice in a row, or shares columns with the one before it, needs their new state
-      if (s_g[k].c0 < s_g[k ^ 1].c1 && s_g[k ^ 1].c0 < s_g[k].c1 && !pass_barrier(q.steps, ++bars, q.status)) return;
+      if (s_g[k].c0 < s_g[k ^ 1].c1 && s_g[k ^ 1].c0 < s_g[k].c1) {
+        darlin_columns_alone(s_g[k ^ 1], s_u[k ^ 1], s_d[k ^ 1], vio_max);
+        columns_left = false;
+        if (!pass_barrier(q.steps, ++bars, q.status)) return;
+      }
     }
     darlin_grad_p1<true>(s_g[k], rows);
-    if (!pass_barrier(q.steps, ++bars, q.status)) return;
+    pass_arrive(q.steps);
+    if (columns_left) darlin_columns_alone(s_g[k ^ 1], s_u[k ^ 1], s_d[k ^ 1], vio_max);
+    if (!pass_wait(q.steps, ++bars, q.status)) return;
     word = fetch(i + 1);
     darlin_margins_alone(s_g[k], s_u[k], s_d[k], rows);
-    if (!pass_barrier(q.steps, ++bars, q.status)) return;
+    pass_arrive(q.steps);
+    if (i + 1 < n) {
+      const PsbDarlinGrad& next = q.grad[place(i + 1)];
+      const u32 c0 = next.c0, c1 = next.c1;
+      prefetch_range(s_g[k].delta, c0, c1);
+      prefetch_range(s_g[k].active, c0, c1);
+      prefetch_range(s_u[k].delta, c0, c1);
+      prefetch_range(s_u[k].w, c0, c1);
+      prefetch_range(s_d[k].w_cur, c0, c1);
+      prefetch_range(s_u[k].active, c0, c1);
+    }
+    if (!pass_wait(q.steps, ++bars, q.status)) return;
   }
   const u32 k = (n - 1) & 1;
   darlin_columns_alone(s_g[k], s_u[k], s_d[k], vio_max);
