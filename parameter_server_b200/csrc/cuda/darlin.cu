@@ -392,16 +392,13 @@ static constexpr int kPassThreads = 1024;
 
 // Grid barrier number `n` (1, 2, ...) of a launch on a word that was zero at its start: one fire-and-forget
 // arrival, then polls until everybody's has landed. Against grid_barrier it saves the sense load and the
-// release by the last to arrive: one trip to L2 instead of three. Bounded like grid_barrier. Between the two halves a
-// CTA does what nobody waits for at this barrier.
-__device__ __forceinline__ void pass_arrive(u32* word) {
-  __syncthreads();
-  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
-}
-__device__ __forceinline__ bool pass_wait(u32* word, u32 n, u32* status) {
+// release by the last to arrive: one trip to L2 instead of three. Bounded like grid_barrier.
+__device__ __forceinline__ bool pass_barrier(u32* word, u32 n, u32* status) {
   __shared__ u32 s_ok;
+  __syncthreads();
   if (threadIdx.x == 0) {
     const u32 target = n * gridDim.x;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
     u32 ok = 1;
     for (u32 it = 0; ld_acquire_gpu(word) < target;) {
       if (++it > kGridWaitIters) { ok = 0; set_status(status, kBarrierTimeout); break; }
@@ -411,10 +408,6 @@ __device__ __forceinline__ bool pass_wait(u32* word, u32 n, u32* status) {
   }
   __syncthreads();
   return s_ok != 0;
-}
-__device__ __forceinline__ bool pass_barrier(u32* word, u32 n, u32* status) {
-  pass_arrive(word);
-  return pass_wait(word, n, status);
 }
 
 // Newton step of one column of a rank that is alone (darlin_update_body), from its gradient sums and state.
@@ -527,17 +520,17 @@ __device__ __forceinline__ void prefetch_range(const T* a, u32 b, u32 e) {
 // A pass of a rank that is alone (S == 1) and owns every column, without delay. Worker and owner are the same GPU: no slices are
 // exchanged and no flags raised, and a block is two phases with a light barrier behind each:
 //
-//   gradient sums of block i
+//   gradient sums of block i, and beside them the column state of block i - 1 (other columns, other staging area)
 //   margins of block i, every nonzero with its column's step worked out on the spot
 //
-// Between arriving at a barrier and waiting for it a CTA sees to what is not on that path: the column state of block
-// i - 1 (other columns, other staging area), and the state of block i + 1's columns on its way to L2, of which a block
-// reads 1.2 MB that were last touched a pass ago. The general path below needs five grid-wide synchronisations per block,
-// two of them through system-scope flags, and gathers label and margin apart. 1.25 M rows, 125 M nonzeros, 256 blocks:
-// 8.4 ms there, 3.91 ms here without the prefetch, 3.70 with it, 3.61 with a CTA's nonzeros adjacent and the same
-// in both phases. Bound by latency: a block of 0.3 M nonzeros is 14 us, two phases of dependent gathers (3 us on average,
-// 5 for the slowest CTA) and two barriers of 1.2 us. (Not faster: the next block's nonzeros in shared memory beforehand,
-// 5.4 ms, since the row gathers then lack L1; in L2 beforehand.)
+// Behind its share of the margins a CTA sends for the state of block i + 1's columns, so that it is in L2 when that block
+// begins: a block reads 1.2 MB of it that were last touched a pass ago. The general path below needs five grid-wide
+// synchronisations per block, two of them through system-scope flags, and gathers label and margin apart. 1.25 M rows,
+// 125 M nonzeros, 256 blocks: 8.4 ms there, 3.91 ms here without the prefetch, 3.61 with it and with a CTA's nonzeros
+// adjacent and the same in both phases. Bound by latency: a block of 0.3 M nonzeros is 14 us, two phases of dependent
+// gathers (3 us on average, 5 for the slowest CTA) and two barriers of 1.2 us. (Not faster: the next block's nonzeros
+// copied to shared memory beforehand, 5.4 ms, since the row gathers then lack L1; the column state between arriving at a
+// barrier and waiting for it, 4.06 ms.)
 __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const PsbDarlinPass q) {
   __shared__ PsbDarlinGrad s_g[2];                 // by step parity
   __shared__ PsbDarlinUpdate s_u[2];
@@ -574,34 +567,28 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const Psb
   if (!pass_barrier(q.steps, ++bars, q.status)) return;
   for (u32 i = 0; i < n; ++i) {
     const u32 k = i & 1;
-    bool columns_left = i > 0;
     if (i > 0) {
       keep(i, word);                               // (the blocks of step i - 2: nobody reads them any more)
+      darlin_columns_alone(s_g[k ^ 1], s_u[k ^ 1], s_d[k ^ 1], vio_max);
       // a block that comes twice in a row, or shares columns with the one before it, needs their new state
-      if (s_g[k].c0 < s_g[k ^ 1].c1 && s_g[k ^ 1].c0 < s_g[k].c1) {
-        darlin_columns_alone(s_g[k ^ 1], s_u[k ^ 1], s_d[k ^ 1], vio_max);
-        columns_left = false;
-        if (!pass_barrier(q.steps, ++bars, q.status)) return;
-      }
+      if (s_g[k].c0 < s_g[k ^ 1].c1 && s_g[k ^ 1].c0 < s_g[k].c1 && !pass_barrier(q.steps, ++bars, q.status)) return;
     }
+    // the next block's columns (needed behind the margins)
+    const PsbDarlinGrad& next = q.grad[place(min(i + 1, n - 1))];
+    const u32 next_c0 = next.c0, next_c1 = next.c1;
     darlin_grad_p1<true>(s_g[k], rows);
-    pass_arrive(q.steps);
-    if (columns_left) darlin_columns_alone(s_g[k ^ 1], s_u[k ^ 1], s_d[k ^ 1], vio_max);
-    if (!pass_wait(q.steps, ++bars, q.status)) return;
+    if (!pass_barrier(q.steps, ++bars, q.status)) return;
     word = fetch(i + 1);
     darlin_margins_alone(s_g[k], s_u[k], s_d[k], rows);
-    pass_arrive(q.steps);
     if (i + 1 < n) {
-      const PsbDarlinGrad& next = q.grad[place(i + 1)];
-      const u32 c0 = next.c0, c1 = next.c1;
-      prefetch_range(s_g[k].delta, c0, c1);
-      prefetch_range(s_g[k].active, c0, c1);
-      prefetch_range(s_u[k].delta, c0, c1);
-      prefetch_range(s_u[k].w, c0, c1);
-      prefetch_range(s_d[k].w_cur, c0, c1);
-      prefetch_range(s_u[k].active, c0, c1);
+      prefetch_range(s_g[k].delta, next_c0, next_c1);
+      prefetch_range(s_g[k].active, next_c0, next_c1);
+      prefetch_range(s_u[k].delta, next_c0, next_c1);
+      prefetch_range(s_u[k].w, next_c0, next_c1);
+      prefetch_range(s_d[k].w_cur, next_c0, next_c1);
+      prefetch_range(s_u[k].active, next_c0, next_c1);
     }
-    if (!pass_wait(q.steps, ++bars, q.status)) return;
+    if (!pass_barrier(q.steps, ++bars, q.status)) return;
   }
   const u32 k = (n - 1) & 1;
   darlin_columns_alone(s_g[k], s_u[k], s_d[k], vio_max);
