@@ -48,7 +48,7 @@
 // average), or a bucket holds more distinct keys than its table can take, a
 // device flag is raised, the remaining steps return at once, and the caller's
 // gated sort-based path (psb_sort_pairs_gated + psb_localize2_gated) does the
-// work instead. Every spin is bounded and reports through the status word.
+// work instead. No step waits inside the kernel for another CTA.
 #include "psb_common.cuh"
 #include "psb_cuda.h"
 #include <type_traits>
@@ -1115,7 +1115,7 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
                                    psb_u64* cold_words, uint32_t* cold_pos, uint32_t* hot_pos,
                                    psb_u64* ukeys, uint32_t* seg_off, uint32_t* csr_col, uint32_t* csc_row,
                                    float* csc_val, uint32_t* flagbits, uint32_t* wordbase,
-                                   uint32_t* n_unique, uint32_t* own_off, void* scratch, uint32_t* status,
+                                   uint32_t* n_unique, uint32_t* own_off, void* scratch, uint32_t* /*status: nothing waits*/,
                                    uint32_t* gate_out, cudaStream_t stream) {
   if (S < 1 || S > 64) return -(int)cudaErrorInvalidValue;
   if (row_ptr == nullptr && fixed_z == 0) return -(int)cudaErrorInvalidValue;
