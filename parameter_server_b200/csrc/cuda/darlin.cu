@@ -530,7 +530,7 @@ __device__ __forceinline__ void prefetch_range(const T* a, u32 b, u32 e) {
 // adjacent and the same in both phases. Bound by latency: a block of 0.3 M nonzeros is 14 us, two phases of dependent
 // gathers (3 us on average, 5 for the slowest CTA) and two barriers of 1.2 us. (Not faster: the next block's nonzeros
 // copied to shared memory beforehand, 5.4 ms, since the row gathers then lack L1; the column state between arriving at a
-// barrier and waiting for it, 4.06 ms.)
+// barrier and waiting for it, 4.06 ms; the 3.61 were taken with it there, and not again since it is back in its place.)
 __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const PsbDarlinPass q) {
   __shared__ PsbDarlinGrad s_g[2];                 // by step parity
   __shared__ PsbDarlinUpdate s_u[2];
