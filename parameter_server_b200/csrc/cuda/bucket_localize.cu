@@ -1131,6 +1131,7 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   p.in = in; p.in_kind = in_kind; p.seed = seed; p.n = n;
   p.lo = low_zero_bits;
   if (row_ptr == nullptr) n_rows = (n + fixed_z - 1) / fixed_z;
+  else n_rows = max(n_rows, 1u);                    // nonzeros without a row are row 0's, as in the sort-based path
   p.packed = (low_zero_bits > 0 && n_rows > 0 && (low_zero_bits >= 32 || ((n_rows - 1) >> low_zero_bits) == 0)) ? 1 : 0;
   p.pay = (p.packed ? 0 : 1) + (vals != nullptr ? 1 : 0);
   if (cold_pos == nullptr || ((((size_t)cold_words) | ((size_t)cold_pos) | ((size_t)hot_pos) | ((size_t)csr_col)) & 15) != 0)

@@ -385,6 +385,25 @@ def test_bucket_localize_long_run_of_empty_rows(cuda_lib, split):
     assert min(ms) < 5.0
 
 
+@pytest.mark.parametrize("method", ["bucket", "sort"])
+@pytest.mark.parametrize("n", [4096, 200_001])
+def test_nonzeros_without_rows_are_row_0s(cuda_lib, n, method):
+    """Row offsets of one element: no row to look for, and nothing of the offsets or the row hints is read."""
+    from parameter_server_b200.ops.localize import LocalBatch
+    rng = np.random.default_rng(n)
+    keys = _rand_keys(n, rng, skew=True)
+    bounds_h, bounds = _bounds(2)
+    b = LocalBatch(1, n, 2, "cuda")
+    b.bucket_scratch.fill_(255)                        # (hints of another minibatch)
+    b.localize(torch.from_numpy(keys.view(np.int64)).cuda(), None, bounds, row_ptr=torch.zeros(1, dtype=torch.int32, device="cuda"),
+               method=method)
+    torch.cuda.synchronize()
+    assert int(b.gate.item()) == 0 and int(b.status.item()) == 0
+    u, inv = np.unique(keys, return_inverse=True)
+    assert np.array_equal(b.ukeys[:len(u)].cpu().numpy().view(np.uint64), u)
+    assert np.array_equal(b.csr_col[:n].cpu().numpy(), inv) and not b.csc_row[:n].any()
+
+
 @pytest.mark.parametrize("values", [False, True])
 @pytest.mark.parametrize("hash_bits,rows", [(40, 3000), (52, 4096), (52, 4097), (24, 3001), (0, 3000)])
 @pytest.mark.parametrize("ragged", [False, True])
