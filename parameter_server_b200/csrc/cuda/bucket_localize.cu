@@ -1127,6 +1127,7 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
     cudaMemsetAsync(gate_out, 0, sizeof(u32), stream);
     return -(int)cudaGetLastError();
   }
+  if (vals == nullptr || csc_val == nullptr) vals = nullptr, csc_val = nullptr;   // values move only from one to the other
   BLP p{};
   p.in = in; p.in_kind = in_kind; p.seed = seed; p.n = n;
   p.lo = low_zero_bits;

@@ -429,6 +429,32 @@ def test_bucket_localize_what_travels_beside_a_key(cuda_lib, ragged, hash_bits, 
     _check_grouped(b, keys, row_ptr, vals, bounds_h, rows)
 
 
+@pytest.mark.parametrize("hash_bits", [0, 40])
+@pytest.mark.parametrize("given", ["neither", "vals", "csc_val", "both"])
+def test_bucket_localize_values_move_only_where_both_sides_are_given(cuda_lib, given, hash_bits):
+    """The C entry with values and no room for them by key, and the other way round: nothing is read or written there."""
+    from parameter_server_b200.ops import _lib
+    from parameter_server_b200.ops.localize import LocalBatch
+    from parameter_server_b200.utils.oracle import hash_id_to_key
+    rng = np.random.default_rng(1)
+    rows, z = 1500, 6
+    ids = (rng.zipf(1.3, rows * z) % (1 << 22)).astype(np.int32)
+    vals = rng.random(rows * z, dtype=np.float32)
+    bounds_h, bounds = _bounds(2)
+    b = LocalBatch(rows, rows * z, 2, "cuda", real_values=True)
+    b.csc_val_buf.fill_(-1)
+    i, v, ptr = torch.from_numpy(ids).cuda(), torch.from_numpy(vals).cuda(), _lib.ptr
+    _lib.check(_lib.lib().psb_bucket_localize(
+        ptr(i), 1, 3 | hash_bits << 56, rows * z, 64 - hash_bits if hash_bits else 0, 0, rows, z, ptr(v) if given in ("vals", "both") else 0,
+        ptr(bounds), 2, ptr(b.keys_a), ptr(b.pos_a), ptr(b.keys_b), ptr(b.ukeys), ptr(b.seg_off), ptr(b.csr_col), ptr(b.csc_row_buf),
+        ptr(b.csc_val_buf) if given in ("csc_val", "both") else 0, ptr(b.flagbits), ptr(b.wordbase), ptr(b.n_unique), ptr(b.own_off),
+        ptr(b.bucket_scratch), ptr(b.status), ptr(b.gate), _lib.stream_ptr()), "bucket localize", kernels=10)
+    torch.cuda.synchronize()
+    b.nnz, b.csc_row, b.csc_val = rows * z, b.csc_row_buf, b.csc_val_buf
+    _check_grouped(b, hash_id_to_key(ids, 3, hash_bits or 64), np.arange(rows + 1) * z, vals if given == "both" else None, bounds_h, rows)
+    assert given == "both" or (b.csc_val_buf == -1).all()
+
+
 @pytest.mark.parametrize("z", [1, 3, 5000])
 def test_bucket_localize_more_slices_than_sms(cuda_lib, z):
     """A slice of the input is at most as long as a nonzero's place in it has bits: from 148 x 2^18 nonzeros on there are
