@@ -76,10 +76,10 @@ static constexpr u32 kPlaceMask = (1u << kPlaceBits) - 1;
 static_assert(kMaxBuckets + kHotMax <= 1u << (32 - kPlaceBits), "a bin fits above the place");
 static constexpr u32 kWalkSplit = 2;              // scatter and finish: CTAs that share a slice
 static constexpr int kHintShift = 5;              // one row hint per 32 positions
-// A bucket's table comes in two sizes. 2^11 home slots (35 KB of shared memory, five CTAs per SM) serve
-// minibatches in which keys repeat, the usual case; 2^12 (55 KB, four per SM) those in which nearly
-// every nonzero has its own key. The sample decides (k_bl_plan), both kernels are launched and the
-// one that was not chosen returns at once.
+// A bucket's table comes in two sizes. 2^11 home slots serve minibatches in which keys repeat, the usual
+// case; 2^12 those in which nearly every nonzero has its own key. Shared memory (and CTAs per SM) with compact keys of
+// 32 bits: 28 KB (six; five with a payload, for its registers) and 54 KB (four); of 64 bits: 36 KB (five) and 71 KB
+// (three). The sample decides (k_bl_plan), both kernels are launched and the one that was not chosen returns at once.
 template <int kBits> struct BucketShape {
   static constexpr u32 kHs = 1u << kBits;                  // home slots
   static constexpr u32 kHsAll = kHs + 2 * kRunMax;         // plus the spill area behind the last home slot
@@ -673,7 +673,7 @@ __device__ __forceinline__ u32 bucket_block_scan(u32 v, u32* s_warp /* 9 words *
 }
 
 // kPay: something travels beside the keys' words (BLP::pay is not 0). Bound by the latencies of its short phases, which
-// five CTAs per SM overlap. 13.1 M nonzeros, 8192 buckets: 117 us, and 222 us with the index of the bucket's first
+// the CTAs of an SM overlap. 13.1 M nonzeros, 8192 buckets: 117 us, and 222 us with the index of the bucket's first
 // key fetched by a look-back over the buckets in front (42 us) and every nonzero's column stored where the nonzero came
 // from (50 us).
 template <typename CK, int kBits, bool kPay>
@@ -1105,14 +1105,12 @@ extern "C" size_t psb_bucket_localize_scratch_bytes(uint32_t max_n) {
 
 // Groups the n nonzeros of a minibatch by key. Inputs as for psb_sort_pairs (in, in_kind, seed);
 // low_zero_bits = number of low key bits that are zero in every key (64 - significant bits of a
-// narrow hashed key); when n_rows - 1 fits in them the row rides in the key word. Work buffers of n x 8 bytes each,
-// 16-byte aligned like csr_col: cold_words (cold keys by bucket), cold_pos (what travels beside them) and hot_pos
-// (places and ranks of the nonzeros). Outputs as for psb_localize2. *gate_out (device word) is
-// set to 1 when the caller must run the gated sort-based path instead (its outputs then replace these).
+// narrow hashed key); when n_rows - 1 fits in them the row rides in the key word. Outputs as for psb_localize2; work buffers,
+// alignment and what may be null: psb_cuda.h.
 extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, uint32_t n, int low_zero_bits,
                                    const uint32_t* row_ptr, uint32_t n_rows, uint32_t fixed_z,
                                    const float* vals, const psb_u64* bounds, int S,
-                                   psb_u64* cold_words, uint32_t* cold_pos, uint32_t* hot_pos,
+                                   psb_u64* cold_words, uint32_t* beside, uint32_t* places,
                                    psb_u64* ukeys, uint32_t* seg_off, uint32_t* csr_col, uint32_t* csc_row,
                                    float* csc_val, uint32_t* flagbits, uint32_t* wordbase,
                                    uint32_t* n_unique, uint32_t* own_off, void* scratch, uint32_t* /*status: nothing waits*/,
@@ -1135,7 +1133,8 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   else n_rows = max(n_rows, 1u);                    // nonzeros without a row are row 0's, as in the sort-based path
   p.packed = (low_zero_bits > 0 && n_rows > 0 && (low_zero_bits >= 32 || ((n_rows - 1) >> low_zero_bits) == 0)) ? 1 : 0;
   p.pay = (p.packed ? 0 : 1) + (vals != nullptr ? 1 : 0);
-  if (cold_pos == nullptr || ((((size_t)cold_words) | ((size_t)cold_pos) | ((size_t)hot_pos) | ((size_t)csr_col)) & 15) != 0)
+  if (cold_words == nullptr || beside == nullptr || places == nullptr ||
+      ((((size_t)cold_words) | ((size_t)beside) | ((size_t)places) | ((size_t)csr_col)) & 15) != 0)
     return -(int)cudaErrorInvalidValue;
   p.NB = bl_num_buckets(n);
   p.nb_bits = 0;
@@ -1162,7 +1161,7 @@ extern "C" int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, ui
   p.shot_key = (u64*)(sc + L.shot_key); p.shot_h = (u32*)(sc + L.shot_h);
   p.bucket_hot_off = (u32*)(sc + L.bucket_hot_off); p.hot_seg = (u32*)(sc + L.hot_seg);
   p.hot_loc = (u32*)(sc + L.hot_loc); p.bucket_d = (u32*)(sc + L.bucket_d); p.row_hint = (u32*)(sc + L.row_hint);
-  p.cold_words = (u64*)cold_words; p.payload = cold_pos; p.place = hot_pos; p.rank = (unsigned short*)(hot_pos + n);
+  p.cold_words = (u64*)cold_words; p.payload = beside; p.place = places; p.rank = (unsigned short*)(places + n);
   p.ukeys = (u64*)ukeys; p.seg_off = seg_off; p.csr_col = csr_col; p.csc_row = csc_row; p.csc_val = csc_val;
   p.flagbits = flagbits; p.wordbase = wordbase; p.n_unique = n_unique;
   p.bounds = (const u64*)bounds; p.S = S; p.own_off = own_off; p.gate_out = gate_out;

@@ -44,11 +44,15 @@ int psb_localize2_gated(const psb_u64* keys_a, const psb_u64* keys_b, const uint
 // Copies a sorted unique key list and sets its length and owner offsets (one launch).
 int psb_set_keys(const psb_u64* keys, uint32_t n, psb_u64* ukeys, uint32_t* n_unique, const psb_u64* bounds, int S,
                  uint32_t* own_off, cudaStream_t stream);
-// Bucket-based localisation (bucket_localize.cu): groups the nonzeros by key without a full sort.
+// Bucket-based localisation (bucket_localize.cu): groups the nonzeros by key without a full sort. Work buffers of
+// n x 8 bytes each, 16-byte aligned, none of them null: cold_words, beside (what travels beside a cold key, then
+// segment starts) and places (a nonzero's bin and place, then its key's rank). csr_col is 16-byte aligned too. Row offsets
+// without rows give every nonzero row 0; values move only where vals and csc_val are both given. status is not used (no
+// step waits); *gate_out = 1: the outputs are not valid and the gated sort-based path has to run.
 size_t psb_bucket_localize_scratch_bytes(uint32_t max_n);
 int psb_bucket_localize(const void* in, int in_kind, psb_u64 seed, uint32_t n, int low_zero_bits,
                         const uint32_t* row_ptr, uint32_t n_rows, uint32_t fixed_z, const float* vals,
-                        const psb_u64* bounds, int S, psb_u64* cold_words, uint32_t* cold_pos, uint32_t* hot_pos,
+                        const psb_u64* bounds, int S, psb_u64* cold_words, uint32_t* beside, uint32_t* places,
                         psb_u64* ukeys, uint32_t* seg_off, uint32_t* csr_col, uint32_t* csc_row, float* csc_val,
                         uint32_t* flagbits, uint32_t* wordbase, uint32_t* n_unique, uint32_t* own_off,
                         void* scratch, uint32_t* status, uint32_t* gate_out, cudaStream_t stream);
