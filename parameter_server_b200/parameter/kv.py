@@ -62,11 +62,14 @@ class DeviceKVMap:
                 b.grad = torch.zeros(max_keys * self.k, dtype=torch.float32, device=self.dev)
         self._next_buf = 0
         self.stream = torch.cuda.Stream(device=self.dev)
-        # The plane's status word as a pull leaves it, copied behind the pull: its wait() then needs no blocking transfer of
-        # its own. (With on_stream and run_behind, and the kernels' tails: push and pull of 1000 keys 133 -> 88 us.)
-        self._status_host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        # The plane's status word as a pull leaves it, copied behind the pull into a word of its own: its wait() then needs
+        # no blocking transfer. (With on_stream and run_behind, and the kernels' tails: push and pull of 1000 keys 133 ->
+        # 88 us.) Only the device writes these words, and in stream order, so that a word may go to another pull while a
+        # discarded one's copy is still to come; a pull that finds none free is waited for as a push is.
+        self._status_host = torch.zeros(64, dtype=torch.int32, pin_memory=True)
         self._status_seen = self._status_host.numpy()
-        self._status_read: set = set()                # timestamps of the requests behind which it was copied
+        self._status_free: List[int] = list(range(len(self._status_seen)))
+        self._status_word: Dict[int, int] = {}        # timestamp of a pull -> its word
 
     @classmethod
     def create(cls, fabric_or_none=None, *, table_capacity: int = 1 << 20, max_keys: int = 1 << 18,
@@ -101,9 +104,17 @@ class DeviceKVMap:
             if ev is not None:
                 self.stream.wait_event(ev)
 
-    def _finish(self, ts: int, callback):
+    def _release_word(self, ts: int):
+        word = self._status_word.pop(ts, None)
+        if word is not None:
+            self._status_free.append(word)
+
+    def _finish(self, ts: int, callback, word: Optional[int] = None):
         ev = torch.cuda.Event()
         ev.record(self.stream)
+        self._release_word(ts)                        # (of an earlier request with this timestamp)
+        if word is not None:
+            self._status_word[ts] = word
         self._events[ts] = ev
         if callback is not None:
             self._callbacks[ts] = callback
@@ -241,22 +252,22 @@ class DeviceKVMap:
             else:
                 self.plane.pull_margin(b, need_applied=self._round, with_margins=False, stream=self.stream)
                 self._results[ts] = b.w_local[:k.numel()].clone()
-        _lib.check(_lib.lib().psb_read_word(self._status_host.data_ptr(), self.plane.status.data_ptr(), self.stream.cuda_stream),
-                   "status", kernels=0)
-        self._status_read.add(ts)
-        self._finish(ts, callback)
+        word = self._status_free.pop() if self._status_free else None
+        if word is not None:
+            _lib.check(_lib.lib().psb_read_word(self._status_host.data_ptr() + 4 * word, self.plane.status.data_ptr(),
+                                                self.stream.cuda_stream), "status", kernels=0)
+        self._finish(ts, callback, word)
         return ts
 
     def wait(self, ts: int):
         ev = self._events.pop(ts, None)
         if ev is not None:
             ev.synchronize()
-        if ev is None or ts not in self._status_read or self._status_seen[0] != 0:
-            try:
-                self.plane.check_status("kv")
-            finally:
-                self._status_seen[0] = 0
-        self._status_read.discard(ts)
+        word = self._status_word.get(ts)
+        good = ev is not None and word is not None and self._status_seen[word] == 0
+        self._release_word(ts)
+        if not good:
+            self.plane.check_status("kv")
         cb = self._callbacks.pop(ts, None)
         if cb is not None:
             cb()
@@ -269,7 +280,7 @@ class DeviceKVMap:
         self._events.pop(ts, None)
         self._callbacks.pop(ts, None)
         self._results.pop(ts, None)
-        self._status_read.discard(ts)
+        self._release_word(ts)
 
     def write_to_file(self, path: str):
         """``key<TAB>value`` per non-zero entry of this shard."""

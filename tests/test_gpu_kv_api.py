@@ -275,6 +275,51 @@ def test_wait_reports_the_status_that_a_pull_left(cuda_lib):
         kv.wait(again)                                 # (behind a push the word is read by wait())
 
 
+def test_no_wait_takes_back_what_another_pull_left(cuda_lib, monkeypatch):
+    """A pull that fails while wait() of another request looks at the status word is still reported by its own wait()."""
+    from parameter_server_b200.ops._lib import PsbCudaError
+    from parameter_server_b200.parameter.kv import DeviceKVVector
+    kv = DeviceKVVector.create(table_capacity=1 << 12, max_keys=1 << 10)
+    keys = torch.arange(1, 6, dtype=torch.int64, device="cuda")
+    pushed, pulled = kv.push(keys, torch.ones(5, device="cuda")), []
+    look = kv.plane.check_status
+
+    def and_then_a_pull_fails(what):
+        look(what)
+        kv.plane.status.fill_(1)
+        pulled.append(kv.pull(keys))
+        torch.cuda.synchronize()
+    with monkeypatch.context() as m:
+        m.setattr(kv.plane, "check_status", and_then_a_pull_fails)
+        kv.wait(pushed)
+    with pytest.raises(PsbCudaError):
+        kv.wait(pulled[0])
+
+
+def test_status_words_of_pulls_that_nobody_waits_for(cuda_lib):
+    """More pulls in flight than there are words, discarded ones, and a push with the timestamp of a pull."""
+    from parameter_server_b200.ops._lib import PsbCudaError
+    from parameter_server_b200.parameter.kv import DeviceKVVector
+    kv = DeviceKVVector.create(table_capacity=1 << 12, max_keys=1 << 10)
+    keys = torch.arange(1, 6, dtype=torch.int64, device="cuda")
+    kv.push(keys, torch.ones(5, device="cuda"))
+    pulls = [kv.pull(keys) for _ in range(150)]
+    for ts in pulls[:50]:
+        kv.discard(ts)
+    kv.plane.status.fill_(1)
+    bad = [kv.pull(keys) for _ in range(100)]
+    with pytest.raises(PsbCudaError):
+        kv.wait(bad[0])
+    for ts in bad[1:] + pulls[50:]:
+        kv.wait(ts)
+        assert kv.result(ts).tolist() == [1.0] * 5
+    assert kv.pull(keys, ts=7000) == kv.push(keys, torch.ones(5, device="cuda"), ts=7000)
+    torch.cuda.synchronize()
+    kv.plane.status.fill_(1)
+    with pytest.raises(PsbCudaError):
+        kv.wait(7000)
+
+
 def test_on_stream_is_left_as_it_was_entered(cuda_lib):
     from parameter_server_b200.ops._lib import on_stream, run_behind
     a, b = torch.cuda.Stream(), torch.cuda.Stream()
