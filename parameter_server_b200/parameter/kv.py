@@ -31,6 +31,7 @@ the CUDA event of request ``t``, and ``wait(ts)`` blocks the host until request
 """
 from __future__ import annotations
 
+import weakref
 from typing import Callable, Dict, List, Optional
 
 import numpy as np
@@ -70,6 +71,9 @@ class DeviceKVMap:
         self._status_seen = self._status_host.numpy()
         self._status_free: List[int] = list(range(len(self._status_seen)))
         self._status_word: Dict[int, int] = {}        # timestamp of a pull -> its word
+        # The allocator of pinned memory does not know of these copies: a container that is dropped with a pull in flight
+        # gives the words back when its stream is idle.
+        weakref.finalize(self, self.stream.synchronize).atexit = False
 
     @classmethod
     def create(cls, fabric_or_none=None, *, table_capacity: int = 1 << 20, max_keys: int = 1 << 18,
