@@ -141,6 +141,12 @@ class DeviceKVMap:
         return (isinstance(values, torch.Tensor) and values.is_cuda and values.dtype == torch.float32
                 and values.is_contiguous() and not values.is_neg() and values.device == self.stream.device)
 
+    def _ready(self, k: torch.Tensor, values) -> bool:
+        """Whether a push need not enter the container's stream: no conversion is to run there, and its device is the
+        current one already (launches go to the current device, whatever their stream)."""
+        return (self._in_place(values) and k.dtype == torch.int64 and k.is_contiguous() and k.device == values.device
+                and torch.cuda.current_device() == self.stream.device.index)
+
     @staticmethod
     def _as_keys(keys, dev) -> torch.Tensor:
         if isinstance(keys, torch.Tensor):
@@ -159,9 +165,7 @@ class DeviceKVMap:
         ts = self._stamp(ts)
         self._begin(wait)
         k = self._as_keys(keys, self.dev)
-        # conversions run on the container's stream; without any the stream need not be entered
-        ready = self._in_place(values) and k.dtype == torch.int64 and k.is_contiguous() and k.device == values.device
-        with _lib.on_stream(None if ready else self.stream):
+        with _lib.on_stream(None if self._ready(k, values) else self.stream):
             rnd = self._push_round_of[ts] = self._push_half(k, values)
             self._apply_half(rnd, channel)
         self._finish(ts, callback)

@@ -1,5 +1,6 @@
 """The values that a device KV container hands to its push kernel, which reads adjacent floats from one address."""
 import contextlib
+import types
 
 import numpy as np
 import pytest
@@ -77,3 +78,23 @@ def test_push_only_leaves_the_caller_its_values(monkeypatch, n, k):
     kv = _container(0, k)
     kv._begin = waited.append
     assert kv.push_only(torch.arange(0), None) == 0        # a round without keys needs no values
+
+
+@pytest.mark.parametrize("current,container", [(0, 0), (0, 1), (1, 0)])
+def test_push_enters_a_stream_of_another_device(monkeypatch, current, container):
+    """Values and keys that are read where they are spare a push the entry into its stream, but not where another device than
+    the container's is the current one: entering makes its device the current one."""
+    from parameter_server_b200.ops import _lib
+    kv = _container(5, 1)
+    kv.stream = types.SimpleNamespace(device=torch.device("cuda", container))
+    kv._time, kv._push_round_of = -1, {}
+    kv._begin = kv._finish = lambda *a: None
+    kv._apply_half = lambda rnd, channel: None
+    kv._in_place = lambda values: True
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current)
+    entered = []
+    monkeypatch.setattr(_lib, "on_stream", lambda s: entered.append(s) or contextlib.nullcontext())
+    kv.push(torch.arange(5), torch.ones(5))
+    assert entered == [None if current == container else kv.stream]
+    kv.push(torch.arange(5, dtype=torch.int32), torch.ones(5))
+    assert entered[1] is kv.stream
