@@ -76,6 +76,10 @@ static constexpr u32 kPlaceMask = (1u << kPlaceBits) - 1;
 static_assert(kMaxBuckets + kHotMax <= 1u << (32 - kPlaceBits), "a bin fits above the place");
 static constexpr u32 kWalkSplit = 2;              // scatter and finish: CTAs that share a slice
 static constexpr int kHintShift = 5;              // one row hint per 32 positions
+// Rows beyond this many positions get their hints from the whole grid: a warp takes 32 rows in turn. (13.1 M nonzeros in
+// rows of 32,000: 498, 491 and 491 us with 2^15, 2^13 and 2^12; 0.39 M in rows of 6000: 79, 78 and 82.)
+static constexpr u32 kLongRow = 1u << 13;
+static constexpr u32 kLongHints = kLongRow >> kHintShift;
 // A bucket's table comes in two sizes. 2^11 home slots serve minibatches in which keys repeat, the usual
 // case; 2^12 those in which nearly every nonzero has its own key. Shared memory (and CTAs per SM) with compact keys of
 // 32 bits: 28 KB (six; five with a payload, for its registers) and 54 KB (four); of 64 bits: 36 KB (five) and 71 KB
@@ -175,6 +179,12 @@ __device__ __forceinline__ u32 row_of_pos(const BLP& p, u32 pos, u32 zinv) {
   return row_search(p.row_ptr, lo, max(lo + 1, hi), pos);
 }
 
+// Positions [b, e) of row r, within the input whatever the offsets are.
+__device__ __forceinline__ void row_range(const BLP& p, u32 r, u32& b, u32& e) {
+  b = r == 0 ? 0u : p.row_ptr[r];
+  e = r + 1 == p.n_rows ? p.n : min(p.n, p.row_ptr[r + 1]);
+}
+
 // ---------------------------------------------------------------- 0. clean scratch
 // Everything that starts as zeros or ones, and the row hints, in one launch instead of one per region.
 __global__ void __launch_bounds__(256) k_bl_clear(const BLP p, uint4* zero, u32 zero4, uint4* ones, u32 ones4, u32 flag_words) {
@@ -185,23 +195,24 @@ __global__ void __launch_bounds__(256) k_bl_clear(const BLP p, uint4* zero, u32 
   for (u32 i = gtid; i < flag_words; i += gsize) p.flagbits[i] = 0;
   if (p.row_ptr != nullptr) {
     // Row hints for steps 4 and 6, up to the block behind the last position: every row writes those of the blocks that
-    // start in it, a long one with its whole warp. (3.9 M nonzeros in 100,000 rows: this kernel 3.2 us; 9.4 with a search
-    // of log2(rows) dependent loads per hint.)
+    // start in it, with its whole warp where they are many. (3.9 M nonzeros in 100,000 rows: this kernel 3.2 us; 9.4 with a
+    // search of log2(rows) dependent loads per hint.) A row beyond kLongRow writes those in front of its first multiple of
+    // kLongRow and one at every multiple; k_bl_sample fills in the rest.
     const u32 lane = threadIdx.x & 31;
     for (u32 r0 = gtid - lane; r0 < p.n_rows; r0 += gsize) {
       const u32 r = r0 + lane;
-      u32 h0 = 0, h1 = 0;
-      if (r < p.n_rows) {
-        const u32 b = r == 0 ? 0u : p.row_ptr[r], e = r + 1 == p.n_rows ? p.n : min(p.n, p.row_ptr[r + 1]);
-        h0 = (b + 31) >> kHintShift;
-        h1 = e > b ? (e + 31) >> kHintShift : h0;
-      }
+      u32 b = 0, e = 0;
+      if (r < p.n_rows) row_range(p, r, b, e);
+      const u32 h0 = (b + 31) >> kHintShift, h1 = e > b ? (e + 31) >> kHintShift : h0;
       const bool longer = h1 > h0 + 16;
       if (!longer) for (u32 h = h0; h < h1; ++h) p.row_hint[h] = r;
       for (u32 m = __ballot_sync(0xffffffffu, longer); m; m &= m - 1) {
         const int first = __ffs(m) - 1;
         const u32 a0 = __shfl_sync(0xffffffffu, h0, first), a1 = __shfl_sync(0xffffffffu, h1, first);
-        for (u32 h = a0 + lane; h < a1; h += 32) p.row_hint[h] = r0 + first;
+        const bool very = __shfl_sync(0xffffffffu, e - b, first) > kLongRow;
+        const u32 mark = (a0 + kLongHints - 1) & ~(kLongHints - 1), a2 = very ? min(a1, mark) : a1;
+        for (u32 h = a0 + lane; h < a2; h += 32) p.row_hint[h] = r0 + first;
+        if (very) for (u32 h = mark + kLongHints * lane; h < a1; h += 32 * kLongHints) p.row_hint[h] = r0 + first;
       }
     }
     if (gtid == 0) p.row_hint[((p.n - 1) >> kHintShift) + 1] = p.n_rows - 1;
@@ -213,6 +224,19 @@ __global__ void __launch_bounds__(256) k_bl_clear(const BLP p, uint4* zero, u32 
 __global__ void __launch_bounds__(256) k_bl_sample(const BLP p) {
   behind_the_step_before();
   const u32 j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p.row_ptr != nullptr) {
+    // Row hints of very long rows: a warp per stretch of kLongRow positions, from the hint at its start. (The localisation of
+    // one row of 13.1 M nonzeros: 538 us with all of its hints written by one warp, 477 so; of 3.9 M 200 and 181.)
+    const u32 lane = threadIdx.x & 31, stretches = (p.n + kLongRow - 1) / kLongRow;
+    for (u32 m = j >> 5; m < stretches; m += gridDim.x * blockDim.x >> 5) {
+      const u32 r = min(p.row_hint[m * kLongHints], p.n_rows - 1);
+      u32 b, e;
+      row_range(p, r, b, e);
+      if (e <= b || e - b <= kLongRow) continue;
+      const u32 h1 = (min(e, m * kLongRow + kLongRow) + 31) >> kHintShift;
+      for (u32 h = m * kLongHints + 1 + lane; h < h1; h += 32) p.row_hint[h] = r;
+    }
+  }
   const bool valid = j < p.samp_m;
   const u64 key = valid ? bl_key_of(p, j * p.samp_stride) : kEmptyKey;
   // equal keys of a warp count once (the most frequent key would otherwise take thousands of

@@ -385,6 +385,26 @@ def test_bucket_localize_long_run_of_empty_rows(cuda_lib, split):
     assert min(ms) < 5.0
 
 
+@pytest.mark.parametrize("lens", [[150_001], [8192], [8193], [16384, 8192, 24_576], [3, 8192, 5, 8193, 1, 16384, 0, 0, 22_501, 7, 70_000, 31],
+                                  [0, 1, 10_000, 0, 0, 8191, 8250, 100, 200_000, 0]])
+def test_bucket_localize_very_long_rows(cuda_lib, lens):
+    """Row hints beyond a warp's share: rows around 8192 positions and far beyond, wherever they begin and end."""
+    from parameter_server_b200.ops.localize import LocalBatch
+    rng = np.random.default_rng(len(lens))
+    lens = np.concatenate([lens, rng.integers(0, 40, 3000)]) if len(lens) > 3 else np.array(lens)
+    row_ptr = np.concatenate([[0], np.cumsum(lens)])
+    rows, nnz = len(lens), int(row_ptr[-1])
+    keys = _rand_keys(nnz, rng, skew=True)
+    bounds_h, bounds = _bounds(2)
+    b = LocalBatch(rows, nnz, 2, "cuda")
+    b.bucket_scratch.fill_(255)
+    b.localize(torch.from_numpy(keys.view(np.int64)).cuda(), None, bounds, row_ptr=torch.from_numpy(row_ptr.astype(np.int32)).cuda(),
+               method="bucket")
+    torch.cuda.synchronize()
+    assert int(b.gate.item()) == 0 and int(b.status.item()) == 0
+    _check_grouped(b, keys, row_ptr, None, bounds_h, rows)
+
+
 @pytest.mark.parametrize("method", ["bucket", "sort"])
 @pytest.mark.parametrize("n", [4096, 200_001])
 def test_nonzeros_without_rows_are_row_0s(cuda_lib, n, method):
