@@ -48,8 +48,10 @@ static constexpr int kGradGroup = 4;
 // by side (k_darlin_pass). index: this CTA's place among them.
 struct Part { u32 index, count; };
 __device__ __forceinline__ Part whole_grid() { return Part{blockIdx.x, gridDim.x}; }
-// Words of 32 nonzeros per CTA of k_darlin_pass_alone: each takes an adjacent part of the block.
-static constexpr u32 kAloneWarps = 32;
+static constexpr int kPassThreads = 1024;         // the pass kernels
+// Words of 32 nonzeros per CTA of k_darlin_pass_alone: each takes an adjacent part of the block, dealt out among its warps.
+static constexpr u32 kAloneWarps = kPassThreads / 32;
+static_assert(kPassThreads % 32 == 0, "whole warps");
 __device__ __forceinline__ u32 part_words(u32 words) { return (words + gridDim.x - 1) / gridDim.x; }
 // kAlone (k_darlin_pass_alone): label and margin of a row are one pair in row_state (one gather instead of
 // two) and the staging area holds (G, U) pairs (one vector atomic per column piece instead of two).
@@ -387,8 +389,6 @@ __device__ __forceinline__ void load_params(P* dst, const P* src) {
   u32* d = reinterpret_cast<u32*>(dst);
   for (u32 i = threadIdx.x; i < sizeof(P) / 4; i += blockDim.x) d[i] = s[i];
 }
-
-static constexpr int kPassThreads = 1024;
 
 // Grid barrier number `n` (1, 2, ...) of a launch on a word that was zero at its start: one fire-and-forget
 // arrival, then polls until everybody's has landed. Against grid_barrier it saves the sense load and the
