@@ -509,28 +509,20 @@ __device__ void darlin_margins_alone(const PsbDarlinGrad& g, const PsbDarlinUpda
   }
 }
 
-// The lines of an array's elements [b, e) on their way to L2.
-template <typename T>
-__device__ __forceinline__ void prefetch_range(const T* a, u32 b, u32 e) {
-  constexpr u32 kPer = 128 / sizeof(T);
-  for (u32 i = b + kPer * (blockIdx.x * kPassThreads + threadIdx.x); i < e; i += kPer * gridDim.x * kPassThreads)
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(a + i));
-}
-
 // A pass of a rank that is alone (S == 1) and owns every column, without delay. Worker and owner are the same GPU: no slices are
 // exchanged and no flags raised, and a block is two phases with a light barrier behind each:
 //
 //   gradient sums of block i, and beside them the column state of block i - 1 (other columns, other staging area)
 //   margins of block i, every nonzero with its column's step worked out on the spot
 //
-// Behind its share of the margins a CTA sends for the state of block i + 1's columns, so that it is in L2 when that block
-// begins: a block reads 1.2 MB of it that were last touched a pass ago. The general path below needs five grid-wide
-// synchronisations per block, two of them through system-scope flags, and gathers label and margin apart. 1.25 M rows,
-// 125 M nonzeros, 256 blocks: 8.4 ms there, 3.91 ms here without the prefetch, 3.61 with it and with a CTA's nonzeros
-// adjacent and the same in both phases. Bound by latency: a block of 0.3 M nonzeros is 14 us, two phases of dependent
-// gathers (3 us on average, 5 for the slowest CTA) and two barriers of 1.2 us. (Not faster: the next block's nonzeros
-// copied to shared memory beforehand, 5.4 ms, since the row gathers then lack L1; the column state between arriving at a
-// barrier and waiting for it, 4.06 ms; the 3.61 were taken with it there, and not again since it is back in its place.)
+// The general path below needs five grid-wide synchronisations per block, two of them through system-scope flags, and gathers
+// label and margin apart: 8.4 ms for a pass over 1.25 M rows, 125 M nonzeros, 256 blocks. Here it is 3.94 ms, and 4.08 with the
+// words of a block dealt out over the grid instead of adjacent for a CTA and the same in both phases (114,000 rows of 65, 256
+// blocks: 2.47 and 2.53; 330,000 of 96, 64 blocks: 1.06 and 1.10). Bound by latency: a block of 0.49 M nonzeros is 15 us, two
+// phases of dependent gathers, each as long as its slowest CTA, and two barriers of 1.2 us. (The row pairs are gathered
+// through L1: a frequent column's rows stand close together, and nothing writes them during a gradient phase.) Not faster:
+// the state of the next block's columns sent for to L2 behind the margins (3.99, 2.56 and 1.06 ms); the next block's
+// nonzeros copied to shared memory beforehand (a third slower, since the row gathers then lack L1).
 __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const PsbDarlinPass q) {
   __shared__ PsbDarlinGrad s_g[2];                 // by step parity
   __shared__ PsbDarlinUpdate s_u[2];
@@ -542,10 +534,9 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const Psb
   static_assert(WG + WU + WD <= kPassThreads, "one word of the three parameter blocks per thread");
   float2* rows = reinterpret_cast<float2*>(q.row_state);
   const u32 gsize = gridDim.x * blockDim.x, gtid = blockIdx.x * blockDim.x + threadIdx.x, t = threadIdx.x;
-  auto place = [&](u32 i) -> size_t { return (size_t)q.order[i] * R + (q.ts_base + i) % R; };
   auto fetch = [&](u32 i) -> u32 {                 // this thread's word of step i's three parameter blocks
     if (i >= n) return 0u;
-    const size_t at = place(i);
+    const size_t at = (size_t)q.order[i] * R + (q.ts_base + i) % R;
     if (t < WG) return reinterpret_cast<const u32*>(&q.grad[at])[t];
     if (t < WG + WU) return reinterpret_cast<const u32*>(&q.update[at])[t - WG];
     if (t < WG + WU + WD) return reinterpret_cast<const u32*>(&q.dual[at])[t - WG - WU];
@@ -573,21 +564,10 @@ __global__ void __launch_bounds__(kPassThreads, 1) k_darlin_pass_alone(const Psb
       // a block that comes twice in a row, or shares columns with the one before it, needs their new state
       if (s_g[k].c0 < s_g[k ^ 1].c1 && s_g[k ^ 1].c0 < s_g[k].c1 && !pass_barrier(q.steps, ++bars, q.status)) return;
     }
-    // the next block's columns (needed behind the margins)
-    const PsbDarlinGrad& next = q.grad[place(min(i + 1, n - 1))];
-    const u32 next_c0 = next.c0, next_c1 = next.c1;
     darlin_grad_p1<true>(s_g[k], rows);
     if (!pass_barrier(q.steps, ++bars, q.status)) return;
     word = fetch(i + 1);
     darlin_margins_alone(s_g[k], s_u[k], s_d[k], rows);
-    if (i + 1 < n) {
-      prefetch_range(s_g[k].delta, next_c0, next_c1);
-      prefetch_range(s_g[k].active, next_c0, next_c1);
-      prefetch_range(s_u[k].delta, next_c0, next_c1);
-      prefetch_range(s_u[k].w, next_c0, next_c1);
-      prefetch_range(s_d[k].w_cur, next_c0, next_c1);
-      prefetch_range(s_u[k].active, next_c0, next_c1);
-    }
     if (!pass_barrier(q.steps, ++bars, q.status)) return;
   }
   const u32 k = (n - 1) & 1;
