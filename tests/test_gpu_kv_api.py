@@ -322,7 +322,7 @@ def test_status_words_of_pulls_that_nobody_waits_for(cuda_lib):
 
 def test_a_dropped_container_gives_its_pinned_words_back_when_idle(cuda_lib):
     """A container dropped with a pull in flight, which still has its status word to write, ends behind it."""
-    import gc
+    import weakref
     from parameter_server_b200.parameter.kv import DeviceKVVector
     kv = DeviceKVVector.create(table_capacity=1 << 12, max_keys=1 << 10)
     keys = torch.arange(1, 6, dtype=torch.int64, device="cuda")
@@ -331,10 +331,10 @@ def test_a_dropped_container_gives_its_pinned_words_back_when_idle(cuda_lib):
     for _ in range(200):                               # about 16 ms in front of the pull
         busy += 1
     kv.pull(keys)
-    stream, words = kv.stream, kv._status_host
+    stream, words, plane = kv.stream, kv._status_host, kv.plane      # (a plane that goes too waits for the device)
+    gone = weakref.ref(kv)
     del kv
-    gc.collect()
-    assert stream.query() and not words.any()
+    assert gone() is None and stream.query() and not words.any()
 
 
 def test_on_stream_is_left_as_it_was_entered(cuda_lib):
